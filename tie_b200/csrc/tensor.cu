@@ -27,9 +27,8 @@
 //     rows, 16-row boxes: only rows the expert really has) and of the sub-block sums;
 //   * two MMA issuer warps issue tcgen05.mma (kind::f16, fp32 accumulate), per 16-wide k step
 //     P += A.B_hi, P += A.B_lo (one MMA over the stacked hi and lo rows when the tile has at most
-//     32 tokens).  A thread can issue only one MMA per ~110-130 cycles whatever its N, so
-//     consecutive super-blocks go to different issuers, each with two of the four accumulator
-//     buffers;
+//     32 tokens); consecutive super-blocks go to different issuers, each with two of the four
+//     accumulator buffers;
 //   * 8 drain warps take a finished super-block out of tensor memory (tcgen05.ld), fold it into
 //     fp32 registers with d (-1 for the min phase), and after the last super-block of a work item
 //     store the rows — while the MMAs of the next super-blocks / work item already run.
@@ -722,19 +721,18 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm16, const __grid_constant_
 		// (pairs: the MMAs of both CTAs are issued by the even-ranked one; its peer's issuer warps idle)
 		// (one issuer alternating between two accumulator buffers was measured slower than two issuers with
 		// one buffer each: the ring round trips of a single consumer are exposed)
-		const uint32_t leader = (lane == 0 && rank == 0) ? 1u : 0u;
 		const bool issuing = rank == 0;
 		auto mma = [&](uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
 			if (PAIR)
-				ptx::mma_f16_ts_pair_if(d, a, b, idesc, accumulate, leader);
+				ptx::mma_f16_ts_pair(d, a, b, idesc, accumulate);
 			else
-				ptx::mma_f16_ts_if(d, a, b, idesc, accumulate, leader);
+				ptx::mma_f16_ts(d, a, b, idesc, accumulate);
 		};
 		auto commit = [&](uint64_t *bar) {
 			if (PAIR)
-				ptx::mma_commit_pair_if(ptx::smem_u32(bar), leader);
+				ptx::mma_commit_pair(ptx::smem_u32(bar));
 			else
-				ptx::mma_commit_if(ptx::smem_u32(bar), leader);
+				ptx::mma_commit(ptx::smem_u32(bar));
 		};
 		int s = 0;
 		uint32_t ph = 0, g = 0, tl = 0, gst = 0;
@@ -794,6 +792,12 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm16, const __grid_constant_
 					const uint32_t ph1 = ph;
 					advance(1);
 					bool ok = tc_wait(ptx::smem_u32(&sh->full[s0]), ph0, abort_flag, status);
+					// (the token loader has to have passed these stages too: were they handed back before it looked,
+					// it would miss that phase of their barrier and wait for ever)
+					if (!PAIR) {
+						ok = ok && tc_wait(ptx::smem_u32(&sh->bfull[s0]), ph0, abort_flag, status);
+						ok = ok && tc_wait(ptx::smem_u32(&sh->bfull[s1]), ph1, abort_flag, status);
+					}
 					ok = ok && tc_wait(ptx::smem_u32(&sh->full[s1]), ph1, abort_flag, status);
 					ok = ok && tc_wait(ptx::smem_u32(&sh->xfull), tl & 1u, abort_flag, status);
 					if (!__all_sync(0xffffffffu, ok)) {
@@ -806,15 +810,18 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm16, const __grid_constant_
 					TCT_TRACE(2, gst - 1);
 					const uint64_t xh = ptx::umma_desc_sw128(xq_hi), xl = ptx::umma_desc_sw128(xq_hi + lo_off);
 					const uint32_t ah = tmem + TC_COL_A + 32u * s0, al = tmem + TC_COL_A + 32u * s1;
-					for (int kk = 0; kk < min_k16; kk++) {
-						mma(dP, ah + 8 * kk, xh + 2 * kk, idesc, kk > 0 ? 1u : 0u);
-						if (!concat)
-							mma(dP, ah + 8 * kk, xl + 2 * kk, idesc, 1u);
-						mma(dP, al + 8 * kk, xh + 2 * kk, idesc_hi, 1u);
+					if (ptx::elect_one()) {
+						for (int kk = 0; kk < min_k16; kk++) {
+							mma(dP, ah + 8 * kk, xh + 2 * kk, idesc, kk > 0 ? 1u : 0u);
+							if (!concat)
+								mma(dP, ah + 8 * kk, xl + 2 * kk, idesc, 1u);
+							mma(dP, al + 8 * kk, xh + 2 * kk, idesc_hi, 1u);
+						}
+						commit(&sh->empty[s1]);	 // both stages
+						commit(&sh->xempty);
+						commit(&sh->pfull[buf]);
 					}
-					commit(&sh->empty[s1]);	 // both stages (a commit costs an MMA's issue time)
-					commit(&sh->xempty);
-					commit(&sh->pfull[buf]);
+					__syncwarp();
 					TCT_TRACE(3, gst - 2);
 					TCT_TRACE(3, gst - 1);
 					TCT_ADD(7, tmp0);
@@ -846,23 +853,28 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm16, const __grid_constant_
 					ptx::tc_fence_after();
 					const uint64_t bh = ptx::umma_desc_sw128(b_hi(bs)), bl = ptx::umma_desc_sw128(b_hi(bs) + lo_off);
 					const uint32_t a = tmem + TC_COL_A + 32u * s;
+					if (ptx::elect_one()) {
 #pragma unroll
-					for (int kk = 0; kk < TC_BK / 16; kk++) {
-						mma(dP, a + 8 * kk, bh + 2 * kk, idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
-						if (!concat)
-							mma(dP, a + 8 * kk, bl + 2 * kk, idesc, 1u);
+						for (int kk = 0; kk < TC_BK / 16; kk++) {
+							mma(dP, a + 8 * kk, bh + 2 * kk, idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
+							if (!concat)
+								mma(dP, a + 8 * kk, bl + 2 * kk, idesc, 1u);
+						}
+						if (q4 & 1)  // stages go back to the producers and the token loader in pairs
+							commit(&sh->empty[s]);
+						if (q4 == TC_SPB - 1) {
+							if (PAIR)  // the super-block's token stages go back to both CTAs' token loaders
+								commit(&sh->bempty[bg & 3u]);
+							commit(&sh->pfull[buf]);
+						}
 					}
-					if (q4 & 1)  // stages go back to the producers and the token loader in pairs
-						commit(&sh->empty[s]);
+					__syncwarp();
 					TCT_ADD(3, ti);
 					TCT_TRACE(3, gst);
 					advance(1);
 				}
 				if (!alive)
 					break;
-				if (PAIR)  // the super-block's token stages go back to both CTAs' token loaders
-					commit(&sh->bempty[bg & 3u]);
-				commit(&sh->pfull[buf]);
 				g++;
 				bg++;
 			}
