@@ -68,10 +68,8 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TRY(dev_alloc(c, &s.hs_hi, 2 * s.rows_pad * F));
 	s.hs_lo = s.hs_hi + s.rows_pad * F;
 	const size_t XH = xq_cols((int)H), XF = xq_cols((int)F);
-	TRY(dev_alloc(c, &s.xq_hi, 2 * s.rows_pad * XH));
-	s.xq_lo = s.xq_hi + s.rows_pad * XH;
-	TRY(dev_alloc(c, &s.hq_hi, 2 * s.rows_pad * XF));
-	s.hq_lo = s.hq_hi + s.rows_pad * XF;
+	TRY(dev_alloc(c, &s.xq, s.rows_pad * XH));
+	TRY(dev_alloc(c, &s.hq, s.rows_pad * XF));
 	TRY(dev_alloc(c, &s.status, 1));
 	TRY(dev_alloc(c, &s.counter, 1));
 	TIE_CUDA_TRY(c, cudaMemset(s.counter, 0, sizeof(int)));
@@ -92,11 +90,8 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TIE_CUDA_TRY(c, cudaMemset(s.xs_lo, 0, s.rows_pad * H * sizeof(__half)));
 	TIE_CUDA_TRY(c, cudaMemset(s.hs_hi, 0, s.rows_pad * F * sizeof(__half)));
 	TIE_CUDA_TRY(c, cudaMemset(s.hs_lo, 0, s.rows_pad * F * sizeof(__half)));
-	// the padding columns of the sub-block sums are read by the tensor path and must stay zero
-	TIE_CUDA_TRY(c, cudaMemset(s.xq_hi, 0, s.rows_pad * XH * sizeof(__half)));
-	TIE_CUDA_TRY(c, cudaMemset(s.xq_lo, 0, s.rows_pad * XH * sizeof(__half)));
-	TIE_CUDA_TRY(c, cudaMemset(s.hq_hi, 0, s.rows_pad * XF * sizeof(__half)));
-	TIE_CUDA_TRY(c, cudaMemset(s.hq_lo, 0, s.rows_pad * XF * sizeof(__half)));
+	TIE_CUDA_TRY(c, cudaMemset(s.xq, 0, s.rows_pad * XH * sizeof(__half)));
+	TIE_CUDA_TRY(c, cudaMemset(s.hq, 0, s.rows_pad * XF * sizeof(__half)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_x), T * H * sizeof(float)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_out), T * H * sizeof(float)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_idx), R * sizeof(int)));
@@ -279,7 +274,7 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	if (use_tc) {
 		const bool sums = L.gate.kind == W_Q4K;	 // the Q4_K "min" term needs the sub-block sums of the inputs
 		TRY(launch_split_rows(c, x_src, c->s.perm, src_div, n_rows, c->cfg.hidden, c->s.xs_hi, c->s.xs_lo,
-				      sums ? c->s.xq_hi : nullptr, sums ? c->s.xq_lo : nullptr));
+				      sums ? c->s.xq : nullptr));
 		prof_mark(c, 3);
 		TRY(launch_tc_gate_up(c, L, n_rows));
 		prof_mark(c, 4);
@@ -679,7 +674,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	void *dev_ptrs[] = {s.x,     s.out,   s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
 			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.status,  s.counter, s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
-			    s.tile_info, s.xq_hi, s.hq_hi, s.dec_sync, c->df_table, s.sort_hist};
+			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist};
 	for (void *p : dev_ptrs)
 		if (p)
 			cudaFree(p);
@@ -1565,22 +1560,10 @@ int tie_cuda_mat_mat(tie_cuda_ctx *c, const void *w_host, const float *x, float 
 	TIE_CUDA_TRY(c, cudaMemsetAsync(s.row_expert, 0, (size_t)batch_len * sizeof(int), c->stream));
 	SortBufs b = {s.counts, s.offsets, s.tile_start, s.active, s.n_active, s.perm, s.tile_info};
 	TRY(launch_sort(c, s.row_expert, batch_len, TC_TOKEN_TILE, 0, 1, b));
-	// the batch, split into fp16 hi + lo (and its sub-block sums for Q4_K), in the tensor's view of the x arrays.
-	// Columns of the sums that the row length leaves unused are read as padding of a 16-deep k step
-	// and must be zero, in this view and, afterwards, in the context's own.
+	// the batch, split into fp16 hi + lo (and its sub-block sums for Q4_K), in the tensor's view of the x arrays
 	const bool sums = reg->dense->kind == W_Q4K;
-	const size_t q_bytes = (size_t)batch_len * xq_cols(in_dim) * sizeof(__half);
-	if (sums) {
-		TIE_CUDA_TRY(c, cudaMemsetAsync(s.xq_hi, 0, q_bytes, c->stream));
-		TIE_CUDA_TRY(c, cudaMemsetAsync(s.xq_hi + v.q_lo_off, 0, q_bytes, c->stream));
-	}
-	TRY(launch_split_rows(c, x_dev, nullptr, 1, batch_len, in_dim, s.xs_hi, s.xs_hi + v.lo_off, sums ? s.xq_hi : nullptr,
-			      sums ? s.xq_hi + v.q_lo_off : nullptr));
+	TRY(launch_split_rows(c, x_dev, nullptr, 1, batch_len, in_dim, s.xs_hi, s.xs_hi + v.lo_off, sums ? s.xq : nullptr));
 	TRY(launch_tc_dense(c, *reg->dense, o_dev));
-	if (sums) {
-		TIE_CUDA_TRY(c, cudaMemsetAsync(s.xq_hi, 0, q_bytes, c->stream));
-		TIE_CUDA_TRY(c, cudaMemsetAsync(s.xq_hi + v.q_lo_off, 0, q_bytes, c->stream));
-	}
 	if (!dev) {
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(o, o_dev, (size_t)batch_len * out_dim * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
 		return check_status(c);

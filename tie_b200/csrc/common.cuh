@@ -34,9 +34,9 @@ enum WKind : int { W_Q4K = 0, W_Q6K_R8 = 1 };
 
 // A stand-alone (dense) tensor's view of the context's split-operand scratch, with row length k.
 struct DenseView {
-	CUtensorMap full[6], half[6];  // [0-2] operand boxes of 16/32/64 rows, [3-5] sub-block sums; (hi, lo) in one box / one half per box
+	CUtensorMap full[6], half[6];  // [0-2] operand boxes of 16/32/64 rows, [3-5] sub-block sums; half: boxes of half the rows, for CTA pairs
 	size_t rows = 0;	       // rows the view holds
-	size_t lo_off = 0, q_lo_off = 0;  // element offsets of the lo halves behind the hi halves
+	size_t lo_off = 0;	       // element offset of the lo halves behind the hi halves
 };
 
 struct DevTensor {
@@ -91,8 +91,8 @@ struct Scratch {
 	__half *xs_hi = nullptr, *xs_lo = nullptr;  // [Rpad][H]  split inputs, sorted order
 	__half *hs_hi = nullptr, *hs_lo = nullptr;  // [Rpad][F]
 	// sums of the rows above over 32-wide sub-blocks, split the same way; 64 columns per 2048 k
-	__half *xq_hi = nullptr, *xq_lo = nullptr;  // [Rpad][xq_cols(H)]
-	__half *hq_hi = nullptr, *hq_lo = nullptr;  // [Rpad][xq_cols(F)]
+	__half *xq = nullptr;  // [Rpad][xq_cols(H)]
+	__half *hq = nullptr;  // [Rpad][xq_cols(F)]
 	unsigned *status = nullptr;		    // [1]
 	int *counter = nullptr;			    // [1] last-CTA counter of the fused decode router (zero at rest)
 	unsigned *dec_sync = nullptr;		    // [2] arrivals and epoch of the one-kernel decode step's grid barriers
@@ -176,7 +176,7 @@ struct tie_cuda_ctx {
 	char cuda_err[1024] = {0};
 	// tensor maps for the tcgen05 path: (x, h, sums of x, sums of h) x (16-, 32-, 64-row boxes)
 	CUtensorMap tmap[12];
-	CUtensorMap tmap_half[12];  // the same with boxes of one half (hi or lo): what a CTA of a pair fetches
+	CUtensorMap tmap_half[12];  // the same with boxes of half the rows: what a CTA of a pair fetches
 	bool tmaps_ok = false;
 	int tc_pairs = 0;	    // CTA pairs the device holds at once (0: the pair kernels are not used)
 	bool tc_no_pair = false;    // this call asked for the single-CTA grouped GEMM (TIE_CUDA_PATH_NO_PAIR)
@@ -272,10 +272,15 @@ __device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float
 	return __fmul_rn(__fmaf_rn(__fsub_rn(y2, y1), frac, y1), u);
 }
 
-// Columns of the sub-block-sum arrays for an input dim k: k/32 sums, padded to whole 64-wide tiles.
+// The sub-block sums of a row of k inputs: 16 halves per 256-wide block — the hi parts of its 8 sums, then
+// their lo parts (one 16-deep MMA step takes both) — padded to whole 64-wide tiles.
 __host__ __device__ __forceinline__ int xq_cols(int k)
 {
-	return ((k / 32 + 63) / 64) * 64;
+	return (k / QK_K * 16 + 63) / 64 * 64;
+}
+__host__ __device__ __forceinline__ int xq_index(int sub_block)
+{
+	return (sub_block >> 3) * 16 + (sub_block & 7);	 // of the hi part; the lo part is 8 further
 }
 
 __device__ __forceinline__ float half_bits_to_float(uint32_t h16)

@@ -259,7 +259,7 @@ constexpr int EP_SPLIT_F4 = 8;	// float4 loads a lane keeps in flight
 // n_rows is on the device.
 __global__ void __launch_bounds__(EP_SPLIT_THREADS)
 ep_split_rows(EpView v, const int *__restrict__ n_rows_dev, const int *__restrict__ seg_base, const int *__restrict__ seg_src,
-	      __half *__restrict__ hi, __half *__restrict__ lo, __half *__restrict__ q_hi, __half *__restrict__ q_lo,
+	      __half *__restrict__ hi, __half *__restrict__ lo, __half *__restrict__ xq,
 	      int q_cols, unsigned *__restrict__ row_dst, unsigned *__restrict__ status)
 {
 	__shared__ int s_base[257], s_src[256];
@@ -341,9 +341,9 @@ ep_split_rows(EpView v, const int *__restrict__ n_rows_dev, const int *__restric
 					if (c < H / 4) {
 						reinterpret_cast<uint2 *>(hi + q * H)[c] = hv;
 						reinterpret_cast<uint2 *>(lo + q * H)[c] = lv;
-						if (q_hi && (lane & 7) == 0) {
-							q_hi[q * q_cols + (c >> 3)] = sh;
-							q_lo[q * q_cols + (c >> 3)] = sl;
+						if (xq && (lane & 7) == 0) {
+							xq[q * q_cols + xq_index(c >> 3)] = sh;
+							xq[q * q_cols + xq_index(c >> 3) + 8] = sl;
 						}
 					}
 				}
@@ -442,8 +442,8 @@ int launch_ep_split_rows(tie_cuda_ctx *c, bool sums)
 {
 	Scratch &s = c->s;
 	ep_split_rows<<<c->sm_count * 8, EP_SPLIT_THREADS, 0, c->stream>>>(c->ep.view, c->ep.n_rows, c->ep.seg_base, c->ep.seg_src,
-									    s.xs_hi, s.xs_lo, sums ? s.xq_hi : nullptr,
-									    sums ? s.xq_lo : nullptr, xq_cols(c->cfg.hidden), c->ep.row_dst,
+									    s.xs_hi, s.xs_lo, sums ? s.xq : nullptr,
+									    xq_cols(c->cfg.hidden), c->ep.row_dst,
 									    s.status);
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;

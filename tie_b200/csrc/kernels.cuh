@@ -47,11 +47,11 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, const int *perm, int src_div, int n_rows,
 		       float *rows_out, int *expert_out, int *inv);
 int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_div, int n_rows, int n_cols, __half *hi,
-		      __half *lo, __half *q_hi, __half *q_lo);
+		      __half *lo, __half *xq);
 int launch_swiglu(tie_cuda_ctx *c, float *gate, const float *up, int n);
 // n_rows_dev != null: the row count is read on the device and n_rows CTAs stride over the rows
-int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *q_hi,
-			__half *q_lo, const int *n_rows_dev = nullptr);
+int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *xq,
+			const int *n_rows_dev = nullptr);
 // tensor.cu
 int tc_setup(tie_cuda_ctx *c);
 int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, int n_experts = -1);  // default: the context's local experts

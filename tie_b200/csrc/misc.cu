@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 // one 16-byte store each; optionally the sum over the 32-wide sub-block the values belong to (four
 // neighbouring lanes hold one sub-block), split the same way.
 __device__ __forceinline__ void split8_store(const float v[8], int k0, __half *__restrict__ hi_row, __half *__restrict__ lo_row,
-					     __half *__restrict__ q_hi_row, __half *__restrict__ q_lo_row, int lane)
+					     __half *__restrict__ q_row, int lane)
 {
 	uint32_t h[4], l[4];
 #pragma unroll
@@ -98,14 +98,14 @@ __device__ __forceinline__ void split8_store(const float v[8], int k0, __half *_
 	}
 	*reinterpret_cast<uint4 *>(hi_row + k0) = make_uint4(h[0], h[1], h[2], h[3]);
 	*reinterpret_cast<uint4 *>(lo_row + k0) = make_uint4(l[0], l[1], l[2], l[3]);
-	if (q_hi_row) {
+	if (q_row) {
 		float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
 		sum += __shfl_xor_sync(0xffffffffu, sum, 1);
 		sum += __shfl_xor_sync(0xffffffffu, sum, 2);
 		if ((lane & 3) == 0) {
 			const __half hs = __float2half_rn(sum);
-			q_hi_row[k0 >> 5] = hs;
-			q_lo_row[k0 >> 5] = __float2half_rn(sum - __half2float(hs));
+			q_row[xq_index(k0 >> 5)] = hs;
+			q_row[xq_index(k0 >> 5) + 8] = __float2half_rn(sum - __half2float(hs));
 		}
 	}
 }
@@ -114,13 +114,13 @@ constexpr int ROWS_WARPS = 8;  // warps per CTA of the row passes: one row per w
 
 // Gather rows into expert-sorted order and split each fp32 value v into fp16 hi + lo
 // (hi = rn16(v), lo = rn16(v - hi)): hi+lo carries 22 significand bits, which the tensor-core
-// scheme needs to stay within the 1e-3 parity bound.  q_hi/q_lo (optional, q_cols per row): the
+// scheme needs to stay within the 1e-3 parity bound.  xq (optional, q_cols per row): the
 // sums of the row over its 32-wide sub-blocks, split the same way (the Q4_K "min" term).
 // A warp takes 1024 columns of a row at a time: eight values per lane and step (16-byte loads and
 // stores), four steps' loads in flight; n_cols must be a multiple of 256.
 __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__restrict__ x, const int *__restrict__ perm, int src_div,
 							      int n_rows, int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
-							      __half *__restrict__ q_hi, __half *__restrict__ q_lo, int q_cols)
+							      __half *__restrict__ xq, int q_cols)
 {
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int upr = (n_cols + 1023) >> 10;	// units of 1024 columns per row
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__res
 		const int src = perm ? (int)rid / src_div : p;
 		const float *xr = x + (size_t)src * n_cols;
 		__half *hr = hi + (size_t)p * n_cols, *lr = lo + (size_t)p * n_cols;
-		__half *qh = q_hi ? q_hi + (size_t)p * q_cols : nullptr, *ql = q_hi ? q_lo + (size_t)p * q_cols : nullptr;
+		__half *qr = xq ? xq + (size_t)p * q_cols : nullptr;
 		{
 			const int k0 = (un - p * upr) * 1024 + lane * 8;
 			float4 v[4][2];
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__res
 				const int k = k0 + i * 256;
 				if (k < n_cols) {  // (uniform over the warp: n_cols is a multiple of 256)
 					const float f[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
-					split8_store(f, k, hr, lr, qh, ql, lane);
+					split8_store(f, k, hr, lr, qr, lane);
 				}
 			}
 		}
@@ -185,8 +185,7 @@ __global__ void __launch_bounds__(256) gather_rows(const float *__restrict__ x, 
 // of 256.
 __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float *__restrict__ gu, int ffn, float scale,
 								     const float *__restrict__ silu, __half *__restrict__ hi,
-								     __half *__restrict__ lo, __half *__restrict__ q_hi,
-								     __half *__restrict__ q_lo, int q_cols,
+								     __half *__restrict__ lo, __half *__restrict__ xq, int q_cols,
 								     const int *__restrict__ n_rows_dev, int n_rows_host)
 {
 	__shared__ float tab[SILU_N];
@@ -200,7 +199,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float
 		const size_t r = un / upr;
 		const float *g = gu + r * 2 * ffn, *u = g + ffn;
 		__half *hr = hi + r * ffn, *lr = lo + r * ffn;
-		__half *qh = q_hi ? q_hi + r * q_cols : nullptr, *ql = q_hi ? q_lo + r * q_cols : nullptr;
+		__half *qr = xq ? xq + r * q_cols : nullptr;
 		{
 			const int k = (int)(un - r * upr) * 256 + lane * 8;
 			const float4 g0 = *reinterpret_cast<const float4 *>(g + k), g1 = *reinterpret_cast<const float4 *>(g + k + 4);
@@ -209,7 +208,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float
 					    swiglu_lut(tab, g0.z, u0.z) * scale, swiglu_lut(tab, g0.w, u0.w) * scale,
 					    swiglu_lut(tab, g1.x, u1.x) * scale, swiglu_lut(tab, g1.y, u1.y) * scale,
 					    swiglu_lut(tab, g1.z, u1.z) * scale, swiglu_lut(tab, g1.w, u1.w) * scale};
-			split8_store(f, k, hr, lr, qh, ql, lane);
+			split8_store(f, k, hr, lr, qr, lane);
 		}
 	}
 }
@@ -249,14 +248,14 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 }
 
 int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_div, int n_rows, int n_cols, __half *hi,
-		      __half *lo, __half *q_hi, __half *q_lo)
+		      __half *lo, __half *xq)
 {
 	if (n_cols % 256)
 		return TIE_CUDA_ENOTSUP;
 	const int want = (n_rows * ((n_cols + 1023) / 1024) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 8;
 	if (n_rows <= 0)
 		return TIE_CUDA_OK;
-	split_rows<<<want < cap ? want : cap, ROWS_WARPS * 32, 0, c->stream>>>(x, perm, src_div, n_rows, n_cols, hi, lo, q_hi, q_lo,
+	split_rows<<<want < cap ? want : cap, ROWS_WARPS * 32, 0, c->stream>>>(x, perm, src_div, n_rows, n_cols, hi, lo, xq,
 										xq_cols(n_cols));
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
@@ -270,15 +269,15 @@ int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, c
 	return TIE_CUDA_OK;
 }
 
-int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *q_hi,
-			__half *q_lo, const int *n_rows_dev)
+int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *xq,
+			const int *n_rows_dev)
 {
 	if (ffn % 256)
 		return TIE_CUDA_ENOTSUP;
 	// (n_rows_dev: the row count is read on the device and n_rows is the grid the caller wants)
 	const int want = (n_rows * (ffn / 256) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 4;
 	const int grid = n_rows_dev ? n_rows : (want < cap ? want : cap);
-	swiglu_split_rows<<<grid > 0 ? grid : 1, ROWS_WARPS * 32, 0, c->stream>>>(gu, ffn, scale, c->silu, hi, lo, q_hi, q_lo, xq_cols(ffn),
+	swiglu_split_rows<<<grid > 0 ? grid : 1, ROWS_WARPS * 32, 0, c->stream>>>(gu, ffn, scale, c->silu, hi, lo, xq, xq_cols(ffn),
 										   n_rows_dev, n_rows);
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;

@@ -31,6 +31,15 @@ __device__ __forceinline__ __half2 bits_h2(uint32_t v)
 	return *reinterpret_cast<__half2 *>(&v);
 }
 
+// (w & mask) | magic in ONE logic instruction.  Two literal constants do not fit one instruction, and left
+// to itself the compiler spends two; the expansion is bound by the logic pipe.
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t mask, uint32_t magic)
+{
+	uint32_t r;
+	asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(mask), "r"(magic));
+	return r;
+}
+
 // Scale constants of one Q4_K sub-block pair (low nibbles: sub-block 2p, high nibbles: 2p+1).
 struct Q4kConsts {
 	__half2 sl, cl;	 // low nibbles:  (1024 + q)    * s      - 1024 s
@@ -53,18 +62,18 @@ __device__ __forceinline__ Q4kConsts q4k_int_consts(int s_lo, int s_hi)
 __device__ __forceinline__ void q4k_int_word(uint32_t w, const Q4kConsts &c, uint32_t lo[2], uint32_t hi[2])
 {
 	const uint32_t w8 = w >> 8;
-	lo[0] = h2_bits(__hfma2(bits_h2((w & 0x000F000Fu) | 0x64006400u), c.sl, c.cl));
-	lo[1] = h2_bits(__hfma2(bits_h2((w8 & 0x000F000Fu) | 0x64006400u), c.sl, c.cl));
-	hi[0] = h2_bits(__hfma2(bits_h2((w & 0x00F000F0u) | 0x64006400u), c.sh, c.ch));
-	hi[1] = h2_bits(__hfma2(bits_h2((w8 & 0x00F000F0u) | 0x64006400u), c.sh, c.ch));
+	lo[0] = h2_bits(__hfma2(bits_h2(and_or(w, 0x000F000Fu, 0x64006400u)), c.sl, c.cl));
+	lo[1] = h2_bits(__hfma2(bits_h2(and_or(w8, 0x000F000Fu, 0x64006400u)), c.sl, c.cl));
+	hi[0] = h2_bits(__hfma2(bits_h2(and_or(w, 0x00F000F0u, 0x64006400u)), c.sh, c.ch));
+	hi[1] = h2_bits(__hfma2(bits_h2(and_or(w8, 0x00F000F0u, 0x64006400u)), c.sh, c.ch));
 }
 
 // Four 6-bit quants held as the bytes of q (0..63 each) -> sc*(q-32) pairs: out[0] = bytes (0, 2),
 // out[1] = bytes (1, 3).  s = half2(sc), c = half2(-96 sc).
 __device__ __forceinline__ void q6k_int_word(uint32_t q, __half2 s, __half2 c, uint32_t out[2])
 {
-	out[0] = h2_bits(__hfma2(bits_h2(((q << 4) & 0x03F003F0u) | 0x54005400u), s, c));
-	out[1] = h2_bits(__hfma2(bits_h2(((q >> 4) & 0x03F003F0u) | 0x54005400u), s, c));
+	out[0] = h2_bits(__hfma2(bits_h2(and_or(q << 4, 0x03F003F0u, 0x54005400u)), s, c));
+	out[1] = h2_bits(__hfma2(bits_h2(and_or(q >> 4, 0x03F003F0u, 0x54005400u)), s, c));
 }
 
 // Position of element k inside its group of 4 in the operand tiles: [k0, k2, k1, k3].

@@ -57,7 +57,22 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 		: "memory");
 	return ok != 0;
 }
-// The same, allowing the hardware to suspend the thread for up to `ns` nanoseconds while the
+// The same without waiting: try_wait may hold the thread for a while when the phase is incomplete.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity)
+{
+	uint32_t ok;
+	asm volatile(
+		"{\n\t"
+		".reg .pred p;\n\t"
+		"mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+		"selp.u32 %0, 1, 0, p;\n\t"
+		"}"
+		: "=r"(ok)
+		: "r"(bar), "r"(parity)
+		: "memory");
+	return ok != 0;
+}
+// As try_wait, allowing the hardware to suspend the thread for up to `ns` nanoseconds while the
 // phase is incomplete (a suspended thread issues nothing; it resumes when the phase completes).
 __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t parity, uint32_t ns)
 {
@@ -108,6 +123,13 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *tma
 		"l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z)
 		: "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *tmap, uint32_t bar, int x, int y, int z, int w)
+{
+	asm volatile(
+		"cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
+		"l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+		: "memory");
+}
 // 1-D bulk copy global -> shared (16-byte aligned addresses, size a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
 {
@@ -118,6 +140,18 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *tmap)
 {
 	asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
+}
+
+// ---- register reallocation between the warpgroups of a CTA (executed by whole warpgroups) ----
+template <int N>
+__device__ __forceinline__ void setmaxnreg_inc()
+{
+	asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void setmaxnreg_dec()
+{
+	asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
 // ---- tensor memory ----
@@ -142,28 +176,31 @@ __device__ __forceinline__ void tc_fence_after()
 	asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]; one thread issues for the CTA.
-__device__ __forceinline__ void mma_f16_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+// Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows of 64 fp16 (128 B), 8-row
+// groups 1024 B apart (stride byte offset), tile base 1024-byte aligned.  Advancing the start address
+// by 32 B selects the next 16-wide k slice inside the swizzled row.
+constexpr uint32_t UMMA_DESC_HI = (1024u >> 4)	 // stride byte offset
+				  | (1u << 14)	 // descriptor version (sm_100)
+				  | (2u << 29);	 // layout: SWIZZLE_128B
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr)
 {
-	asm volatile(
-		"{\n\t"
-		".reg .pred p;\n\t"
-		"setp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-		"}" ::"r"(d_tmem),
-		"l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-		: "memory");
+	return (smem_addr & 0x3FFFFu) >> 4;  // start address; leading byte offset: unused for swizzled K-major
 }
-// Same with the A operand in tensor memory (lane = row, two 16-bit k elements per column).
-__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+
+// D[tmem] (+)= A[tmem] * B[smem]; one thread issues for the CTA.
+// A: (lane = row, two 16-bit k elements per column).  bdesc is the
+// low word of the B descriptor (umma_desc_lo); its high word is the same for every operand tile here.
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
 	asm volatile(
 		"{\n\t"
 		".reg .pred p;\n\t"
+		".reg .b64 d;\n\t"
+		"mov.b64 d, {%2, %5};\n\t"
 		"setp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d, %3, p;\n\t"
 		"}" ::"r"(d_tmem),
-		"r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+		"r"(a_tmem), "r"(bdesc), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI)
 		: "memory");
 }
 // One lane of the (converged) warp, always the same one.  MMAs and commits are issued under a branch
@@ -184,9 +221,16 @@ __device__ __forceinline__ bool elect_one()
 	return p != 0;
 }
 // 4 consecutive 32-bit columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d)
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t v[4])
 {
-	asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(a), "r"(b), "r"(c), "r"(d)
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+		     : "memory");
+}
+// 8 consecutive 32-bit columns.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t v[8])
+{
+	asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+		     "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
 		     : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait()
@@ -280,6 +324,13 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap
 		"l"(reinterpret_cast<uint64_t>(tmap)), "r"(leader_addr(local_bar)), "r"(x), "r"(y), "r"(z)
 		: "memory");
 }
+__device__ __forceinline__ void tma_load_4d_pair(uint32_t dst, const CUtensorMap *tmap, uint32_t local_bar, int x, int y, int z, int w)
+{
+	asm volatile(
+		"cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
+		"l"(reinterpret_cast<uint64_t>(tmap)), "r"(leader_addr(local_bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+		: "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_result, uint32_t ncols)
 {
 	asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_result), "r"(ncols) : "memory");
@@ -293,15 +344,17 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 	asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // D[tmem of both CTAs] (+)= A[tmem of both CTAs] * B[shared memory of both CTAs]; one thread of the leader issues.
-__device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc, uint32_t idesc, uint32_t accumulate)
 {
 	asm volatile(
 		"{\n\t"
 		".reg .pred p;\n\t"
+		".reg .b64 d;\n\t"
+		"mov.b64 d, {%2, %5};\n\t"
 		"setp.ne.b32 p, %4, 0;\n\t"
-		"tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+		"tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], d, %3, p;\n\t"
 		"}" ::"r"(d_tmem),
-		"r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
+		"r"(a_tmem), "r"(bdesc), "r"(idesc), "r"(accumulate), "n"(UMMA_DESC_HI)
 		: "memory");
 }
 // One arrival on the barrier at this address in BOTH CTAs of the pair once the MMAs issued so far retire.
@@ -311,20 +364,6 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar)
 		"tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
 		"h"((uint16_t)3)
 		: "memory");
-}
-
-// Shared-memory matrix descriptor, K-major operand, 128-byte swizzle: rows of 64 fp16 (128 B),
-// 8-row groups 1024 B apart (stride byte offset), tile base 1024-byte aligned.  Advancing the
-// start address by 32 B selects the next 16-wide k slice inside the swizzled row.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr)
-{
-	uint64_t d = 0;
-	d |= (uint64_t)((smem_addr & 0x3FFFFu) >> 4);	// start address
-	d |= (uint64_t)0 << 16;				// leading byte offset: unused for swizzled K-major
-	d |= (uint64_t)(1024u >> 4) << 32;		// stride byte offset
-	d |= (uint64_t)1 << 46;				// descriptor version (sm_100)
-	d |= (uint64_t)2 << 61;				// layout: SWIZZLE_128B
-	return d;
 }
 
 // Instruction descriptor for kind::f16: fp16 A and B (both K-major), fp32 accumulate, M x N tile.
