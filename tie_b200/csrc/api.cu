@@ -71,6 +71,8 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TRY(dev_alloc(c, &s.xq, s.rows_pad * XH));
 	TRY(dev_alloc(c, &s.hq, s.rows_pad * XF));
 	TRY(dev_alloc(c, &s.status, 1));
+	TRY(dev_alloc(c, &s.route_counter, (T + 3) / 4));
+	TIE_CUDA_TRY(c, cudaMemset(s.route_counter, 0, (T + 3) / 4 * sizeof(int)));
 	TRY(dev_alloc(c, &s.counter, 1));
 	TIE_CUDA_TRY(c, cudaMemset(s.counter, 0, sizeof(int)));
 	TRY(dev_alloc(c, &s.dec_sync, 2));
@@ -320,11 +322,11 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 			return TIE_CUDA_OK;
 		}
 	}
-	// decode (1-4 tokens): three launches — router with fused selection, gate/up, down + combine
+	// decode and small batches: three launches — router with fused selection, gate/up, down + combine
 	if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR && !(flags & TIE_CUDA_PATH_LEGACY_STREAM) &&
 	    decode_supported(c, L, n_tokens)) {
-		if (lfm2)  // the LFM2 selection is a kernel of its own
-			TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, 1));
+		if (lfm2 || n_tokens > 4)
+			TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
 		else
 			TRY(launch_router_decode_fused(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w));
 		prof_mark(c, 1);
@@ -641,6 +643,8 @@ int tie_cuda_init(tie_cuda_ctx **out, const tie_cuda_config *cfg)
 		return fail(rc);
 	if ((rc = router_setup(c)) != TIE_CUDA_OK)
 		return fail(rc);
+	if ((rc = decode_setup(c)) != TIE_CUDA_OK)
+		return fail(rc);
 	*out = c;
 	return TIE_CUDA_OK;
 }
@@ -674,7 +678,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	void *dev_ptrs[] = {s.x,     s.out,   s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
 			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.status,  s.counter, s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
-			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist};
+			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
 		if (p)
 			cudaFree(p);
@@ -781,8 +785,21 @@ int tie_cuda_last_active_experts(tie_cuda_ctx *c)
 {
 	if (!c)
 		return TIE_CUDA_EINVAL;
-	if (c->last_direct_rows >= 0)
-		return c->last_direct_rows;
+	if (c->last_direct_rows >= 0) {	 // rows that were not sorted: count the experts of the selection
+		const size_t rows = (size_t)c->last_direct_rows;
+		TIE_CUDA_TRY(c, cudaMemcpyAsync(c->pin_idx, c->s.topk_idx, rows * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+		TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+		bool seen[256] = {false};
+		int distinct = 0;
+		for (size_t i = 0; i < rows; i++) {
+			const int le = c->pin_idx[i] - c->first_expert;
+			if (le >= 0 && le < c->n_local && !seen[le]) {
+				seen[le] = true;
+				distinct++;
+			}
+		}
+		return distinct;
+	}
 	int n = 0;
 	TIE_CUDA_TRY(c, cudaMemcpyAsync(&n, c->s.n_active, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));

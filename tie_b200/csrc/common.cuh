@@ -94,6 +94,7 @@ struct Scratch {
 	__half *xq = nullptr;  // [Rpad][xq_cols(H)]
 	__half *hq = nullptr;  // [Rpad][xq_cols(F)]
 	unsigned *status = nullptr;		    // [1]
+	int *route_counter = nullptr;		    // [(T + 3) / 4] CTAs done per token tile of the batched router (zero at rest)
 	int *counter = nullptr;			    // [1] last-CTA counter of the fused decode router (zero at rest)
 	unsigned *dec_sync = nullptr;		    // [2] arrivals and epoch of the one-kernel decode step's grid barriers
 	int *row_expert = nullptr;		    // [R] staging for expert_rows

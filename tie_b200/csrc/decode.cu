@@ -1,53 +1,42 @@
-// Decode path (1-4 tokens): the expert mat-vecs with each CTA's whole weight tile staged in
-// shared memory by bulk asynchronous copies.
+// Decode and small batches (up to 31 tokens of this model's shape): the expert mat-vecs of every
+// (token, slot) row on its own — no dispatch sort, no grouping — with the exact mma.sync products of
+// mma_dot.cuh.
 //
-// Reference: process_expert_task (engine.c:916-964) for the 8 selected experts of a token and the
-// weighted combine (model_qwen3.c:458-467).  At batch 1 the block is a pure stream of 25.5 MB of
-// packed weights, so the only thing that matters is how many bytes are in flight: a CTA issues
-// ONE bulk copy per weight matrix for its complete row tile (the rows of a tile are contiguous
-// in the GGUF layout; up to ~110 KB per CTA, all outstanding at once), stages the activation
-// while the copy flies, waits on the mbarrier and then reduces from shared memory with the same
-// per-lane block algebra as the streaming kernels (partdot.cuh).
+// Reference: process_expert_task (engine.c:916-964) for the selected experts of a token and the
+// weighted combine (model_qwen3.c:458-467).
 //
-//   decode_gate_up       CTA = ((token, slot), row tile): gate and up tiles -> SwiGLU -> h
-//   decode_down_combine  CTA = (token, 16-row tile): the tiles of ALL the token's experts are
-//                        fetched at once; rows are reduced slot by slot and accumulated as
-//                        acc = fma(w_j, row_j, acc), j ascending from zero — the reference's
-//                        combine — so no per-slot output and no separate combine pass exist.
+//   decode_gate_up       CTA = (16 output rows, (token, slot)), warp = one super-block of the input row:
+//                        gate and up products, summed over the warps -> SwiGLU -> h
+//   decode_down_combine  CTA = (16 output rows, token), warp = one slot: the packed rows of all slots are
+//                        requested (one bulk copy per slot) before the wait for h; a warp's super-blocks add up in
+//                        order, the slots are combined as acc = fma(w_j, row_j, acc), j ascending from
+//                        zero — the reference's combine — so no per-slot output and no combine pass exist.
+//
+// What bounds it: at 1-4 tokens latency (three dependent launches, 2-3 us each), above that the expansion of
+// the packed weights (about 230 instructions per warp for 16 rows x 256 Q4_K weights, 450 for Q6_K).
+// Rows that share an expert expand it once each: at 13 tokens 104 rows use 82 experts, at 31 tokens 248
+// rows 111.
 #include "common.cuh"
 #include "kernels.cuh"
-#include "partdot.cuh"
+#include "mma_dot.cuh"
 #include "tc_ptx.cuh"
 #include "decode_common.cuh"
 
 namespace tie {
 
-constexpr int DEC_MAX_CHUNKS = 8;
+constexpr int DEC_MAX_NB = 8;  // super-blocks per row
 
-template <WKind KIND, int K>
-__global__ void __launch_bounds__(DEC_GU_THREADS, 1)
-decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert,
-	       int rows_per_tile, const float *__restrict__ x, int top_k, const int *__restrict__ topk_idx, float *__restrict__ h,
-	       int first_expert, int n_local, const float *__restrict__ silu, unsigned *__restrict__ status, int n_expert_all)
+// Sum of a row's products over its super-blocks, in order (decode_fused.cu adds in the same order).
+template <WKind KIND>
+__global__ void __launch_bounds__(DEC_MAX_NB * 32, 2)
+decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert, int nb,
+	       const float *__restrict__ x, int top_k, const int *__restrict__ topk_idx, float *__restrict__ h, int first_expert,
+	       int n_local, const float *__restrict__ silu, unsigned *__restrict__ status, int n_expert_all)
 {
-	constexpr int PARTS = K / 64;
-	constexpr int LPR = PARTS > 16 ? 32 : (PARTS > 8 ? 16 : (PARTS > 4 ? 8 : 4));
-	constexpr int RPW = 32 / LPR;
-	constexpr int NB = K / QK_K;
-	constexpr int ROWS_PER_PASS = (DEC_GU_THREADS / 32) * RPW;
-	constexpr int CH = ROWS_PER_PASS > 16 ? ROWS_PER_PASS : 16;  // rows per copy chunk (own barrier): a pass never spans two
-	extern __shared__ __align__(128) uint8_t dsm[];
-	__shared__ uint64_t bar[DEC_MAX_CHUNKS];
+	__shared__ __align__(16) uint8_t img[DEC_MAX_NB][XImage<KIND>::BYTES];
+	__shared__ float red[DEC_MAX_NB][2][16];
 	const int slot = blockIdx.y;  // (token, j)
-	const int r0 = blockIdx.x * rows_per_tile;
-	const int r1 = min(r0 + rows_per_tile, rows_per_expert);
-	const int n_chunks = (r1 - r0 + CH - 1) / CH;
-	if (threadIdx.x == 0) {
-		for (int c = 0; c < n_chunks; c++)
-			ptx::mbar_init(ptx::smem_u32(&bar[c]), 1);
-		ptx::fence_barrier_init();
-		ptx::fence_proxy_async_smem();
-	}
+	const int r0 = blockIdx.x * 16;
 	pdl_wait();	// the router's top-k (and x) are visible from here on
 	pdl_trigger();	// the down kernel may start fetching its weights
 	const int ge = topk_idx[slot];
@@ -58,168 +47,114 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 			atomicOr(status, ST_BAD_EXPERT);
 		return;
 	}
-	const uint32_t tile_bytes = (uint32_t)(tile_offset<KIND>(NB, r1) - tile_offset<KIND>(NB, r0));
-	uint8_t *sg = dsm, *su = dsm + tile_bytes;
-	float *xs = reinterpret_cast<float *>(dsm + 2 * (size_t)tile_bytes);
-	if (threadIdx.x == 0) {
-		const size_t base = (size_t)le * expert_stride;
-		for (int c = 0; c < n_chunks; c++) {
-			const int c0 = r0 + c * CH, c1 = min(c0 + CH, r1);
-			const size_t o0 = tile_offset<KIND>(NB, c0), o1 = tile_offset<KIND>(NB, c1);
-			const uint32_t bytes = (uint32_t)(o1 - o0), rel = (uint32_t)(o0 - tile_offset<KIND>(NB, r0));
-			const uint32_t ba = ptx::smem_u32(&bar[c]);
-			ptx::mbar_arrive_expect_tx(ba, 2 * bytes);
-			bulk_g2s(ptx::smem_u32(sg + rel), wg + base + o0, bytes, ba);
-			bulk_g2s(ptx::smem_u32(su + rel), wu + base + o0, bytes, ba);
-		}
+	const int lane = threadIdx.x & 31, b = threadIdx.x >> 5;
+	const size_t off = (size_t)le * expert_stride + tile_offset<KIND>(nb, r0);
+	MmaRows<KIND> g, u;
+	g.load(wg + off, nb, b, lane);
+	u.load(wu + off, nb, b, lane);
+	const float4 *xp = reinterpret_cast<const float4 *>(x + (size_t)(slot / top_k) * nb * QK_K + b * QK_K) + 2 * lane;
+	const float4 x0 = xp[0], x1 = xp[1];
+	const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+	const float inv = x_image<KIND>(v, img[b], lane);
+	float2 r, s;
+	g.dot(img[b], inv, lane, r, s);
+	if ((lane & 3) == 0) {
+		red[b][0][lane >> 2] = r.x * s.x;
+		red[b][0][(lane >> 2) + 8] = r.y * s.y;
 	}
-	const float *xrow = x + (size_t)(slot / top_k) * K;
-	stage_x_lane_major<KIND, LPR>(xrow, xs, PARTS, threadIdx.x, DEC_GU_THREADS);
-	__syncthreads();  // also publishes the barrier initialisation
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int sub = lane / LPR, part = lane % LPR;
-	const bool lane_on = part < PARTS;
-	float xr[64], sx[4];
-	if (lane_on)
-		load_x_lane_major<KIND, LPR>(xs, part, xr, sx);
-	// PartDot addresses rows from the start of an expert: shift the tile bases accordingly
-	const uint8_t *vg = sg - tile_offset<KIND>(NB, r0), *vu = su - tile_offset<KIND>(NB, r0);
-	float *hrow = h + (size_t)slot * rows_per_expert;
-	int waited = -1;
-	// (the SwiGLU table look-ups of all passes go out together at the end: lane p of a row keeps the
-	// sums of pass p, which every lane of the row holds after the reduction)
-	const bool defer = (r1 - r0 + ROWS_PER_PASS - 1) / ROWS_PER_PASS <= LPR;
-	float keep_g = 0.f, keep_u = 0.f;
-	int keep_row = -1, pass = 0;
-	for (int rp = r0; rp < r1; rp += ROWS_PER_PASS, pass++) {
-		const int chunk = (rp - r0) / CH;
-		if (chunk != waited) {	// rows of a pass share a chunk; chunks arrive in order
-			if (!dec_wait(ptx::smem_u32(&bar[chunk]), status))
-				return;
-			waited = chunk;
-		}
-		const int row = rp + warp * RPW + sub;
-		float vgv = 0.f, vuv = 0.f;
-		if (lane_on && row < r1) {
-			vgv = PartDot<KIND>::dot(PartDot<KIND>::template load<true>(vg, NB, row, part), part, xr, sx);
-			vuv = PartDot<KIND>::dot(PartDot<KIND>::template load<true>(vu, NB, row, part), part, xr, sx);
-		}
-#pragma unroll
-		for (int o = LPR / 2; o > 0; o >>= 1) {
-			vgv += __shfl_xor_sync(0xffffffffu, vgv, o);
-			vuv += __shfl_xor_sync(0xffffffffu, vuv, o);
-		}
-		if (defer) {
-			if (part == pass && row < r1) {
-				keep_g = vgv;
-				keep_u = vuv;
-				keep_row = row;
-			}
-		} else if (part == 0 && row < r1) {
-			hrow[row] = swiglu_lut(silu, vgv, vuv);
-		}
+	u.dot(img[b], inv, lane, r, s);
+	if ((lane & 3) == 0) {
+		red[b][1][lane >> 2] = r.x * s.x;
+		red[b][1][(lane >> 2) + 8] = r.y * s.y;
 	}
-	if (keep_row >= 0)
-		hrow[keep_row] = swiglu_lut(silu, keep_g, keep_u);
+	__syncthreads();
+	if (threadIdx.x < 32) {
+		float sum = red[0][lane >> 4][lane & 15];
+		for (int i = 1; i < nb; i++)
+			sum = __fadd_rn(sum, red[i][lane >> 4][lane & 15]);
+		const float up = __shfl_down_sync(0xffffffffu, sum, 16);
+		if (lane < 16)
+			h[(size_t)slot * rows_per_expert + r0 + lane] = swiglu_lut(silu, sum, up);
+	}
 }
 
-template <WKind KIND, int K>
-__global__ void __launch_bounds__(DEC_THREADS, 1)
-decode_down_combine(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_expert, int rows_per_tile,
-		    const float *__restrict__ h, int top_k, const int *__restrict__ topk_idx, const float *__restrict__ topk_w,
-		    const float *__restrict__ residual, float *__restrict__ out, int first_expert, int n_local,
-		    unsigned *__restrict__ status)
+// The product of slot j's 16 staged rows with its h row, in this warp: lane (g, t = 0, 1) ends up with rows g, g + 8.
+template <WKind KIND>
+__device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const float *hrow, uint8_t *img, int lane)
 {
-	constexpr int PARTS = K / 64;
-	constexpr int LPR = PARTS > 16 ? 32 : (PARTS > 8 ? 16 : (PARTS > 4 ? 8 : 4));
-	constexpr int RPW = 32 / LPR;
-	constexpr int NB = K / QK_K;
-	constexpr int ROWS_PER_PASS = (DEC_THREADS / 32) * RPW;
-	constexpr int MAX_PASSES = 4;
-	constexpr int XS_T = LPR * 64;	// floats of one lane-major activation row
+	float2 out = make_float2(0.f, 0.f);
+	for (int b = 0; b < nb; b++) {
+		const float4 *hp = reinterpret_cast<const float4 *>(hrow + b * QK_K) + 2 * lane;
+		const float4 h0 = hp[0], h1 = hp[1];
+		const float v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+		const float inv = x_image<KIND>(v, img, lane);
+		MmaRows<KIND> w;
+		w.load_smem(tile, nb, b, lane);
+		float2 r, s;
+		w.dot(img, inv, lane, r, s);
+		out.x = __fmaf_rn(s.x, r.x, out.x);
+		out.y = __fmaf_rn(s.y, r.y, out.y);
+	}
+	return out;
+}
+
+template <WKind KIND>
+__global__ void __launch_bounds__(MAX_TOP_K * 32, 2)
+decode_down_combine(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_expert, int nb, const float *__restrict__ h,
+		    int top_k, const int *__restrict__ topk_idx, const float *__restrict__ topk_w, const float *__restrict__ residual,
+		    float *__restrict__ out, int first_expert, int n_local, unsigned *__restrict__ status)
+{
 	extern __shared__ __align__(128) uint8_t dsm[];
+	__shared__ __align__(16) uint8_t img[MAX_TOP_K][XImage<KIND>::BYTES];
 	__shared__ uint64_t bar[MAX_TOP_K];  // one per slot: a slot's rows are reduced as soon as its tile lands
-	__shared__ int s_le[MAX_TOP_K];
-	__shared__ float s_w[MAX_TOP_K];
-	const int t = blockIdx.y;
-	const int r0 = blockIdx.x * rows_per_tile;
-	const int r1 = min(r0 + rows_per_tile, rows_per_expert);
-	const uint32_t tile_bytes = (uint32_t)(tile_offset<KIND>(NB, r1) - tile_offset<KIND>(NB, r0));
-	float *hs = reinterpret_cast<float *>(dsm + (size_t)top_k * tile_bytes);  // two lane-major rows (double buffer)
+	__shared__ float red[MAX_TOP_K][16];
+	__shared__ int s_bad;
+	const int t = blockIdx.y, r0 = blockIdx.x * 16;
+	const uint32_t tile_bytes = (uint32_t)tile_offset<KIND>(nb, 16);
+	const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
 	// The selection was written two kernels ago and the weights never change: the tiles of all the
 	// token's experts are requested BEFORE waiting for the gate/up kernel, so this fetch overlaps it.
 	if (threadIdx.x == 0) {
-		for (int j = 0; j < top_k; j++)
-			ptx::mbar_init(ptx::smem_u32(&bar[j]), 1);
+		for (int k = 0; k < top_k; k++)
+			ptx::mbar_init(ptx::smem_u32(&bar[k]), 1);
 		ptx::fence_barrier_init();
 		ptx::fence_proxy_async_smem();
-		bool bad = false;
-		for (int j = 0; j < top_k; j++) {
-			const int le = topk_idx[t * top_k + j] - first_expert;
-			s_le[j] = le;
-			s_w[j] = topk_w[t * top_k + j];
-			bad |= (le < 0 || le >= n_local);
-		}
-		if (bad) {
-			s_le[0] = -1;
+		s_bad = 0;
+	}
+	__syncthreads();
+	if (lane == 0) {
+		const int le = topk_idx[t * top_k + j] - first_expert;
+		if (le < 0 || le >= n_local) {
+			s_bad = 1;
 			if (blockIdx.x == 0)
 				atomicOr(status, ST_BAD_EXPERT);
 		} else {
-			for (int j = 0; j < top_k; j++) {
-				const uint32_t ba = ptx::smem_u32(&bar[j]);
-				ptx::mbar_arrive_expect_tx(ba, tile_bytes);
-				bulk_g2s(ptx::smem_u32(dsm + (size_t)j * tile_bytes),
-					 wd + (size_t)s_le[j] * expert_stride + tile_offset<KIND>(NB, r0), tile_bytes, ba);
-			}
+			const uint32_t ba = ptx::smem_u32(&bar[j]);
+			ptx::mbar_arrive_expect_tx(ba, tile_bytes);
+			bulk_g2s(ptx::smem_u32(dsm + (size_t)j * tile_bytes), wd + (size_t)le * expert_stride + tile_offset<KIND>(nb, r0), tile_bytes, ba);
 		}
 	}
 	pdl_wait();  // h of the gate/up kernel is visible from here on
-	const float *hrow = h + (size_t)t * top_k * K;
-	stage_x_lane_major<KIND, LPR>(hrow, hs, PARTS, threadIdx.x, DEC_THREADS);
 	__syncthreads();
-	if (s_le[0] < 0)
-		return;
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int sub = lane / LPR, part = lane % LPR;
-	const bool lane_on = part < PARTS;
-	float acc[MAX_PASSES];
-#pragma unroll
-	for (int p = 0; p < MAX_PASSES; p++)
-		acc[p] = 0.f;
-	for (int j = 0; j < top_k; j++) {
-		float xr[64], sx[4];
-		if (lane_on)
-			load_x_lane_major<KIND, LPR>(hs + (size_t)(j & 1) * XS_T, part, xr, sx);
-		if (j + 1 < top_k)  // next slot's activation into the other buffer (last read two slots ago)
-			stage_x_lane_major<KIND, LPR>(hrow + (size_t)(j + 1) * K, hs + (size_t)((j + 1) & 1) * XS_T, PARTS, threadIdx.x, DEC_THREADS);
-		if (!dec_wait(ptx::smem_u32(&bar[j]), status))
-			return;
-		const uint8_t *vd = dsm + (size_t)j * tile_bytes - tile_offset<KIND>(NB, r0);
-		const float wj = s_w[j];
-#pragma unroll
-		for (int p = 0; p < MAX_PASSES; p++) {
-			const int row = r0 + p * ROWS_PER_PASS + warp * RPW + sub;
-			if (r0 + p * ROWS_PER_PASS >= r1)
-				break;
-			float v = 0.f;
-			if (lane_on && row < r1)
-				v = PartDot<KIND>::dot(PartDot<KIND>::template load<true>(vd, NB, row, part), part, xr, sx);
-#pragma unroll
-			for (int o = LPR / 2; o > 0; o >>= 1)
-				v += __shfl_xor_sync(0xffffffffu, v, o);
-			acc[p] = __fmaf_rn(wj, v, acc[p]);  // model_qwen3.c:458-467, slot order, from zero
-		}
-		__syncthreads();  // the staged row of slot j+1 is complete; buffer j&1 is free again
+	const bool bad = s_bad != 0;
+	const bool mine = topk_idx[t * top_k + j] - first_expert >= 0 && topk_idx[t * top_k + j] - first_expert < n_local;
+	const bool ok = !mine || dec_wait(ptx::smem_u32(&bar[j]), status);
+	if (!__syncthreads_and(ok) || bad)
+		return;	 // (every tile that was requested has landed, or its wait has run out)
+	const float2 v = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane);
+	if ((lane & 3) == 0) {
+		red[j][lane >> 2] = v.x;
+		red[j][(lane >> 2) + 8] = v.y;
 	}
-#pragma unroll
-	for (int p = 0; p < MAX_PASSES; p++) {
-		const int row = r0 + p * ROWS_PER_PASS + warp * RPW + sub;
-		if (part == 0 && row < r1 && r0 + p * ROWS_PER_PASS < r1) {
-			float v = acc[p];
-			if (residual)
-				v = __fadd_rn(residual[(size_t)t * rows_per_expert + row], v);
-			out[(size_t)t * rows_per_expert + row] = v;
-		}
+	__syncthreads();
+	if (threadIdx.x < 16) {
+		float acc = 0.f;
+		for (int k = 0; k < top_k; k++)
+			acc = __fmaf_rn(topk_w[t * top_k + k], red[k][threadIdx.x], acc);  // model_qwen3.c:458-467, slot order, from zero
+		const size_t at = (size_t)t * rows_per_expert + r0 + threadIdx.x;
+		if (residual)
+			acc = __fadd_rn(residual[at], acc);
+		out[at] = acc;
 	}
 }
 
@@ -231,52 +166,33 @@ decode_down_combine(const uint8_t *__restrict__ wd, size_t expert_stride, int ro
 // bit-identical to the one-GPU decode kernels.  A peer's y rows of the previous step may only be
 // overwritten once that peer has started this step (its pub flag): the CTA waits for all pub
 // flags first (bounded; they are words of this rank's own region).
-template <WKind KIND, int K>
-__global__ void __launch_bounds__(DEC_THREADS, 1)
-decode_down_peer(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_expert, int rows_per_tile,
-		 const float *__restrict__ h, int top_k, const int *__restrict__ topk_idx, const EpView v,
-		 const unsigned *__restrict__ step_dev, long long budget, int first_expert, int n_local, unsigned *__restrict__ status)
+template <WKind KIND>
+__global__ void __launch_bounds__(MAX_TOP_K * 32, 2)
+decode_down_peer(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_expert, int nb, const float *__restrict__ h, int top_k,
+		 const int *__restrict__ topk_idx, const EpView v, const unsigned *__restrict__ step_dev, long long budget, int first_expert,
+		 int n_local, unsigned *__restrict__ status)
 {
-	constexpr int PARTS = K / 64;
-	constexpr int LPR = PARTS > 16 ? 32 : (PARTS > 8 ? 16 : (PARTS > 4 ? 8 : 4));
-	constexpr int RPW = 32 / LPR;
-	constexpr int NB = K / QK_K;
-	constexpr int ROWS_PER_PASS = (DEC_THREADS / 32) * RPW;
-	constexpr int MAX_PASSES = 4;
 	extern __shared__ __align__(128) uint8_t dsm[];
+	__shared__ __align__(16) uint8_t img[MAX_TOP_K][XImage<KIND>::BYTES];
 	__shared__ uint64_t bar[MAX_TOP_K];
-	__shared__ int s_le[MAX_TOP_K];
-	const int t = blockIdx.y;
-	const int r0 = blockIdx.x * rows_per_tile;
-	const int r1 = min(r0 + rows_per_tile, rows_per_expert);
-	const uint32_t tile_bytes = (uint32_t)(tile_offset<KIND>(NB, r1) - tile_offset<KIND>(NB, r0));
-	float *hs = reinterpret_cast<float *>(dsm + (size_t)top_k * tile_bytes);
+	const int t = blockIdx.y, r0 = blockIdx.x * 16;
+	const uint32_t tile_bytes = (uint32_t)tile_offset<KIND>(nb, 16);
+	const int lane = threadIdx.x & 31, j = threadIdx.x >> 5;
 	if (threadIdx.x == 0) {
-		for (int j = 0; j < top_k; j++)
-			ptx::mbar_init(ptx::smem_u32(&bar[j]), 1);
+		for (int k = 0; k < top_k; k++)
+			ptx::mbar_init(ptx::smem_u32(&bar[k]), 1);
 		ptx::fence_barrier_init();
 		ptx::fence_proxy_async_smem();
-		bool bad = false;
-		for (int j = 0; j < top_k; j++) {
-			const int ge = topk_idx[t * top_k + j];
-			const int le = ge - first_expert;
-			bad |= (ge < 0 || ge >= v.n_expert);
-			s_le[j] = (le >= 0 && le < n_local) ? le : -1;
-		}
-		if (bad) {
-			for (int j = 0; j < top_k; j++)
-				s_le[j] = -1;
-			if (blockIdx.x == 0)
-				atomicOr(status, ST_BAD_EXPERT);
-		}
-		for (int j = 0; j < top_k; j++) {
-			if (s_le[j] < 0)
-				continue;
-			const uint32_t ba = ptx::smem_u32(&bar[j]);
-			ptx::mbar_arrive_expect_tx(ba, tile_bytes);
-			bulk_g2s(ptx::smem_u32(dsm + (size_t)j * tile_bytes), wd + (size_t)s_le[j] * expert_stride + tile_offset<KIND>(NB, r0),
-				 tile_bytes, ba);
-		}
+	}
+	__syncthreads();
+	const int ge = topk_idx[t * top_k + j], le = ge - first_expert;
+	const bool bad = ge < 0 || ge >= v.n_expert, mine = !bad && le >= 0 && le < n_local;
+	if (bad && lane == 0 && blockIdx.x == 0)
+		atomicOr(status, ST_BAD_EXPERT);
+	if (mine && lane == 0) {
+		const uint32_t ba = ptx::smem_u32(&bar[j]);
+		ptx::mbar_arrive_expect_tx(ba, tile_bytes);
+		bulk_g2s(ptx::smem_u32(dsm + (size_t)j * tile_bytes), wd + (size_t)le * expert_stride + tile_offset<KIND>(nb, r0), tile_bytes, ba);
 	}
 	pdl_wait();  // h of the gate/up kernel is visible from here on
 	// every rank has started this step: its y rows of the previous step are combined and may be overwritten
@@ -297,48 +213,22 @@ decode_down_peer(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_
 			__nanosleep(100);
 		}
 	}
-	ok = __syncthreads_and(ok);  // (also publishes the barrier initialisation and s_le)
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int sub = lane / LPR, part = lane % LPR;
-	const bool lane_on = part < PARTS;
+	ok = __syncthreads_and(ok);
 	if (!ok && threadIdx.x == 0)
 		atomicOr(status, ST_WAIT_TIMEOUT);
-	for (int j = 0; j < top_k; j++) {
-		if (s_le[j] < 0)
-			continue;  // (uniform over the CTA)
-		if (!ok) {  // leave, but not with copies in flight
-			if (threadIdx.x == 0)
-				dec_wait(ptx::smem_u32(&bar[j]), status);
-			continue;
-		}
-		stage_x_lane_major<KIND, LPR>(h + (size_t)(t * top_k + j) * K, hs, PARTS, threadIdx.x, DEC_THREADS);
-		__syncthreads();
-		float xr[64], sx[4];
-		if (lane_on)
-			load_x_lane_major<KIND, LPR>(hs, part, xr, sx);
-		if (!dec_wait(ptx::smem_u32(&bar[j]), status))
-			ok = false;
-		ok = __syncthreads_and(ok);  // hs is free again; a failed wait is seen by all
-		if (!ok)
-			continue;
-		const uint8_t *vd = dsm + (size_t)j * tile_bytes - tile_offset<KIND>(NB, r0);
-#pragma unroll
-		for (int p = 0; p < MAX_PASSES; p++) {
-			const int row = r0 + p * ROWS_PER_PASS + warp * RPW + sub;
-			if (r0 + p * ROWS_PER_PASS >= r1)
-				break;
-			float val = 0.f;
-			if (lane_on && row < r1)
-				val = PartDot<KIND>::dot(PartDot<KIND>::template load<true>(vd, NB, row, part), part, xr, sx);
-#pragma unroll
-			for (int o = LPR / 2; o > 0; o >>= 1)
-				val += __shfl_xor_sync(0xffffffffu, val, o);
-			if (part == 0 && row < r1) {
-				const size_t at = (size_t)(t * top_k + j) * rows_per_expert + row;
-				for (int r = 0; r < v.n_ranks; r++)
-					reinterpret_cast<float *>(v.peer[r] + v.off_y)[at] = val;
-			}
-		}
+	// (a wait for the copies in any case: nobody leaves with copies in flight)
+	const bool landed = !mine || dec_wait(ptx::smem_u32(&bar[j]), status);
+	if (!__syncthreads_and(landed) || !ok || __syncthreads_or(bad))
+		return;
+	if (!mine)
+		return;
+	const float2 r = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane);
+	// lanes of t = 0 hold row g, their neighbours of t = 1 store row g + 8
+	if ((lane & 3) < 2) {
+		const size_t at = (size_t)(t * top_k + j) * rows_per_expert + r0 + (lane >> 2) + 8 * (lane & 1);
+		const float val = lane & 1 ? r.y : r.x;
+		for (int k = 0; k < v.n_ranks; k++)
+			reinterpret_cast<float *>(v.peer[k] + v.off_y)[at] = val;
 	}
 }
 
@@ -346,151 +236,77 @@ decode_down_peer(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_
 
 constexpr int DEC_MAX_SMEM = 200 * 1024;
 
-template <WKind KIND>
-static size_t row_bytes_of(int k)
+static size_t dec_down_smem(const Layer &L, int top_k)
 {
-	return (size_t)(k / QK_K) * (KIND == W_Q4K ? Q4K_BYTES : Q6K_BYTES);
+	const int nb = L.down.k / QK_K;
+	return (size_t)top_k * (L.down.kind == W_Q4K ? tile_offset<W_Q4K>(nb, 16) : tile_offset<W_Q6K_R8>(nb, 16));
 }
-
-template <WKind KIND, int K>
-static int launch_dec_gu_t(tie_cuda_ctx *c, const Layer &L, const float *x, int n_rows, int n_expert_all)
-{
-	const int rows = L.gate.rows;
-	const size_t rb = row_bytes_of<KIND>(K);
-	int want_tiles = max(1, c->sm_count / max(1, n_rows));
-	int rpt = (rows + want_tiles - 1) / want_tiles;
-	rpt = ((rpt + 7) / 8) * 8;
-	const int max_rpt = (int)(((DEC_MAX_SMEM - 2 * K * 4) / 2 / rb) / 8 * 8);
-	rpt = max(8, min(rpt, max_rpt));
-	const int tiles = (rows + rpt - 1) / rpt;
-	rpt = min(rpt, 8 * 16);	 // at most DEC_MAX_CHUNKS copy chunks of 16 rows
-	const size_t smem = 2 * (size_t)rpt * rb + (size_t)2 * K * 4;  // lane-major x needs LPR*64 <= 2K floats
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_gate_up<KIND, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(tiles, n_rows);
-	cfg.blockDim = dim3(DEC_GU_THREADS);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = c->stream;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, decode_gate_up<KIND, K>, (const uint8_t *)L.gate.ptr, (const uint8_t *)L.up.ptr,
-					   L.gate.expert_stride, rows, rpt, x, c->cfg.top_k, (const int *)c->s.topk_idx, c->s.h,
-					   c->first_expert, c->n_local, (const float *)c->silu, c->s.status, n_expert_all));
-	c->launches++;
-	return TIE_CUDA_OK;
-}
-
-template <WKind KIND, int K>
-static int launch_dec_dn_t(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out)
-{
-	const int rows = L.down.rows, top_k = c->cfg.top_k;
-	const size_t rb = row_bytes_of<KIND>(K);
-	const int rpt = 16;
-	const size_t smem = (size_t)top_k * rpt * rb + (size_t)2 * 2 * K * 4;  // weight tiles + two lane-major h rows
-	if (smem > (size_t)DEC_MAX_SMEM)
-		return TIE_CUDA_ENOTSUP;
-	const int tiles = (rows + rpt - 1) / rpt;
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<KIND, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(tiles, n_tokens);
-	cfg.blockDim = dim3(DEC_THREADS);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = c->stream;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, decode_down_combine<KIND, K>, (const uint8_t *)L.down.ptr, L.down.expert_stride, rows,
-					   rpt, (const float *)c->s.h, top_k, (const int *)c->s.topk_idx, (const float *)c->s.topk_w,
-					   residual, out, c->first_expert, c->n_local, c->s.status));
-	c->launches++;
-	return TIE_CUDA_OK;
-}
-
-template <WKind KIND, int K>
-static int launch_dec_dn_peer_t(tie_cuda_ctx *c, const Layer &L, int n_tokens)
-{
-	const int rows = L.down.rows, top_k = c->cfg.top_k;
-	const size_t rb = row_bytes_of<KIND>(K);
-	const int rpt = 16;
-	const size_t smem = (size_t)top_k * rpt * rb + (size_t)2 * 2 * K * 4;
-	if (smem > (size_t)DEC_MAX_SMEM)
-		return TIE_CUDA_ENOTSUP;
-	const int tiles = (rows + rpt - 1) / rpt;
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_peer<KIND, K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3(tiles, n_tokens);
-	cfg.blockDim = dim3(DEC_THREADS);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = c->stream;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, decode_down_peer<KIND, K>, (const uint8_t *)L.down.ptr, L.down.expert_stride, rows, rpt,
-					   (const float *)c->s.h, top_k, (const int *)c->s.topk_idx, c->ep.view,
-					   (const unsigned *)c->ep.step_dev, c->ep.wait_cycles, c->first_expert, c->n_local, c->s.status));
-	c->launches++;
-	return TIE_CUDA_OK;
-}
-
-#define TIE_DEC_DIMS(X) X(256) X(512) X(768) X(1024) X(2048)
 
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
-	auto ok_dim = [](int k) { return k == 256 || k == 512 || k == 768 || k == 1024 || k == 2048; };
-	return n_tokens <= 4 && L.gate.kind == L.up.kind && ok_dim(L.gate.k) && ok_dim(L.down.k) && L.down.rows % 16 == 0 &&
-	       L.gate.rows % 8 == 0;
+	// every (token, slot) row by itself up to the batch where the experts' rows are grouped (two rows per
+	// expert on average, run_experts)
+	const int n_rows = n_tokens * c->cfg.top_k;
+	return (n_tokens <= 4 || n_rows < 2 * c->n_local) && n_rows <= 65535 && L.gate.kind == L.up.kind &&
+	       L.gate.k <= DEC_MAX_NB * QK_K && L.gate.rows % 16 == 0 && L.down.rows % 16 == 0 && L.down.k <= DEC_MAX_NB * QK_K &&
+	       dec_down_smem(L, c->cfg.top_k) <= (size_t)DEC_MAX_SMEM;
+}
+
+template <class... P, class... A>
+static int launch_pdl(tie_cuda_ctx *c, void (*kern)(P...), dim3 grid, int threads, size_t smem, A... args)
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = dim3(threads);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = c->stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+	c->launches++;
+	return TIE_CUDA_OK;
+}
+
+// Opt-in shared-memory sizes, once per context.
+int decode_setup(tie_cuda_ctx *c)
+{
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<W_Q4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<W_Q6K_R8>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_peer<W_Q4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_peer<W_Q6K_R8>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
+	return TIE_CUDA_OK;
 }
 
 // x [n_tokens][hidden] -> h [(token, slot)][ffn] (sorted nowhere: rows are the top-k entries themselves)
 int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n_tokens, bool foreign_slots_ok)
 {
-	const int n_rows = n_tokens * c->cfg.top_k;
-	const int nea = foreign_slots_ok ? c->cfg.n_expert : 0;
-	switch (L.gate.k) {
-#define X(KK)                                                                                                   \
-	case KK:                                                                                                \
-		return L.gate.kind == W_Q4K ? launch_dec_gu_t<W_Q4K, KK>(c, L, x, n_rows, nea) : launch_dec_gu_t<W_Q6K_R8, KK>(c, L, x, n_rows, nea);
-		TIE_DEC_DIMS(X)
-#undef X
-	default:
-		return TIE_CUDA_ENOTSUP;
-	}
+	const int n_rows = n_tokens * c->cfg.top_k, nb = L.gate.k / QK_K;
+	auto kern = L.gate.kind == W_Q4K ? decode_gate_up<W_Q4K> : decode_gate_up<W_Q6K_R8>;
+	return launch_pdl(c, kern, dim3(L.gate.rows / 16, n_rows), 32 * nb, 0, L.gate.ptr, L.up.ptr, L.gate.expert_stride, L.gate.rows, nb, x,
+			  c->cfg.top_k, c->s.topk_idx, c->s.h, c->first_expert, c->n_local, c->silu, c->s.status,
+			  foreign_slots_ok ? c->cfg.n_expert : 0);
 }
 
 // h -> out [n_tokens][hidden] (= residual + sum_j w_j * down_j(h_j))
 int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out)
 {
-	switch (L.down.k) {
-#define X(KK)                                                                                                          \
-	case KK:                                                                                                       \
-		return L.down.kind == W_Q4K ? launch_dec_dn_t<W_Q4K, KK>(c, L, n_tokens, residual, out)                \
-					    : launch_dec_dn_t<W_Q6K_R8, KK>(c, L, n_tokens, residual, out);
-		TIE_DEC_DIMS(X)
-#undef X
-	default:
-		return TIE_CUDA_ENOTSUP;
-	}
+	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
+	auto kern = L.down.kind == W_Q4K ? decode_down_combine<W_Q4K> : decode_down_combine<W_Q6K_R8>;
+	return launch_pdl(c, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
+			  L.down.rows, nb, c->s.h, top_k, c->s.topk_idx, c->s.topk_w, residual, out, c->first_expert, c->n_local, c->s.status);
 }
 
 // h (local slots) -> the y rows of every rank's region (expert-parallel decode on replicated tokens)
 int launch_decode_down_peer(tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
-	switch (L.down.k) {
-#define X(KK)                                                                                              \
-	case KK:                                                                                           \
-		return L.down.kind == W_Q4K ? launch_dec_dn_peer_t<W_Q4K, KK>(c, L, n_tokens) : launch_dec_dn_peer_t<W_Q6K_R8, KK>(c, L, n_tokens);
-		TIE_DEC_DIMS(X)
-#undef X
-	default:
-		return TIE_CUDA_ENOTSUP;
-	}
+	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
+	auto kern = L.down.kind == W_Q4K ? decode_down_peer<W_Q4K> : decode_down_peer<W_Q6K_R8>;
+	return launch_pdl(c, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
+			  L.down.rows, nb, c->s.h, top_k, c->s.topk_idx, c->ep.view, c->ep.step_dev, c->ep.wait_cycles, c->first_expert,
+			  c->n_local, c->s.status);
 }
 
 }  // namespace tie

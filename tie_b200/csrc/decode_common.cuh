@@ -7,10 +7,6 @@
 
 namespace tie {
 
-constexpr int DEC_THREADS = 256;
-// gate/up: 16 warps per SM — the reduction out of shared memory is latency-bound (dependent
-// unpack -> fma chains), so twice the warps per scheduler halve its time
-constexpr int DEC_GU_THREADS = 512;
 constexpr long long DEC_WAIT_CYCLES = 1ll << 30;
 
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)

@@ -26,7 +26,7 @@
 // waits (bounded) for its own copies in flight and returns.
 #include "common.cuh"
 #include "kernels.cuh"
-#include "partdot.cuh"
+#include "mma_dot.cuh"
 #include "tc_ptx.cuh"
 #include "decode_common.cuh"
 #include "router_topk.cuh"
@@ -35,9 +35,9 @@
 
 namespace tie {
 
-constexpr int DF_THREADS = 512;
+constexpr int DF_THREADS = 768;	// 24 warps: two products of 16 rows x one super-block each for gate/up, one for down
+constexpr int DF_WARPS = DF_THREADS / 32;
 constexpr int DF_MAX_CHUNKS = 8;
-constexpr int DF_MAX_PASSES = 4;
 constexpr long long DF_WAIT_CYCLES = 1ll << 30;
 
 struct DfShared {
@@ -50,6 +50,7 @@ struct DfShared {
 	int ok;
 	int dn_req[MAX_TOP_K];	// the down tile of slot j has been requested
 	float inv;  // 1 / rms of the row (RMSNorm in the kernel)
+	float x_inv[8];	 // per super-block of x: the factor that undoes its image's scaling
 };
 
 struct DfArgs {
@@ -67,7 +68,7 @@ struct DfArgs {
 	unsigned *status, *sync;  // sync[0]: arrivals, sync[1]: epoch
 	int n_expert, top_k, first_expert, n_local;
 	int rpt_gu, tiles_gu, rpt_dn, tiles_dn;
-	uint32_t off_b, off_c, off_v, off_n;  // shared-memory offsets: down tiles, staged x, slot products, normed x
+	uint32_t off_b, off_c, off_v, off_n;  // shared-memory offsets: down tiles, images of x, products, normed x
 };
 
 __device__ __forceinline__ unsigned df_ld_acquire(const unsigned *p)
@@ -99,46 +100,26 @@ __device__ __forceinline__ bool df_grid_barrier(unsigned *counter, unsigned targ
 	return sh->ok != 0;
 }
 
-template <WKind KIND, int LPR>
-__device__ __forceinline__ void df_stage_lane_major_cg(const float *xrow, float *xs_t, int parts, int tid)
-{
-	// as stage_x_lane_major, with loads that bypass L1: the row was written by other CTAs of this grid
-	for (int d = tid; d < 16 * parts; d += DF_THREADS) {
-		const int r4 = d / parts, p = d % parts;
-		const int k = PartDot<KIND>::src_index(p, 4 * r4);
-		*reinterpret_cast<float4 *>(xs_t + (size_t)(r4 * LPR + p) * 4) = __ldcg(reinterpret_cast<const float4 *>(xrow + k));
-	}
-}
-
-template <int KDIM>
-struct DfDims {
-	static constexpr int PARTS = KDIM / 64;
-	static constexpr int LPR = PARTS > 16 ? 32 : (PARTS > 8 ? 16 : (PARTS > 4 ? 8 : 4));
-	static constexpr int RPW = 32 / LPR;
-	static constexpr int NB = KDIM / QK_K;
-	static constexpr int RPP = (DF_THREADS / 32) * RPW;  // rows per pass of the whole CTA
-};
-
 template <WKind KG, int K, WKind KD, int F>
 __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 {
-	using DK = DfDims<K>;
-	using DF = DfDims<F>;
-	constexpr int CH = DK::RPP > 16 ? DK::RPP : 16;	 // rows per gate/up copy chunk (own barrier)
+	constexpr int NBK = K / QK_K, NBF = F / QK_K;
+	constexpr int CH = 16;	// rows per gate/up copy chunk (own barrier): one MMA tile
 	extern __shared__ __align__(128) uint8_t dsm[];
 	__shared__ DfShared sh;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int cta = blockIdx.x, G = gridDim.x;
 	const int top_k = a.top_k;
-	float *xs = reinterpret_cast<float *>(dsm + a.off_c);  // x, lane-major, for the gate/up reduction
+	uint8_t *ximg = dsm + a.off_c;			    // images of x's super-blocks, for gate/up
+	float *prod = reinterpret_cast<float *>(dsm + a.off_v);	 // products before they are added up
 
 	const bool gu_role = cta < top_k * a.tiles_gu, dn_role = cta < a.tiles_dn;
 	const int slot = cta / a.tiles_gu;
 	const int g0 = (cta % a.tiles_gu) * a.rpt_gu, g1 = min(g0 + a.rpt_gu, F);
 	const int d0 = cta * a.rpt_dn, d1 = min(d0 + a.rpt_dn, K);
 	const int n_chunks = gu_role ? (g1 - g0 + CH - 1) / CH : 0;
-	const uint32_t tile_gu = (uint32_t)(tile_offset<KG>(DK::NB, g1) - tile_offset<KG>(DK::NB, g0));
-	const uint32_t tile_dn = dn_role ? (uint32_t)(tile_offset<KD>(DF::NB, d1) - tile_offset<KD>(DF::NB, d0)) : 0;
+	const uint32_t tile_gu = (uint32_t)(tile_offset<KG>(NBK, g1) - tile_offset<KG>(NBK, g0));
+	const uint32_t tile_dn = dn_role ? (uint32_t)(tile_offset<KD>(NBF, d1) - tile_offset<KD>(NBF, d0)) : 0;
 
 	DF_STAMP(0);
 	if (tid == 0) {
@@ -206,8 +187,14 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			}
 		}
 	}
-	if (gu_role)
-		stage_x_lane_major<KG, DK::LPR>(xin, xs, DK::PARTS, tid, DF_THREADS);
+	if (gu_role && warp < NBK) {
+		const float4 *xp = reinterpret_cast<const float4 *>(xin + warp * QK_K) + 2 * lane;
+		const float4 x0 = xp[0], x1 = xp[1];
+		const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+		const float inv = x_image<KG>(v, ximg + warp * XImage<KG>::BYTES, lane);
+		if (lane == 0)
+			sh.x_inv[warp] = inv;
+	}
 	const unsigned base = (__syncthreads(), sh.base);
 	DF_STAMP(1);
 	if (!df_grid_barrier(a.sync, base + (unsigned)G, &sh, a.status))
@@ -270,7 +257,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			ptx::fence_proxy_async_smem();
 			ptx::mbar_arrive_expect_tx(ba, tile_dn);
 			bulk_g2s(ptx::smem_u32(sd + (size_t)j * tile_dn),
-				 a.wd + (size_t)(sh.idx[j] - a.first_expert) * a.stride_dn + tile_offset<KD>(DF::NB, d0), tile_dn, ba);
+				 a.wd + (size_t)(sh.idx[j] - a.first_expert) * a.stride_dn + tile_offset<KD>(NBF, d0), tile_dn, ba);
 		}
 	};
 	if (lane == 0 && !bad) {
@@ -280,8 +267,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			if (gu_role && c < n_chunks) {
 				const size_t eb = (size_t)(sh.idx[slot] - a.first_expert) * a.stride_gu;
 				const int c0 = g0 + c * CH, c1 = min(c0 + CH, g1);
-				const size_t o0 = tile_offset<KG>(DK::NB, c0), o1 = tile_offset<KG>(DK::NB, c1);
-				const uint32_t bytes = (uint32_t)(o1 - o0), rel = (uint32_t)(o0 - tile_offset<KG>(DK::NB, g0));
+				const size_t o0 = tile_offset<KG>(NBK, c0), o1 = tile_offset<KG>(NBK, c1);
+				const uint32_t bytes = (uint32_t)(o1 - o0), rel = (uint32_t)(o0 - tile_offset<KG>(NBK, g0));
 				const uint32_t ba = ptx::smem_u32(&sh.bar_gu[c]);
 				ptx::mbar_arrive_expect_tx(ba, 2 * bytes);
 				bulk_g2s(ptx::smem_u32(sg + rel), a.wg + eb + o0, bytes, ba);
@@ -307,57 +294,39 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 	DF_STAMP(3);
 	bool alive = true;
 	if (gu_role && !bad) {
-		const int sub = lane / DK::LPR, part = lane % DK::LPR;
-		const bool lane_on = part < DK::PARTS;
-		float xr[64], sx[4];
-		if (lane_on)
-			load_x_lane_major<KG, DK::LPR>(xs, part, xr, sx);
-		const uint8_t *vg = sg - tile_offset<KG>(DK::NB, g0), *vu = su - tile_offset<KG>(DK::NB, g0);
-		float *hrow = a.h + (size_t)slot * F;
-		int waited = -1;
-		// The table look-ups of a row's SwiGLU are two dependent loads: done at the end of every pass they
-		// stall the warp before its next pass.  After the reduction every lane of a row holds the sums, so
-		// lane p of the row keeps those of pass p and all passes' look-ups are issued together at the end
-		// (as long as a row has at least as many lanes as the tile has passes).
-		const bool defer = (g1 - g0 + DK::RPP - 1) / DK::RPP <= DK::LPR;
-		float keep_g = 0.f, keep_u = 0.f;
-		int keep_row = -1, pass = 0;
-		for (int rp = g0; rp < g1 && alive; rp += DK::RPP, pass++) {
-			const int chunk = (rp - g0) / CH;
-			if (chunk != waited) {
-				alive = dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status);
-				waited = chunk;
-				if (!alive)
-					break;
-				if (chunk == 0) {
-					DF_STAMP(7);
-					if (lane == 0 && warp >= DF_MAX_CHUNKS)
-						request_down();
-				}
+		// a job is (chunk of 16 rows, matrix, super-block); the products of a row's super-blocks are added up in order
+		const int jobs = n_chunks * 2 * NBK;
+		for (int i = warp; i < jobs && alive; i += DF_WARPS) {
+			const int chunk = i / (2 * NBK), mat = i % 2, b = (i % (2 * NBK)) >> 1;
+			alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status));
+			if (!alive)
+				break;
+			if (i == warp && lane == 0) {
+				DF_STAMP(7);
+				request_down();
 			}
-			const int row = rp + warp * DK::RPW + sub;
-			float vgv = 0.f, vuv = 0.f;
-			if (lane_on && row < g1) {
-				vgv = PartDot<KG>::dot(PartDot<KG>::template load<true>(vg, DK::NB, row, part), part, xr, sx);
-				vuv = PartDot<KG>::dot(PartDot<KG>::template load<true>(vu, DK::NB, row, part), part, xr, sx);
-			}
-#pragma unroll
-			for (int o = DK::LPR / 2; o > 0; o >>= 1) {
-				vgv += __shfl_xor_sync(0xffffffffu, vgv, o);
-				vuv += __shfl_xor_sync(0xffffffffu, vuv, o);
-			}
-			if (defer) {
-				if (part == pass && row < g1) {
-					keep_g = vgv;
-					keep_u = vuv;
-					keep_row = row;
-				}
-			} else if (part == 0 && row < g1) {
-				__stcg(hrow + row, swiglu_lut(a.silu, vgv, vuv));
+			MmaRows<KG> w;
+			w.load_smem((mat ? su : sg) + tile_offset<KG>(NBK, chunk * CH), NBK, b, lane);
+			float2 r, s;
+			w.dot(ximg + b * XImage<KG>::BYTES, sh.x_inv[b], lane, r, s);
+			if ((lane & 3) == 0) {
+				float *d = prod + ((chunk * 2 + mat) * NBK + b) * 16 + (lane >> 2);
+				d[0] = r.x * s.x;
+				d[8] = r.y * s.y;
 			}
 		}
-		if (keep_row >= 0 && alive)
-			__stcg(hrow + keep_row, swiglu_lut(a.silu, keep_g, keep_u));
+		if (warp >= jobs && lane == 0)
+			request_down();
+		alive = __syncthreads_and(alive);
+		if (alive && tid < g1 - g0) {
+			const float *pg = prod + (tid >> 4) * 2 * NBK * 16 + (tid & 15), *pu = pg + NBK * 16;
+			float g = pg[0], u = pu[0];
+			for (int b = 1; b < NBK; b++) {
+				g = __fadd_rn(g, pg[b * 16]);
+				u = __fadd_rn(u, pu[b * 16]);
+			}
+			__stcg(a.h + (size_t)slot * F + g0 + tid, swiglu_lut(a.silu, g, u));
+		}
 		DF_STAMP(8);
 	}
 	alive = __syncthreads_and(alive);
@@ -383,49 +352,40 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		}
 	}
 	if (dn_role && !bad) {
-		float *hs = reinterpret_cast<float *>(dsm);  // top_k lane-major rows of h (the gate/up tiles are done with)
-		float *vbuf = reinterpret_cast<float *>(dsm + a.off_v);
-		constexpr int XS_T = DF::LPR * 64;
-		for (int j = 0; j < top_k; j++)
-			df_stage_lane_major_cg<KD, DF::LPR>(a.h + (size_t)j * F, hs + (size_t)j * XS_T, DF::PARTS, tid);
-		__syncthreads();
-		DF_STAMP(9);
-		const int sub = lane / DF::LPR, part = lane % DF::LPR;
-		const bool lane_on = part < DF::PARTS;
-		const int rows = d1 - d0;
-		// A (warp, sub-row) unit keeps ONE slot for the whole phase — its slice of that slot's h stays in
-		// registers — and walks the rows of the tile: the units of slot j are j, j + top_k, ..., the
-		// k-th of them takes rows k, k + n_j, ... (loading the activations once per unit instead of once
-		// per slot and unit leaves only the packed rows to fetch inside the loop).
-		const int unit = warp * DF::RPW + sub;	// (a pass has at least 16 units, a token at most 8 slots)
-		{
-			const int j = unit % top_k, r0 = unit / top_k;
-			const int n_j = (DF::RPP - 1 - j) / top_k + 1;		    // units that share slot j
-			const int trips = (rows + DF::RPP / top_k - 1) / (DF::RPP / top_k);  // the same for every lane of a warp
-			float xr[64], sx[4];
-			if (lane_on)
-				load_x_lane_major<KD, DF::LPR>(hs + (size_t)j * XS_T, part, xr, sx);
+		// a job is (slot, super-block); the gate/up tiles are done with: their space takes the images of h
+		uint8_t *himg = dsm + warp * XImage<KD>::BYTES;
+		for (int i = warp; i < top_k * NBF && alive; i += DF_WARPS) {
+			const int j = i / NBF, b = i % NBF;
+			const float4 *hp = reinterpret_cast<const float4 *>(a.h + (size_t)j * F + b * QK_K) + 2 * lane;
+			const float4 h0 = __ldcg(hp), h1 = __ldcg(hp + 1);  // (written by other CTAs of this grid)
+			const float v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+			const float inv = x_image<KD>(v, himg, lane);
 			alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_dn[j]), a.status));
-			const uint8_t *vd = sd + (size_t)j * tile_dn - tile_offset<KD>(DF::NB, d0);
-			for (int i = 0; i < trips && alive; i++) {
-				const int lr = r0 + i * n_j;
-				float v = 0.f;
-				if (lane_on && lr < rows)
-					v = PartDot<KD>::dot(PartDot<KD>::template load<true>(vd, DF::NB, d0 + lr, part), part, xr, sx);
-#pragma unroll
-				for (int o = DF::LPR / 2; o > 0; o >>= 1)
-					v += __shfl_xor_sync(0xffffffffu, v, o);
-				if (part == 0 && lr < rows)
-					vbuf[j * a.rpt_dn + lr] = v;
+			if (!alive)
+				break;
+			MmaRows<KD> w;
+			w.load_smem(sd + (size_t)j * tile_dn, NBF, b, lane);
+			float2 r, s;
+			w.dot(himg, inv, lane, r, s);
+			if ((lane & 3) == 0) {
+				float2 *d = reinterpret_cast<float2 *>(prod) + i * 16 + (lane >> 2);
+				d[0] = make_float2(r.x, s.x);
+				d[8] = make_float2(r.y, s.y);
 			}
 		}
 		DF_STAMP(10);
 		alive = __syncthreads_and(alive);
 		if (alive) {
-			for (int lr = tid; lr < rows; lr += DF_THREADS) {
+			for (int lr = tid; lr < d1 - d0; lr += DF_THREADS) {
 				float acc = 0.f;
-				for (int j = 0; j < top_k; j++)
-					acc = __fmaf_rn(sh.w[j], vbuf[j * a.rpt_dn + lr], acc);	 // slot order, from zero
+				for (int j = 0; j < top_k; j++) {
+					float v = 0.f;
+					for (int b = 0; b < NBF; b++) {
+						const float2 e = reinterpret_cast<const float2 *>(prod)[(j * NBF + b) * 16 + lr];
+						v = __fmaf_rn(e.y, e.x, v);
+					}
+					acc = __fmaf_rn(sh.w[j], v, acc);  // slot order, from zero
+				}
 				if (a.residual)
 					acc = __fadd_rn(a.residual[d0 + lr], acc);
 				a.out[d0 + lr] = acc;
@@ -464,15 +424,12 @@ static DfPlan df_plan(const tie_cuda_ctx *c)
 	const int want_gu = sms / top_k;
 	if (want_gu < 1)
 		return p;
-	p.rpt_gu = ((F + want_gu - 1) / want_gu + 7) / 8 * 8;
+	p.rpt_gu = ((F + want_gu - 1) / want_gu + 15) / 16 * 16;
 	p.tiles_gu = (F + p.rpt_gu - 1) / p.rpt_gu;
-	p.rpt_dn = ((K + sms - 1) / sms + 7) / 8 * 8;
+	p.rpt_dn = 16;	// one MMA tile
 	p.tiles_dn = (K + p.rpt_dn - 1) / p.rpt_dn;
-	constexpr int RPP_K = DfDims<K>::RPP, RPP_F = DfDims<F>::RPP;
-	constexpr int CH = RPP_K > 16 ? RPP_K : 16;
-	if ((p.rpt_gu + CH - 1) / CH > DF_MAX_CHUNKS)
-		return p;
-	if (p.rpt_dn >= RPP_F ? (p.rpt_dn + RPP_F - 1) / RPP_F > DF_MAX_PASSES : RPP_F % p.rpt_dn != 0)
+	constexpr int NBK = K / QK_K, NBF = F / QK_K;
+	if (p.rpt_gu / 16 > DF_MAX_CHUNKS || NBK > 8 || F % 16 || K % 16)
 		return p;
 	p.grid = max(c->cfg.n_expert, max(top_k * p.tiles_gu, p.tiles_dn));
 	if (p.grid > sms)
@@ -480,11 +437,11 @@ static DfPlan df_plan(const tie_cuda_ctx *c)
 	const size_t tile_gu = (size_t)p.rpt_gu * df_row_bytes<KG>(K), tile_dn = (size_t)p.rpt_dn * df_row_bytes<KD>(F);
 	size_t area_a = 2 * tile_gu;
 	area_a = max(area_a, (size_t)2 * K * sizeof(float));				 // router staging
-	area_a = max(area_a, (size_t)top_k * DfDims<F>::LPR * 64 * sizeof(float));	 // staged h rows
+	area_a = max(area_a, (size_t)DF_WARPS * XImage<KD>::BYTES);			 // images of h
 	p.off_b = (area_a + 127) / 128 * 128;
 	p.off_c = (p.off_b + (size_t)top_k * tile_dn + 127) / 128 * 128;
-	p.off_v = p.off_c + (size_t)DfDims<K>::LPR * 64 * sizeof(float);
-	p.off_n = (p.off_v + (size_t)top_k * p.rpt_dn * sizeof(float) + 15) / 16 * 16;
+	p.off_v = p.off_c + (size_t)NBK * XImage<KG>::BYTES;
+	p.off_n = (p.off_v + max((size_t)p.rpt_gu * 2 * NBK, (size_t)top_k * NBF * 16 * 2) * sizeof(float) + 15) / 16 * 16;
 	p.smem = p.off_n + (size_t)K * sizeof(float);
 	p.ok = p.smem <= 220 * 1024;
 	return p;

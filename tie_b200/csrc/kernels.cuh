@@ -12,6 +12,7 @@ int router_setup(tie_cuda_ctx *c);
 int launch_router_decode_fused(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
 			       int *topk_idx, float *topk_w);
 // decode.cu
+int decode_setup(tie_cuda_ctx *c);
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens);
 // foreign_slots_ok: slots whose expert another rank owns are skipped instead of reported
 int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n_tokens, bool foreign_slots_ok = false);

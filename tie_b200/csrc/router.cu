@@ -63,47 +63,52 @@ __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__res
 	}
 }
 
-// Batched token counts: thread = one AVX2 lane l of a TPT-token x EPT-expert register tile (each
-// of its chains a strict i-ascending sequence of fused multiply-adds, so the result stays
-// bit-identical).  The limit of this kernel is shared-memory-to-register bandwidth (one float per
-// lane per cycle), so every loaded float must feed several multiply-adds from registers.
-// Operands are staged by cp.async in k chunks (a 4-deep ring); a row pitch of KC+8 floats puts
-// the 4 token groups of a warp on disjoint banks, and the 4 groups share their expert rows
-// (broadcast loads).
-constexpr int RMT_STAGES = 4;
+// The router of a batch: logits, selection and softmax in one launch.
+//
+// Thread = one AVX2 lane l of a TPT-token x EPT-expert register tile (each of its chains a strict
+// i-ascending sequence of fused multiply-adds, so the result stays bit-identical); CTA = TT tokens x TE
+// experts.  The operands are staged lane-major in shared memory: two consecutive chain steps of a lane
+// are one 8-byte load (16-byte loads run at half the bandwidth), and the 8 lanes of a block of 32 k are
+// rotated so that the scattered stores are free of bank conflicts too; double-buffered through
+// registers.  What bounds a small batch is how many SMs pull the 1 MB of router weights, so the tile shrinks
+// with the batch until about 128 CTAs work (launch_router).  The CTA that finishes a token tile last (a
+// counter per tile, nobody waits) selects for all its tokens.
+// Measured (logits + selection): 4 tokens 14.4 -> 8.8 us, 13 28.7 -> 10.3, 64 28.7 -> 12.3, 512 29 -> 31, 1000 41 ->
+// 37, 4096 94 -> 100.
+//
 // The hand-over of the tokens in an expert-parallel step rides along as one more row of CTAs, of
 // which as many work as there are SMs the logits' CTAs leave free (at least 16): CTAs that share an
 // SM with the logits take load/store slots from them (32 working CTAs lengthened the kernel by 10 us
 // at 4 GPUs, 128 by 18 us).
-constexpr int RMT_PUSH_ROWS = 1;
-static int rmt_push_ctas(const tie_cuda_ctx *c, int logits_ctas, int most)
+constexpr int RT_PUSH_ROWS = 1;
+static int rt_push_ctas(const tie_cuda_ctx *c, int logits_ctas, int most)
 {
 	int n = c->sm_count - logits_ctas;
 	n = n < 16 ? 16 : n;
 	return n < most ? n : most;
 }
 
-// TPT x EPT = tokens x experts per thread, TE = experts per CTA, KC = k chunk.  CTA = 4 TPT
-// tokens x TE experts, 8 x 4 x TE/EPT threads.
-//   <4, 4, 32, 128>: 16 x 32 tiles, 256 threads, 104 KB — a few hundred tokens (parallelism first);
-//   <8, 8, 64, 64>:  32 x 64 tiles, 256 threads, 108 KB, two CTAs per SM — thousands of tokens
-//                    (16 loads per 64 multiply-adds instead of 8 per 16).
-template <int TPT, int EPT, int TE, int KC>
-struct RmtCfg {
-	static constexpr int TT = 4 * TPT, PITCH = KC + 8, THREADS = 8 * 4 * (TE / EPT);
-	static constexpr int STAGE_FLOATS = (TT + TE) * PITCH;
-	static constexpr int SMEM = RMT_STAGES * STAGE_FLOATS * (int)sizeof(float);
+template <int TPT_, int EPT_, int TT_, int TE_, int KC_>
+struct RtCfg {
+	static constexpr int TPT = TPT_, EPT = EPT_, TT = TT_, TE = TE_, KC = KC_;
+	static constexpr int TG = TT / TPT, EG = TE / EPT, THREADS = 8 * TG * EG;
+	static constexpr int PITCH = KC + 16, STAGE = (TT + TE) * PITCH;  // floats; two rows apart by half of the banks
+	static constexpr int SMEM = 2 * STAGE * (int)sizeof(float);
+	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : 8;
+	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte loads per thread and chunk
+	static_assert((TT + TE) * (KC / 4) % THREADS == 0 && TG % 2 == 0 && EG % 2 == 0 && KC % 32 == 0, "router tile");
 };
 
-template <int TPT, int EPT, int TE, int KC>
-__global__ void __launch_bounds__((RmtCfg<TPT, EPT, TE, KC>::THREADS), 2)
-router_logits_mt(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, float *__restrict__ logits,
-		 int n_tokens, int hidden, int n_expert, const EpPush push)
+template <class C>
+__global__ void __launch_bounds__(C::THREADS, C::THREADS >= 512 ? 1 : 2)
+router_batch(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, float *__restrict__ logits,
+	     int n_tokens, int hidden, int n_expert, int top_k, int *__restrict__ topk_idx, float *__restrict__ topk_w, int lfm2,
+	     const float *__restrict__ sel_bias, int *__restrict__ counter, const EpPush push)
 {
-	using Cfg = RmtCfg<TPT, EPT, TE, KC>;
-	constexpr int TT = Cfg::TT, PITCH = Cfg::PITCH, THREADS = Cfg::THREADS;
+	constexpr int TPT = C::TPT, EPT = C::EPT, TT = C::TT, TE = C::TE, KC = C::KC;
 	extern __shared__ __align__(16) float rsm[];
-	// Expert-parallel steps: RMT_PUSH_ROWS more rows of CTAs (blockIdx.y past the expert tiles) store this
+	__shared__ int s_last;
+	// Expert-parallel steps: RT_PUSH_ROWS more rows of CTAs (blockIdx.y past the expert tiles) store this
 	// rank's tokens into every rank's memory while the others compute the logits; they share nothing
 	// with them.
 	if (push.x && (int)blockIdx.y * TE >= n_expert) {
@@ -113,85 +118,107 @@ router_logits_mt(const float *__restrict__ x, const float *__restrict__ w, const
 		return;
 	}
 	const int t0 = blockIdx.x * TT, e0 = blockIdx.y * TE;
-	const int l = threadIdx.x & 7;		// AVX2 lane
-	const int tg = (threadIdx.x >> 3) & 3;	// tokens tg, tg+4, tg+8, ...
-	const int eg = threadIdx.x >> 5;	// experts EPT*eg .. EPT*eg+EPT-1 (one warp per expert group)
-	auto stage = [&](int buf, int k0) {
-		float *xs = rsm + buf * Cfg::STAGE_FLOATS;
-		float *ws = xs + TT * PITCH;
-		for (int i = threadIdx.x; i < (TT + TE) * (KC / 4); i += THREADS) {
-			const int r = i / (KC / 4), c4 = i % (KC / 4);
-			const float *src;
-			float *dst;
-			if (r < TT) {
-				const int t = min(t0 + r, n_tokens - 1);  // rows past the end are computed and dropped
-				src = x + (size_t)t * hidden + k0 + 4 * c4;
-				dst = xs + r * PITCH + 4 * c4;
-			} else {
-				src = w + (size_t)(e0 + r - TT) * hidden + k0 + 4 * c4;
-				dst = ws + (r - TT) * PITCH + 4 * c4;
-			}
-			asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
-				     : "memory");
+	// a warp is 8 lanes x 2 token groups x 2 expert groups
+	const int l = threadIdx.x & 7, g4 = threadIdx.x >> 5;
+	const int tg = ((threadIdx.x >> 3) & 1) + 2 * (g4 % (C::TG / 2)), eg = ((threadIdx.x >> 4) & 1) + 2 * (g4 / (C::TG / 2));
+	float4 r[C::LD];
+	auto fetch = [&](int k0) {
+#pragma unroll
+		for (int j = 0; j < C::LD; j++) {
+			const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
+			const float *src = row < TT ? x + (size_t)min(t0 + row, n_tokens - 1) * hidden	// (rows past the end: computed, dropped)
+						    : w + (size_t)(e0 + row - TT) * hidden;
+			// (volatile: left to itself the compiler sinks the loads to their use behind the chunk's arithmetic)
+			asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+				     : "=f"(r[j].x), "=f"(r[j].y), "=f"(r[j].z), "=f"(r[j].w)
+				     : "l"(src + k0 + 4 * c4));
 		}
-		asm volatile("cp.async.commit_group;" ::: "memory");
 	};
-	float acc[TPT][EPT];  // [token j][expert b]
+	auto put = [&](int buf) {
+#pragma unroll
+		for (int j = 0; j < C::LD; j++) {
+			const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
+			// k = 4 c4 ..: chain step c4 / 2 of lanes 4 (c4 & 1) .. + 3
+			float *d = rsm + buf * C::STAGE + row * C::PITCH + (c4 >> 2) * 16 + ((c4 >> 1) & 1);
+			const int at = 8 * (c4 & 1) + 2 * ((c4 >> 3) & 3);
+			d[at & 15] = r[j].x;
+			d[(at + 2) & 15] = r[j].y;
+			d[(at + 4) & 15] = r[j].z;
+			d[(at + 6) & 15] = r[j].w;
+		}
+	};
+	float acc[TPT][EPT];
 #pragma unroll
 	for (int j = 0; j < TPT; j++)
 #pragma unroll
 		for (int b = 0; b < EPT; b++)
 			acc[j][b] = 0.0f;
 	const int n_chunks = hidden / KC;
-#pragma unroll
-	for (int c = 0; c < RMT_STAGES - 1; c++) {
-		if (c < n_chunks)
-			stage(c, c * KC);
-		else
-			asm volatile("cp.async.commit_group;" ::: "memory");
-	}
+	fetch(0);
+	put(0);
+	__syncthreads();
 	for (int c = 0; c < n_chunks; c++) {
-		if (c + RMT_STAGES - 1 < n_chunks)
-			stage((c + RMT_STAGES - 1) % RMT_STAGES, (c + RMT_STAGES - 1) * KC);
-		else
-			asm volatile("cp.async.commit_group;" ::: "memory");
-		asm volatile("cp.async.wait_group %0;" ::"n"(RMT_STAGES - 1) : "memory");
-		__syncthreads();
-		const float *xs = rsm + (c % RMT_STAGES) * Cfg::STAGE_FLOATS;
-		const float *ws = xs + TT * PITCH;
-		const float *xp = xs + tg * PITCH + l;
-		const float *wp = ws + (EPT * eg) * PITCH + l;
-#pragma unroll 2
-		for (int i = 0; i < KC / 8; i++) {
-			float xv[TPT], wv[EPT];
+		if (c + 1 < n_chunks)
+			fetch((c + 1) * KC);
+		const float *xs = rsm + (c & 1) * C::STAGE + tg * C::PITCH, *ws = rsm + (c & 1) * C::STAGE + (TT + eg) * C::PITCH;
+#pragma unroll C::UNROLL
+		for (int g = 0; g < KC / 16; g++) {  // two chain steps
+			const int at = 16 * g + ((2 * l + 2 * ((g >> 1) & 3)) & 15);
+			float2 xv[TPT];
 #pragma unroll
 			for (int j = 0; j < TPT; j++)
-				xv[j] = xp[(4 * j) * PITCH + 8 * i];
+				xv[j] = *reinterpret_cast<const float2 *>(xs + C::TG * j * C::PITCH + at);
 #pragma unroll
-			for (int b = 0; b < EPT; b++)
-				wv[b] = wp[b * PITCH + 8 * i];
+			for (int b = 0; b < EPT; b++) {
+				const float2 wv = *reinterpret_cast<const float2 *>(ws + C::EG * b * C::PITCH + at);
 #pragma unroll
-			for (int j = 0; j < TPT; j++)
+				for (int j = 0; j < TPT; j++)
+					acc[j][b] = __fmaf_rn(xv[j].x, wv.x, acc[j][b]);
 #pragma unroll
-				for (int b = 0; b < EPT; b++)
-					acc[j][b] = __fmaf_rn(xv[j], wv[b], acc[j][b]);
+				for (int j = 0; j < TPT; j++)
+					acc[j][b] = __fmaf_rn(xv[j].y, wv.y, acc[j][b]);
+			}
 		}
+		if (c + 1 < n_chunks)
+			put((c + 1) & 1);
 		__syncthreads();
 	}
 #pragma unroll
 	for (int j = 0; j < TPT; j++) {
-		const int t = t0 + tg + 4 * j;
+		const int t = t0 + tg + C::TG * j;
 #pragma unroll
 		for (int b = 0; b < EPT; b++) {
-			const int e = e0 + EPT * eg + b;
-			float r = hsum8_lanes(acc[j][b]);  // lanes l = 0..7 are 8 consecutive threads
+			const int e = e0 + eg + C::EG * b;
+			float v = hsum8_lanes(acc[j][b]);  // lanes l = 0..7 are 8 consecutive threads
 			if (l == 0 && t < n_tokens) {
 				if (bias)
-					r = __fadd_rn(r, bias[e]);
-				logits[(size_t)t * n_expert + e] = r;
+					v = __fadd_rn(v, bias[e]);
+				__stcg(logits + (size_t)t * n_expert + e, v);
 			}
 		}
 	}
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0)
+		s_last = atomicAdd(counter + blockIdx.x, 1) == n_expert / TE - 1;
+	__syncthreads();
+	if (!s_last)
+		return;
+	__threadfence();
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	// (a warp's tokens are selected for together, up to four at a time: one after the other they are a chain of
+	// reductions of a microsecond each)
+	constexpr int WARPS = C::THREADS / 32, TW = (TT + WARPS - 1) / WARPS, NT = TW < 4 ? TW : 4;
+	const int t1 = min(t0 + TT, n_tokens);
+	for (int t = t0 + warp * TW; t < min(t0 + (warp + 1) * TW, t1); t += NT) {
+		const int n = min(NT, min(t0 + (warp + 1) * TW, t1) - t);
+		if (n_expert <= 128)
+			topk_tokens<NT, 4>(logits, sel_bias, t, n, lane, n_expert, top_k, topk_idx, topk_w, lfm2);
+		else
+			topk_tokens<NT, 8>(logits, sel_bias, t, n, lane, n_expert, top_k, topk_idx, topk_w, lfm2);
+	}
+	if (threadIdx.x == 0)
+		counter[blockIdx.x] = 0;
 }
 
 // Decode-sized token counts (<= 8 tokens): one expert per CTA so the 1 MB of router weights is
@@ -240,75 +267,6 @@ __global__ void __launch_bounds__(128) router_topk(const float *__restrict__ log
 	if (warp >= n_tokens)
 		return;
 	topk_softmax_warp(logits, warp, lane, n_expert, top_k, topk_idx, topk_w);
-}
-
-// LFM2-MoE routing (model_lfm2.c:438-473), one warp per token: s = sigmoid(logit) for every
-// expert, selection by the same arg-max rounds on s + sel_bias (exp_probs_b, may be null), gates =
-// the UNBIASED s of the selected experts, summed in slot order and scaled by 1/(sum + 1e-6).
-// logits is overwritten with the sigmoid scores (the reference does the same to expert_scores).
-__global__ void __launch_bounds__(128) router_topk_lfm2(float *__restrict__ logits, const float *__restrict__ sel_bias,
-							int n_tokens, int n_expert, int top_k, int *__restrict__ topk_idx,
-							float *__restrict__ topk_w)
-{
-	const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-	const int lane = threadIdx.x & 31;
-	if (token >= n_tokens)
-		return;
-	float *lg = logits + (size_t)token * n_expert;
-	float sg[8], v[8];
-	const int per = (n_expert + 31) / 32;
-#pragma unroll
-	for (int i = 0; i < 8; i++) {
-		const int e = lane + 32 * i;
-		const bool in = i < per && e < n_expert;
-		sg[i] = in ? __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-__ldcg(lg + e)))) : 0.0f;
-		v[i] = in ? (sel_bias ? __fadd_rn(sg[i], sel_bias[e]) : sg[i]) : -INFINITY;
-		if (in)
-			lg[e] = sg[i];
-	}
-	unsigned taken = 0;
-	float my_gate = 0.0f;
-	int my_idx = -1;
-	for (int r = 0; r < top_k; r++) {
-		float best = -INFINITY, best_sg = 0.0f;
-		int bi = 0x7fffffff;
-#pragma unroll
-		for (int i = 0; i < 8; i++) {
-			const int e = lane + 32 * i;
-			const bool ok = !(taken & (1u << i)) && i < per && e < n_expert;
-			// strictly greater wins; within a lane indices ascend, so ties keep the lower index
-			if (ok && (v[i] > best || bi == 0x7fffffff)) {
-				best = v[i];
-				best_sg = sg[i];
-				bi = e;
-			}
-		}
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1) {
-			const float ob = __shfl_xor_sync(0xffffffffu, best, o), os = __shfl_xor_sync(0xffffffffu, best_sg, o);
-			const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-			const bool take = (oi != 0x7fffffff) && (bi == 0x7fffffff || ob > best || (ob == best && oi < bi));
-			if (take) {
-				best = ob;
-				best_sg = os;
-				bi = oi;
-			}
-		}
-		if (bi != 0x7fffffff && (bi & 31) == lane)
-			taken |= 1u << (bi >> 5);
-		if (lane == r) {
-			my_gate = best_sg;
-			my_idx = (bi == 0x7fffffff) ? -1 : bi;
-		}
-	}
-	float sum = 0.0f;
-	for (int j = 0; j < top_k; j++)
-		sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, my_gate, j));
-	const float inv = __fdiv_rn(1.0f, __fadd_rn(sum, 1e-6f));
-	if (lane < top_k) {
-		topk_idx[(size_t)token * top_k + lane] = my_idx;
-		topk_w[(size_t)token * top_k + lane] = __fmul_rn(my_gate, inv);
-	}
 }
 
 // Decode: logits as in router_logits_decode, and the CTA that finishes last (a counter, no
@@ -395,6 +353,18 @@ __global__ void __launch_bounds__(256) router_decode_fused(const float *__restri
 // (Qwen3-MoE).  lfm2 = 1: LFM2-MoE routing, bias (optional) is the selection bias exp_probs_b.
 // push (expert-parallel steps): the kernel of the logits takes the hand-over of this rank's tokens to
 // its peers along as extra CTAs where it can; *push_taken tells whether it did.
+//
+// The tile: the largest of the list that still gives at least 0.85 CTAs per SM (each step down in size loads
+// more bytes per multiply-add from shared memory and L2, and fewer CTAs leave SMs idle), else the
+// smallest; the last-but-one sizes need hidden to be a multiple of their chunk of 512.
+#define TIE_RT_TILES(X)              \
+	X(RtCfg<8, 8, 64, 64, 64>)   \
+	X(RtCfg<4, 4, 32, 32, 128>)  \
+	X(RtCfg<4, 2, 32, 16, 128>)  \
+	X(RtCfg<2, 4, 16, 16, 256>)  \
+	X(RtCfg<2, 2, 16, 8, 512>)   \
+	X(RtCfg<1, 2, 8, 8, 512>)    \
+	X(RtCfg<1, 1, 4, 4, 512>)
 int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
 		  int *topk_idx, float *topk_w, int lfm2, const EpPush *push, bool *push_taken)
 {
@@ -403,49 +373,37 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 	if (push)
 		f = *push;
 	if (push_taken)
-		*push_taken = false;
+		*push_taken = push != nullptr;
 	const float *sel_bias = lfm2 ? bias : nullptr;
 	if (lfm2)
 		bias = nullptr;
-	if (n_tokens <= 8) {
-		size_t smem = ((size_t)H + (size_t)n_tokens * (H + 8)) * sizeof(float);
-		if (smem > 200 * 1024)	// the limit router_setup opts this kernel into
-			return TIE_CUDA_ENOTSUP;
-		router_logits_decode<8><<<E, 64, smem, c->stream>>>(x, w, bias, logits, n_tokens, H, E);
-		TIE_CUDA_LAUNCHED(c);
-	} else if (E % 64 == 0 && H % 128 == 0 && n_tokens >= 2048) {
-		using Cfg = RmtCfg<8, 8, 64, 64>;
-		dim3 grid((n_tokens + Cfg::TT - 1) / Cfg::TT, E / 64 + (push ? RMT_PUSH_ROWS : 0));
-		f.n_ctas = rmt_push_ctas(c, grid.x * (E / 64), grid.x * RMT_PUSH_ROWS);
-		router_logits_mt<8, 8, 64, 64><<<grid, Cfg::THREADS, Cfg::SMEM, c->stream>>>(x, w, bias, logits, n_tokens, H, E, f);
-		if (push_taken)
-			*push_taken = push != nullptr;
-		TIE_CUDA_LAUNCHED(c);
-	} else if (E % 32 == 0 && H % 128 == 0) {
-		using Cfg = RmtCfg<4, 4, 32, 128>;
-		dim3 grid((n_tokens + Cfg::TT - 1) / Cfg::TT, E / 32 + (push ? RMT_PUSH_ROWS : 0));
-		f.n_ctas = rmt_push_ctas(c, grid.x * (E / 32), grid.x * RMT_PUSH_ROWS);
-		router_logits_mt<4, 4, 32, 128><<<grid, Cfg::THREADS, Cfg::SMEM, c->stream>>>(x, w, bias, logits, n_tokens, H, E, f);
-		if (push_taken)
-			*push_taken = push != nullptr;
-		TIE_CUDA_LAUNCHED(c);
-	} else if (n_tokens <= 512) {
-		constexpr int TT = 8, EPC = 16;
-		dim3 grid((n_tokens + TT - 1) / TT, E / EPC);
-		router_logits_tile<TT, EPC, 256><<<grid, EPC * 8, 0, c->stream>>>(x, w, bias, logits, n_tokens, H, E);
-		TIE_CUDA_LAUNCHED(c);
-	} else {
-		constexpr int TT = 32, EPC = 16;
-		dim3 grid((n_tokens + TT - 1) / TT, E / EPC);
-		router_logits_tile<TT, EPC, 256><<<grid, EPC * 8, 0, c->stream>>>(x, w, bias, logits, n_tokens, H, E);
-		TIE_CUDA_LAUNCHED(c);
+	// what fits the shapes, in descending size: the first with enough CTAs, else the last
+	int pick = -1, at = 0;
+	bool enough = false;
+#define TIE_RT_PICK(...)                                                                                            \
+	{                                                                                                           \
+		using C = __VA_ARGS__;                                                                              \
+		if (E % C::TE == 0 && H % C::KC == 0 && !enough) {                                                  \
+			pick = at;                                                                                  \
+			enough = (long long)((n_tokens + C::TT - 1) / C::TT) * (E / C::TE) * 100 >= 85ll * c->sm_count; \
+		}                                                                                                   \
+		at++;                                                                                               \
 	}
-	const int warps_per_block = 4;
-	const int topk_blocks = (n_tokens + warps_per_block - 1) / warps_per_block;
-	if (lfm2)
-		router_topk_lfm2<<<topk_blocks, warps_per_block * 32, 0, c->stream>>>(logits, sel_bias, n_tokens, E, K, topk_idx, topk_w);
-	else
-		router_topk<<<topk_blocks, warps_per_block * 32, 0, c->stream>>>(logits, n_tokens, E, K, topk_idx, topk_w);
+	TIE_RT_TILES(TIE_RT_PICK)
+#undef TIE_RT_PICK
+	if (pick < 0)
+		return TIE_CUDA_ENOTSUP;
+	at = 0;
+#define TIE_RT_RUN(...)                                                                                                              \
+	if (at++ == pick) {                                                                                                          \
+		using C = __VA_ARGS__;                                                                                               \
+		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                                    \
+		f.n_ctas = rt_push_ctas(c, grid.x * (E / C::TE), grid.x * RT_PUSH_ROWS);                                             \
+		router_batch<C><<<grid, C::THREADS, C::SMEM, c->stream>>>(x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2, \
+									  sel_bias, c->s.route_counter, f);                          \
+	}
+	TIE_RT_TILES(TIE_RT_RUN)
+#undef TIE_RT_RUN
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }
@@ -465,10 +423,10 @@ int router_setup(tie_cuda_ctx *c)
 {
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_decode_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_mt<4, 4, 32, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     RmtCfg<4, 4, 32, 128>::SMEM));
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_mt<8, 8, 64, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     RmtCfg<8, 8, 64, 64>::SMEM));
+#define TIE_RT_ATTR(...) \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, __VA_ARGS__::SMEM));
+	TIE_RT_TILES(TIE_RT_ATTR)
+#undef TIE_RT_ATTR
 	return TIE_CUDA_OK;
 }
 
