@@ -6,19 +6,24 @@
 // SM together).  Here one cooperative grid (one CTA per SM, all co-resident) walks the phases
 // with two grid-wide barriers:
 //
-//   R  CTA e < n_expert: logit e, the AVX2 lane order replayed (8 chains of sequential fused
-//      multiply-adds, hsum tree: bit-exact, as router_decode_fused); every CTA meanwhile stages
-//      x for its gate/up tile
+//   R  CTA e < n_expert: logit e by warp 0, the AVX2 lane order replayed (8 chains of sequential fused
+//      multiply-adds, hsum tree: bit-exact, as router_decode_fused); other warps meanwhile make the
+//      images of x (mma_dot.cuh) for its gate/up tile
 //   -- barrier --
-//      every CTA selects the experts itself from the 128 logits (one thread per expert counts
-//      the experts ahead of it: cheaper than a broadcast), then requests, all at once, its gate
-//      and up tiles AND the down tiles of all selected experts for its 16 output rows (bulk
-//      copies, ~190 KB in flight per SM, one issuing thread per copy group)
-//   G  CTA (slot, row tile): gate . x, up . x, table SwiGLU -> h (global, 24 KB)
+//      every CTA selects the experts itself from the logits (one warp, hardware max/min reductions:
+//      cheaper than a broadcast), then requests its gate and up tiles and, once those land, the down
+//      tiles of all selected experts for its 16 output rows (bulk copies, ~190 KB per SM, one issuing
+//      thread per copy group); the gate weights are computed while the tiles are on their way
+//   G  CTA (slot, row tile): a warp takes 16 rows x one super-block of gate or up; table SwiGLU -> h
 //   -- barrier --
-//   D  CTA (row tile): the down tiles are long there; slots are spread over the warp groups, the
-//      per-slot dot products meet in shared memory and are combined in slot order from zero,
+//   D  CTA (row tile): a warp takes one (slot, super-block); the products meet in shared memory and are
+//      added up per slot in super-block order, then over the slots from zero,
 //      acc = fma(w_j, v_j, acc) (model_qwen3.c:458-467), + residual
+//
+// Bound by latency: of 22.6 us per block in a stack, 4.7 are RMSNorm + router chains, 3 the two grid
+// barriers, 1.7 the selection, 2 the first tile's arrival, 4 gate/up, 3 down, 3.4 launch and tail (the
+// 25.5 MB themselves would take 3.9).  28.9 us with scalar reductions and the row and the router matrix
+// loaded one after the other.
 //
 // The barriers count arrivals in a device word that only grows (targets are relative to an epoch
 // the last CTA of every launch advances), so the launch arguments never change and the kernel
@@ -44,8 +49,7 @@ struct DfShared {
 	uint64_t bar_gu[DF_MAX_CHUNKS];
 	uint64_t bar_dn[MAX_TOP_K];
 	int idx[MAX_TOP_K];
-	float w[MAX_TOP_K], score[MAX_TOP_K];
-	float lg[256];	// the logits (n_expert <= 256)
+	float w[MAX_TOP_K];
 	unsigned base;
 	int ok;
 	int dn_req[MAX_TOP_K];	// the down tile of slot j has been requested
@@ -122,7 +126,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 	const uint32_t tile_dn = dn_role ? (uint32_t)(tile_offset<KD>(NBF, d1) - tile_offset<KD>(NBF, d0)) : 0;
 
 	DF_STAMP(0);
-	if (tid == 0) {
+	if (tid == DF_THREADS - 1) {  // (not in a warp that the norm or the router waits for)
 		for (int c = 0; c < DF_MAX_CHUNKS; c++)
 			ptx::mbar_init(ptx::smem_u32(&sh.bar_gu[c]), 1);
 		for (int j = 0; j < MAX_TOP_K; j++) {
@@ -133,17 +137,24 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		sh.base = df_ld_acquire(a.sync + 1);
 	}
 
+	// The row and the CTA's row of the router matrix are both on their way before anything is computed.
+	float *ws = reinterpret_cast<float *>(dsm), *xn = reinterpret_cast<float *>(dsm + a.off_n);
+	static_assert(K / 4 <= DF_THREADS, "one 16-byte load per thread");
+	if (tid < K / 4) {
+		const float4 xv = __ldcg(reinterpret_cast<const float4 *>(a.x) + tid);	// (the row is overwritten in place at the end)
+		float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
+		if (cta < a.n_expert)
+			wv = __ldg(reinterpret_cast<const float4 *>(a.router_w + (size_t)cta * K) + tid);
+		reinterpret_cast<float4 *>(xn)[tid] = xv;
+		reinterpret_cast<float4 *>(ws)[tid] = wv;
+	}
+	__syncthreads();
 	// ---------------- (RMSNorm of the row, every CTA for itself: rms_norm_f32_f32_f32_avx2, math_avx2.c:56-97) ----------------
-	const float *xin = a.x;
 	if (a.norm_eps >= 0.0f) {
-		float *xn = reinterpret_cast<float *>(dsm + a.off_n);
-		for (int i = tid; i < K / 4; i += DF_THREADS)
-			reinterpret_cast<float4 *>(xn)[i] = __ldcg(reinterpret_cast<const float4 *>(a.x) + i);  // (the row is overwritten in place at the end)
-		__syncthreads();
 		if (warp == 0) {
 			float acc = 0.0f;
 			if (lane < 8) {
-#pragma unroll 16
+#pragma unroll 32
 				for (int i = 0; i < K / 8; i++) {
 					const float v = xn[8 * i + lane];
 					acc = __fmaf_rn(v, v, acc);
@@ -158,42 +169,31 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		for (int i = tid; i < K; i += DF_THREADS)
 			xn[i] = __fmul_rn(__fmul_rn(xn[i], a.norm_w ? a.norm_w[i] : 1.0f), inv);
 		__syncthreads();
-		xin = xn;
 	}
 
-	// ---------------- R: one router logit per CTA ----------------
-	if (cta < a.n_expert) {
-		float *ws = reinterpret_cast<float *>(dsm), *xr = ws + K;
-		const float4 *w4 = reinterpret_cast<const float4 *>(a.router_w + (size_t)cta * K);
-		const float4 *x4 = reinterpret_cast<const float4 *>(xin);
-		for (int i = tid; i < K / 4; i += DF_THREADS) {
-			const float4 wv = __ldg(w4 + i), xv = x4[i];
-			reinterpret_cast<float4 *>(ws)[i] = wv;
-			reinterpret_cast<float4 *>(xr)[i] = xv;
+	// ---------------- R: one router logit per CTA (warp 0), the images of x beside it ----------------
+	if (warp == 0 && cta < a.n_expert) {
+		float acc = 0.0f;
+		if (lane < 8) {
+#pragma unroll 32
+			for (int i = 0; i < K / 8; i++)
+				acc = __fmaf_rn(xn[8 * i + lane], ws[8 * i + lane], acc);
 		}
-		__syncthreads();
-		if (warp == 0) {
-			float acc = 0.0f;
-			if (lane < 8) {
-#pragma unroll 16
-				for (int i = 0; i < K / 8; i++)
-					acc = __fmaf_rn(xr[8 * i + lane], ws[8 * i + lane], acc);
-			}
-			float r = hsum8_lanes(acc);
-			if (lane == 0) {
-				if (a.bias)
-					r = __fadd_rn(r, a.bias[cta]);
-				__stcg(a.logits + cta, r);
-			}
+		float r = hsum8_lanes(acc);
+		if (lane == 0) {
+			if (a.bias)
+				r = __fadd_rn(r, a.bias[cta]);
+			__stcg(a.logits + cta, r);
 		}
 	}
-	if (gu_role && warp < NBK) {
-		const float4 *xp = reinterpret_cast<const float4 *>(xin + warp * QK_K) + 2 * lane;
+	if (gu_role && warp >= 8 && warp < 8 + NBK) {
+		const int b = warp - 8;
+		const float4 *xp = reinterpret_cast<const float4 *>(xn + b * QK_K) + 2 * lane;
 		const float4 x0 = xp[0], x1 = xp[1];
 		const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-		const float inv = x_image<KG>(v, ximg + warp * XImage<KG>::BYTES, lane);
+		const float inv = x_image<KG>(v, ximg + b * XImage<KG>::BYTES, lane);
 		if (lane == 0)
-			sh.x_inv[warp] = inv;
+			sh.x_inv[b] = inv;
 	}
 	const unsigned base = (__syncthreads(), sh.base);
 	DF_STAMP(1);
@@ -202,34 +202,15 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 	DF_STAMP(2);
 
 	// ---------------- selection (every CTA for itself) and all weight requests ----------------
-	// find_top_k (engine.c:891-914) orders by (score descending, index ascending) — a total order, so
-	// the slot of an expert is the number of experts ahead of it: one thread per expert counts them.
-	if (tid < a.n_expert)
-		sh.lg[tid] = __ldcg(a.logits + tid);
-	__syncthreads();
-	if (tid < a.n_expert) {
-		const float v = sh.lg[tid];
-		int rank = 0;
-		for (int e = 0; e < a.n_expert; e++) {
-			const float o = sh.lg[e];
-			rank += (o > v || (o == v && e < tid)) ? 1 : 0;
-		}
-		if (rank < top_k) {
-			sh.idx[rank] = tid;
-			sh.score[rank] = v;
-		}
-	}
-	__syncthreads();
-	if (warp == 0) {  // softmax (engine.c:864-888) with the arithmetic of topk_softmax_warp
-		const float my_score = lane < top_k ? sh.score[lane] : 0.0f;
-		const float mx = __shfl_sync(0xffffffffu, my_score, 0);
-		const float ex = (lane < top_k) ? expf(__fsub_rn(my_score, mx)) : 0.0f;
-		float sum = 0.0f;
-		for (int j = 0; j < top_k; j++)
-			sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, ex, j));
-		const float inv = __fdiv_rn(1.0f, sum);
+	if (warp == 0) {
+		unsigned key[1][8];
+#pragma unroll
+		for (int i = 0; i < 8; i++)
+			key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
+		int mine[1];
+		topk_warp<1, 8>(key, lane, top_k, mine);
 		if (lane < top_k)
-			sh.w[lane] = __fmul_rn(ex, inv);
+			sh.idx[lane] = mine[0];
 	}
 	__syncthreads();
 	bool bad = false;
@@ -237,18 +218,13 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		const int le = sh.idx[j] - a.first_expert;
 		bad |= (le < 0 || le >= a.n_local);
 	}
-	if (cta == 0 && tid < top_k) {
-		a.topk_idx[tid] = sh.idx[tid];
-		a.topk_w[tid] = sh.w[tid];
-	}
 	if (bad && cta == 0 && tid == 0)
 		atomicOr(a.status, ST_BAD_EXPERT);
 	uint8_t *sg = dsm, *su = dsm + tile_gu, *sd = dsm + a.off_b;
 	// one issuing thread per copy group (issuing a bulk copy costs ~100 cycles): warp c < 8 the
-	// gate/up chunk c, warp 8 + j the down tile of slot j.  The down tiles are requested once the
-	// first gate/up chunk has landed: asked for together with the gate/up tiles they shared the HBM
-	// bandwidth with them and the first chunk arrived a microsecond later; they still have the whole
-	// gate/up phase to arrive in.
+	// gate/up chunk c, warp 8 + j the down tile of slot j.  The down tiles are requested when the warp's
+	// last gate/up chunk has landed: asked for earlier they share the HBM bandwidth with the gate/up
+	// tiles, and they still have a product, a grid barrier and the image of h to arrive in.
 	auto request_down = [&]() {  // lane 0 of warp 8 + j
 		const int j = warp - DF_MAX_CHUNKS;
 		if (dn_role && j >= 0 && j < top_k) {
@@ -278,6 +254,23 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			request_down();	 // (a CTA without gate/up rows: nothing to wait for)
 		}
 	}
+	if (warp == DF_WARPS - 1) {  // softmax (engine.c:864-888) with the arithmetic of topk_tokens, while the tiles are on their way
+		const int e = lane < top_k ? sh.idx[lane] : -1;
+		const float score = e >= 0 ? __ldcg(a.logits + e) : 0.0f;
+		const float mx = __shfl_sync(0xffffffffu, score, 0);
+		const float ex = (lane < top_k) ? expf(__fsub_rn(score, mx)) : 0.0f;
+		float sum = 0.0f;
+		for (int j = 0; j < top_k; j++)
+			sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, ex, j));
+		const float w = __fmul_rn(ex, __fdiv_rn(1.0f, sum));
+		if (lane < top_k) {
+			sh.w[lane] = w;
+			if (cta == 0) {
+				a.topk_idx[lane] = e;
+				a.topk_w[lane] = w;
+			}
+		}
+	}
 	// waits (bounded) for every copy this CTA requested: before it gives up, and harmless otherwise
 	auto drain = [&]() {
 		if (bad)
@@ -301,10 +294,10 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status));
 			if (!alive)
 				break;
-			if (i == warp && lane == 0) {
+			if (i == warp && lane == 0)
 				DF_STAMP(7);
+			if (i + DF_WARPS >= jobs && lane == 0)	// the warp's last
 				request_down();
-			}
 			MmaRows<KG> w;
 			w.load_smem((mat ? su : sg) + tile_offset<KG>(NBK, chunk * CH), NBK, b, lane);
 			float2 r, s;
