@@ -1573,14 +1573,10 @@ int tie_cuda_mat_mat(tie_cuda_ctx *c, const void *w_host, const float *x, float 
 		x_dev = s.x;
 		o_dev = s.y;
 	}
-	// one "expert" owning every row: the tile table of the grouped product, rows in input order
-	TIE_CUDA_TRY(c, cudaMemsetAsync(s.row_expert, 0, (size_t)batch_len * sizeof(int), c->stream));
-	SortBufs b = {s.counts, s.offsets, s.tile_start, s.active, s.n_active, s.perm, s.tile_info};
-	TRY(launch_sort(c, s.row_expert, batch_len, TC_TOKEN_TILE, 0, 1, b));
 	// the batch, split into fp16 hi + lo (and its sub-block sums for Q4_K), in the tensor's view of the x arrays
 	const bool sums = reg->dense->kind == W_Q4K;
 	TRY(launch_split_rows(c, x_dev, nullptr, 1, batch_len, in_dim, s.xs_hi, s.xs_hi + v.lo_off, sums ? s.xq : nullptr));
-	TRY(launch_tc_dense(c, *reg->dense, o_dev));
+	TRY(launch_tc_dense(c, *reg->dense, batch_len, o_dev));
 	if (!dev) {
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(o, o_dev, (size_t)batch_len * out_dim * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
 		return check_status(c);

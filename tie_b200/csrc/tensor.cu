@@ -178,18 +178,19 @@ constexpr int TC_ITEMS = 128;
 // m_items: work items per token tile (128-row tiles, or pairs of them); a CTA of a pair takes the
 // tile 2 * item + its rank.  Packed: expert, first row, rows, first weight row | matrix << 30.
 template <bool PAIR>
-__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int rows_per_matrix, uint32_t rank)
+__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int rows_per_matrix,
+					  uint32_t rank)
 {
 	const int slot = t / m_items, mi = t - slot * m_items;
-	const int4 ti = __ldg(tile_info + slot);
+	const int4 ti = tile_info ? __ldg(tile_info + slot) : make_int4(0, slot * TC_NT, min(TC_NT, n_rows - slot * TC_NT), 0);
 	const int m = (PAIR ? 2 * mi + (int)rank : mi) * TC_BM, sel = m >= rows_per_matrix ? 1 : 0;
 	return make_int4(ti.x, ti.y, ti.z, (m - sel * rows_per_matrix) | sel << 30);
 }
 template <bool PAIR>
 __device__ __forceinline__ TcItem tc_item(int t, int tl, const int4 *s_items, int m_items, const int4 *__restrict__ tile_info,
-					  int rows_per_matrix, uint32_t rank)
+					  int n_rows, int rows_per_matrix, uint32_t rank)
 {
-	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR>(t, m_items, tile_info, rows_per_matrix, rank);
+	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR>(t, m_items, tile_info, n_rows, rows_per_matrix, rank);
 	TcItem it;
 	it.le = ti.x;
 	it.row0 = ti.y;
@@ -321,11 +322,9 @@ struct Expander<W_Q6K_R8> {
 // Every role walks the same sequence of super-blocks, numbered through the work items of the CTA: n % 2
 // selects the accumulator buffer and the pair of ring slots.
 //
-// A launch covers the super-blocks [sb0, sb0 + k_dim / 256) of rows that hold nb_total of them
-// (k_dim is the launch's share of the input dimension); accumulate != 0 adds to what y already
-// holds.  The expert products pass (0, k / 256, 0); a dense Q4_K tensor with more than 2048 inputs
-// runs as several launches of at most 8 super-blocks (the min phase takes the sub-block sums of
-// one 64-wide tile).
+// The sub-block sums (Q4_K) come in segments of 8 super-blocks: the expert products have one per work item, a
+// dense tensor with more than 2048 inputs several.  tile_info null (dense tensors): no tables, the
+// token tiles are n_local rows cut in order.
 //
 // PEER (expert parallelism over peer memory, down product only): sorted row p belongs to row
 // dst.row[p] & 0xFFFFFF of rank dst.row[p] >> 24 and is stored there, into that rank's memory
@@ -339,7 +338,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		const uint8_t *__restrict__ w1, size_t expert_stride, int k_dim, const int4 *__restrict__ tile_info,
 		const int *__restrict__ tile_start, int n_local, int m_tiles, float *__restrict__ y, const int *__restrict__ perm,
 		int out_stride, float out_scale, unsigned *__restrict__ status, int rows_per_matrix, const EpDst dst,
-		const int sb0, const int nb_total, const int accumulate, const int xq_depth)
+		const int xq_depth)
 {
 	static_assert(!(RAW && PEER), "peer destinations exist for the down product only");
 	using Sm = TcSmem<KIND, PAIR>;
@@ -355,7 +354,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	const int stride_t = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 	const int m_items = PAIR ? m_tiles / 2 : m_tiles;
 	if (threadIdx.x == 0)
-		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : tile_start[n_local] * m_items;
+		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + TC_NT - 1) / TC_NT) * m_items;
 	__syncthreads();
 	// (a CTA of a pair never returns early: its peer would wait for it at the cluster barrier below)
 	const int total = s_total;
@@ -364,7 +363,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	if (threadIdx.x < TC_ITEMS) {
 		const int t = walker + threadIdx.x * stride_t;
 		if (t < total)
-			s_items[threadIdx.x] = tc_decode<PAIR>(t, m_items, tile_info, rows_per_matrix, rank);
+			s_items[threadIdx.x] = tc_decode<PAIR>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
 	}
 	const int nb = k_dim / QK_K;
 
@@ -513,7 +512,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		bool alive = true;
 		int dtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, dtl++) {
-			const TcItem item = tc_item<PAIR>(t, dtl, s_items, m_items, tile_info, rows_per_matrix, rank);
+			const TcItem item = tc_item<PAIR>(t, dtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 			const int mrow = item.m0 + lrow;
 			// tokens (accumulator columns) of this warp: half of the tile's range, 16 or 32
 			const bool wide = item.n_mma > 32;
@@ -558,14 +557,14 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			const uint8_t *grp = nullptr;
 			float dnext = 0.0f;
 			if (!Q4) {
-				grp = (item.mat_sel ? w1 : w0) + (size_t)item.le * expert_stride + (size_t)(mrow >> 3) * q6k_r8_group_bytes(nb_total);
-				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb_total, mrow & 7, sb0))));
+				grp = (item.mat_sel ? w1 : w0) + (size_t)item.le * expert_stride + (size_t)(mrow >> 3) * q6k_r8_group_bytes(nb);
+				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, 0))));
 			}
 			for (int sbi = 0; sbi < nb; sbi++, n++) {
 				float scale = dnext;
 				if (!Q4 && sbi + 1 < nb)
 					dnext = half_bits_to_float(
-						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb_total, mrow & 7, sb0 + sbi + 1))));
+						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
 				const uint32_t buf = n % TC_NBUF;
 				if (!tc_wait_warp(ptx::smem_u32(&sh->pfull[buf]), (n / TC_NBUF) & 1u, abort_flag, status, lane)) {
 					alive = false;
@@ -600,8 +599,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					} else if (PEER) {
 						dst.y[(unsigned)rj >> 24][(size_t)(rj & 0xFFFFFF) * out_stride + mrow] = acc[j] * out_scale;
 					} else {
-						float *yp = yr + (size_t)rj * out_stride;
-						*yp = accumulate ? __fadd_rn(*yp, acc[j] * out_scale) : acc[j] * out_scale;
+						yr[(size_t)rj * out_stride] = acc[j] * out_scale;
 					}
 				}
 				if (RAW)
@@ -627,13 +625,13 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				else
 					ptx::mma_commit(ptx::smem_u32(bar));
 			};
-			uint32_t n = 0, tl = 0;	 // super-blocks, work items so far
+			uint32_t n = 0, tl = 0, xs_n = 0;  // super-blocks, work items, segments of sums so far
 			bool alive = true;
 			auto wait = [&](uint64_t *bar, uint32_t parity) {
 				alive = alive && tc_wait(ptx::smem_u32(bar), parity, abort_flag, status);
 			};
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 				const uint32_t idesc = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, item.n_mma);
 				const uint32_t lo_off = (uint32_t)((PAIR ? 8 : 16) << item.box) * 128u;
 				for (int sbi = 0; sbi < nb && alive; sbi++, n++) {
@@ -655,7 +653,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					}
 					ptx::tc_fence_after();
 					const uint32_t dP = tmem + TC_COL_P + TC_NT * buf, bt = b_group(q);
-					const uint32_t xs = ptx::umma_desc_lo(xq_buf(tl & 1u) + (uint32_t)(sbi >> 2) * lo_off) + 2u * (sbi & 3);
+					const uint32_t xs = ptx::umma_desc_lo(xq_buf(xs_n & 1u) + (uint32_t)((sbi >> 2) & 1) * lo_off) + 2u * (sbi & 3);
 					// (dmin m)_hi (half 0), (dmin m)_lo (half 1) times the block's sums, hi and lo side by side in k
 					auto min_mma = [&](int h, uint32_t acc) {
 						mma(tmem + TC_COL_M, tmem + TC_COL_A + UNIT * (j0 + h) + 64u, xs, idesc, acc);
@@ -670,29 +668,31 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 							mma(dP, a + 8 * kk, bh + 2 * kk, idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
 							mma(dP, a + 8 * kk, bl + 2 * kk, idesc, 1u);
 						}
-						if ((q4 & 1) && (!Q4 || sbi > 0)) {
+						if ((q4 & 1) && (!Q4 || (sbi & 7) != 0)) {
 							if (Q4)
 								min_mma(q4 >> 1, 1u);
 							commit(&sh->empty[j0 + (q4 >> 1)]);
 						}
 					}
-					if (Q4 && sbi == 0) {
-						// the item's first min sums: behind the stages, so that neither the sums' landing nor the drain of
-						// the previous item's accumulator holds those up
-						wait(&sh->xfull[tl & 1u], (tl >> 1) & 1u);
-						if (tl >= 1)
+					if (Q4 && (sbi & 7) == 0) {
+						// the first min sums of a segment: behind the stages, so that neither the sums' landing nor the
+						// drain of the previous item's accumulator holds those up
+						wait(&sh->xfull[xs_n & 1u], (xs_n >> 1) & 1u);
+						if (sbi == 0 && tl >= 1)
 							wait(&sh->mempty, (tl & 1u) ^ 1u);
 						if (!alive)
 							break;
 						ptx::tc_fence_after();
-						min_mma(0, 0u);
+						min_mma(0, sbi > 0 ? 1u : 0u);
 						commit(&sh->empty[j0]);
 						min_mma(1, 1u);
 						commit(&sh->empty[j0 + 1]);
 					}
 					commit(&sh->bempty[q]);
-					if (Q4 && sbi == nb - 1)
-						commit(&sh->xempty[tl & 1u]);
+					if (Q4 && ((sbi & 7) == 7 || sbi == nb - 1)) {
+						commit(&sh->xempty[xs_n & 1u]);
+						xs_n++;
+					}
 					commit(&sh->pfull[buf]);
 				}
 			}
@@ -704,31 +704,33 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	} else if (warp == W_TOK) {
 		// ================= token loader: token operand and sub-block sums (TMA) =================
 		if (ptx::elect_one()) {
-			uint32_t tl = 0, n = 0;
+			uint32_t tl = 0, n = 0, xs_n = 0;
 			bool alive = true;
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 				// one box per super-block: four stages of 64 k x (hi, lo) x the CTA's token rows.  The CTAs of a pair
 				// take the first and the second half of the tile's n_mma columns; all the bytes are counted on
 				// the leader's barrier, whose token loader announces them.
 				const uint32_t row_bytes = (uint32_t)(16 << item.box) * 128u;  // of one 64-wide column tile, both CTAs
 				const int row0 = item.row0 + (PAIR ? (int)rank * (item.n_mma >> 1) : 0);
 				const CUtensorMap *tmp = item.box == 0 ? &tm0 : (item.box == 1 ? &tm1 : &tm2);
-				if (Q4) {  // the sub-block sums of the work item (two buffers)
-					if (tl >= 2u && !tc_wait<100>(ptx::smem_u32(&sh->xempty[tl & 1u]), ((tl >> 1) & 1u) ^ 1u, abort_flag, status)) {
-						alive = false;
-						break;
-					}
-					const uint32_t xb = ptx::smem_u32(&sh->xfull[tl & 1u]);
-					const CUtensorMap *tqp = item.box == 0 ? &tq0 : (item.box == 1 ? &tq1 : &tq2);
-					if (rank == 0)
-						ptx::mbar_arrive_expect_tx(xb, (uint32_t)xq_depth * row_bytes);
-					if (PAIR)
-						ptx::tma_load_3d_pair(xq_buf(tl & 1u), tqp, xb, 0, row0, sb0 >> 2);
-					else
-						ptx::tma_load_3d(xq_buf(tl & 1u), tqp, xb, 0, row0, sb0 >> 2);
-				}
 				for (int sbi = 0; sbi < nb; sbi++, n++) {
+					if (Q4 && (sbi & 7) == 0) {  // a segment of the sub-block sums (two buffers)
+						const uint32_t xi = xs_n & 1u;
+						if (xs_n >= 2u && !tc_wait<100>(ptx::smem_u32(&sh->xempty[xi]), ((xs_n >> 1) & 1u) ^ 1u, abort_flag, status)) {
+							alive = false;
+							break;
+						}
+						const uint32_t xb = ptx::smem_u32(&sh->xfull[xi]);
+						const CUtensorMap *tqp = item.box == 0 ? &tq0 : (item.box == 1 ? &tq1 : &tq2);
+						if (rank == 0)
+							ptx::mbar_arrive_expect_tx(xb, (uint32_t)xq_depth * row_bytes);
+						if (PAIR)
+							ptx::tma_load_3d_pair(xq_buf(xi), tqp, xb, 0, row0, sbi >> 2);
+						else
+							ptx::tma_load_3d(xq_buf(xi), tqp, xb, 0, row0, sbi >> 2);
+						xs_n++;
+					}
 					const uint32_t q = n & (Ring::GROUPS - 1);
 					if (n >= (uint32_t)Ring::GROUPS &&
 					    !tc_wait<100>(ptx::smem_u32(&sh->bempty[q]), ((n / Ring::GROUPS) & 1u) ^ 1u, abort_flag, status)) {
@@ -739,9 +741,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					if (rank == 0)
 						ptx::mbar_arrive_expect_tx(fb, 2u * TC_SPB * row_bytes);
 					if (PAIR)
-						ptx::tma_load_4d_pair(b_group(q), tmp, fb, 0, row0, 0, (sb0 + sbi) * TC_SPB);
+						ptx::tma_load_4d_pair(b_group(q), tmp, fb, 0, row0, 0, sbi * TC_SPB);
 					else
-						ptx::tma_load_4d(b_group(q), tmp, fb, 0, row0, 0, (sb0 + sbi) * TC_SPB);
+						ptx::tma_load_4d(b_group(q), tmp, fb, 0, row0, 0, sbi * TC_SPB);
 				}
 			}
 		}
@@ -752,7 +754,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		bool alive = true;
 		int wtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, wtl++) {
-			const TcItem item = tc_item<PAIR>(t, wtl, s_items, m_items, tile_info, rows_per_matrix, rank);
+			const TcItem item = tc_item<PAIR>(t, wtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 			for (int sbi = 0; sbi < nb; sbi++) {
 				if (wc >= (uint32_t)Sm::NWB && !tc_wait_warp<100>(ptx::smem_u32(&sh->wempty[wb]), wph ^ 1u, abort_flag, status, lane)) {
 					alive = false;
@@ -762,10 +764,10 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				if (ptx::elect_one()) {
 					ptx::mbar_arrive_expect_tx(bar, Sm::WBUF);
 					if (Q4)	 // box = (one block, 128 rows)
-						ptx::tma_load_2d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, (sb0 + sbi) * Q4K_BYTES,
+						ptx::tma_load_2d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, sbi * Q4K_BYTES,
 								 item.le * rows_per_matrix + item.m0);
 					else  // box = (one record, 8 rows of a group, 16 groups)
-						ptx::tma_load_3d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, (sb0 + sbi) * TC_Q6_ROW, 0,
+						ptx::tma_load_3d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, sbi * TC_Q6_ROW, 0,
 								 (item.le * rows_per_matrix + item.m0) >> 3);
 				}
 				wc++;
@@ -978,12 +980,11 @@ int tc_setup(tie_cuda_ctx *c)
 // arr: 0 = the split inputs x (gate/up), 1 = the split activations h (down).
 template <WKind KIND, bool RAW, bool PEER = false>
 static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1, int arr, float *y, float out_scale,
-		       bool sorted_out = false, const EpDst *dst = nullptr, int n_experts = -1, const DenseView *view = nullptr,
-		       int sb0 = 0, int n_sb = 0, int accumulate = 0)
+		       bool sorted_out = false, const EpDst *dst = nullptr, int dense_rows = 0, const DenseView *view = nullptr)
 {
 	Scratch &s = c->s;
-	if (n_experts <= 0)
-		n_experts = c->n_local;
+	const int4 *tile_info = dense_rows ? nullptr : s.tile_info;
+	const int n_experts = dense_rows ? dense_rows : c->n_local;
 	const int m_tiles = (RAW ? 2 : 1) * t0.rows / TC_BM;
 	const CUtensorMap &w0m = t0.map;
 	const CUtensorMap &w1m = t1 ? t1->map : t0.map;
@@ -991,8 +992,7 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	const int *perm = sorted_out ? nullptr : s.perm;
 	const int out_stride = RAW ? 2 * t0.rows : t0.rows;
 	const EpDst d = dst ? *dst : EpDst();
-	const int nb_total = t0.k / QK_K;
-	const int k_dim = (n_sb > 0 ? n_sb : nb_total) * QK_K;
+	const int k_dim = t0.k;
 	const int xqd = xq_depth((size_t)xq_cols(t0.k));
 	// a dense tensor brings the maps of its own view of the operand scratch (entries 0-2 operand, 3-5 sums)
 	const CUtensorMap *mh = view ? view->half : c->tmap_half + arr * 3, *mhq = view ? view->half + 3 : c->tmap_half + (2 + arr) * 3;
@@ -1015,23 +1015,22 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
 		TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, grouped_gemm_sb<KIND, RAW, PEER, true>, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m,
-						   (const uint8_t *)t0.ptr, w1p, t0.expert_stride, k_dim, (const int4 *)s.tile_info,
+						   (const uint8_t *)t0.ptr, w1p, t0.expert_stride, k_dim, tile_info,
 						   (const int *)s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d,
-						   sb0, nb_total, accumulate, xqd));
+						   xqd));
 		c->launches++;
 		return TIE_CUDA_OK;
 	}
 	grouped_gemm_sb<KIND, RAW, PEER><<<c->sm_count, TC_THREADS, TcSmem<KIND, false>::SMEM, c->stream>>>(
-		mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p, t0.expert_stride, k_dim, s.tile_info, s.tile_start, n_experts,
-		m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d, sb0, nb_total, accumulate, xqd);
+		mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p, t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts,
+		m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d, xqd);
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }
 
 static bool tc_tensor_ok(const DevTensor &t)
 {
-	// Q4_K needs all sub-block sums of a row in one 64-wide tile (k <= 2048)
-	return t.has_map && t.rows % TC_BM == 0 && t.k % QK_K == 0 && (t.kind != W_Q4K || t.k <= 2048);
+	return t.has_map && t.rows % TC_BM == 0 && t.k % QK_K == 0;
 }
 
 bool tc_supported(const tie_cuda_ctx *c, const Layer &L)
@@ -1107,19 +1106,10 @@ int tc_make_dense_view(tie_cuda_ctx *c, DevTensor &t)
 	return TIE_CUDA_OK;
 }
 
-int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, float *y)
+int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y)
 {
-	const int nb = t.k / QK_K;
-	// Q4_K: at most 8 super-blocks (64 sub-block sums) per launch; later launches add to y
-	const int step = t.kind == W_Q4K ? 8 : nb;
-	for (int sb0 = 0; sb0 < nb; sb0 += step) {
-		const int n_sb = nb - sb0 < step ? nb - sb0 : step;
-		int rc = t.kind == W_Q4K ? launch_tc_t<W_Q4K, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, 1, t.view, sb0, n_sb, sb0 > 0)
-					 : launch_tc_t<W_Q6K_R8, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, 1, t.view, sb0, n_sb, sb0 > 0);
-		if (rc)
-			return rc;
-	}
-	return TIE_CUDA_OK;
+	return t.kind == W_Q4K ? launch_tc_t<W_Q4K, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view)
+			       : launch_tc_t<W_Q6K_R8, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view);
 }
 
 // The down product of an expert-parallel step: row p goes to the rank and row dst->row[p] names.
