@@ -27,8 +27,9 @@
 //   * a token loader thread issues TMA tile loads of the token operand (hi/lo fp16, expert-sorted
 //     rows: only rows the expert really has) and of the sub-block sums, into rings of their own;
 //   * one MMA issuer thread walks the super-blocks: per 16-wide k step P += A.B_hi, P += A.B_lo into the
-//     same accumulator columns (one column per token), a super-block per accumulator buffer, two
-//     buffers of 64 columns in turn, and the block's min sums into a third;
+//     same accumulator columns (one column per token; tiles of up to 32 tokens: one MMA over hi and lo
+//     rows, into columns side by side), a super-block per accumulator buffer, two buffers of 64
+//     columns in turn, and the block's min sums into a third;
 //   * 8 drain warps take a finished super-block out of tensor memory (tcgen05.ld), hand the buffer back
 //     at once, fold the values into fp32 registers with d (-1 for the min sums), and after the last
 //     super-block of a work item store the rows — while the MMAs of the next super-blocks / work
@@ -45,6 +46,8 @@
 // Barriers that collect arrivals from both CTAs live in the leader (remote mbarrier arrivals; TMA
 // loads of the peer count their bytes there); the MMA completions are committed to both CTAs at
 // once.  No copy is delivered to more than one CTA.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "tc_dequant.cuh"
@@ -514,43 +517,53 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		for (int t = walker; t < total && alive; t += stride_t, dtl++) {
 			const TcItem item = tc_item<PAIR>(t, dtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 			const int mrow = item.m0 + lrow;
-			// tokens (accumulator columns) of this warp: half of the tile's range, 16 or 32
+			// tokens of this warp: half of the tile's range.  A narrow tile (up to 32 tokens) has its hi and lo
+			// products in accumulator columns of their own (one MMA for both), which for a pair lie
+			// [hi lo] per CTA's half of the tokens.
 			const bool wide = item.n_mma > 32;
-			const int ntok = wide ? 32 : 16;
+			const int ntok = wide ? 32 : item.n_mma >> 1;
 			const int tok0 = chalf * ntok;
-			const bool on = tok0 < item.n_mma;  // (warp-uniform, as wide is)
+			const uint32_t c_hi = PAIR ? chalf * item.n_mma : tok0, c_lo = PAIR ? c_hi + ntok : item.n_mma + tok0;
 			float acc[TC_NT / 2];
 #pragma unroll
 			for (int j = 0; j < TC_NT / 2; j++)
 				acc[j] = 0.0f;
 			// acc += scale * the warp's columns of an accumulator; the buffer is handed back once they are in registers
-			auto fold = [&](uint32_t col, float scale, uint64_t *bar) {
+			// (columns past the warp's tokens are read along and dropped)
+			auto fold = [&](uint32_t col, bool stacked, float scale, uint64_t *bar) {
 				uint32_t v[16];
-				if (on) {
+				if (wide) {
 					ptx::tmem_ld16(tlane + col + tok0, v);
 					ptx::tmem_ld_wait();
-					if (wide) {
 #pragma unroll
-						for (int j = 0; j < 16; j++)
-							acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
-						ptx::tmem_ld16(tlane + col + tok0 + 16, v);
-						ptx::tmem_ld_wait();
-					}
+					for (int j = 0; j < 16; j++)
+						acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
+					ptx::tmem_ld16(tlane + col + tok0 + 16, v);
+					ptx::tmem_ld_wait();
+				} else if (stacked) {
+					uint32_t u[16];
+					ptx::tmem_ld16(tlane + col + c_hi, v);
+					ptx::tmem_ld16(tlane + col + c_lo, u);
+					ptx::tmem_ld_wait();
+#pragma unroll
+					for (int j = 0; j < 16; j++)
+						v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+				} else {
+					ptx::tmem_ld16(tlane + col + tok0, v);
+					ptx::tmem_ld_wait();
 				}
 				ptx::tc_fence_before();
 				__syncwarp();
 				if (lane == 0)
 					arrive_issuer(bar);
-				if (on) {
-					if (wide) {
+				if (wide) {
 #pragma unroll
-						for (int j = 0; j < 16; j++)
-							acc[16 + j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[16 + j]);
-					} else {
+					for (int j = 0; j < 16; j++)
+						acc[16 + j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[16 + j]);
+				} else {
 #pragma unroll
-						for (int j = 0; j < 16; j++)
-							acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
-					}
+					for (int j = 0; j < 16; j++)
+						acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
 				}
 			};
 			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead
@@ -573,13 +586,13 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				ptx::tc_fence_after();
 				if (Q4)
 					scale = ds[(n & (TC_NDS - 1)) * TC_BM + lrow];
-				fold(TC_COL_P + TC_NT * buf, scale, &sh->pempty[buf]);
+				fold(TC_COL_P + TC_NT * buf, true, scale, &sh->pempty[buf]);
 			}
 			if (!alive)
 				break;
 			// the min sums (Q4_K) were complete with the last super-block
 			if (Q4)
-				fold(TC_COL_M, -1.0f, &sh->mempty);
+				fold(TC_COL_M, false, -1.0f, &sh->mempty);
 			// rows of this work item: lanes hold consecutive output columns (coalesced 128-byte stores)
 			const int n_rows = min(ntok, item.n_valid - tok0);
 			int rid = 0;
@@ -633,7 +646,11 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
 				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 				const uint32_t idesc = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, item.n_mma);
+				const uint32_t idesc2 = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, 2 * item.n_mma);
 				const uint32_t lo_off = (uint32_t)((PAIR ? 8 : 16) << item.box) * 128u;
+				// up to 32 tokens fill their box, so the lo rows follow the hi rows and one MMA of twice the columns
+				// takes both (this thread paces narrow tiles: its instructions count)
+				const bool stacked = item.n_mma <= 32;
 				for (int sbi = 0; sbi < nb && alive; sbi++, n++) {
 					const uint32_t buf = n % TC_NBUF, j0 = 2u * (n & 1u), uph = (n >> 1) & 1u;
 					const uint32_t q = n & (Ring::GROUPS - 1), bph = (n / Ring::GROUPS) & 1u, pph = ((n / TC_NBUF) & 1u) ^ 1u;
@@ -658,22 +675,29 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					auto min_mma = [&](int h, uint32_t acc) {
 						mma(tmem + TC_COL_M, tmem + TC_COL_A + UNIT * (j0 + h) + 64u, xs, idesc, acc);
 					};
+					auto stages = [&](auto both) {
 #pragma unroll
-					for (int q4 = 0; q4 < TC_SPB; q4++) {
-						const uint32_t bh = ptx::umma_desc_lo(bt + q4 * 2u * lo_off);
-						const uint32_t bl = bh + (lo_off >> 4);
-						const uint32_t a = tmem + TC_COL_A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1);
+						for (int q4 = 0; q4 < TC_SPB; q4++) {
+							const uint32_t bh = ptx::umma_desc_lo(bt + q4 * 2u * lo_off);
+							const uint32_t bl = bh + (lo_off >> 4);
+							const uint32_t a = tmem + TC_COL_A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1);
 #pragma unroll
-						for (int kk = 0; kk < TC_BK / 16; kk++) {
-							mma(dP, a + 8 * kk, bh + 2 * kk, idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
-							mma(dP, a + 8 * kk, bl + 2 * kk, idesc, 1u);
+							for (int kk = 0; kk < TC_BK / 16; kk++) {
+								mma(dP, a + 8 * kk, bh + 2 * kk, both.value ? idesc2 : idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
+								if (!both.value)
+									mma(dP, a + 8 * kk, bl + 2 * kk, idesc, 1u);
+							}
+							if ((q4 & 1) && (!Q4 || (sbi & 7) != 0)) {
+								if (Q4)
+									min_mma(q4 >> 1, 1u);
+								commit(&sh->empty[j0 + (q4 >> 1)]);
+							}
 						}
-						if ((q4 & 1) && (!Q4 || (sbi & 7) != 0)) {
-							if (Q4)
-								min_mma(q4 >> 1, 1u);
-							commit(&sh->empty[j0 + (q4 >> 1)]);
-						}
-					}
+					};
+					if (stacked)
+						stages(std::true_type());
+					else
+						stages(std::false_type());
 					if (Q4 && (sbi & 7) == 0) {
 						// the first min sums of a segment: behind the stages, so that neither the sums' landing nor the
 						// drain of the previous item's accumulator holds those up
