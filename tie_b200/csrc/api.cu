@@ -54,7 +54,7 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TRY(dev_alloc(c, &s.counts, E));
 	TRY(dev_alloc(c, &s.offsets, E + 1));
 	TRY(dev_alloc(c, &s.tile_start, E + 1));
-	TRY(dev_alloc(c, &s.tile_info, E + R / TC_TOKEN_TILE + 1));
+	TRY(dev_alloc(c, &s.tile_info, E + R / 32 + 1));
 	TRY(dev_alloc(c, &s.active, E));
 	TRY(dev_alloc(c, &s.n_active, 1));
 	TRY(dev_alloc(c, &s.perm, R));
@@ -267,7 +267,9 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	}
 	c->tc_no_pair = (flags & TIE_CUDA_PATH_NO_PAIR) != 0;
 	const int direct = (!use_tc && n_rows <= c->cfg.top_k && src_div == c->cfg.top_k) ? 1 : 0;
-	const int n_tile = TC_TOKEN_TILE;
+	// tiles of 32 tokens where hardly any expert has more rows than that (the next tile would expand its
+	// weights again), else of 64
+	const int n_tile = n_rows <= 24 * c->n_local ? 32 : TC_TOKEN_TILE;
 	c->last_direct_rows = direct ? n_rows : -1;
 	c->last_used_tc = use_tc;
 	if (!direct)
@@ -278,11 +280,11 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 		TRY(launch_split_rows(c, x_src, c->s.perm, src_div, n_rows, c->cfg.hidden, c->s.xs_hi, c->s.xs_lo,
 				      sums ? c->s.xq : nullptr));
 		prof_mark(c, 3);
-		TRY(launch_tc_gate_up(c, L, n_rows));
+		TRY(launch_tc_gate_up(c, L, n_tile));
 		prof_mark(c, 4);
 		TRY(launch_tc_swiglu(c, L, n_rows));
 		prof_mark(c, 5);
-		TRY(launch_tc_down(c, L, n_rows, y));
+		TRY(launch_tc_down(c, L, n_tile, y));
 		prof_mark(c, 6);
 	} else {
 		prof_mark(c, 3);
@@ -1365,7 +1367,7 @@ int tie_cuda_ep_compute(tie_cuda_ctx *c, int layer, unsigned flags)
 	TRY(launch_ep_index(c));
 	TRY(launch_ep_split_rows(c, L->gate.kind == W_Q4K));
 	prof_mark(c, 3);
-	TRY(launch_tc_gate_up(c, *L, 0));
+	TRY(launch_tc_gate_up(c, *L, TC_TOKEN_TILE));
 	prof_mark(c, 4);
 	TRY(launch_tc_swiglu(c, *L, c->sm_count * 8, ep.n_rows));
 	prof_mark(c, 5);

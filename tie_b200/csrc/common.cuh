@@ -17,7 +17,7 @@ constexpr int QK_K = 256;	  // gguf.h:100
 constexpr int Q4K_BYTES = 144;	  // sizeof(block_q4_k), gguf.h:108-113
 constexpr int Q6K_BYTES = 210;	  // sizeof(block_q6_k), gguf.h:101-106
 constexpr int MAX_TOP_K = 8;
-constexpr int TC_TOKEN_TILE = 64;  // rows of one expert per token tile of the tensor-core path
+constexpr int TC_TOKEN_TILE = 64;  // rows of one expert per token tile of the tensor-core path (or 32: run_experts)
 constexpr int SILU_N = TIE_CUDA_SILU_TABLE_SIZE;
 constexpr int SORT_SLICE = 256;   // rows per CTA of the dispatch sort
 
@@ -80,7 +80,7 @@ struct Scratch {
 	int *counts = nullptr;	    // [E]
 	int *offsets = nullptr;	    // [E+1]
 	int *tile_start = nullptr;  // [E+1]
-	int4 *tile_info = nullptr;  // [E + R/TC_TOKEN_TILE + 1]  token tiles: (expert, first sorted row, rows, 0)
+	int4 *tile_info = nullptr;  // [E + R/32 + 1]  token tiles: (expert, first sorted row, rows, 0)
 	int *active = nullptr;	    // [E]  compact list of experts with rows
 	int *n_active = nullptr;    // [1]
 	int *perm = nullptr;	    // [R]  sorted position -> row id

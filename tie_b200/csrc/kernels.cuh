@@ -60,10 +60,10 @@ bool tc_dense_supported(const tie_cuda_ctx *c, const DevTensor &t);
 int tc_make_dense_view(tie_cuda_ctx *c, DevTensor &t);
 int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y);
 bool tc_supported(const tie_cuda_ctx *c, const Layer &L);
-int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_rows);
+// n_tile: the token tiles of the sort, 32 or 64 rows
+int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile);
 int launch_tc_swiglu(tie_cuda_ctx *c, const Layer &L, int n_rows, const int *n_rows_dev = nullptr);
-// sorted_out: y[p] instead of y[perm[p]]
-int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_rows, float *y, bool sorted_out = false);
+int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_tile, float *y);
 int launch_tc_down_peer(tie_cuda_ctx *c, const Layer &L, const EpDst &dst);
 // ep.cu
 int launch_ep_signal(tie_cuda_ctx *c, int which);

@@ -58,7 +58,6 @@ namespace tie {
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;
 constexpr int TC_SPB = QK_K / TC_BK;	  // stages per super-block
-constexpr int TC_NT = TC_TOKEN_TILE;	  // tokens per tile (N of the MMAs, at most)
 constexpr int TC_PWARPS = 16;		  // producer warps: four groups of 128 threads
 constexpr int TC_DWARPS = 8;		  // drain warps
 constexpr int TC_THREADS = (TC_PWARPS + TC_DWARPS + 3) * 32;  // + MMA issuer + token loader + weight loader
@@ -67,26 +66,34 @@ constexpr int TC_THREADS = (TC_PWARPS + TC_DWARPS + 3) * 32;  // + MMA issuer + 
 constexpr int TC_LREGS = 72, TC_PREGS = 64, TC_DREGS = 88;
 static_assert(32 * (TC_PWARPS * TC_PREGS + TC_DWARPS * TC_DREGS) + 3 * 32 * TC_LREGS <= TC_THREADS * TC_LREGS, "register split");
 constexpr int TC_UNITS = 4;  // slots of the weight ring in tensor memory, one per producer group: half a super-block each
-constexpr int TC_NBUF = 2;   // accumulator buffers
 constexpr int TC_NDS = 8;    // block-factor hand-off buffers (producers -> drain warps)
 constexpr long long TC_WAIT_CYCLES = 1ll << 30;	 // about half a second of SM clocks
 constexpr float TC_H_SCALE = 1.0f / 256.0f;	 // keeps SwiGLU outputs inside fp16 range; exact (power of two)
 
-// tensor-memory columns
-constexpr uint32_t TC_COL_P = 0;    // TC_NBUF x 64: partial sums of one super-block
-constexpr uint32_t TC_COL_M = 128;  // 64: the min sums of a work item (Q4_K)
-constexpr uint32_t TC_COL_A = 192;  // TC_UNITS x (64 + 8): weight ring
+// Tensor-memory columns.  NT: tokens per tile (N of the MMAs, at most), 32 or 64 by the rows per expert
+// (run_experts).  What paces narrow tiles is the round trip of an accumulator (MMA, commit, drain, hand-back:
+// about 1800 cycles) and the drain's row stores at the end of an item, so tiles of up to 32 tokens get four
+// accumulators, and their items go to two sets of drain warps in turn (64 tokens: gate/up 76 -> 71 us, down
+// 56 -> 50).
 constexpr uint32_t TC_TMEM_COLS = 512;
-static_assert(TC_NBUF * TC_NT <= TC_COL_M && TC_COL_M + TC_NT <= TC_COL_A && TC_COL_A + TC_UNITS * 72 <= TC_TMEM_COLS,
-	      "tensor memory budget");
+constexpr int TC_NBUF_MAX = 4;
+template <WKind KIND, int NT>
+struct TcCols {
+	static constexpr bool Q4 = KIND == W_Q4K;
+	static constexpr int NBUF = NT == 32 || !Q4 ? 4 : 2;  // accumulators of one super-block
+	static constexpr int NM = NT == 32 ? 2 : 1;	      // ... of the min sums of a work item (Q4_K)
+	static constexpr uint32_t UNIT = 64 + (Q4 ? 8 : 0);   // one unit of the weight ring
+	static constexpr uint32_t M = NBUF * NT, A = M + (Q4 ? NM * NT : 0);
+	static_assert(A + TC_UNITS * UNIT <= TC_TMEM_COLS, "tensor memory budget");
+};
 
 // shared memory
 constexpr int TC_B_BYTES = 128 * 1024;	// token ring: groups of four stages of (hi, lo) x 64 k x the CTA's token rows
-constexpr int TC_BG_MAX = 4;
-template <bool PAIR>
+constexpr int TC_BG_MAX = 8;
+template <bool PAIR, int NT>
 struct TcRing {
-	static constexpr int ROWS = PAIR ? TC_NT / 2 : TC_NT;		// token rows a CTA holds, at most
-	static constexpr int GROUP = TC_SPB * 2 * ROWS * TC_BK * 2;	// 32 KB / 64 KB
+	static constexpr int ROWS = PAIR ? NT / 2 : NT;			// token rows a CTA holds, at most
+	static constexpr int GROUP = TC_SPB * 2 * ROWS * TC_BK * 2;	// 16 .. 64 KB
 	static constexpr int GROUPS = TC_B_BYTES / GROUP;
 	static_assert(GROUPS <= TC_BG_MAX && (GROUPS & (GROUPS - 1)) == 0, "token ring");
 };
@@ -95,7 +102,7 @@ struct TcRing {
 // of 9 and 13 x 16 bytes: 16-byte reads by 32 consecutive rows are bank-conflict free.
 constexpr int TC_Q6_ROW = Q6K_RECORD;
 constexpr int TC_NWB_MAX = 4, TC_NWF_MAX = 6;
-template <WKind KIND, bool PAIR>
+template <WKind KIND, bool PAIR, int NT>
 struct TcSmem {
 	static constexpr bool Q4 = KIND == W_Q4K;
 	static constexpr int NWB = Q4 && PAIR ? 4 : 3;	// packed super-blocks in flight
@@ -103,7 +110,7 @@ struct TcSmem {
 	// producer groups take every other super-block, so an odd number of buffers gets two barriers each.
 	static constexpr int NWF = NWB % 2 ? 2 * NWB : NWB;
 	static constexpr int WBUF = TC_BM * (Q4 ? Q4K_BYTES : TC_Q6_ROW);
-	static constexpr int XQ = Q4 ? 2 * TcRing<PAIR>::ROWS * 128 : 0;  // sub-block sums of a work item (Q4_K): two 64-wide tiles
+	static constexpr int XQ = Q4 ? 2 * TcRing<PAIR, NT>::ROWS * 128 : 0;  // sub-block sums of a work item (Q4_K): two 64-wide tiles
 	static constexpr int OFF_W = TC_B_BYTES;
 	static constexpr int OFF_XQ = OFF_W + NWB * WBUF;
 	static constexpr int OFF_DS = OFF_XQ + 2 * XQ;	// block factors (Q4_K)
@@ -120,11 +127,11 @@ struct TcShared {
 	uint64_t bempty[TC_BG_MAX];	// ... and consumed
 	uint64_t wfull[TC_NWF_MAX];	// packed super-block landed
 	uint64_t wempty[TC_NWB_MAX];	// ... and expanded
-	uint64_t pfull[TC_NBUF];	// accumulator buffer complete (one super-block)
-	uint64_t pempty[TC_NBUF];	// accumulator buffer read out by the drain warps
+	uint64_t pfull[2][TC_NBUF_MAX];	// accumulator complete (one super-block), per set of drain warps
+	uint64_t pempty[TC_NBUF_MAX];	// accumulator read out by the drain warps
 	uint64_t xfull[2];		// sub-block sums of a work item landed
 	uint64_t xempty[2];		// ... and consumed
-	uint64_t mempty;		// min sums of a work item read out by the drain warps
+	uint64_t mempty[2];		// min sums of a work item read out by the drain warps
 	uint64_t fin;			// every commit has landed
 	uint32_t tmem_base;
 	uint32_t abort;
@@ -180,20 +187,20 @@ struct TcItem {
 constexpr int TC_ITEMS = 128;
 // m_items: work items per token tile (128-row tiles, or pairs of them); a CTA of a pair takes the
 // tile 2 * item + its rank.  Packed: expert, first row, rows, first weight row | matrix << 30.
-template <bool PAIR>
+template <bool PAIR, int NT>
 __device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int rows_per_matrix,
 					  uint32_t rank)
 {
 	const int slot = t / m_items, mi = t - slot * m_items;
-	const int4 ti = tile_info ? __ldg(tile_info + slot) : make_int4(0, slot * TC_NT, min(TC_NT, n_rows - slot * TC_NT), 0);
+	const int4 ti = tile_info ? __ldg(tile_info + slot) : make_int4(0, slot * NT, min(NT, n_rows - slot * NT), 0);
 	const int m = (PAIR ? 2 * mi + (int)rank : mi) * TC_BM, sel = m >= rows_per_matrix ? 1 : 0;
 	return make_int4(ti.x, ti.y, ti.z, (m - sel * rows_per_matrix) | sel << 30);
 }
-template <bool PAIR>
+template <bool PAIR, int NT>
 __device__ __forceinline__ TcItem tc_item(int t, int tl, const int4 *s_items, int m_items, const int4 *__restrict__ tile_info,
 					  int n_rows, int rows_per_matrix, uint32_t rank)
 {
-	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR>(t, m_items, tile_info, n_rows, rows_per_matrix, rank);
+	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR, NT>(t, m_items, tile_info, n_rows, rows_per_matrix, rank);
 	TcItem it;
 	it.le = ti.x;
 	it.row0 = ti.y;
@@ -332,7 +339,7 @@ struct Expander<W_Q6K_R8> {
 // PEER (expert parallelism over peer memory, down product only): sorted row p belongs to row
 // dst.row[p] & 0xFFFFFF of rank dst.row[p] >> 24 and is stored there, into that rank's memory
 // (dst.y[rank], plain stores over NVLink, 128 contiguous bytes per warp and row).
-template <WKind KIND, bool RAW, bool PEER = false, bool PAIR = false>
+template <WKind KIND, bool RAW, bool PEER = false, bool PAIR = false, int NT = TC_TOKEN_TILE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
 		const __grid_constant__ CUtensorMap tm2, const __grid_constant__ CUtensorMap tq0,
@@ -344,10 +351,14 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		const int xq_depth)
 {
 	static_assert(!(RAW && PEER), "peer destinations exist for the down product only");
-	using Sm = TcSmem<KIND, PAIR>;
-	using Ring = TcRing<PAIR>;
+	using Sm = TcSmem<KIND, PAIR, NT>;
+	using Ring = TcRing<PAIR, NT>;
+	using Cols = TcCols<KIND, NT>;
+	constexpr int NBUF = Cols::NBUF;
+	constexpr bool SETS = NT == 32;	 // two sets of drain warps, taking the work items in turn
+	constexpr int FOLDERS = SETS ? TC_DWARPS / 2 : TC_DWARPS;  // drain warps that read an accumulator
 	constexpr bool Q4 = KIND == W_Q4K;
-	constexpr uint32_t UNIT = 64 + (Q4 ? 8 : 0);  // tensor-memory columns of one unit of the weight ring
+	constexpr uint32_t UNIT = Cols::UNIT;
 	extern __shared__ uint8_t smem_raw[];
 	__shared__ int s_total;
 	__shared__ int4 s_items[TC_ITEMS];
@@ -357,7 +368,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	const int stride_t = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 	const int m_items = PAIR ? m_tiles / 2 : m_tiles;
 	if (threadIdx.x == 0)
-		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + TC_NT - 1) / TC_NT) * m_items;
+		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
 	__syncthreads();
 	// (a CTA of a pair never returns early: its peer would wait for it at the cluster barrier below)
 	const int total = s_total;
@@ -366,7 +377,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	if (threadIdx.x < TC_ITEMS) {
 		const int t = walker + threadIdx.x * stride_t;
 		if (t < total)
-			s_items[threadIdx.x] = tc_decode<PAIR>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
+			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
 	}
 	const int nb = k_dim / QK_K;
 
@@ -395,15 +406,16 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			ptx::mbar_init(ptx::smem_u32(&sh->wfull[s]), 1);
 		for (int s = 0; s < Sm::NWB; s++)
 			ptx::mbar_init(ptx::smem_u32(&sh->wempty[s]), 8);
-		for (int s = 0; s < TC_NBUF; s++) {
-			ptx::mbar_init(ptx::smem_u32(&sh->pfull[s]), 1);
-			ptx::mbar_init(ptx::smem_u32(&sh->pempty[s]), (PAIR ? 2 : 1) * TC_DWARPS);
+		for (int s = 0; s < NBUF; s++) {
+			ptx::mbar_init(ptx::smem_u32(&sh->pfull[0][s]), 1);
+			ptx::mbar_init(ptx::smem_u32(&sh->pfull[1][s]), 1);
+			ptx::mbar_init(ptx::smem_u32(&sh->pempty[s]), (PAIR ? 2 : 1) * FOLDERS);
 		}
 		for (int s = 0; s < 2; s++) {
 			ptx::mbar_init(ptx::smem_u32(&sh->xfull[s]), 1);
 			ptx::mbar_init(ptx::smem_u32(&sh->xempty[s]), 1);
+			ptx::mbar_init(ptx::smem_u32(&sh->mempty[s]), (PAIR ? 2 : 1) * FOLDERS);
 		}
-		ptx::mbar_init(ptx::smem_u32(&sh->mempty), (PAIR ? 2 : 1) * TC_DWARPS);
 		ptx::mbar_init(ptx::smem_u32(&sh->fin), 1);
 		sh->abort = 0;
 		ptx::fence_barrier_init();
@@ -457,7 +469,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		// first piece is expanded in registers BEFORE the slot is waited for.
 		ptx::setmaxnreg_dec<TC_PREGS>();
 		const int row = threadIdx.x & 127, grp = threadIdx.x >> 7, half = grp & 1;
-		const uint32_t slot = tmem + ((uint32_t)((warp & 3) * 32) << 16) + TC_COL_A + UNIT * grp;
+		const uint32_t slot = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cols::A + UNIT * grp;
 		const uint32_t full = ptx::smem_u32(&sh->full[grp]), empty = ptx::smem_u32(&sh->empty[grp]);
 		const uint32_t n_sb = walker < total ? (uint32_t)((total - 1 - walker) / stride_t + 1) * (uint32_t)nb : 0u;
 		bool alive = true;
@@ -508,31 +520,38 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	} else if (warp < W_MMA) {
 		// ================= drain warps: partial sums of a super-block -> fp32 rows =================
 		ptx::setmaxnreg_inc<TC_DREGS>();
-		const int dw = warp - TC_PWARPS, quad = warp & 3, chalf = dw >> 2;
+		const int dw = warp - TC_PWARPS, quad = warp & 3, part = dw >> 2;
 		const int lrow = quad * 32 + lane;
 		const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16);
-		uint32_t n = 0;	 // super-blocks so far
+		const int set = SETS ? part : 0;
+		uint32_t n = 0;	   // super-blocks so far
+		uint32_t pph = 0;  // SETS, per accumulator: parity of this set's next wait (it takes only its items' uses)
 		bool alive = true;
 		int dtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, dtl++) {
-			const TcItem item = tc_item<PAIR>(t, dtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+			if (SETS && (dtl & 1) != set) {	 // the other set's item
+				n += nb;
+				continue;
+			}
+			const TcItem item = tc_item<PAIR, NT>(t, dtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 			const int mrow = item.m0 + lrow;
-			// tokens of this warp: half of the tile's range.  A narrow tile (up to 32 tokens) has its hi and lo
-			// products in accumulator columns of their own (one MMA for both), which for a pair lie
-			// [hi lo] per CTA's half of the tokens.
-			const bool wide = item.n_mma > 32;
-			const int ntok = wide ? 32 : item.n_mma >> 1;
-			const int tok0 = chalf * ntok;
-			const uint32_t c_hi = PAIR ? chalf * item.n_mma : tok0, c_lo = PAIR ? c_hi + ntok : item.n_mma + tok0;
-			float acc[TC_NT / 2];
+			// tokens of this warp: with two sets the whole tile, else half of it (the first or the second by part).
+			// Where twice the columns fit an accumulator, the hi and lo products have columns of their own (one MMA
+			// for both), which for a pair lie [hi lo] per CTA's half of the tokens.
+			const bool stacked = 2 * item.n_mma <= NT;
+			const int ntok = SETS ? item.n_mma : (item.n_mma > 32 ? 32 : item.n_mma >> 1);
+			const int tok0 = SETS ? 0 : part * ntok;
+			const bool two = ntok == 32;
+			const uint32_t c_hi = PAIR ? part * item.n_mma : tok0, c_lo = PAIR ? c_hi + ntok : item.n_mma + tok0;  // (not SETS)
+			float acc[32];
 #pragma unroll
-			for (int j = 0; j < TC_NT / 2; j++)
+			for (int j = 0; j < 32; j++)
 				acc[j] = 0.0f;
 			// acc += scale * the warp's columns of an accumulator; the buffer is handed back once they are in registers
 			// (columns past the warp's tokens are read along and dropped)
-			auto fold = [&](uint32_t col, bool stacked, float scale, uint64_t *bar) {
+			auto fold = [&](uint32_t col, bool both, float scale, uint64_t *bar) {
 				uint32_t v[16];
-				if (wide) {
+				if (two) {
 					ptx::tmem_ld16(tlane + col + tok0, v);
 					ptx::tmem_ld_wait();
 #pragma unroll
@@ -540,14 +559,22 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
 					ptx::tmem_ld16(tlane + col + tok0 + 16, v);
 					ptx::tmem_ld_wait();
-				} else if (stacked) {
+				} else if (both) {
 					uint32_t u[16];
-					ptx::tmem_ld16(tlane + col + c_hi, v);
-					ptx::tmem_ld16(tlane + col + c_lo, u);
+					ptx::tmem_ld16(tlane + col + (SETS ? 0u : c_hi), v);
+					ptx::tmem_ld16(tlane + col + (SETS ? 16u : c_lo), u);
 					ptx::tmem_ld_wait();
+					if (SETS && PAIR) {  // [hi lo] of tokens 0 .. 7, then of 8 .. 15
 #pragma unroll
-					for (int j = 0; j < 16; j++)
-						v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+						for (int j = 0; j < 8; j++) {
+							v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(v[8 + j]));
+							v[8 + j] = __float_as_uint(__uint_as_float(u[j]) + __uint_as_float(u[8 + j]));
+						}
+					} else {
+#pragma unroll
+						for (int j = 0; j < 16; j++)
+							v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+					}
 				} else {
 					ptx::tmem_ld16(tlane + col + tok0, v);
 					ptx::tmem_ld_wait();
@@ -556,7 +583,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				__syncwarp();
 				if (lane == 0)
 					arrive_issuer(bar);
-				if (wide) {
+				if (two) {
 #pragma unroll
 					for (int j = 0; j < 16; j++)
 						acc[16 + j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[16 + j]);
@@ -578,21 +605,23 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				if (!Q4 && sbi + 1 < nb)
 					dnext = half_bits_to_float(
 						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
-				const uint32_t buf = n % TC_NBUF;
-				if (!tc_wait_warp(ptx::smem_u32(&sh->pfull[buf]), (n / TC_NBUF) & 1u, abort_flag, status, lane)) {
+				const uint32_t buf = n % NBUF;
+				if (!tc_wait_warp(ptx::smem_u32(&sh->pfull[set][buf]), SETS ? (pph >> buf) & 1u : (n / NBUF) & 1u, abort_flag, status, lane)) {
 					alive = false;
 					break;
 				}
+				if (SETS)
+					pph ^= 1u << buf;
 				ptx::tc_fence_after();
 				if (Q4)
 					scale = ds[(n & (TC_NDS - 1)) * TC_BM + lrow];
-				fold(TC_COL_P + TC_NT * buf, true, scale, &sh->pempty[buf]);
+				fold(NT * buf, stacked, scale, &sh->pempty[buf]);
 			}
 			if (!alive)
 				break;
 			// the min sums (Q4_K) were complete with the last super-block
 			if (Q4)
-				fold(TC_COL_M, false, -1.0f, &sh->mempty);
+				fold(Cols::M + NT * set, false, -1.0f, &sh->mempty[set]);
 			// rows of this work item: lanes hold consecutive output columns (coalesced 128-byte stores)
 			const int n_rows = min(ntok, item.n_valid - tok0);
 			int rid = 0;
@@ -604,7 +633,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			}
 			float *yr = RAW ? y + (size_t)(item.row0 + tok0) * out_stride + (size_t)item.mat_sel * rows_per_matrix + mrow : y + mrow;
 #pragma unroll
-			for (int j = 0; j < TC_NT / 2; j++) {
+			for (int j = 0; j < 32; j++) {
 				const int rj = RAW ? 0 : __shfl_sync(0xffffffffu, rid, j);
 				if (j < n_rows) {
 					if (RAW) {
@@ -644,24 +673,25 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				alive = alive && tc_wait(ptx::smem_u32(bar), parity, abort_flag, status);
 			};
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 				const uint32_t idesc = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, item.n_mma);
 				const uint32_t idesc2 = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, 2 * item.n_mma);
 				const uint32_t lo_off = (uint32_t)((PAIR ? 8 : 16) << item.box) * 128u;
-				// up to 32 tokens fill their box, so the lo rows follow the hi rows and one MMA of twice the columns
-				// takes both (this thread paces narrow tiles: its instructions count)
-				const bool stacked = item.n_mma <= 32;
+				// a tile whose hi and lo products fit an accumulator side by side fills its box, so the lo rows follow the
+				// hi rows and one MMA of twice the columns takes both
+				const bool stacked = 2 * item.n_mma <= NT;
+				const uint32_t dset = SETS ? tl & 1u : 0u;  // the set of drain warps that takes the item
 				for (int sbi = 0; sbi < nb && alive; sbi++, n++) {
-					const uint32_t buf = n % TC_NBUF, j0 = 2u * (n & 1u), uph = (n >> 1) & 1u;
-					const uint32_t q = n & (Ring::GROUPS - 1), bph = (n / Ring::GROUPS) & 1u, pph = ((n / TC_NBUF) & 1u) ^ 1u;
+					const uint32_t buf = n % NBUF, j0 = 2u * (n & 1u), uph = (n >> 1) & 1u;
+					const uint32_t q = n & (Ring::GROUPS - 1), bph = (n / Ring::GROUPS) & 1u, pph = ((n / NBUF) & 1u) ^ 1u;
 					bool ready = ptx::mbar_try_wait(ptx::smem_u32(&sh->bfull[q]), bph);
 					ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->full[j0]), uph);
 					ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->full[j0 + 1]), uph);
-					if (n >= (uint32_t)TC_NBUF)
+					if (n >= (uint32_t)NBUF)
 						ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->pempty[buf]), pph);
 					if (!ready) {
 						wait(&sh->bfull[q], bph);
-						if (n >= (uint32_t)TC_NBUF)
+						if (n >= (uint32_t)NBUF)
 							wait(&sh->pempty[buf], pph);
 						wait(&sh->full[j0], uph);
 						wait(&sh->full[j0 + 1], uph);
@@ -669,18 +699,18 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 							break;
 					}
 					ptx::tc_fence_after();
-					const uint32_t dP = tmem + TC_COL_P + TC_NT * buf, bt = b_group(q);
+					const uint32_t dP = tmem + NT * buf, bt = b_group(q);
 					const uint32_t xs = ptx::umma_desc_lo(xq_buf(xs_n & 1u) + (uint32_t)((sbi >> 2) & 1) * lo_off) + 2u * (sbi & 3);
 					// (dmin m)_hi (half 0), (dmin m)_lo (half 1) times the block's sums, hi and lo side by side in k
 					auto min_mma = [&](int h, uint32_t acc) {
-						mma(tmem + TC_COL_M, tmem + TC_COL_A + UNIT * (j0 + h) + 64u, xs, idesc, acc);
+						mma(tmem + Cols::M + NT * dset, tmem + Cols::A + UNIT * (j0 + h) + 64u, xs, idesc, acc);
 					};
 					auto stages = [&](auto both) {
 #pragma unroll
 						for (int q4 = 0; q4 < TC_SPB; q4++) {
 							const uint32_t bh = ptx::umma_desc_lo(bt + q4 * 2u * lo_off);
 							const uint32_t bl = bh + (lo_off >> 4);
-							const uint32_t a = tmem + TC_COL_A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1);
+							const uint32_t a = tmem + Cols::A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1);
 #pragma unroll
 							for (int kk = 0; kk < TC_BK / 16; kk++) {
 								mma(dP, a + 8 * kk, bh + 2 * kk, both.value ? idesc2 : idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
@@ -702,8 +732,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						// the first min sums of a segment: behind the stages, so that neither the sums' landing nor the
 						// drain of the previous item's accumulator holds those up
 						wait(&sh->xfull[xs_n & 1u], (xs_n >> 1) & 1u);
-						if (sbi == 0 && tl >= 1)
-							wait(&sh->mempty, (tl & 1u) ^ 1u);
+						if (sbi == 0 && tl >= (uint32_t)Cols::NM)
+							wait(&sh->mempty[dset], ((SETS ? tl >> 1 : tl) & 1u) ^ 1u);
 						if (!alive)
 							break;
 						ptx::tc_fence_after();
@@ -717,7 +747,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						commit(&sh->xempty[xs_n & 1u]);
 						xs_n++;
 					}
-					commit(&sh->pfull[buf]);
+					commit(&sh->pfull[dset][buf]);
 				}
 			}
 			// the last commits have to land in both CTAs' barriers before either CTA may leave
@@ -731,7 +761,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			uint32_t tl = 0, n = 0, xs_n = 0;
 			bool alive = true;
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 				// one box per super-block: four stages of 64 k x (hi, lo) x the CTA's token rows.  The CTAs of a pair
 				// take the first and the second half of the tile's n_mma columns; all the bytes are counted on
 				// the leader's barrier, whose token loader announces them.
@@ -778,7 +808,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		bool alive = true;
 		int wtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, wtl++) {
-			const TcItem item = tc_item<PAIR>(t, wtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+			const TcItem item = tc_item<PAIR, NT>(t, wtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
 			for (int sbi = 0; sbi < nb; sbi++) {
 				if (wc >= (uint32_t)Sm::NWB && !tc_wait_warp<100>(ptx::smem_u32(&sh->wempty[wb]), wph ^ 1u, abort_flag, status, lane)) {
 					alive = false;
@@ -956,20 +986,24 @@ int tc_setup(tie_cuda_ctx *c)
 				return rc;
 		}
 #define TC_ATTR(KIND, RAW) \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<KIND, false>::SMEM))
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<KIND, false, 64>::SMEM)); \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, false, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
+					     TcSmem<KIND, false, 32>::SMEM));                                                                         \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, false, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
+					     TcSmem<KIND, true, 32>::SMEM))
 	TC_ATTR(W_Q4K, false);
 	TC_ATTR(W_Q4K, true);
 	TC_ATTR(W_Q6K_R8, false);
 	TC_ATTR(W_Q6K_R8, true);
 #undef TC_ATTR
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q4K, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     TcSmem<W_Q4K, false>::SMEM));
+					     TcSmem<W_Q4K, false, 64>::SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q6K_R8, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     TcSmem<W_Q6K_R8, false>::SMEM));
+					     TcSmem<W_Q6K_R8, false, 64>::SMEM));
 	// the CTA-pair forms; how many pairs the device holds at once sizes their (persistent) grids
 #define TC_ATTR_PAIR(KIND, RAW, PEER)                                                                                          \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, PEER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-					     TcSmem<KIND, true>::SMEM));                                                       \
+					     TcSmem<KIND, true, 64>::SMEM));                                                   \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, PEER, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 0))
 	TC_ATTR_PAIR(W_Q4K, false, false);
 	TC_ATTR_PAIR(W_Q4K, true, false);
@@ -982,7 +1016,7 @@ int tc_setup(tie_cuda_ctx *c)
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(c->sm_count & ~1);
 		cfg.blockDim = dim3(TC_THREADS);
-		cfg.dynamicSmemBytes = TcSmem<W_Q4K, true>::SMEM;
+		cfg.dynamicSmemBytes = TcSmem<W_Q4K, true, 64>::SMEM;
 		cudaLaunchAttribute attr[1];
 		attr[0].id = cudaLaunchAttributeClusterDimension;
 		attr[0].val.clusterDim.x = 2;
@@ -1002,7 +1036,7 @@ int tc_setup(tie_cuda_ctx *c)
 }
 
 // arr: 0 = the split inputs x (gate/up), 1 = the split activations h (down).
-template <WKind KIND, bool RAW, bool PEER = false>
+template <WKind KIND, bool RAW, bool PEER = false, int NT = TC_TOKEN_TILE>
 static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1, int arr, float *y, float out_scale,
 		       bool sorted_out = false, const EpDst *dst = nullptr, int dense_rows = 0, const DenseView *view = nullptr)
 {
@@ -1029,7 +1063,7 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(2 * c->tc_pairs);
 		cfg.blockDim = dim3(TC_THREADS);
-		cfg.dynamicSmemBytes = TcSmem<KIND, true>::SMEM;
+		cfg.dynamicSmemBytes = TcSmem<KIND, true, NT>::SMEM;
 		cfg.stream = c->stream;
 		cudaLaunchAttribute attr[1];
 		attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1038,14 +1072,14 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 		attr[0].val.clusterDim.z = 1;
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
-		TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, grouped_gemm_sb<KIND, RAW, PEER, true>, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m,
+		TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m,
 						   (const uint8_t *)t0.ptr, w1p, t0.expert_stride, k_dim, tile_info,
 						   (const int *)s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d,
 						   xqd));
 		c->launches++;
 		return TIE_CUDA_OK;
 	}
-	grouped_gemm_sb<KIND, RAW, PEER><<<c->sm_count, TC_THREADS, TcSmem<KIND, false>::SMEM, c->stream>>>(
+	grouped_gemm_sb<KIND, RAW, PEER, false, NT><<<c->sm_count, TC_THREADS, TcSmem<KIND, false, NT>::SMEM, c->stream>>>(
 		mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p, t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts,
 		m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d, xqd);
 	TIE_CUDA_LAUNCHED(c);
@@ -1063,11 +1097,13 @@ bool tc_supported(const tie_cuda_ctx *c, const Layer &L)
 }
 
 // xs_hi/xs_lo (and xq for Q4_K) must hold the split inputs in sorted order; the sort must
-// have been run with TC_TOKEN_TILE.  Gate and up run as independent 128-row tiles; the raw fp32
+// have been run with n_tile (32 or 64).  Gate and up run as independent 128-row tiles; the raw fp32
 // products go to the scratch s.y as [row][gate | up].
-int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_rows)
+int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile)
 {
-	(void)n_rows;
+	if (n_tile == 32)
+		return (L.gate.kind == W_Q4K) ? launch_tc_t<W_Q4K, true, false, 32>(c, L.gate, &L.up, 0, c->s.y, 1.0f)
+					      : launch_tc_t<W_Q6K_R8, true, false, 32>(c, L.gate, &L.up, 0, c->s.y, 1.0f);
 	return (L.gate.kind == W_Q4K) ? launch_tc_t<W_Q4K, true>(c, L.gate, &L.up, 0, c->s.y, 1.0f)
 				      : launch_tc_t<W_Q6K_R8, true>(c, L.gate, &L.up, 0, c->s.y, 1.0f);
 }
@@ -1081,13 +1117,15 @@ int launch_tc_swiglu(tie_cuda_ctx *c, const Layer &L, int n_rows, const int *n_r
 				   n_rows_dev);
 }
 
-// reads hs_hi/hs_lo; writes y[perm[p]] (sorted_out: y[p]).
-int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_rows, float *y, bool sorted_out)
+// reads hs_hi/hs_lo; writes y[perm[p]].
+int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_tile, float *y)
 {
-	(void)n_rows;
-	if (L.down.kind == W_Q4K)
-		return launch_tc_t<W_Q4K, false>(c, L.down, nullptr, 1, y, 1.0f / TC_H_SCALE, sorted_out);
-	return launch_tc_t<W_Q6K_R8, false>(c, L.down, nullptr, 1, y, 1.0f / TC_H_SCALE, sorted_out);
+	const float scale = 1.0f / TC_H_SCALE;
+	if (n_tile == 32)
+		return L.down.kind == W_Q4K ? launch_tc_t<W_Q4K, false, false, 32>(c, L.down, nullptr, 1, y, scale)
+					    : launch_tc_t<W_Q6K_R8, false, false, 32>(c, L.down, nullptr, 1, y, scale);
+	return L.down.kind == W_Q4K ? launch_tc_t<W_Q4K, false>(c, L.down, nullptr, 1, y, scale)
+				    : launch_tc_t<W_Q6K_R8, false>(c, L.down, nullptr, 1, y, scale);
 }
 
 // A dense tensor (one "expert") on the grouped product: y[p][row] = sum_k w[row][k] x[p][k].  The
@@ -1132,6 +1170,10 @@ int tc_make_dense_view(tie_cuda_ctx *c, DevTensor &t)
 
 int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y)
 {
+	// tiles of 64 rows share a weight tile's expansion; tiles of 32 where those leave SMs idle
+	if ((n_rows + 63) / 64 * (t.rows / TC_BM) <= c->sm_count / 2)
+		return t.kind == W_Q4K ? launch_tc_t<W_Q4K, false, false, 32>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view)
+				       : launch_tc_t<W_Q6K_R8, false, false, 32>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view);
 	return t.kind == W_Q4K ? launch_tc_t<W_Q4K, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view)
 			       : launch_tc_t<W_Q6K_R8, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view);
 }
