@@ -6,10 +6,12 @@
 
 #include <atomic>
 #include <mutex>
+#include <new>
 
 #include "common.cuh"
 #include "ep_dev.cuh"
 #include "kernels.cuh"
+#include "copy_pool.h"
 
 using namespace tie;
 
@@ -46,7 +48,11 @@ int alloc_scratch(tie_cuda_ctx *c)
 	s.rows_cap = R;
 	s.rows_pad = R + 256;
 	TRY(dev_alloc(c, &s.x, T * H));
-	TRY(dev_alloc(c, &s.out, T * H));
+	// the status word lies right in front of the output rows, on the device and in the pinned staging: one copy
+	// brings both to the host
+	TRY(dev_alloc(c, &s.out_base, OUT_PAD + T * H));
+	s.out = s.out_base + OUT_PAD;
+	s.status = reinterpret_cast<unsigned *>(s.out) - 1;
 	TRY(dev_alloc(c, &s.logits, T * E));
 	TRY(dev_alloc(c, &s.bias, E));
 	TRY(dev_alloc(c, &s.topk_idx, R));
@@ -70,7 +76,6 @@ int alloc_scratch(tie_cuda_ctx *c)
 	const size_t XH = xq_cols((int)H), XF = xq_cols((int)F);
 	TRY(dev_alloc(c, &s.xq, s.rows_pad * XH));
 	TRY(dev_alloc(c, &s.hq, s.rows_pad * XF));
-	TRY(dev_alloc(c, &s.status, 1));
 	TRY(dev_alloc(c, &s.route_counter, (T + 3) / 4));
 	TIE_CUDA_TRY(c, cudaMemset(s.route_counter, 0, (T + 3) / 4 * sizeof(int)));
 	TRY(dev_alloc(c, &s.counter, 1));
@@ -95,7 +100,8 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TIE_CUDA_TRY(c, cudaMemset(s.xq, 0, s.rows_pad * XH * sizeof(__half)));
 	TIE_CUDA_TRY(c, cudaMemset(s.hq, 0, s.rows_pad * XF * sizeof(__half)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_x), T * H * sizeof(float)));
-	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_out), T * H * sizeof(float)));
+	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_out_base), (OUT_PAD + T * H) * sizeof(float)));
+	c->pin_out = c->pin_out_base + OUT_PAD;
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_idx), R * sizeof(int)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_w), R * sizeof(float)));
 	TIE_CUDA_TRY(c, cudaMallocHost(reinterpret_cast<void **>(&c->pin_logits), T * E * sizeof(float)));
@@ -431,6 +437,91 @@ size_t align_up(size_t v, size_t a)
 	return (v + a - 1) / a * a;
 }
 
+// Pageable host buffers of a batch: the copies between them and the pinned staging were most of a call (333 tokens:
+// 2.7 MB each way, about 190 us per direction from one thread beside 50 us of DMA and 190 us of kernels).  They are
+// cut in chunks that the caller's thread and a few helper threads copy while the DMA of earlier chunks runs.
+// Below COPY_MIN waking the helpers costs more than the copy.
+constexpr size_t COPY_MIN = 256 << 10;
+
+struct CopyPlan {
+	size_t chunk;
+	int n;
+};
+CopyPlan copy_plan(size_t bytes)
+{
+	size_t chunk = align_up((bytes + COPY_CHUNKS - 1) / COPY_CHUNKS, 4096);
+	if (chunk < (64u << 10))
+		chunk = 64u << 10;
+	return {chunk, (int)((bytes + chunk - 1) / chunk)};
+}
+
+int copy_in_chunks(tie_cuda_ctx *c, const void *x, size_t bytes)
+{
+	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // the previous call's copies out of the staging are done
+	if (!c->copy_pool && !(c->copy_pool = new (std::nothrow) CopyPool()))
+		return TIE_CUDA_ENOMEM;
+	const CopyPlan p = copy_plan(bytes);
+	CopyPool &pool = *c->copy_pool;
+	pool.begin(reinterpret_cast<char *>(c->pin_x), static_cast<const char *>(x), bytes, p.chunk, p.n, p.n);
+	cudaError_t e = cudaSuccess;
+	for (int sent = 0; sent < p.n && e == cudaSuccess;) {
+		int have = sent;
+		while (have < p.n && pool.done(have))
+			have++;
+		if (have == sent) {
+			pool.step();
+			continue;
+		}
+		const size_t o = (size_t)sent * p.chunk, end = have == p.n ? bytes : (size_t)have * p.chunk;
+		e = cudaMemcpyAsync(reinterpret_cast<char *>(c->s.x) + o, reinterpret_cast<char *>(c->pin_x) + o, end - o, cudaMemcpyHostToDevice,
+				    c->stream);
+		sent = have;
+	}
+	pool.end();
+	TIE_CUDA_TRY(c, e);
+	return TIE_CUDA_OK;
+}
+
+// After the kernels have been enqueued: result and status to the host; returns the call's status.
+int copy_out_chunks(tie_cuda_ctx *c, void *out, size_t bytes)
+{
+	const CopyPlan p = copy_plan(bytes);
+	for (int i = 0; i < p.n; i++) {
+		const size_t o = (size_t)i * p.chunk, end = i == p.n - 1 ? bytes : o + p.chunk;
+		if (i == 0)  // (the first chunk brings the status word that lies in front of it)
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->pin_out_base, c->s.out_base, OUT_PAD * sizeof(float) + end, cudaMemcpyDeviceToHost, c->stream));
+		else
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(reinterpret_cast<char *>(c->pin_out) + o, reinterpret_cast<char *>(c->s.out) + o, end - o,
+							cudaMemcpyDeviceToHost, c->stream));
+		if (!c->copy_ev[i])
+			TIE_CUDA_TRY(c, cudaEventCreateWithFlags(&c->copy_ev[i], cudaEventDisableTiming));
+		TIE_CUDA_TRY(c, cudaEventRecord(c->copy_ev[i], c->stream));
+	}
+	TIE_CUDA_TRY(c, cudaEventSynchronize(c->copy_ev[0]));
+	const int rc = report_status(c, *(reinterpret_cast<volatile unsigned *>(c->pin_out) - 1));
+	if (rc)
+		return rc;
+	CopyPool &pool = *c->copy_pool;
+	int landed = 1;
+	pool.begin(static_cast<char *>(out), reinterpret_cast<char *>(c->pin_out), bytes, p.chunk, p.n, landed);
+	cudaError_t e = cudaSuccess;
+	while (landed < p.n) {
+		e = cudaEventQuery(c->copy_ev[landed]);
+		if (e == cudaSuccess) {
+			pool.allow(++landed);
+			continue;
+		}
+		if (e != cudaErrorNotReady)
+			break;
+		pool.step();
+	}
+	while (e == cudaSuccess && pool.step())
+		;
+	pool.end();
+	TIE_CUDA_TRY(c, e == cudaErrorNotReady ? cudaSuccess : e);
+	return TIE_CUDA_OK;
+}
+
 void ep_close_peers(tie_cuda_ctx *c)
 {
 	EpState &ep = c->ep;
@@ -677,14 +768,14 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 		delete[] c->layers;
 	}
 	Scratch &s = c->s;
-	void *dev_ptrs[] = {s.x,     s.out,   s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
-			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.status,  s.counter, s.row_expert, c->silu,  c->row_x,
+	void *dev_ptrs[] = {s.x,     s.out_base, s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
+			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.counter, s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
 			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
 		if (p)
 			cudaFree(p);
-	void *pin_ptrs[] = {c->pin_x, c->pin_out, c->pin_idx, c->pin_w, c->pin_logits, c->pin_status};
+	void *pin_ptrs[] = {c->pin_x, c->pin_out_base, c->pin_idx, c->pin_w, c->pin_logits, c->pin_status};
 	for (void *p : pin_ptrs)
 		if (p)
 			cudaFreeHost(p);
@@ -721,6 +812,10 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	}
 	free(c->regs);
 	ep_release(c);
+	for (cudaEvent_t ev : c->copy_ev)
+		if (ev)
+			cudaEventDestroy(ev);
+	delete c->copy_pool;
 	delete c;
 }
 
@@ -881,26 +976,36 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 	// host pointers: pinned user memory is copied directly, pageable memory goes through the
 	// context's pinned staging buffers
 	const bool x_pinned = is_pinned_host(x), out_pinned = is_pinned_host(out);
+	if (!x_pinned && !out_pinned && bytes >= COPY_MIN) {
+		TRY(copy_in_chunks(c, x, bytes));
+		GraphKey k = {1, layer, n_tokens, c->s.x, c->s.out, bias_dev, nullptr, kflags | TIE_CUDA_DEVICE};
+		TRY(run_maybe_graphed(c, graph, k, [&]() { return moe_ffn_device(c, *L, c->s.x, c->s.out, n_tokens, bias_dev, nullptr, flags); }));
+		return copy_out_chunks(c, out, bytes);
+	}
 	const void *src = x;
-	void *dst = out;
 	if (!x_pinned) {
 		TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
 		memcpy(c->pin_x, x, bytes);
 		src = c->pin_x;
 	}
-	if (!out_pinned)
-		dst = c->pin_out;
-	GraphKey k = {2, layer, n_tokens, src, dst, bias_dev, nullptr, kflags};
+	GraphKey k = {2, layer, n_tokens, src, out_pinned ? out : c->pin_out, bias_dev, nullptr, kflags};
 	TRY(run_maybe_graphed(c, graph, k, [&]() -> int {
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(c->s.x, src, bytes, cudaMemcpyHostToDevice, c->stream));
 		TRY(moe_ffn_device(c, *L, c->s.x, c->s.out, n_tokens, bias_dev, nullptr, flags));
-		TIE_CUDA_TRY(c, cudaMemcpyAsync(dst, c->s.out, bytes, cudaMemcpyDeviceToHost, c->stream));
-		TIE_CUDA_TRY(c, cudaMemcpyAsync(c->pin_status, c->s.status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+		if (out_pinned) {
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(out, c->s.out, bytes, cudaMemcpyDeviceToHost, c->stream));
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->pin_status, c->s.status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+		} else {
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->pin_out_base, c->s.out_base, OUT_PAD * sizeof(float) + bytes, cudaMemcpyDeviceToHost,
+							c->stream));
+		}
 		return TIE_CUDA_OK;
 	}));
-	TRY(check_status_pinned(c));
-	if (!out_pinned)
-		memcpy(out, c->pin_out, bytes);
+	if (out_pinned)
+		return check_status_pinned(c);
+	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+	TRY(report_status(c, *(reinterpret_cast<volatile unsigned *>(c->pin_out) - 1)));
+	memcpy(out, c->pin_out, bytes);
 	return TIE_CUDA_OK;
 }
 

@@ -20,6 +20,10 @@ constexpr int MAX_TOP_K = 8;
 constexpr int TC_TOKEN_TILE = 64;  // rows of one expert per token tile of the tensor-core path (or 32: run_experts)
 constexpr int SILU_N = TIE_CUDA_SILU_TABLE_SIZE;
 constexpr int SORT_SLICE = 256;   // rows per CTA of the dispatch sort
+constexpr int OUT_PAD = 64;	  // floats in front of the output rows: the status word is the last of them
+constexpr int COPY_CHUNKS = 16;	  // pageable host batches are copied in at most this many chunks
+
+class CopyPool;	 // copy_pool.h
 
 // Device status word bits (set by kernels instead of trapping).
 constexpr unsigned ST_BAD_EXPERT = 1u;	  // expert id outside this context's range
@@ -72,6 +76,7 @@ struct DfLayer {
 // Scratch arena of one context, sized for max_tokens.
 struct Scratch {
 	float *x = nullptr;	    // [T][H]   staged input (host mode) / normed input (block mode)
+	float *out_base = nullptr;  // [OUT_PAD + T*H]: the status word, then out
 	float *out = nullptr;	    // [T][H]   staged output
 	float *logits = nullptr;    // [T][E]
 	float *bias = nullptr;	    // [E]
@@ -93,7 +98,7 @@ struct Scratch {
 	// sums of the rows above over 32-wide sub-blocks, split the same way; 64 columns per 2048 k
 	__half *xq = nullptr;  // [Rpad][xq_cols(H)]
 	__half *hq = nullptr;  // [Rpad][xq_cols(F)]
-	unsigned *status = nullptr;		    // [1]
+	unsigned *status = nullptr;		    // [1], the word in front of out
 	int *route_counter = nullptr;		    // [(T + 3) / 4] CTAs done per token tile of the batched router (zero at rest)
 	int *counter = nullptr;			    // [1] last-CTA counter of the fused decode router (zero at rest)
 	unsigned *dec_sync = nullptr;		    // [2] arrivals and epoch of the one-kernel decode step's grid barriers
@@ -153,7 +158,9 @@ struct tie_cuda_ctx {
 	tie::Scratch s;
 	int first_expert = 0, n_local = 0;
 	// pinned staging for host-pointer calls
-	float *pin_x = nullptr, *pin_out = nullptr;
+	float *pin_x = nullptr, *pin_out_base = nullptr, *pin_out = nullptr;  // (pin_out_base: as Scratch::out_base)
+	tie::CopyPool *copy_pool = nullptr;	    // helper threads for pageable batches, started at the first one
+	cudaEvent_t copy_ev[tie::COPY_CHUNKS] = {nullptr};
 	int *pin_idx = nullptr;
 	float *pin_w = nullptr, *pin_logits = nullptr;
 	unsigned *pin_status = nullptr;
