@@ -269,7 +269,7 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	} else if (path == TIE_CUDA_PATH_STREAM) {
 		use_tc = false;
 	} else {
-		use_tc = tc_supported(c, L) && n_rows >= 2 * c->n_local;
+		use_tc = tc_supported(c, L) && 2 * n_rows > c->n_local;  // (below: decode_supported, decode.cu)
 	}
 	c->tc_no_pair = (flags & TIE_CUDA_PATH_NO_PAIR) != 0;
 	const int direct = (!use_tc && n_rows <= c->cfg.top_k && src_div == c->cfg.top_k) ? 1 : 0;

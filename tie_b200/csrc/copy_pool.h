@@ -1,11 +1,13 @@
 // A few threads that copy memory in chunks beside the calling thread: what tie_cuda_moe_ffn moves between pageable
-// host buffers and the pinned staging.  One owner (the context's calling thread) at a time; the helpers sleep
-// between copies.
+// host buffers and the pinned staging.  One owner (the context's calling thread) at a time; after a copy the
+// helpers stay awake for SPIN_US (a call copies in, computes, copies out: waking a sleeping thread costs as much as
+// copying a chunk), then sleep.
 #pragma once
 
 #include <string.h>
 
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <mutex>
 #include <thread>
@@ -13,12 +15,12 @@
 namespace tie {
 
 class CopyPool {
-	static constexpr int MAX_CHUNKS = 64, MAX_HELPERS = 3;
+	static constexpr int MAX_CHUNKS = 64, MAX_HELPERS = 3, SPIN_US = 400;
 	std::mutex mutex_;
 	std::condition_variable wake_, idle_;
 	std::thread helpers_[MAX_HELPERS];
 	int n_helpers_ = 0, inside_ = 0;  // helpers inside the current job (under mutex_)
-	uint64_t job_ = 0;		  // (under mutex_)
+	std::atomic<uint64_t> job_{0};	  // (written under mutex_)
 	bool open_ = false, quit_ = false;
 	char *dst_ = nullptr;
 	const char *src_ = nullptr;
@@ -32,10 +34,17 @@ class CopyPool {
 		uint64_t seen = 0;
 		std::unique_lock<std::mutex> lk(mutex_);
 		for (;;) {
-			wake_.wait(lk, [&] { return quit_ || (open_ && job_ != seen); });
+			if (seen) {
+				lk.unlock();
+				const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(SPIN_US);
+				while (job_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until)
+					std::this_thread::yield();
+				lk.lock();
+			}
+			wake_.wait(lk, [&] { return quit_ || (open_ && job_.load(std::memory_order_relaxed) != seen); });
 			if (quit_)
 				return;
-			seen = job_;
+			seen = job_.load(std::memory_order_relaxed);
 			inside_++;
 			lk.unlock();
 			while (left_.load(std::memory_order_acquire) > 0)
@@ -90,7 +99,7 @@ public:
 			allowed_.store(allowed, std::memory_order_relaxed);
 			left_.store(n, std::memory_order_release);
 			open_ = true;
-			job_++;
+			job_.fetch_add(1, std::memory_order_release);
 		}
 		wake_.notify_all();
 	}

@@ -197,14 +197,15 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 			}
 		}
 	}
-	__threadfence();
 	__syncthreads();
-	if (threadIdx.x == 0)
+	if (threadIdx.x == 0) {	 // (one fence for the CTA: the barrier has ordered its stores before this thread)
+		__threadfence();
 		s_last = atomicAdd(counter + blockIdx.x, 1) == n_expert / TE - 1;
+		__threadfence();
+	}
 	__syncthreads();
 	if (!s_last)
 		return;
-	__threadfence();
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	// (a warp's tokens are selected for together, up to four at a time: one after the other they are a chain of
 	// reductions of a microsecond each)
