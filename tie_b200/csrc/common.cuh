@@ -324,49 +324,4 @@ __host__ __device__ __forceinline__ size_t q6k_r8_d_off(int nb, int r8, int b)
 	return (size_t)8 * nb * Q6K_RECORD + (size_t)(r8 * nb + b) * 2;
 }
 
-// Programmatic dependent launch: a kernel launched with the attribute may start while its
-// predecessor still runs; pdl_wait() blocks until the predecessor's memory is visible,
-// pdl_trigger() lets the successor start.  Both are no-ops in an ordinary launch.
-__device__ __forceinline__ void pdl_wait()
-{
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_trigger()
-{
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-// The kernels of a call form a chain of such launches: each waits before its first access to memory that
-// another kernel writes or reads, and only then lets its successor start (so at most one successor is
-// resident early, and every CTA of a kernel has started before any of its successor's).  A small batch's chain of
-// nine kernels spends about a microsecond less per boundary.
-template <class... P, class... A>
-int launch_pdl_cluster(tie_cuda_ctx *c, int cluster, void (*kern)(P...), dim3 grid, int threads, size_t smem, const A &...args)
-{
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = grid;
-	cfg.blockDim = dim3(threads);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = c->stream;
-	cudaLaunchAttribute attr[2];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	if (cluster > 1) {
-		attr[1].id = cudaLaunchAttributeClusterDimension;
-		attr[1].val.clusterDim.x = cluster;
-		attr[1].val.clusterDim.y = 1;
-		attr[1].val.clusterDim.z = 1;
-		cfg.numAttrs = 2;
-	}
-	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
-	c->launches++;
-	return TIE_CUDA_OK;
-}
-template <class... P, class... A>
-int launch_pdl(tie_cuda_ctx *c, void (*kern)(P...), dim3 grid, int threads, size_t smem, const A &...args)
-{
-	return launch_pdl_cluster(c, 1, kern, grid, threads, smem, args...);
-}
-
 }  // namespace tie

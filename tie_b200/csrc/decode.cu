@@ -253,6 +253,24 @@ bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 	       dec_down_smem(L, c->cfg.top_k) <= (size_t)DEC_MAX_SMEM;
 }
 
+template <class... P, class... A>
+static int launch_pdl(tie_cuda_ctx *c, void (*kern)(P...), dim3 grid, int threads, size_t smem, A... args)
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = dim3(threads);
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = c->stream;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	attr[0].val.programmaticStreamSerializationAllowed = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+	c->launches++;
+	return TIE_CUDA_OK;
+}
+
 // Opt-in shared-memory sizes, once per context.
 int decode_setup(tie_cuda_ctx *c)
 {

@@ -11,8 +11,6 @@ namespace tie {
 __global__ void __launch_bounds__(128) rms_norm_rows(const float *__restrict__ x, const float *__restrict__ w,
 						     float *__restrict__ o, int n_tokens, int n, float eps)
 {
-	pdl_wait();
-	pdl_trigger();
 	extern __shared__ float sm[];
 	const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int t = blockIdx.x * (blockDim.x >> 5) + wib;
@@ -48,8 +46,6 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 						    int hidden, const float *__restrict__ residual, float *__restrict__ out,
 						    const int *__restrict__ pos)
 {
-	pdl_wait();
-	pdl_trigger();
 	const int t = blockIdx.x;
 	float wj[MAX_TOP_K];
 	size_t yrow[MAX_TOP_K];
@@ -126,8 +122,6 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__res
 							      int n_rows, int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
 							      __half *__restrict__ xq, int q_cols)
 {
-	pdl_wait();
-	pdl_trigger();
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int upr = (n_cols + 1023) >> 10;	// units of 1024 columns per row
 	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_rows * upr; un += gridDim.x * ROWS_WARPS) {
@@ -198,8 +192,6 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float
 	for (int i = threadIdx.x; i < SILU_N / 4; i += blockDim.x)
 		reinterpret_cast<float4 *>(tab)[i] = __ldg(reinterpret_cast<const float4 *>(silu) + i);
 	__syncthreads();
-	pdl_wait();  // (the table above is constant)
-	pdl_trigger();
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const size_t n_rows = n_rows_dev ? (size_t)*n_rows_dev : (size_t)n_rows_host;
 	const size_t upr = (size_t)(ffn >> 8);
@@ -242,13 +234,17 @@ int launch_rms_norm(tie_cuda_ctx *c, const float *x, const float *w, float *o, i
 	size_t smem = (size_t)wpb * H * sizeof(float);
 	if (smem > 48 * 1024)  // the kernel runs within the default dynamic shared-memory limit
 		return TIE_CUDA_ENOTSUP;
-	return launch_pdl(c, rms_norm_rows, dim3((n_tokens + wpb - 1) / wpb), wpb * 32, smem, x, w, o, n_tokens, H, c->cfg.norm_eps);
+	rms_norm_rows<<<(n_tokens + wpb - 1) / wpb, wpb * 32, smem, c->stream>>>(x, w, o, n_tokens, H, c->cfg.norm_eps);
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_tokens, const float *residual, float *out,
 		   const int *pos)
 {
-	return launch_pdl(c, combine_rows, dim3(n_tokens), 256, 0, y, topk_w, c->cfg.top_k, c->cfg.hidden, residual, out, pos);
+	combine_rows<<<n_tokens, 256, 0, c->stream>>>(y, topk_w, c->cfg.top_k, c->cfg.hidden, residual, out, pos);
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_div, int n_rows, int n_cols, __half *hi,
@@ -259,8 +255,10 @@ int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_
 	const int want = (n_rows * ((n_cols + 1023) / 1024) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 8;
 	if (n_rows <= 0)
 		return TIE_CUDA_OK;
-	return launch_pdl(c, split_rows, dim3(want < cap ? want : cap), ROWS_WARPS * 32, 0, x, perm, src_div, n_rows, n_cols, hi, lo, xq,
-			  xq_cols(n_cols));
+	split_rows<<<want < cap ? want : cap, ROWS_WARPS * 32, 0, c->stream>>>(x, perm, src_div, n_rows, n_cols, hi, lo, xq,
+										xq_cols(n_cols));
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, const int *perm, int src_div, int n_rows,
@@ -279,8 +277,10 @@ int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, f
 	// (n_rows_dev: the row count is read on the device and n_rows is the grid the caller wants)
 	const int want = (n_rows * (ffn / 256) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 4;
 	const int grid = n_rows_dev ? n_rows : (want < cap ? want : cap);
-	return launch_pdl(c, swiglu_split_rows, dim3(grid > 0 ? grid : 1), ROWS_WARPS * 32, 0, gu, ffn, scale, c->silu, hi, lo, xq,
-			  xq_cols(ffn), n_rows_dev, n_rows);
+	swiglu_split_rows<<<grid > 0 ? grid : 1, ROWS_WARPS * 32, 0, c->stream>>>(gu, ffn, scale, c->silu, hi, lo, xq, xq_cols(ffn),
+										   n_rows_dev, n_rows);
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_swiglu(tie_cuda_ctx *c, float *gate, const float *up, int n)

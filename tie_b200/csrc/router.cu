@@ -105,8 +105,6 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 	     int n_tokens, int hidden, int n_expert, int top_k, int *__restrict__ topk_idx, float *__restrict__ topk_w, int lfm2,
 	     const float *__restrict__ sel_bias, int *__restrict__ counter, const EpPush push)
 {
-	pdl_wait();
-	pdl_trigger();
 	constexpr int TPT = C::TPT, EPT = C::EPT, TT = C::TT, TE = C::TE, KC = C::KC;
 	extern __shared__ __align__(16) float rsm[];
 	__shared__ int s_last;
@@ -402,12 +400,13 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 		using C = __VA_ARGS__;                                                                                               \
 		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                                    \
 		f.n_ctas = rt_push_ctas(c, grid.x * (E / C::TE), grid.x * RT_PUSH_ROWS);                                             \
-		return launch_pdl(c, router_batch<C>, grid, C::THREADS, C::SMEM, x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2,   \
-				  sel_bias, c->s.route_counter, f);                                                                  \
+		router_batch<C><<<grid, C::THREADS, C::SMEM, c->stream>>>(x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2, \
+									  sel_bias, c->s.route_counter, f);                          \
 	}
 	TIE_RT_TILES(TIE_RT_RUN)
 #undef TIE_RT_RUN
-	return TIE_CUDA_ENOTSUP;
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_router_decode_fused(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,

@@ -58,8 +58,6 @@ __device__ __forceinline__ int sort_my_row(const int *__restrict__ row_expert, i
 __global__ void __launch_bounds__(SORT_THREADS) sort_hist(const int *__restrict__ row_expert, int n_rows, int first_expert,
 							  int n_local, int *__restrict__ hist, unsigned *__restrict__ status)
 {
-	pdl_wait();
-	pdl_trigger();
 	__shared__ int cnt[SORT_WARPS][SORT_MAX_E];
 	unsigned same;
 	sort_my_row(row_expert, n_rows, first_expert, n_local, cnt, same, status);
@@ -79,8 +77,6 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_scatter(const int *__restri
 							     int *__restrict__ active, int *__restrict__ n_active, int *__restrict__ perm,
 							     int4 *__restrict__ tile_info, int *__restrict__ inv, int owner_div, int top_k)
 {
-	pdl_wait();
-	pdl_trigger();
 	__shared__ int cnt[SORT_WARPS][SORT_MAX_E];  // rows of expert e in warp w's 32 rows; then: where they start
 	__shared__ int wsum[3][SORT_WARPS];
 	unsigned same;
@@ -181,8 +177,6 @@ __global__ void __launch_bounds__(SORT_SMALL) sort_small(const int *__restrict__
 							 int *__restrict__ tile_start, int *__restrict__ active, int *__restrict__ n_active,
 							 int *__restrict__ perm, int4 *__restrict__ tile_info, unsigned *__restrict__ status)
 {
-	pdl_wait();
-	pdl_trigger();
 	__shared__ short cnt[SORT_SMALL / 32][SORT_MAX_E];  // rows of expert e in warp w's 32 rows; then: rows before warp w
 	__shared__ int start[SORT_MAX_E];
 	__shared__ int wsum[3][SORT_WARPS];
@@ -272,19 +266,21 @@ int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, 
 		return TIE_CUDA_ENOTSUP;
 	if (n_rows <= SORT_SMALL && !b.inv && !b.owner_div) {
 		const int threads = n_rows <= SORT_MAX_E ? SORT_MAX_E : (n_rows + 31) / 32 * 32;
-		return launch_pdl(c, sort_small, dim3(1), threads, 0, row_expert, n_rows, first_expert, n_expert, n_tile, b.counts, b.offsets,
-				  b.tile_start, b.active, b.n_active, b.perm, b.tile_info, c->s.status);
+		sort_small<<<1, threads, 0, c->stream>>>(row_expert, n_rows, first_expert, n_expert, n_tile, b.counts, b.offsets, b.tile_start,
+							 b.active, b.n_active, b.perm, b.tile_info, c->s.status);
+		TIE_CUDA_LAUNCHED(c);
+		return TIE_CUDA_OK;
 	}
 	const int n_slices = n_rows > 0 ? (n_rows + SORT_SLICE - 1) / SORT_SLICE : 1;  // (no rows: one CTA writes the empty tables)
 	if ((size_t)n_slices * n_expert > c->s.sort_hist_cap)
 		return TIE_CUDA_EINVAL;
-	int rc = launch_pdl(c, sort_hist, dim3(n_slices), SORT_THREADS, 0, row_expert, n_rows, first_expert, n_expert, c->s.sort_hist,
-			    c->s.status);
-	if (rc)
-		return rc;
-	return launch_pdl(c, sort_scatter, dim3(n_slices), SORT_THREADS, 0, row_expert, n_rows, first_expert, n_expert, c->s.sort_hist, n_tile,
-			  b.counts, b.offsets, b.tile_start, b.active, b.n_active, b.perm, b.tile_info, b.inv, b.top_k > 0 ? b.owner_div : 0,
-			  b.top_k);
+	sort_hist<<<n_slices, SORT_THREADS, 0, c->stream>>>(row_expert, n_rows, first_expert, n_expert, c->s.sort_hist, c->s.status);
+	TIE_CUDA_LAUNCHED(c);
+	sort_scatter<<<n_slices, SORT_THREADS, 0, c->stream>>>(row_expert, n_rows, first_expert, n_expert, c->s.sort_hist, n_tile, b.counts,
+								b.offsets, b.tile_start, b.active, b.n_active, b.perm, b.tile_info, b.inv,
+								b.top_k > 0 ? b.owner_div : 0, b.top_k);
+	TIE_CUDA_LAUNCHED(c);
+	return TIE_CUDA_OK;
 }
 
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile)
