@@ -253,24 +253,6 @@ bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 	       dec_down_smem(L, c->cfg.top_k) <= (size_t)DEC_MAX_SMEM;
 }
 
-template <class... P, class... A>
-static int launch_pdl(tie_cuda_ctx *c, void (*kern)(P...), dim3 grid, int threads, size_t smem, A... args)
-{
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = grid;
-	cfg.blockDim = dim3(threads);
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = c->stream;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
-	c->launches++;
-	return TIE_CUDA_OK;
-}
-
 // Opt-in shared-memory sizes, once per context.
 int decode_setup(tie_cuda_ctx *c)
 {
@@ -286,7 +268,7 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 {
 	const int n_rows = n_tokens * c->cfg.top_k, nb = L.gate.k / QK_K;
 	auto kern = L.gate.kind == W_Q4K ? decode_gate_up<W_Q4K> : decode_gate_up<W_Q6K_R8>;
-	return launch_pdl(c, kern, dim3(L.gate.rows / 16, n_rows), 32 * nb, 0, L.gate.ptr, L.up.ptr, L.gate.expert_stride, L.gate.rows, nb, x,
+	return launch_kernel(c, true, 1, kern, dim3(L.gate.rows / 16, n_rows), 32 * nb, 0, L.gate.ptr, L.up.ptr, L.gate.expert_stride, L.gate.rows, nb, x,
 			  c->cfg.top_k, c->s.topk_idx, c->s.h, c->first_expert, c->n_local, c->silu, c->s.status,
 			  foreign_slots_ok ? c->cfg.n_expert : 0);
 }
@@ -296,7 +278,7 @@ int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, co
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
 	auto kern = L.down.kind == W_Q4K ? decode_down_combine<W_Q4K> : decode_down_combine<W_Q6K_R8>;
-	return launch_pdl(c, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
+	return launch_kernel(c, true, 1, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
 			  L.down.rows, nb, c->s.h, top_k, c->s.topk_idx, c->s.topk_w, residual, out, c->first_expert, c->n_local, c->s.status);
 }
 
@@ -305,7 +287,7 @@ int launch_decode_down_peer(tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
 	auto kern = L.down.kind == W_Q4K ? decode_down_peer<W_Q4K> : decode_down_peer<W_Q6K_R8>;
-	return launch_pdl(c, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
+	return launch_kernel(c, true, 1, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
 			  L.down.rows, nb, c->s.h, top_k, c->s.topk_idx, c->ep.view, c->ep.step_dev, c->ep.wait_cycles, c->first_expert,
 			  c->n_local, c->s.status);
 }

@@ -41,16 +41,4 @@ __host__ __device__ __forceinline__ size_t tile_offset(int nb, int r0)
 	return KIND == W_Q4K ? (size_t)r0 * nb * Q4K_BYTES : (size_t)(r0 >> 3) * q6k_r8_group_bytes(nb);
 }
 
-// Programmatic dependent launch: a kernel launched with the attribute may start while its
-// predecessor still runs; pdl_wait() blocks until the predecessor's memory is visible,
-// pdl_trigger() lets the successor start.  Both are no-ops in an ordinary launch.
-__device__ __forceinline__ void pdl_wait()
-{
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_trigger()
-{
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 }  // namespace tie

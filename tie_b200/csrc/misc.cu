@@ -122,6 +122,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__res
 							      int n_rows, int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
 							      __half *__restrict__ xq, int q_cols)
 {
+	pdl_trigger();	// (a dense product launched behind this pass sets itself up meanwhile)
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int upr = (n_cols + 1023) >> 10;	// units of 1024 columns per row
 	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_rows * upr; un += gridDim.x * ROWS_WARPS) {

@@ -367,18 +367,6 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	const int walker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
 	const int stride_t = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 	const int m_items = PAIR ? m_tiles / 2 : m_tiles;
-	if (threadIdx.x == 0)
-		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
-	__syncthreads();
-	// (a CTA of a pair never returns early: its peer would wait for it at the cluster barrier below)
-	const int total = s_total;
-	if (!PAIR && walker >= total)
-		return;
-	if (threadIdx.x < TC_ITEMS) {
-		const int t = walker + threadIdx.x * stride_t;
-		if (t < total)
-			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
-	}
 	const int nb = k_dim / QK_K;
 
 	const uint32_t raw = ptx::smem_u32(smem_raw);
@@ -446,7 +434,17 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		if (RAW)
 			ptx::prefetch_tmap(&tw1);
 	}
+	pdl_wait();  // what the kernels before this one wrote is visible from here on
+	if (threadIdx.x == 0)
+		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
 	ptx::tc_fence_before();
+	__syncthreads();
+	const int total = s_total;  // (a CTA without work items goes through the motions: it holds tensor memory, its peer waits for it)
+	if (threadIdx.x < TC_ITEMS) {
+		const int t = walker + threadIdx.x * stride_t;
+		if (t < total)
+			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
+	}
 	__syncthreads();
 	if (PAIR)
 		ptx::cluster_sync_all();  // both CTAs' barriers are initialised before either signals the other's
@@ -1059,31 +1057,17 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	// least 4 super-blocks.  Measured at 64 / 512 / 4096 tokens: rows of 8 super-blocks (gate/up) 68 / 79 / 355 us
 	// paired, 70 / 92 / 410 single (a pair fetches half the token bytes per CTA); rows of 3 (down) 59 / 73 / 310
 	// paired, 55 / 70 / 294 single (the hand-offs between two SMs are not amortised over so few).
+	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles : 1 << 30;	// (known for a dense tensor: no idle CTAs)
 	if (c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K) {
-		cudaLaunchConfig_t cfg = {};
-		cfg.gridDim = dim3(2 * c->tc_pairs);
-		cfg.blockDim = dim3(TC_THREADS);
-		cfg.dynamicSmemBytes = TcSmem<KIND, true, NT>::SMEM;
-		cfg.stream = c->stream;
-		cudaLaunchAttribute attr[1];
-		attr[0].id = cudaLaunchAttributeClusterDimension;
-		attr[0].val.clusterDim.x = 2;
-		attr[0].val.clusterDim.y = 1;
-		attr[0].val.clusterDim.z = 1;
-		cfg.attrs = attr;
-		cfg.numAttrs = 1;
-		TIE_CUDA_TRY(c, cudaLaunchKernelEx(&cfg, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m,
-						   (const uint8_t *)t0.ptr, w1p, t0.expert_stride, k_dim, tile_info,
-						   (const int *)s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d,
-						   xqd));
-		c->launches++;
-		return TIE_CUDA_OK;
+		return launch_kernel(c, dense_rows > 0, 2, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
+				     TcSmem<KIND, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
+				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
+				     s.status, t0.rows, d, xqd);
 	}
-	grouped_gemm_sb<KIND, RAW, PEER, false, NT><<<c->sm_count, TC_THREADS, TcSmem<KIND, false, NT>::SMEM, c->stream>>>(
-		mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p, t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts,
-		m_tiles, y, perm, out_stride, out_scale, s.status, t0.rows, d, xqd);
-	TIE_CUDA_LAUNCHED(c);
-	return TIE_CUDA_OK;
+	return launch_kernel(c, dense_rows > 0, 1, grouped_gemm_sb<KIND, RAW, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
+			     TcSmem<KIND, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
+			     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status,
+			     t0.rows, d, xqd);
 }
 
 static bool tc_tensor_ok(const DevTensor &t)
