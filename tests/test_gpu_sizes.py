@@ -1,0 +1,128 @@
+"""Sizes where one form of a kernel hands over to another, or where a tile has a remainder: token
+tiles of the router, of the grouped products and of the dispatch sort, the step from the per-row
+decode kernels to the grouped ones, and the copies of pageable host buffers.  Against the CPU
+restatement, or bit for bit against another route to the same kernels.
+"""
+import numpy as np
+import pytest
+
+from tie_b200 import synth, workloads
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-3
+
+
+def bits(a):
+    return np.ascontiguousarray(a, dtype=np.float32).view(np.uint32)
+
+
+@pytest.fixture(scope="module")
+def be(layer0, ref_silu_table):
+    from tie_b200 import moe
+    b = moe.MoeBackend(max_tokens=1100, silu_table=ref_silu_table)
+    b.upload_layer(0, layer0, keep_host=True)
+    yield b
+    b.close()
+
+
+@pytest.fixture(scope="module")
+def port0(port_lib, layer0, ref_silu_table):
+    return port_lib.PortMoe(layer0, silu=ref_silu_table)
+
+
+# The smaller expert shape of the grouped products: 4 super-blocks per gate / up row (pairs of CTAs), 1 per
+# down row; Q6_K down, and the same with all three tensors as Q4_K.
+@pytest.fixture(scope="module", params=["q6k_down", "q4k_down"])
+def grouped(request, port_lib, ref_silu_table):
+    from tie_b200 import moe
+    s = synth.MoeShape(hidden=1024, n_expert=32, top_k=4, ffn_dim=256)
+    layer = synth.make_layer(workloads.BASE_SEED + 5, s)
+    if request.param == "q4k_down":
+        n_down = s.n_expert * s.hidden * (s.ffn_dim // 256)
+        layer = synth.MoeLayer(s, layer.router_w, layer.gate, layer.up, synth.q4k_blocks(5, synth.STREAM_DOWN, n_down),
+                               gate_type=synth.GGML_Q4_K, up_type=synth.GGML_Q4_K, down_type=synth.GGML_Q4_K)
+    b = moe.MoeBackend(hidden=s.hidden, n_expert=s.n_expert, top_k=s.top_k, ffn_dim=s.ffn_dim, max_tokens=512, silu_table=ref_silu_table)
+    b.upload_layer(0, layer, keep_host=True)
+    yield b, port_lib.PortMoe(layer, silu=ref_silu_table), s
+    b.close()
+
+
+# A tile of the batched router is 4, 8, 16, 32 or 64 tokens wide, by how many CTAs the batch makes.
+@pytest.mark.parametrize("n_tokens", [5, 13, 31, 33, 65, 129, 257, 511, 1023, 1100])
+def test_router_tiles_and_both_selections(be, port0, n_tokens):
+    x = synth.make_x(0, n_tokens, first_token=7)
+    idx, w, logits = be.route(0, x)
+    i_r, w_r, l_r = port0.route(x)
+    assert np.array_equal(bits(logits), bits(l_r)) and np.array_equal(idx, i_r)
+    assert np.abs(w - w_r).max() <= 2e-7
+    idx, w, _ = be.route(0, x, lfm2=True)
+    i_r, w_r, _ = port0.route_lfm2(x)
+    assert np.array_equal(idx, i_r)
+    assert np.abs(w / w_r - 1).max() < 2e-6
+
+
+# 8 tokens are the last batch of the per-row kernels with 128 experts and top-8.
+@pytest.mark.parametrize("n_tokens", [6, 8, 9, 12])
+def test_per_row_and_grouped_products_around_the_change(be, port0, n_tokens):
+    x = synth.make_x(0, n_tokens, first_token=90)
+    ref, ref_idx, _ = port0.moe_ffn(x)
+    out = be.moe_ffn(0, x)
+    assert workloads.rel_rms_err(out, ref).max() < (1e-5 if n_tokens <= 8 else TOL)
+    assert be.last_active_experts() == len(np.unique(ref_idx))
+
+
+# Rows per expert at the edges of 16-, 32- and 64-row tiles: tiles of 32 up to 24 rows an expert on average, of 64
+# above; the dispatch sort is one CTA up to 1024 rows.
+_EDGES = [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65]
+
+
+@pytest.mark.parametrize("flags", [0, "no_pair"])
+@pytest.mark.parametrize("counts", [_EDGES, _EDGES + [48] * 9, _EDGES + [127, 128, 129, 1, 47], [32] * 32, [32] * 31 + [31], [32] * 31 + [33]],
+                         ids=["337rows", "769rows", "769rows_wide", "1024rows", "1023rows", "1025rows"])
+def test_grouped_tile_edges(grouped, counts, flags):
+    import torch
+    from tie_b200 import moe
+    b, port, s = grouped
+    row_expert = np.repeat(np.arange(len(counts), dtype=np.int32), counts)
+    row_expert = row_expert[np.random.default_rng(11).permutation(row_expert.size)]
+    rows = synth.make_x(13, row_expert.size, s.hidden)
+    ref = port.expert_rows(rows, row_expert)
+    x, e = torch.from_numpy(rows).cuda(), torch.from_numpy(row_expert).cuda()
+    y = torch.full_like(x, float("nan"))
+    b.expert_rows_ptr(0, x, e, row_expert.size, y, moe.DEVICE | moe.PATH_TENSOR | (moe.PATH_NO_PAIR if flags else 0))
+    assert workloads.rel_rms_err(y.cpu().numpy(), ref).max() < TOL
+
+
+# One registered tensor: its batch in tiles of 64, or of 32 where 64 leave SMs idle; Q4_K rows beyond 2048 inputs
+# (9 super-blocks: a second segment of the input sums).
+@pytest.mark.parametrize("ggml_type,in_dim,out_dim", [(12, 2304, 256), (14, 512, 256), (12, 256, 9472)])
+@pytest.mark.parametrize("batch", [1, 32, 33, 64, 65, 129])
+def test_dense_batches(be, port_lib, ggml_type, in_dim, out_dim, batch):
+    nb = out_dim * (in_dim // 256)
+    w = np.ascontiguousarray(synth.q4k_blocks(78, 9, nb) if ggml_type == 12 else synth.q6k_blocks(78, 9, nb))
+    be.register_tensor(w, ggml_type, in_dim)
+    x = synth.make_x(4, batch, in_dim)
+    rows = sorted({0, batch // 2, batch - 1, min(31, batch - 1), min(32, batch - 1)})
+    ref = np.stack([port_lib.mat_vec(x[i], w, ggml_type, in_dim, out_dim) for i in rows])
+    got = be.mat_mat(w, x, np.full((batch, out_dim), np.nan, dtype=np.float32), batch, in_dim, out_dim)
+    scale = np.sqrt((ref.astype(np.float64) ** 2).mean(axis=1, keepdims=True))
+    assert (np.abs(got[rows] - ref) / scale).max() < TOL
+    assert np.isfinite(got).all()
+
+
+# Pageable buffers of 256 KB (32 tokens) and more go through the chunked copies; pinned ones do not.
+@pytest.mark.parametrize("n_tokens", [1, 31, 32, 33, 333])
+@pytest.mark.parametrize("pinned", [(False, False), (True, False), (False, True), (True, True)])
+def test_host_buffers_pageable_and_pinned(be, n_tokens, pinned):
+    import torch
+    from tie_b200 import moe
+    x = torch.from_numpy(synth.make_x(0, n_tokens, first_token=400))
+    want = torch.empty(n_tokens, 2048, device="cuda")
+    be.moe_ffn_ptr(0, x.cuda(), want, n_tokens, moe.DEVICE)
+    xh = x.pin_memory() if pinned[0] else x
+    out = torch.full((n_tokens, 2048), float("nan"), pin_memory=pinned[1])
+    for _ in range(2):
+        be.moe_ffn_ptr(0, xh, out, n_tokens, moe.HOST)
+        assert np.array_equal(bits(out.numpy()), bits(want.cpu().numpy()))
+        out.fill_(float("nan"))

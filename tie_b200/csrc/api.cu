@@ -714,9 +714,6 @@ int tie_cuda_init(tie_cuda_ctx **out, const tie_cuda_config *cfg)
 	c->layers = new (std::nothrow) Layer[cfg->n_layers];
 	if (!c->layers)
 		return fail(TIE_CUDA_ENOMEM);
-	if (cudaMalloc(reinterpret_cast<void **>(&c->df_table), sizeof(DfLayer) * cfg->n_layers) != cudaSuccess ||
-	    cudaMemset(c->df_table, 0, sizeof(DfLayer) * cfg->n_layers) != cudaSuccess)
-		return fail(TIE_CUDA_ENOMEM);
 	float *tab = static_cast<float *>(malloc(SILU_N * sizeof(float)));
 	if (!tab)
 		return fail(TIE_CUDA_ENOMEM);
@@ -771,7 +768,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	void *dev_ptrs[] = {s.x,     s.out_base, s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
 			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.counter, s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
-			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
+			    s.tile_info, s.xq, s.hq, s.dec_sync, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
 		if (p)
 			cudaFree(p);
@@ -937,8 +934,6 @@ int tie_cuda_upload_moe_layer(tie_cuda_ctx *c, int layer, const void *router_w_f
 	TRY(add_reg(c, gate_exps, L.gate.bytes, L.gate.ptr, gate_type, L.gate.kind, F, H));
 	TRY(add_reg(c, up_exps, L.up.bytes, L.up.ptr, up_type, L.up.kind, F, H));
 	TRY(add_reg(c, down_exps, L.down.bytes, L.down.ptr, down_type, L.down.kind, H, F));
-	const DfLayer entry = {L.gate.ptr, L.up.ptr, L.down.ptr, L.router_w, ffn_norm_w ? L.norm_w : nullptr};
-	TIE_CUDA_TRY(c, cudaMemcpy(c->df_table + layer, &entry, sizeof(entry), cudaMemcpyHostToDevice));
 	L.uploaded = true;
 	return TIE_CUDA_OK;
 }
@@ -1132,27 +1127,8 @@ int tie_cuda_moe_stack_inplace(tie_cuda_ctx *c, int first_layer, int n_layers, f
 					 TIE_CUDA_PATH_NO_PAIR);
 	const bool decode_paths = (pflags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR &&
 				  !(pflags & (TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2));
-	// (one token through all layers in ONE launch is tried first where the layers share tensor types;
-	// launch_decode_fused_stack reports "not supported" while that kernel is not built)
-	const Layer &L0 = c->layers[first_layer];
-	bool one_launch = n_tokens == 1 && n_layers > 1 && decode_paths && decode_fused_supported(c, L0, 1);
-	for (int l = first_layer + 1; l < first_layer + n_layers && one_launch; l++) {
-		const Layer &L = c->layers[l];
-		one_launch = L.gate.kind == L0.gate.kind && L.up.kind == L0.up.kind && L.down.kind == L0.down.kind &&
-			     L.gate.expert_stride == L0.gate.expert_stride && L.down.expert_stride == L0.down.expert_stride;
-	}
 	GraphKey k = {8, first_layer, n_tokens, hidden_dev, nullptr, nullptr, reinterpret_cast<const void *>((size_t)n_layers), pflags};
 	TRY(run_maybe_graphed(c, flags & TIE_CUDA_GRAPH, k, [&]() -> int {
-		if (one_launch) {
-			const int rc = launch_decode_fused_stack(c, first_layer, n_layers, hidden_dev);
-			if (rc != TIE_CUDA_ENOTSUP) {
-				if (!rc) {
-					c->last_used_tc = false;
-					c->last_direct_rows = c->cfg.top_k;
-				}
-				return rc;
-			}
-		}
 		for (int l = first_layer; l < first_layer + n_layers; l++) {
 			Layer &L = c->layers[l];
 			if (decode_paths && decode_fused_supported(c, L, n_tokens)) {

@@ -65,14 +65,6 @@ struct Layer {
 	const void *router_host = nullptr;
 };
 
-// Weights of one layer as the one-token decode kernel reads them when it walks a stack of layers
-// (device pointers; one entry per layer in the context's device table).
-struct DfLayer {
-	const uint8_t *wg, *wu, *wd;
-	const float *router_w;
-	const float *norm_w;  // or null: weight 1
-};
-
 // Scratch arena of one context, sized for max_tokens.
 struct Scratch {
 	float *x = nullptr;	    // [T][H]   staged input (host mode) / normed input (block mode)
@@ -154,7 +146,6 @@ struct tie_cuda_ctx {
 	cudaStream_t stream = nullptr;
 	float *silu = nullptr;	// device [8192]
 	tie::Layer *layers = nullptr;
-	tie::DfLayer *df_table = nullptr;  // device [n_layers]: the layers' weight pointers (stack decode)
 	tie::Scratch s;
 	int first_expert = 0, n_local = 0;
 	// pinned staging for host-pointer calls
@@ -240,13 +231,6 @@ namespace tie {
 	} while (0)
 
 // ---- device helpers ----
-__device__ __forceinline__ float warp_sum(float v)
-{
-#pragma unroll
-	for (int o = 16; o > 0; o >>= 1)
-		v += __shfl_xor_sync(0xffffffffu, v, o);
-	return v;
-}
 
 // get_scale_min_k4 (math_scalar.c:91-100) on the 12 packed bytes held as three 32-bit words.
 __device__ __forceinline__ void q4k_scale_min(const uint32_t sc[3], int j, int &s, int &m)

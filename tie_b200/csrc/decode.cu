@@ -1,4 +1,4 @@
-// Decode and small batches (up to 31 tokens of this model's shape): the expert mat-vecs of every
+// Decode and small batches (up to 8 tokens of this model's shape): the expert mat-vecs of every
 // (token, slot) row on its own — no dispatch sort, no grouping — with the exact mma.sync products of
 // mma_dot.cuh.
 //
@@ -14,8 +14,7 @@
 //
 // What bounds it: at 1-4 tokens latency (three dependent launches, 2-3 us each), above that the expansion of
 // the packed weights (about 230 instructions per warp for 16 rows x 256 Q4_K weights, 450 for Q6_K).
-// Rows that share an expert expand it once each: at 13 tokens 104 rows use 82 experts, at 31 tokens 248
-// rows 111.
+// Rows that share an expert expand it once each (at 8 tokens 64 rows use about 51 experts).
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma_dot.cuh"

@@ -549,12 +549,4 @@ int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const f
 	return df_dispatch(c, L, x, bias, residual, out, false, norm_w, norm_eps, next);
 }
 
-// One token through consecutive layers as ONE launch: not built (the layer loop inside the kernel
-// pushed the reductions' activation registers into local memory and doubled the step's time); the
-// caller runs the per-layer kernels from one CUDA graph instead.
-int launch_decode_fused_stack(tie_cuda_ctx *, int, int, float *)
-{
-	return TIE_CUDA_ENOTSUP;
-}
-
 }  // namespace tie

@@ -28,51 +28,10 @@ __device__ __forceinline__ float byte_to_float(uint32_t word, int k, float bias)
 template <WKind KIND>
 struct PartDot;
 
-// Lane-major staging of an activation row in shared memory: the r-th value (r = 0..63) of part p
-// is stored at ((r/4) * LPR + p) * 4 + r%4, so that the 128-bit reads of a warp (same r, all
-// parts) touch consecutive 16-byte words — no bank conflicts, unlike reading 64 contiguous floats
-// per lane.  src_index(p, r) gives the element of the row that value is.
-template <WKind KIND, int LPR>
-__device__ __forceinline__ void stage_x_lane_major(const float *__restrict__ xrow, float *__restrict__ xs_t, int parts, int tid,
-						   int nthreads)
-{
-	for (int d = tid; d < 16 * parts; d += nthreads) {  // one float4 per (r4, part)
-		const int r4 = d / parts, p = d % parts;
-		const int k = PartDot<KIND>::src_index(p, 4 * r4);
-		*reinterpret_cast<float4 *>(xs_t + (size_t)(r4 * LPR + p) * 4) = *reinterpret_cast<const float4 *>(xrow + k);
-	}
-}
-template <WKind KIND, int LPR>
-__device__ __forceinline__ void load_x_lane_major(const float *__restrict__ xs_t, int part, float xr[64], float sx[4])
-{
-#pragma unroll
-	for (int r4 = 0; r4 < 16; r4++) {
-		const float4 v = *reinterpret_cast<const float4 *>(xs_t + (size_t)(r4 * LPR + part) * 4);
-		xr[4 * r4] = v.x;
-		xr[4 * r4 + 1] = v.y;
-		xr[4 * r4 + 2] = v.z;
-		xr[4 * r4 + 3] = v.w;
-	}
-	PartDot<KIND>::sums(xr, sx);
-}
-
 // ---- Q4_K: part = (block b, quarter p): qs[32p .. 32p+32), low nibbles = sub-block 2p
 //      (elements 64p+i), high nibbles = sub-block 2p+1 (elements 64p+32+i) — math_scalar.c:216-255.
 template <>
 struct PartDot<W_Q4K> {
-	__device__ static __forceinline__ int src_index(int part, int r) { return 64 * part + r; }
-	__device__ static __forceinline__ void sums(const float xr[64], float sx[4])
-	{
-		float s0 = 0.f, s1 = 0.f;
-#pragma unroll
-		for (int i = 0; i < 8; i++) {
-			s0 += (xr[4 * i] + xr[4 * i + 1]) + (xr[4 * i + 2] + xr[4 * i + 3]);
-			s1 += (xr[32 + 4 * i] + xr[32 + 4 * i + 1]) + (xr[32 + 4 * i + 2] + xr[32 + 4 * i + 3]);
-		}
-		sx[0] = s0;
-		sx[1] = s1;
-		sx[2] = sx[3] = 0.f;
-	}
 	// xr[0..63] = x[64*part .. 64*part+63]; sx[0] = sum xr[0..31], sx[1] = sum xr[32..63]
 	__device__ static __forceinline__ void load_x(const float *xrow, int part, float xr[64], float sx[4])
 	{
@@ -139,11 +98,6 @@ struct PartDot<W_Q4K> {
 //      (l, l+32, l+64, l+96 within the half) — math_scalar.c:257-287.
 template <>
 struct PartDot<W_Q6K_R8> {
-	__device__ static __forceinline__ int src_index(int part, int r)
-	{
-		return 256 * (part >> 2) + 128 * ((part >> 1) & 1) + 16 * (part & 1) + 32 * (r >> 4) + (r & 15);
-	}
-	__device__ static __forceinline__ void sums(const float[64], float sx[4]) { sx[0] = sx[1] = sx[2] = sx[3] = 0.f; }
 	// xr[16*j + i] = x[256b + 128n + 16*l16 + 32*j + i]
 	__device__ static __forceinline__ void load_x(const float *xrow, int part, float xr[64], float sx[4])
 	{

@@ -76,10 +76,4 @@ __device__ __forceinline__ void q6k_int_word(uint32_t q, __half2 s, __half2 c, u
 	out[1] = h2_bits(__hfma2(bits_h2(and_or(q >> 4, 0x03F003F0u, 0x54005400u)), s, c));
 }
 
-// Position of element k inside its group of 4 in the operand tiles: [k0, k2, k1, k3].
-__host__ __device__ __forceinline__ int tc_kperm(int k)
-{
-	return (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1);
-}
-
 }  // namespace tie

@@ -13,13 +13,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p)
 	return (uint32_t)__cvta_generic_to_shared(p);
 }
 
-__device__ __forceinline__ uint64_t globaltimer_ns()
-{
-	uint64_t t;
-	asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-	return t;
-}
-
 // ---- mbarrier ----
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count)
 {
@@ -57,21 +50,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 		: "memory");
 	return ok != 0;
 }
-// The same without waiting: try_wait may hold the thread for a while when the phase is incomplete.
-__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity)
-{
-	uint32_t ok;
-	asm volatile(
-		"{\n\t"
-		".reg .pred p;\n\t"
-		"mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		"selp.u32 %0, 1, 0, p;\n\t"
-		"}"
-		: "=r"(ok)
-		: "r"(bar), "r"(parity)
-		: "memory");
-	return ok != 0;
-}
 // As try_wait, allowing the hardware to suspend the thread for up to `ns` nanoseconds while the
 // phase is incomplete (a suspended thread issues nothing; it resumes when the phase completes).
 __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t parity, uint32_t ns)
@@ -87,25 +65,6 @@ __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t par
 		: "r"(bar), "r"(parity), "r"(ns)
 		: "memory");
 	return ok != 0;
-}
-
-// ---- cp.async: per-thread asynchronous copies global -> shared ----
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
-{
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void *src)
-{
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit()
-{
-	asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-	asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ---- TMA: 2-D tile load global -> shared, completion counted on an mbarrier ----
@@ -129,13 +88,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *tma
 		"cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
 		"l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
 		: "memory");
-}
-// 1-D bulk copy global -> shared (16-byte aligned addresses, size a multiple of 16 bytes).
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar)
-{
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
-		     "r"(bytes), "r"(bar)
-		     : "memory");
 }
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *tmap)
 {
@@ -285,35 +237,6 @@ __device__ __forceinline__ uint32_t leader_addr(uint32_t local_smem_addr)
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t local_bar)
 {
 	asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(local_bar)) : "memory");
-}
-// try_wait that also orders the peer CTA's writes (its tensor-memory stores, its arrivals).
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t parity)
-{
-	uint32_t ok;
-	asm volatile(
-		"{\n\t"
-		".reg .pred p;\n\t"
-		"mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-		"selp.u32 %0, 1, 0, p;\n\t"
-		"}"
-		: "=r"(ok)
-		: "r"(bar), "r"(parity)
-		: "memory");
-	return ok != 0;
-}
-__device__ __forceinline__ bool mbar_try_wait_suspend_cluster(uint32_t bar, uint32_t parity, uint32_t ns)
-{
-	uint32_t ok;
-	asm volatile(
-		"{\n\t"
-		".reg .pred p;\n\t"
-		"mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-		"selp.u32 %0, 1, 0, p;\n\t"
-		"}"
-		: "=r"(ok)
-		: "r"(bar), "r"(parity), "r"(ns)
-		: "memory");
-	return ok != 0;
 }
 // TMA tile load into THIS CTA's shared memory whose completion bytes are counted on the barrier at
 // the same address in the LEADER CTA (no multicast: one destination, one barrier).

@@ -29,7 +29,8 @@
 //   * one MMA issuer thread walks the super-blocks: per 16-wide k step P += A.B_hi, P += A.B_lo into the
 //     same accumulator columns (one column per token; tiles of up to 32 tokens: one MMA over hi and lo
 //     rows, into columns side by side), a super-block per accumulator buffer, two buffers of 64
-//     columns in turn, and the block's min sums into a third;
+//     columns in turn (NT = 32, launches of narrow tiles: four of 32), and the block's min sums into a
+//     buffer of their own;
 //   * 8 drain warps take a finished super-block out of tensor memory (tcgen05.ld), hand the buffer back
 //     at once, fold the values into fp32 registers with d (-1 for the min sums), and after the last
 //     super-block of a work item store the rows — while the MMAs of the next super-blocks / work
@@ -143,15 +144,14 @@ static_assert(sizeof(TcShared) <= 512, "barrier block");
 // hardware suspend it between polls, so that waiting roles do not take issue slots from the
 // producers.
 // BACKOFF_NS > 0: roles that can afford a few hundred cycles of extra latency also sleep between polls.
-// CL: the barrier collects arrivals of the peer CTA of a pair (acquire at cluster scope).
-template <int BACKOFF_NS = 0, bool CL = false>
+template <int BACKOFF_NS = 0>
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile uint32_t *abort_flag, unsigned *status)
 {
-	if (CL ? ptx::mbar_try_wait_cluster(bar, parity) : ptx::mbar_try_wait(bar, parity))
+	if (ptx::mbar_try_wait(bar, parity))
 		return true;
 	const long long t0 = clock64();
 	uint32_t spins = 0;
-	while (!(CL ? ptx::mbar_try_wait_suspend_cluster(bar, parity, 20000u) : ptx::mbar_try_wait_suspend(bar, parity, 20000u))) {
+	while (!ptx::mbar_try_wait_suspend(bar, parity, 20000u)) {
 		if (BACKOFF_NS > 0)
 			__nanosleep(BACKOFF_NS);
 		if (*abort_flag)
