@@ -91,7 +91,9 @@ def test_grouped_tile_edges(grouped, counts, flags):
     x, e = torch.from_numpy(rows).cuda(), torch.from_numpy(row_expert).cuda()
     y = torch.full_like(x, float("nan"))
     b.expert_rows_ptr(0, x, e, row_expert.size, y, moe.DEVICE | moe.PATH_TENSOR | (moe.PATH_NO_PAIR if flags else 0))
-    assert workloads.rel_rms_err(y.cpu().numpy(), ref).max() < TOL
+    # (a row whose gates are all far below zero has no output to speak of: relative to the usual row then)
+    rms = np.sqrt((ref.astype(np.float64) ** 2).mean(1))
+    assert (np.abs(y.cpu().numpy() - ref).max(1) / np.maximum(rms, 1e-2 * np.median(rms))).max() < TOL
 
 
 # One registered tensor: its batch in tiles of 64, or of 32 where 64 leave SMs idle; Q4_K rows beyond 2048 inputs
