@@ -15,6 +15,7 @@
 #include "kernels.cuh"
 
 #include "router_topk.cuh"
+#include "tc_ptx.cuh"
 
 namespace tie {
 
@@ -67,14 +68,13 @@ __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__res
 //
 // Thread = one AVX2 lane l of a TPT-token x EPT-expert register tile (each of its chains a strict
 // i-ascending sequence of fused multiply-adds, so the result stays bit-identical); CTA = TT tokens x TE
-// experts.  The operands are staged lane-major in shared memory: two consecutive chain steps of a lane
-// are one 8-byte load (16-byte loads run at half the bandwidth), and the 8 lanes of a block of 32 k are
-// rotated so that the scattered stores are free of bank conflicts too; double-buffered through
-// registers.  What bounds a small batch is how many SMs pull the 1 MB of router weights, so the tile shrinks
-// with the batch until about 128 CTAs work (launch_router).  The CTA that finishes a token tile last (a
-// counter per tile, nobody waits) selects for all its tokens.
-// Measured (logits + selection): 4 tokens 14.4 -> 8.8 us, 13 28.7 -> 10.3, 64 28.7 -> 12.3, 512 29 -> 31, 1000 41 ->
-// 37, 4096 94 -> 100.
+// experts.  The operands' rows are staged as they are, by asynchronous copies two chunks ahead; a row pitch of
+// 8 words mod 32 keeps a warp's loads (8 lanes x 2 rows) free of bank conflicts.  What bounds a small batch is
+// how many SMs pull the 1 MB of router weights, a large one the multiply-adds and the shared-memory loads
+// beside them (wider loads move no more per cycle), so the tile grows with the batch (TIE_RT_TILES).  The
+// CTA that finishes a token tile last (a counter per tile, nobody waits) selects for all its tokens.
+// Measured (logits + selection): 4 tokens 14.4 -> 8.8 us, 13 28.7 -> 10.3, 64 28.7 -> 12.3, 333 29 -> 26, 512 29 -> 26.7,
+// 1000 41 -> 37, 2000 68 -> 54, 4096 94 -> 93.
 //
 // The hand-over of the tokens in an expert-parallel step rides along as one more row of CTAs, of
 // which as many work as there are SMs the logits' CTAs leave free (at least 16): CTAs that share an
@@ -92,10 +92,10 @@ template <int TPT_, int EPT_, int TT_, int TE_, int KC_>
 struct RtCfg {
 	static constexpr int TPT = TPT_, EPT = EPT_, TT = TT_, TE = TE_, KC = KC_;
 	static constexpr int TG = TT / TPT, EG = TE / EPT, THREADS = 8 * TG * EG;
-	static constexpr int PITCH = KC + 16, STAGE = (TT + TE) * PITCH;  // floats; two rows apart by half of the banks
-	static constexpr int SMEM = 2 * STAGE * (int)sizeof(float);
+	static constexpr int PITCH = KC + 8, STAGE = (TT + TE) * PITCH;  // floats; two rows apart by a quarter of the banks
+	static constexpr int STAGES = 3, SMEM = STAGES * STAGE * (int)sizeof(float);
 	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : 8;
-	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte loads per thread and chunk
+	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte copies per thread and chunk
 	static_assert((TT + TE) * (KC / 4) % THREADS == 0 && TG % 2 == 0 && EG % 2 == 0 && KC % 32 == 0, "router tile");
 };
 
@@ -121,31 +121,18 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 	// a warp is 8 lanes x 2 token groups x 2 expert groups
 	const int l = threadIdx.x & 7, g4 = threadIdx.x >> 5;
 	const int tg = ((threadIdx.x >> 3) & 1) + 2 * (g4 % (C::TG / 2)), eg = ((threadIdx.x >> 4) & 1) + 2 * (g4 / (C::TG / 2));
-	float4 r[C::LD];
-	auto fetch = [&](int k0) {
+	const int n_chunks = hidden / KC;
+	auto fetch = [&](int c) {  // (one group a call, an empty one past the end)
+		if (c < n_chunks) {
 #pragma unroll
-		for (int j = 0; j < C::LD; j++) {
-			const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
-			const float *src = row < TT ? x + (size_t)min(t0 + row, n_tokens - 1) * hidden	// (rows past the end: computed, dropped)
-						    : w + (size_t)(e0 + row - TT) * hidden;
-			// (volatile: left to itself the compiler sinks the loads to their use behind the chunk's arithmetic)
-			asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-				     : "=f"(r[j].x), "=f"(r[j].y), "=f"(r[j].z), "=f"(r[j].w)
-				     : "l"(src + k0 + 4 * c4));
+			for (int j = 0; j < C::LD; j++) {
+				const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
+				const float *src = row < TT ? x + (size_t)min(t0 + row, n_tokens - 1) * hidden	// (rows past the end: computed, dropped)
+							    : w + (size_t)(e0 + row - TT) * hidden;
+				ptx::cp_async16(ptx::smem_u32(rsm + (c % C::STAGES) * C::STAGE + row * C::PITCH + 4 * c4), src + c * KC + 4 * c4);
+			}
 		}
-	};
-	auto put = [&](int buf) {
-#pragma unroll
-		for (int j = 0; j < C::LD; j++) {
-			const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
-			// k = 4 c4 ..: chain step c4 / 2 of lanes 4 (c4 & 1) .. + 3
-			float *d = rsm + buf * C::STAGE + row * C::PITCH + (c4 >> 2) * 16 + ((c4 >> 1) & 1);
-			const int at = 8 * (c4 & 1) + 2 * ((c4 >> 3) & 3);
-			d[at & 15] = r[j].x;
-			d[(at + 2) & 15] = r[j].y;
-			d[(at + 4) & 15] = r[j].z;
-			d[(at + 6) & 15] = r[j].w;
-		}
+		ptx::cp_async_commit();
 	};
 	float acc[TPT][EPT];
 #pragma unroll
@@ -153,35 +140,29 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 #pragma unroll
 		for (int b = 0; b < EPT; b++)
 			acc[j][b] = 0.0f;
-	const int n_chunks = hidden / KC;
-	fetch(0);
-	put(0);
-	__syncthreads();
+#pragma unroll
+	for (int c = 0; c < C::STAGES - 1; c++)
+		fetch(c);
 	for (int c = 0; c < n_chunks; c++) {
-		if (c + 1 < n_chunks)
-			fetch((c + 1) * KC);
-		const float *xs = rsm + (c & 1) * C::STAGE + tg * C::PITCH, *ws = rsm + (c & 1) * C::STAGE + (TT + eg) * C::PITCH;
+		ptx::cp_async_wait<C::STAGES - 2>();
+		__syncthreads();  // (chunk c is here for everyone, and everyone is done with the buffer of chunk c - 1)
+		fetch(c + C::STAGES - 1);
+		const float *buf = rsm + (c % C::STAGES) * C::STAGE + l, *xs = buf + tg * C::PITCH, *ws = buf + (TT + eg) * C::PITCH;
 #pragma unroll C::UNROLL
-		for (int g = 0; g < KC / 16; g++) {  // two chain steps
-			const int at = 16 * g + ((2 * l + 2 * ((g >> 1) & 3)) & 15);
-			float2 xv[TPT];
+		for (int g = 0; g < KC / 8; g++) {
+			float xv[TPT], wv[EPT];
 #pragma unroll
 			for (int j = 0; j < TPT; j++)
-				xv[j] = *reinterpret_cast<const float2 *>(xs + C::TG * j * C::PITCH + at);
+				xv[j] = xs[C::TG * j * C::PITCH + 8 * g];
 #pragma unroll
-			for (int b = 0; b < EPT; b++) {
-				const float2 wv = *reinterpret_cast<const float2 *>(ws + C::EG * b * C::PITCH + at);
+			for (int b = 0; b < EPT; b++)
+				wv[b] = ws[C::EG * b * C::PITCH + 8 * g];
+#pragma unroll
+			for (int b = 0; b < EPT; b++)
 #pragma unroll
 				for (int j = 0; j < TPT; j++)
-					acc[j][b] = __fmaf_rn(xv[j].x, wv.x, acc[j][b]);
-#pragma unroll
-				for (int j = 0; j < TPT; j++)
-					acc[j][b] = __fmaf_rn(xv[j].y, wv.y, acc[j][b]);
-			}
+					acc[j][b] = __fmaf_rn(xv[j], wv[b], acc[j][b]);
 		}
-		if (c + 1 < n_chunks)
-			put((c + 1) & 1);
-		__syncthreads();
 	}
 #pragma unroll
 	for (int j = 0; j < TPT; j++) {
@@ -355,17 +336,18 @@ __global__ void __launch_bounds__(256) router_decode_fused(const float *__restri
 // push (expert-parallel steps): the kernel of the logits takes the hand-over of this rank's tokens to
 // its peers along as extra CTAs where it can; *push_taken tells whether it did.
 //
-// The tile: the largest of the list that still gives at least 0.85 CTAs per SM (each step down in size loads
-// more bytes per multiply-add from shared memory and L2, and fewer CTAs leave SMs idle), else the
-// smallest; the last-but-one sizes need hidden to be a multiple of their chunk of 512.
-#define TIE_RT_TILES(X)              \
-	X(RtCfg<8, 8, 64, 64, 64>)   \
-	X(RtCfg<4, 4, 32, 32, 128>)  \
-	X(RtCfg<4, 2, 32, 16, 128>)  \
-	X(RtCfg<2, 4, 16, 16, 256>)  \
-	X(RtCfg<2, 2, 16, 8, 512>)   \
-	X(RtCfg<1, 2, 8, 8, 512>)    \
-	X(RtCfg<1, 1, 4, 4, 512>)
+// The tiles, with what a launch of them takes: a + b n tenths of a microsecond when every SM has n CTAs (measured at
+// 2048 inputs, 128 experts).  launch_router takes the cheapest for its batch: a tile with more products per
+// operand load costs less per token, and more for the batch that leaves it half empty or one CTA over.
+#define TIE_RT_TILES(X)                            \
+	X(100, 820, RtCfg<8, 8, 64, 64, 64>)   \
+	X(70, 465, RtCfg<8, 4, 32, 64, 64>)    \
+	X(145, 223, RtCfg<4, 8, 16, 64, 64>)   \
+	X(105, 140, RtCfg<4, 4, 16, 32, 64>)   \
+	X(104, 101, RtCfg<2, 4, 16, 16, 256>)  \
+	X(85, 70, RtCfg<2, 2, 8, 16, 256>)     \
+	X(70, 53, RtCfg<1, 2, 8, 8, 512>)      \
+	X(65, 31, RtCfg<1, 1, 4, 4, 512>)
 int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
 		  int *topk_idx, float *topk_w, int lfm2, const EpPush *push, bool *push_taken)
 {
@@ -378,24 +360,25 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 	const float *sel_bias = lfm2 ? bias : nullptr;
 	if (lfm2)
 		bias = nullptr;
-	// what fits the shapes, in descending size: the first with enough CTAs, else the last
 	int pick = -1, at = 0;
-	bool enough = false;
-#define TIE_RT_PICK(...)                                                                                            \
-	{                                                                                                           \
-		using C = __VA_ARGS__;                                                                              \
-		if (E % C::TE == 0 && H % C::KC == 0 && !enough) {                                                  \
-			pick = at;                                                                                  \
-			enough = (long long)((n_tokens + C::TT - 1) / C::TT) * (E / C::TE) * 100 >= 85ll * c->sm_count; \
-		}                                                                                                   \
-		at++;                                                                                               \
+	long long best = 0;
+#define TIE_RT_PICK(A, B, ...)                                                                             \
+	{                                                                                                  \
+		using C = __VA_ARGS__;                                                                     \
+		const long long ctas = (long long)((n_tokens + C::TT - 1) / C::TT) * (E / C::TE);          \
+		const long long cost = A + B * ((ctas + c->sm_count - 1) / c->sm_count);                   \
+		if (E % C::TE == 0 && H % C::KC == 0 && (pick < 0 || cost < best)) {                       \
+			pick = at;                                                                         \
+			best = cost;                                                                       \
+		}                                                                                          \
+		at++;                                                                                      \
 	}
 	TIE_RT_TILES(TIE_RT_PICK)
 #undef TIE_RT_PICK
 	if (pick < 0)
 		return TIE_CUDA_ENOTSUP;
 	at = 0;
-#define TIE_RT_RUN(...)                                                                                                              \
+#define TIE_RT_RUN(A, B, ...)                                                                                                              \
 	if (at++ == pick) {                                                                                                          \
 		using C = __VA_ARGS__;                                                                                               \
 		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                                    \
@@ -424,7 +407,7 @@ int router_setup(tie_cuda_ctx *c)
 {
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_decode_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-#define TIE_RT_ATTR(...) \
+#define TIE_RT_ATTR(A, B, ...) \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, __VA_ARGS__::SMEM));
 	TIE_RT_TILES(TIE_RT_ATTR)
 #undef TIE_RT_ATTR
