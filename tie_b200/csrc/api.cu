@@ -714,6 +714,8 @@ int tie_cuda_init(tie_cuda_ctx **out, const tie_cuda_config *cfg)
 	c->layers = new (std::nothrow) Layer[cfg->n_layers];
 	if (!c->layers)
 		return fail(TIE_CUDA_ENOMEM);
+	if (cudaMalloc(reinterpret_cast<void **>(&c->df_table), sizeof(DfLayer) * cfg->n_layers) != cudaSuccess)
+		return fail(TIE_CUDA_ENOMEM);
 	float *tab = static_cast<float *>(malloc(SILU_N * sizeof(float)));
 	if (!tab)
 		return fail(TIE_CUDA_ENOMEM);
@@ -768,7 +770,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	void *dev_ptrs[] = {s.x,     s.out_base, s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
 			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.counter, s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
-			    s.tile_info, s.xq, s.hq, s.dec_sync, s.sort_hist, s.route_counter};
+			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
 		if (p)
 			cudaFree(p);
@@ -934,6 +936,8 @@ int tie_cuda_upload_moe_layer(tie_cuda_ctx *c, int layer, const void *router_w_f
 	TRY(add_reg(c, gate_exps, L.gate.bytes, L.gate.ptr, gate_type, L.gate.kind, F, H));
 	TRY(add_reg(c, up_exps, L.up.bytes, L.up.ptr, up_type, L.up.kind, F, H));
 	TRY(add_reg(c, down_exps, L.down.bytes, L.down.ptr, down_type, L.down.kind, H, F));
+	const DfLayer entry = df_layer(L);
+	TIE_CUDA_TRY(c, cudaMemcpy(c->df_table + layer, &entry, sizeof(entry), cudaMemcpyHostToDevice));
 	L.uploaded = true;
 	return TIE_CUDA_OK;
 }
@@ -1097,7 +1101,7 @@ int tie_cuda_moe_block_inplace(tie_cuda_ctx *c, int layer, float *hidden_dev, in
 		if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR &&
 		    !(flags & (TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2)) &&
 		    decode_fused_supported(c, *L, n_tokens)) {
-			const int rc = launch_decode_fused(c, *L, hidden_dev, nullptr, hidden_dev, hidden_dev, L->norm_w, c->cfg.norm_eps);
+			const int rc = launch_decode_fused_blocks(c, *L, 1, hidden_dev);
 			if (rc != TIE_CUDA_ENOTSUP) {
 				if (!rc) {
 					c->last_used_tc = false;
@@ -1132,11 +1136,16 @@ int tie_cuda_moe_stack_inplace(tie_cuda_ctx *c, int first_layer, int n_layers, f
 		for (int l = first_layer; l < first_layer + n_layers; l++) {
 			Layer &L = c->layers[l];
 			if (decode_paths && decode_fused_supported(c, L, n_tokens)) {
-				const Layer *next = l + 1 < first_layer + n_layers ? &c->layers[l + 1] : nullptr;
-				const int rc = launch_decode_fused(c, L, hidden_dev, nullptr, hidden_dev, hidden_dev, L.norm_w, c->cfg.norm_eps, next);
+				// one token: one launch for as many blocks as share a kernel
+				int n = 1;
+				while (l + n < first_layer + n_layers && c->layers[l + n].gate.kind == L.gate.kind &&
+				       c->layers[l + n].up.kind == L.up.kind)
+					n++;
+				const int rc = launch_decode_fused_blocks(c, L, n, hidden_dev);
 				if (rc != TIE_CUDA_ENOTSUP) {
 					if (rc)
 						return rc;
+					l += n - 1;
 					continue;
 				}
 			}

@@ -65,6 +65,15 @@ struct Layer {
 	const void *router_host = nullptr;
 };
 
+// Weights of one layer as the one-token decode kernel reads them (device pointers).
+struct DfLayer {
+	const uint8_t *wg, *wu, *wd;
+	const float *router_w;
+	const float *norm_w;  // or null: weight 1
+	size_t stride_dn;     // bytes per expert of wd
+	int down_q6k;	      // wd is W_Q6K_R8, else W_Q4K
+};
+
 // Scratch arena of one context, sized for max_tokens.
 struct Scratch {
 	float *x = nullptr;	    // [T][H]   staged input (host mode) / normed input (block mode)
@@ -146,6 +155,7 @@ struct tie_cuda_ctx {
 	cudaStream_t stream = nullptr;
 	float *silu = nullptr;	// device [8192]
 	tie::Layer *layers = nullptr;
+	tie::DfLayer *df_table = nullptr;  // device [n_layers]: df_layer of the uploaded ones
 	tie::Scratch s;
 	int first_expert = 0, n_local = 0;
 	// pinned staging for host-pointer calls

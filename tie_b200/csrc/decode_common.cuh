@@ -17,11 +17,11 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
 }
 
 // Bounded wait for the staged tiles; on timeout the status word is flagged and false returned.
-__device__ __forceinline__ bool dec_wait(uint32_t bar, unsigned *status)
+__device__ __forceinline__ bool dec_wait(uint32_t bar, unsigned *status, uint32_t parity = 0)
 {
 	long long t0 = 0;
 	uint32_t spins = 0;
-	while (!ptx::mbar_try_wait(bar, 0)) {
+	while (!ptx::mbar_try_wait(bar, parity)) {
 		if ((++spins & 1023u) == 0) {
 			const long long now = clock64();
 			if (t0 == 0)

@@ -19,8 +19,12 @@
 //   D  CTA (row tile): a warp takes one (slot, super-block); the products meet in shared memory and are
 //      added up per slot in super-block order, then over the slots from zero,
 //      acc = fma(w_j, v_j, acc) (model_qwen3.c:458-467), + residual
+//   -- barrier, the next block of a stack --
 //
-// Bound by latency: of 22.6 us per block in a stack, 4.7 are RMSNorm + router chains, 3 the two grid
+// A stack of blocks is one launch (the blocks may differ in the kind of the down tensor): a third barrier costs less
+// than the end of a grid and the start of the next, 22.7 -> 21.1 us a block.
+//
+// Bound by latency: of 22.6 us for one block, 4.7 are RMSNorm + router chains, 3 the two grid
 // barriers, 1.7 the selection, 2 the first tile's arrival, 4 gate/up, 3 down, 3.4 launch and tail (the
 // 25.5 MB themselves would take 3.9).  28.9 us with scalar reductions and the row and the router matrix
 // loaded one after the other.
@@ -55,20 +59,18 @@ struct DfShared {
 	int dn_req[MAX_TOP_K];	// the down tile of slot j has been requested
 	float inv;  // 1 / rms of the row (RMSNorm in the kernel)
 	float x_inv[8];	 // per super-block of x: the factor that undoes its image's scaling
+	DfLayer lay;
 };
 
 struct DfArgs {
-	const uint8_t *wg, *wu, *wd;
-	size_t stride_gu, stride_dn;  // bytes per expert
-	const float *x, *router_w, *bias, *residual, *silu;
-	const float *norm_w;  // norm_eps >= 0: x is the un-normed hidden row, RMSNorm (weights norm_w or 1) happens in the kernel
-	float norm_eps;
+	DfLayer first;		  // the (first) block's weights
+	const DfLayer *layers;	  // n_layers > 1: all of them, and x == residual == out
+	int n_layers;
+	size_t stride_gu;  // bytes per expert
+	const float *x, *bias, *residual, *silu;
+	float norm_eps;	 // >= 0: x is the un-normed hidden row, RMSNorm (weights norm_w or 1) happens in the kernel
 	float *logits, *h, *out, *topk_w;
 	int *topk_idx;
-	// bytes the NEXT launch reads first (the following block's router matrix), or nullptr: requested into
-	// L2 while this block's down products run; whole 16-byte units
-	const uint8_t *next;
-	uint32_t next_bytes;
 	unsigned *status, *sync;  // sync[0]: arrivals, sync[1]: epoch
 	int n_expert, top_k, first_expert, n_local;
 	int rpt_gu, tiles_gu, rpt_dn, tiles_dn;
@@ -104,7 +106,35 @@ __device__ __forceinline__ bool df_grid_barrier(unsigned *counter, unsigned targ
 	return sh->ok != 0;
 }
 
-template <WKind KG, int K, WKind KD, int F>
+// D, its products: a job is (slot, super-block); the gate/up tiles are done with, their space takes the images of h.
+template <WKind KD, int F>
+__device__ __forceinline__ bool df_down(uint8_t *dsm, const uint8_t *sd, float *prod, const float *h, int top_k, uint32_t tile_dn, int warp,
+					int lane, DfShared &sh, unsigned *status, uint32_t parity)
+{
+	constexpr int NBF = F / QK_K;
+	uint8_t *himg = dsm + warp * XImage<KD>::BYTES;
+	for (int i = warp; i < top_k * NBF; i += DF_WARPS) {
+		const int j = i / NBF, b = i % NBF;
+		const float4 *hp = reinterpret_cast<const float4 *>(h + (size_t)j * F + b * QK_K) + 2 * lane;
+		const float4 h0 = __ldcg(hp), h1 = __ldcg(hp + 1);  // (written by other CTAs of this grid)
+		const float v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+		const float inv = x_image<KD>(v, himg, lane);
+		if (!__all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_dn[j]), status, parity)))
+			return false;
+		MmaRows<KD> w;
+		w.load_smem(sd + (size_t)j * tile_dn, NBF, b, lane);
+		float2 r, s;
+		w.dot(himg, inv, lane, r, s);
+		if ((lane & 3) == 0) {
+			float2 *d = reinterpret_cast<float2 *>(prod) + i * 16 + (lane >> 2);
+			d[0] = make_float2(r.x, s.x);
+			d[8] = make_float2(r.y, s.y);
+		}
+	}
+	return true;
+}
+
+template <WKind KG, int K, int F>
 __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 {
 	constexpr int NBK = K / QK_K, NBF = F / QK_K;
@@ -123,7 +153,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 	const int d0 = cta * a.rpt_dn, d1 = min(d0 + a.rpt_dn, K);
 	const int n_chunks = gu_role ? (g1 - g0 + CH - 1) / CH : 0;
 	const uint32_t tile_gu = (uint32_t)(tile_offset<KG>(NBK, g1) - tile_offset<KG>(NBK, g0));
-	const uint32_t tile_dn = dn_role ? (uint32_t)(tile_offset<KD>(NBF, d1) - tile_offset<KD>(NBF, d0)) : 0;
 
 	DF_STAMP(0);
 	if (tid == DF_THREADS - 1) {  // (not in a warp that the norm or the router waits for)
@@ -134,264 +163,271 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			sh.dn_req[j] = 0;
 		}
 		ptx::fence_barrier_init();
+		sh.lay = a.first;
 		sh.base = df_ld_acquire(a.sync + 1);
 	}
+	unsigned target = 0;  // grid barriers, relative to the epoch
+	bool alive = true;
+	for (int layer = 0;; layer++) {
+		const uint32_t parity = (uint32_t)layer & 1u;  // (every copy barrier completes once a layer)
 
-	// The row and the CTA's row of the router matrix are both on their way before anything is computed.
-	float *ws = reinterpret_cast<float *>(dsm), *xn = reinterpret_cast<float *>(dsm + a.off_n);
-	static_assert(K / 4 <= DF_THREADS, "one 16-byte load per thread");
-	if (tid < K / 4) {
-		const float4 xv = __ldcg(reinterpret_cast<const float4 *>(a.x) + tid);	// (the row is overwritten in place at the end)
-		float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
-		if (cta < a.n_expert)
-			wv = __ldg(reinterpret_cast<const float4 *>(a.router_w + (size_t)cta * K) + tid);
-		reinterpret_cast<float4 *>(xn)[tid] = xv;
-		reinterpret_cast<float4 *>(ws)[tid] = wv;
-	}
-	__syncthreads();
-	// ---------------- (RMSNorm of the row, every CTA for itself: rms_norm_f32_f32_f32_avx2, math_avx2.c:56-97) ----------------
-	if (a.norm_eps >= 0.0f) {
-		if (warp == 0) {
+		// The row and the CTA's row of the router matrix are both on their way before anything is computed.
+		float *ws = reinterpret_cast<float *>(dsm), *xn = reinterpret_cast<float *>(dsm + a.off_n);
+		static_assert(K / 4 <= DF_THREADS, "one 16-byte load per thread");
+		if (tid < K / 4) {
+			const float4 xv = __ldcg(reinterpret_cast<const float4 *>(a.x) + tid);	// (the row is overwritten in place at the end)
+			float4 wv = make_float4(0.f, 0.f, 0.f, 0.f);
+			if (cta < a.n_expert)
+				wv = __ldg(reinterpret_cast<const float4 *>((layer ? sh.lay.router_w : a.first.router_w) + (size_t)cta * K) + tid);
+			reinterpret_cast<float4 *>(xn)[tid] = xv;
+			reinterpret_cast<float4 *>(ws)[tid] = wv;
+		}
+		__syncthreads();
+		// ---------------- (RMSNorm of the row, every CTA for itself: rms_norm_f32_f32_f32_avx2, math_avx2.c:56-97) ----------------
+		if (a.norm_eps >= 0.0f) {
+			if (warp == 0) {
+				float acc = 0.0f;
+				if (lane < 8) {
+#pragma unroll 32
+					for (int i = 0; i < K / 8; i++) {
+						const float v = xn[8 * i + lane];
+						acc = __fmaf_rn(v, v, acc);
+					}
+				}
+				const float ss = hsum8_lanes(acc);  // (l + l4), then + 1, then + 2: the reference's tree
+				if (lane == 0)
+					sh.inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), a.norm_eps)));
+			}
+			__syncthreads();
+			const float inv = sh.inv, *norm_w = sh.lay.norm_w;
+			for (int i = tid; i < K; i += DF_THREADS)
+				xn[i] = __fmul_rn(__fmul_rn(xn[i], norm_w ? norm_w[i] : 1.0f), inv);
+			__syncthreads();
+		}
+
+		// ---------------- R: one router logit per CTA (warp 0), the images of x beside it ----------------
+		if (warp == 0 && cta < a.n_expert) {
 			float acc = 0.0f;
 			if (lane < 8) {
 #pragma unroll 32
-				for (int i = 0; i < K / 8; i++) {
-					const float v = xn[8 * i + lane];
-					acc = __fmaf_rn(v, v, acc);
-				}
+				for (int i = 0; i < K / 8; i++)
+					acc = __fmaf_rn(xn[8 * i + lane], ws[8 * i + lane], acc);
 			}
-			const float ss = hsum8_lanes(acc);  // (l + l4), then + 1, then + 2: the reference's tree
+			float r = hsum8_lanes(acc);
+			if (lane == 0) {
+				if (a.bias)
+					r = __fadd_rn(r, a.bias[cta]);
+				__stcg(a.logits + cta, r);
+			}
+		}
+		if (gu_role && warp >= 8 && warp < 8 + NBK) {
+			const int b = warp - 8;
+			const float4 *xp = reinterpret_cast<const float4 *>(xn + b * QK_K) + 2 * lane;
+			const float4 x0 = xp[0], x1 = xp[1];
+			const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+			const float inv = x_image<KG>(v, ximg + b * XImage<KG>::BYTES, lane);
 			if (lane == 0)
-				sh.inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)K), a.norm_eps)));
+				sh.x_inv[b] = inv;
 		}
-		__syncthreads();
-		const float inv = sh.inv;
-		for (int i = tid; i < K; i += DF_THREADS)
-			xn[i] = __fmul_rn(__fmul_rn(xn[i], a.norm_w ? a.norm_w[i] : 1.0f), inv);
-		__syncthreads();
-	}
+		if (layer == 0)
+			target = (__syncthreads(), sh.base);
+		DF_STAMP(1);
+		if (!df_grid_barrier(a.sync, target += (unsigned)G, &sh, a.status))
+			return;	 // nothing of this CTA is in flight yet
+		DF_STAMP(2);
 
-	// ---------------- R: one router logit per CTA (warp 0), the images of x beside it ----------------
-	if (warp == 0 && cta < a.n_expert) {
-		float acc = 0.0f;
-		if (lane < 8) {
-#pragma unroll 32
-			for (int i = 0; i < K / 8; i++)
-				acc = __fmaf_rn(xn[8 * i + lane], ws[8 * i + lane], acc);
-		}
-		float r = hsum8_lanes(acc);
-		if (lane == 0) {
-			if (a.bias)
-				r = __fadd_rn(r, a.bias[cta]);
-			__stcg(a.logits + cta, r);
-		}
-	}
-	if (gu_role && warp >= 8 && warp < 8 + NBK) {
-		const int b = warp - 8;
-		const float4 *xp = reinterpret_cast<const float4 *>(xn + b * QK_K) + 2 * lane;
-		const float4 x0 = xp[0], x1 = xp[1];
-		const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-		const float inv = x_image<KG>(v, ximg + b * XImage<KG>::BYTES, lane);
-		if (lane == 0)
-			sh.x_inv[b] = inv;
-	}
-	const unsigned base = (__syncthreads(), sh.base);
-	DF_STAMP(1);
-	if (!df_grid_barrier(a.sync, base + (unsigned)G, &sh, a.status))
-		return;	 // nothing of this CTA is in flight yet
-	DF_STAMP(2);
-
-	// ---------------- selection (every CTA for itself) and all weight requests ----------------
-	if (warp == 0) {
-		unsigned key[1][8];
+		// ---------------- selection (every CTA for itself) and all weight requests ----------------
+		if (warp == 0) {
+			unsigned key[1][8];
 #pragma unroll
-		for (int i = 0; i < 8; i++)
-			key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
-		int mine[1];
-		topk_warp<1, 8>(key, lane, top_k, mine);
-		if (lane < top_k)
-			sh.idx[lane] = mine[0];
-	}
-	__syncthreads();
-	bool bad = false;
-	for (int j = 0; j < top_k; j++) {
-		const int le = sh.idx[j] - a.first_expert;
-		bad |= (le < 0 || le >= a.n_local);
-	}
-	if (bad && cta == 0 && tid == 0)
-		atomicOr(a.status, ST_BAD_EXPERT);
-	uint8_t *sg = dsm, *su = dsm + tile_gu, *sd = dsm + a.off_b;
-	// one issuing thread per copy group (issuing a bulk copy costs ~100 cycles): warp c < 8 the
-	// gate/up chunk c, warp 8 + j the down tile of slot j.  The down tiles are requested when the warp's
-	// last gate/up chunk has landed: asked for earlier they share the HBM bandwidth with the gate/up
-	// tiles, and they still have a product, a grid barrier and the image of h to arrive in.
-	auto request_down = [&]() {  // lane 0 of warp 8 + j
-		const int j = warp - DF_MAX_CHUNKS;
-		if (dn_role && j >= 0 && j < top_k) {
-			const uint32_t ba = ptx::smem_u32(&sh.bar_dn[j]);
-			sh.dn_req[j] = 1;
-			ptx::fence_proxy_async_smem();
-			ptx::mbar_arrive_expect_tx(ba, tile_dn);
-			bulk_g2s(ptx::smem_u32(sd + (size_t)j * tile_dn),
-				 a.wd + (size_t)(sh.idx[j] - a.first_expert) * a.stride_dn + tile_offset<KD>(NBF, d0), tile_dn, ba);
+			for (int i = 0; i < 8; i++)
+				key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
+			int mine[1];
+			topk_warp<1, 8>(key, lane, top_k, mine);
+			if (lane < top_k)
+				sh.idx[lane] = mine[0];
 		}
-	};
-	if (lane == 0 && !bad) {
-		ptx::fence_proxy_async_smem();	// the tile area held the router's staging
-		if (warp < DF_MAX_CHUNKS) {
-			const int c = warp;
-			if (gu_role && c < n_chunks) {
-				const size_t eb = (size_t)(sh.idx[slot] - a.first_expert) * a.stride_gu;
-				const int c0 = g0 + c * CH, c1 = min(c0 + CH, g1);
-				const size_t o0 = tile_offset<KG>(NBK, c0), o1 = tile_offset<KG>(NBK, c1);
-				const uint32_t bytes = (uint32_t)(o1 - o0), rel = (uint32_t)(o0 - tile_offset<KG>(NBK, g0));
-				const uint32_t ba = ptx::smem_u32(&sh.bar_gu[c]);
-				ptx::mbar_arrive_expect_tx(ba, 2 * bytes);
-				bulk_g2s(ptx::smem_u32(sg + rel), a.wg + eb + o0, bytes, ba);
-				bulk_g2s(ptx::smem_u32(su + rel), a.wu + eb + o0, bytes, ba);
+		__syncthreads();
+		bool bad = false;
+		for (int j = 0; j < top_k; j++) {
+			const int le = sh.idx[j] - a.first_expert;
+			bad |= (le < 0 || le >= a.n_local);
+		}
+		if (bad && cta == 0 && tid == 0)
+			atomicOr(a.status, ST_BAD_EXPERT);
+		const bool dn_q6k = sh.lay.down_q6k;
+		const uint32_t tile_dn = !dn_role ? 0
+						  : (uint32_t)(dn_q6k ? tile_offset<W_Q6K_R8>(NBF, d1) - tile_offset<W_Q6K_R8>(NBF, d0)
+								      : tile_offset<W_Q4K>(NBF, d1) - tile_offset<W_Q4K>(NBF, d0));
+		uint8_t *sg = dsm, *su = dsm + tile_gu, *sd = dsm + a.off_b;
+		// one issuing thread per copy group (issuing a bulk copy costs ~100 cycles): warp c < 8 the
+		// gate/up chunk c, warp 8 + j the down tile of slot j.  The down tiles are requested when the warp's
+		// last gate/up chunk has landed: asked for earlier they share the HBM bandwidth with the gate/up
+		// tiles, and they still have a product, a grid barrier and the image of h to arrive in.
+		auto request_down = [&]() {  // lane 0 of warp 8 + j
+			const int j = warp - DF_MAX_CHUNKS;
+			if (dn_role && j >= 0 && j < top_k) {
+				const uint32_t ba = ptx::smem_u32(&sh.bar_dn[j]);
+				sh.dn_req[j] = 1;
+				ptx::fence_proxy_async_smem();
+				ptx::mbar_arrive_expect_tx(ba, tile_dn);
+				bulk_g2s(ptx::smem_u32(sd + (size_t)j * tile_dn),
+					 sh.lay.wd + (size_t)(sh.idx[j] - a.first_expert) * sh.lay.stride_dn +
+						 (dn_q6k ? tile_offset<W_Q6K_R8>(NBF, d0) : tile_offset<W_Q4K>(NBF, d0)),
+					 tile_dn, ba);
 			}
-		} else if (!gu_role) {
-			request_down();	 // (a CTA without gate/up rows: nothing to wait for)
-		}
-	}
-	if (warp == DF_WARPS - 1) {  // softmax (engine.c:864-888) with the arithmetic of topk_tokens, while the tiles are on their way
-		const int e = lane < top_k ? sh.idx[lane] : -1;
-		const float score = e >= 0 ? __ldcg(a.logits + e) : 0.0f;
-		const float mx = __shfl_sync(0xffffffffu, score, 0);
-		const float ex = (lane < top_k) ? expf(__fsub_rn(score, mx)) : 0.0f;
-		float sum = 0.0f;
-		for (int j = 0; j < top_k; j++)
-			sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, ex, j));
-		const float w = __fmul_rn(ex, __fdiv_rn(1.0f, sum));
-		if (lane < top_k) {
-			sh.w[lane] = w;
-			if (cta == 0) {
-				a.topk_idx[lane] = e;
-				a.topk_w[lane] = w;
-			}
-		}
-	}
-	// waits (bounded) for every copy this CTA requested: before it gives up, and harmless otherwise
-	auto drain = [&]() {
-		if (bad)
-			return;
-		for (int c = 0; c < n_chunks; c++)
-			dec_wait(ptx::smem_u32(&sh.bar_gu[c]), a.status);
-		if (dn_role)
-			for (int j = 0; j < top_k; j++)
-				if (sh.dn_req[j])
-					dec_wait(ptx::smem_u32(&sh.bar_dn[j]), a.status);
-	};
-
-	// ---------------- G: gate, up, SwiGLU ----------------
-	DF_STAMP(3);
-	bool alive = true;
-	if (gu_role && !bad) {
-		// a job is (chunk of 16 rows, matrix, super-block); the products of a row's super-blocks are added up in order
-		const int jobs = n_chunks * 2 * NBK;
-		for (int i = warp; i < jobs && alive; i += DF_WARPS) {
-			const int chunk = i / (2 * NBK), mat = i % 2, b = (i % (2 * NBK)) >> 1;
-			alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status));
-			if (!alive)
-				break;
-			if (i == warp && lane == 0)
-				DF_STAMP(7);
-			if (i + DF_WARPS >= jobs && lane == 0)	// the warp's last
-				request_down();
-			MmaRows<KG> w;
-			w.load_smem((mat ? su : sg) + tile_offset<KG>(NBK, chunk * CH), NBK, b, lane);
-			float2 r, s;
-			w.dot(ximg + b * XImage<KG>::BYTES, sh.x_inv[b], lane, r, s);
-			if ((lane & 3) == 0) {
-				float *d = prod + ((chunk * 2 + mat) * NBK + b) * 16 + (lane >> 2);
-				d[0] = r.x * s.x;
-				d[8] = r.y * s.y;
-			}
-		}
-		if (warp >= jobs && lane == 0)
-			request_down();
-		alive = __syncthreads_and(alive);
-		if (alive && tid < g1 - g0) {
-			const float *pg = prod + (tid >> 4) * 2 * NBK * 16 + (tid & 15), *pu = pg + NBK * 16;
-			float g = pg[0], u = pu[0];
-			for (int b = 1; b < NBK; b++) {
-				g = __fadd_rn(g, pg[b * 16]);
-				u = __fadd_rn(u, pu[b * 16]);
-			}
-			__stcg(a.h + (size_t)slot * F + g0 + tid, swiglu_lut(a.silu, g, u));
-		}
-		DF_STAMP(8);
-	}
-	alive = __syncthreads_and(alive);
-	DF_STAMP(4);
-	if (!alive) {  // a copy never landed: leave, but not with copies in flight
-		if (tid == 0)
-			drain();
-		return;
-	}
-	if (!df_grid_barrier(a.sync, base + 2u * (unsigned)G, &sh, a.status)) {
-		if (tid == 0)
-			drain();
-		return;
-	}
-
-	// ---------------- D: down + combine ----------------
-	DF_STAMP(5);
-	if (a.next && tid == 0) {  // this CTA's share of the next block's first bytes -> L2
-		const uint32_t per = ((a.next_bytes + G - 1) / G + 15u) & ~15u, o = per * (uint32_t)cta;
-		if (o < a.next_bytes) {
-			const uint32_t n = min(per, a.next_bytes - o);
-			asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a.next + o), "r"(n) : "memory");
-		}
-	}
-	if (dn_role && !bad) {
-		// a job is (slot, super-block); the gate/up tiles are done with: their space takes the images of h
-		uint8_t *himg = dsm + warp * XImage<KD>::BYTES;
-		for (int i = warp; i < top_k * NBF && alive; i += DF_WARPS) {
-			const int j = i / NBF, b = i % NBF;
-			const float4 *hp = reinterpret_cast<const float4 *>(a.h + (size_t)j * F + b * QK_K) + 2 * lane;
-			const float4 h0 = __ldcg(hp), h1 = __ldcg(hp + 1);  // (written by other CTAs of this grid)
-			const float v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-			const float inv = x_image<KD>(v, himg, lane);
-			alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_dn[j]), a.status));
-			if (!alive)
-				break;
-			MmaRows<KD> w;
-			w.load_smem(sd + (size_t)j * tile_dn, NBF, b, lane);
-			float2 r, s;
-			w.dot(himg, inv, lane, r, s);
-			if ((lane & 3) == 0) {
-				float2 *d = reinterpret_cast<float2 *>(prod) + i * 16 + (lane >> 2);
-				d[0] = make_float2(r.x, s.x);
-				d[8] = make_float2(r.y, s.y);
-			}
-		}
-		DF_STAMP(10);
-		alive = __syncthreads_and(alive);
-		if (alive) {
-			for (int lr = tid; lr < d1 - d0; lr += DF_THREADS) {
-				float acc = 0.f;
-				for (int j = 0; j < top_k; j++) {
-					float v = 0.f;
-					for (int b = 0; b < NBF; b++) {
-						const float2 e = reinterpret_cast<const float2 *>(prod)[(j * NBF + b) * 16 + lr];
-						v = __fmaf_rn(e.y, e.x, v);
-					}
-					acc = __fmaf_rn(sh.w[j], v, acc);  // slot order, from zero
+		};
+		if (lane == 0 && !bad) {
+			ptx::fence_proxy_async_smem();	// the tile area held the router's staging
+			if (warp < DF_MAX_CHUNKS) {
+				const int c = warp;
+				if (gu_role && c < n_chunks) {
+					const size_t eb = (size_t)(sh.idx[slot] - a.first_expert) * a.stride_gu;
+					const int c0 = g0 + c * CH, c1 = min(c0 + CH, g1);
+					const size_t o0 = tile_offset<KG>(NBK, c0), o1 = tile_offset<KG>(NBK, c1);
+					const uint32_t bytes = (uint32_t)(o1 - o0), rel = (uint32_t)(o0 - tile_offset<KG>(NBK, g0));
+					const uint32_t ba = ptx::smem_u32(&sh.bar_gu[c]);
+					ptx::mbar_arrive_expect_tx(ba, 2 * bytes);
+					bulk_g2s(ptx::smem_u32(sg + rel), sh.lay.wg + eb + o0, bytes, ba);
+					bulk_g2s(ptx::smem_u32(su + rel), sh.lay.wu + eb + o0, bytes, ba);
 				}
-				if (a.residual)
-					acc = __fadd_rn(a.residual[d0 + lr], acc);
-				a.out[d0 + lr] = acc;
+			} else if (!gu_role) {
+				request_down();	 // (a CTA without gate/up rows: nothing to wait for)
 			}
 		}
-	}
-	__syncthreads();
-	DF_STAMP(6);
-	if (tid == 0) {
-		drain();
-		// the last CTA out advances the epoch for the next launch
-		if (alive && atomicAdd(a.sync, 1u) == base + 3u * (unsigned)G - 1u)
-			atomicExch(a.sync + 1, base + 3u * (unsigned)G);
+		if (warp == DF_WARPS - 1) {  // softmax (engine.c:864-888) with the arithmetic of topk_tokens, while the tiles are on their way
+			const int e = lane < top_k ? sh.idx[lane] : -1;
+			const float score = e >= 0 ? __ldcg(a.logits + e) : 0.0f;
+			const float mx = __shfl_sync(0xffffffffu, score, 0);
+			const float ex = (lane < top_k) ? expf(__fsub_rn(score, mx)) : 0.0f;
+			float sum = 0.0f;
+			for (int j = 0; j < top_k; j++)
+				sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, ex, j));
+			const float w = __fmul_rn(ex, __fdiv_rn(1.0f, sum));
+			if (lane < top_k) {
+				sh.w[lane] = w;
+				if (cta == 0) {
+					a.topk_idx[lane] = e;
+					a.topk_w[lane] = w;
+				}
+			}
+		}
+		// waits (bounded) for every copy this CTA requested: before it gives up, and harmless otherwise
+		auto drain = [&]() {
+			if (bad)
+				return;
+			for (int c = 0; c < n_chunks; c++)
+				dec_wait(ptx::smem_u32(&sh.bar_gu[c]), a.status, parity);
+			if (dn_role)
+				for (int j = 0; j < top_k; j++)
+					if (sh.dn_req[j])
+						dec_wait(ptx::smem_u32(&sh.bar_dn[j]), a.status, parity);
+		};
+
+		// ---------------- G: gate, up, SwiGLU ----------------
+		DF_STAMP(3);
+		if (gu_role && !bad) {
+			// a job is (chunk of 16 rows, matrix, super-block); the products of a row's super-blocks are added up in order
+			const int jobs = n_chunks * 2 * NBK;
+			for (int i = warp; i < jobs && alive; i += DF_WARPS) {
+				const int chunk = i / (2 * NBK), mat = i % 2, b = (i % (2 * NBK)) >> 1;
+				alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status, parity));
+				if (!alive)
+					break;
+				if (i == warp && lane == 0)
+					DF_STAMP(7);
+				if (i + DF_WARPS >= jobs && lane == 0)	// the warp's last
+					request_down();
+				MmaRows<KG> w;
+				w.load_smem((mat ? su : sg) + tile_offset<KG>(NBK, chunk * CH), NBK, b, lane);
+				float2 r, s;
+				w.dot(ximg + b * XImage<KG>::BYTES, sh.x_inv[b], lane, r, s);
+				if ((lane & 3) == 0) {
+					float *d = prod + ((chunk * 2 + mat) * NBK + b) * 16 + (lane >> 2);
+					d[0] = r.x * s.x;
+					d[8] = r.y * s.y;
+				}
+			}
+			if (warp >= jobs && lane == 0)
+				request_down();
+			alive = __syncthreads_and(alive);
+			if (alive && tid < g1 - g0) {
+				const float *pg = prod + (tid >> 4) * 2 * NBK * 16 + (tid & 15), *pu = pg + NBK * 16;
+				float g = pg[0], u = pu[0];
+				for (int b = 1; b < NBK; b++) {
+					g = __fadd_rn(g, pg[b * 16]);
+					u = __fadd_rn(u, pu[b * 16]);
+				}
+				__stcg(a.h + (size_t)slot * F + g0 + tid, swiglu_lut(a.silu, g, u));
+			}
+			DF_STAMP(8);
+		}
+		alive = __syncthreads_and(alive);
+		DF_STAMP(4);
+		if (!alive) {  // a copy never landed: leave, but not with copies in flight
+			if (tid == 0)
+				drain();
+			return;
+		}
+		if (!df_grid_barrier(a.sync, target += (unsigned)G, &sh, a.status)) {
+			if (tid == 0)
+				drain();
+			return;
+		}
+
+		// ---------------- D: down + combine ----------------
+		DF_STAMP(5);
+		const bool more = layer + 1 < a.n_layers && !bad;  // (bad is the same in every CTA: they all selected alike)
+		if (more && tid == 0) {	 // this CTA's share of the next block's router matrix -> L2
+			const uint32_t bytes = (uint32_t)a.n_expert * K * sizeof(float), per = ((bytes + G - 1) / G + 15u) & ~15u, o = per * (uint32_t)cta;
+			if (o < bytes) {
+				const uint32_t n = min(per, bytes - o);
+				asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<const uint8_t *>(a.layers[layer + 1].router_w) + o), "r"(n)
+					     : "memory");
+			}
+		}
+		if (dn_role && !bad) {
+			alive = dn_q6k ? df_down<W_Q6K_R8, F>(dsm, sd, prod, a.h, top_k, tile_dn, warp, lane, sh, a.status, parity)
+				       : df_down<W_Q4K, F>(dsm, sd, prod, a.h, top_k, tile_dn, warp, lane, sh, a.status, parity);
+			DF_STAMP(10);
+			alive = __syncthreads_and(alive);
+			if (alive) {
+				for (int lr = tid; lr < d1 - d0; lr += DF_THREADS) {
+					float acc = 0.f;
+					for (int j = 0; j < top_k; j++) {
+						float v = 0.f;
+						for (int b = 0; b < NBF; b++) {
+							const float2 e = reinterpret_cast<const float2 *>(prod)[(j * NBF + b) * 16 + lr];
+							v = __fmaf_rn(e.y, e.x, v);
+						}
+						acc = __fmaf_rn(sh.w[j], v, acc);  // slot order, from zero
+					}
+					if (a.residual)
+						acc = __fadd_rn(__ldcg(a.residual + d0 + lr), acc);
+					__stcg(a.out + d0 + lr, acc);
+				}
+			}
+		}
+		__syncthreads();
+		DF_STAMP(6);
+		if (!alive || !more) {
+			if (tid == 0) {
+				drain();
+				// the last CTA out advances the epoch for the next launch
+				target += (unsigned)G;
+				if (alive && atomicAdd(a.sync, 1u) == target - 1u)
+					atomicExch(a.sync + 1, target);
+			}
+			return;
+		}
+		if (tid == DF_THREADS - 1) {
+			sh.lay = a.layers[layer + 1];
+			for (int j = 0; j < MAX_TOP_K; j++)
+				sh.dn_req[j] = 0;
+		}
+		// the row is complete, and the next block may overwrite h, the logits and the tiles
+		if (!df_grid_barrier(a.sync, target += (unsigned)G, &sh, a.status))
+			return;	 // (every copy of this CTA has been waited for)
 	}
 }
 
@@ -409,7 +445,7 @@ struct DfPlan {
 	bool ok;
 };
 
-template <WKind KG, int K, WKind KD, int F>
+template <WKind KG, int K, int F>
 static DfPlan df_plan(const tie_cuda_ctx *c)
 {
 	DfPlan p = {};
@@ -427,10 +463,10 @@ static DfPlan df_plan(const tie_cuda_ctx *c)
 	p.grid = max(c->cfg.n_expert, max(top_k * p.tiles_gu, p.tiles_dn));
 	if (p.grid > sms)
 		return p;
-	const size_t tile_gu = (size_t)p.rpt_gu * df_row_bytes<KG>(K), tile_dn = (size_t)p.rpt_dn * df_row_bytes<KD>(F);
+	const size_t tile_gu = (size_t)p.rpt_gu * df_row_bytes<KG>(K), tile_dn = (size_t)p.rpt_dn * df_row_bytes<W_Q6K_R8>(F);  // (the larger kind)
 	size_t area_a = 2 * tile_gu;
 	area_a = max(area_a, (size_t)2 * K * sizeof(float));				 // router staging
-	area_a = max(area_a, (size_t)DF_WARPS * XImage<KD>::BYTES);			 // images of h
+	area_a = max(area_a, (size_t)DF_WARPS * max(XImage<W_Q4K>::BYTES, XImage<W_Q6K_R8>::BYTES));  // images of h
 	p.off_b = (area_a + 127) / 128 * 128;
 	p.off_c = (p.off_b + (size_t)top_k * tile_dn + 127) / 128 * 128;
 	p.off_v = p.off_c + (size_t)NBK * XImage<KG>::BYTES;
@@ -440,24 +476,27 @@ static DfPlan df_plan(const tie_cuda_ctx *c)
 	return p;
 }
 
-template <WKind KG, int K, WKind KD, int F>
-static int df_launch(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
-		     bool query_only, const float *norm_w, float norm_eps, const Layer *next)
+DfLayer df_layer(const Layer &L)
 {
-	const DfPlan p = df_plan<KG, K, KD, F>(c);
+	return {L.gate.ptr, L.up.ptr, L.down.ptr, L.router_w, L.norm_w, L.down.expert_stride, L.down.kind == W_Q6K_R8};
+}
+
+template <WKind KG, int K, int F>
+static int df_launch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float *x, const float *bias, const float *residual, float *out,
+		     bool query_only, bool norm)
+{
+	const DfPlan p = df_plan<KG, K, F>(c);
 	if (!p.ok)
 		return TIE_CUDA_ENOTSUP;
 	if (query_only)
 		return TIE_CUDA_OK;
 	Scratch &s = c->s;
 	DfArgs a = {};
-	a.wg = L.gate.ptr;
-	a.wu = L.up.ptr;
-	a.wd = L.down.ptr;
+	a.first = df_layer(L);
+	a.layers = c->df_table + (&L - c->layers);
+	a.n_layers = n_layers;
 	a.stride_gu = L.gate.expert_stride;
-	a.stride_dn = L.down.expert_stride;
 	a.x = x;
-	a.router_w = L.router_w;
 	a.bias = bias;
 	a.residual = residual;
 	a.silu = c->silu;
@@ -480,13 +519,8 @@ static int df_launch(tie_cuda_ctx *c, const Layer &L, const float *x, const floa
 	a.off_c = (uint32_t)p.off_c;
 	a.off_v = (uint32_t)p.off_v;
 	a.off_n = (uint32_t)p.off_n;
-	a.norm_w = norm_w;
-	a.norm_eps = norm_eps;
-	if (next && next->router_w) {
-		a.next = reinterpret_cast<const uint8_t *>(next->router_w);
-		a.next_bytes = (uint32_t)((size_t)c->cfg.n_expert * K * sizeof(float));
-	}
-	auto kern = decode1_fused<KG, K, KD, F>;
+	a.norm_eps = norm ? c->cfg.norm_eps : -1.0f;
+	auto kern = decode1_fused<KG, K, F>;
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3(p.grid);
@@ -513,22 +547,16 @@ static int df_launch(tie_cuda_ctx *c, const Layer &L, const float *x, const floa
 // The (hidden, ffn_dim) pairs the one-kernel step is built for.
 #define TIE_DF_SHAPES(X) X(2048, 768) X(512, 256)
 
-static int df_dispatch(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
-		       bool query_only, const float *norm_w = nullptr, float norm_eps = -1.0f, const Layer *next = nullptr)
+static int df_dispatch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float *x, const float *bias, const float *residual, float *out,
+		       bool query_only, bool norm)
 {
 	if (L.gate.kind != L.up.kind)
 		return TIE_CUDA_ENOTSUP;
 	const int K = c->cfg.hidden, F = c->cfg.ffn_dim;
-#define X(KK, FF)                                                                                                              \
-	if (K == KK && F == FF) {                                                                                              \
-		if (L.gate.kind == W_Q4K && L.down.kind == W_Q6K_R8)                                                           \
-			return df_launch<W_Q4K, KK, W_Q6K_R8, FF>(c, L, x, bias, residual, out, query_only, norm_w, norm_eps, next);                    \
-		if (L.gate.kind == W_Q4K && L.down.kind == W_Q4K)                                                              \
-			return df_launch<W_Q4K, KK, W_Q4K, FF>(c, L, x, bias, residual, out, query_only, norm_w, norm_eps, next);                      \
-		if (L.gate.kind == W_Q6K_R8 && L.down.kind == W_Q6K_R8)                                                        \
-			return df_launch<W_Q6K_R8, KK, W_Q6K_R8, FF>(c, L, x, bias, residual, out, query_only, norm_w, norm_eps, next);                \
-		return df_launch<W_Q6K_R8, KK, W_Q4K, FF>(c, L, x, bias, residual, out, query_only, norm_w, norm_eps, next);                           \
-	}
+#define X(KK, FF)                                                                                                               \
+	if (K == KK && F == FF)                                                                                                 \
+		return L.gate.kind == W_Q4K ? df_launch<W_Q4K, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm) \
+					    : df_launch<W_Q6K_R8, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm);
 	TIE_DF_SHAPES(X)
 #undef X
 	return TIE_CUDA_ENOTSUP;
@@ -538,15 +566,18 @@ bool decode_fused_supported(tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	if (n_tokens != 1 || !c->coop_ok || c->cfg.top_k > MAX_TOP_K || c->cfg.n_expert > 256)
 		return false;
-	return df_dispatch(c, L, nullptr, nullptr, nullptr, nullptr, true) == TIE_CUDA_OK;
+	return df_dispatch(c, L, 1, nullptr, nullptr, nullptr, nullptr, true, false) == TIE_CUDA_OK;
 }
 
-// norm_eps >= 0: x is the un-normed hidden row; the kernel applies RMSNorm (norm_w, or weight 1) first.
-// next: the block that runs after this one (its router matrix is requested into L2 meanwhile), or nullptr.
-int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
-			const float *norm_w, float norm_eps, const Layer *next)
+int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out)
 {
-	return df_dispatch(c, L, x, bias, residual, out, false, norm_w, norm_eps, next);
+	return df_dispatch(c, L, 1, x, bias, residual, out, false, false);
+}
+
+// hidden += block(RMSNorm(hidden)), for n_layers consecutive blocks from L on (same gate / up kind, decode_fused_supported).
+int launch_decode_fused_blocks(tie_cuda_ctx *c, const Layer &L, int n_layers, float *hidden)
+{
+	return df_dispatch(c, L, n_layers, hidden, nullptr, hidden, hidden, false, true);
 }
 
 }  // namespace tie
