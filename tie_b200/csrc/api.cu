@@ -5,6 +5,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <chrono>
 #include <mutex>
 #include <new>
 
@@ -310,16 +311,22 @@ int get_layer(tie_cuda_ctx *c, int layer, Layer **L)
 	return TIE_CUDA_OK;
 }
 
+// One token as one cooperative kernel?
+bool one_kernel_step(tie_cuda_ctx *c, const Layer &L, int n_tokens, unsigned flags)
+{
+	return (flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR &&
+	       !(flags & (TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2)) &&
+	       decode_fused_supported(c, L, n_tokens);
+}
+
 int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_tokens, const float *bias_dev,
-		   const float *residual, unsigned flags)
+		   const float *residual, unsigned flags, unsigned *host_status = nullptr)
 {
 	Scratch &s = c->s;
 	const int lfm2 = (flags & TIE_CUDA_ROUTE_LFM2) ? 1 : 0;
 	prof_mark(c, 0);
-	const bool decode_paths = (flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR && !(flags & TIE_CUDA_PATH_LEGACY_STREAM);
-	// one token: the whole block as one cooperative kernel
-	if (decode_paths && !lfm2 && !(flags & TIE_CUDA_PATH_DECODE_CHAIN) && decode_fused_supported(c, L, n_tokens)) {
-		const int rc = launch_decode_fused(c, L, x, bias_dev, residual, out);
+	if (one_kernel_step(c, L, n_tokens, flags)) {
+		const int rc = launch_decode_fused(c, L, x, bias_dev, residual, out, host_status);
 		if (rc != TIE_CUDA_ENOTSUP) {  // (not supported after all: the chain below)
 			if (rc)
 				return rc;
@@ -426,6 +433,7 @@ int h2d(tie_cuda_ctx *c, void *dst, const void *src, size_t bytes, void *pin)
 	} else {
 		// the staging buffer is reused by the next call: make sure the previous copy out of it is done
 		TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+		c->pin_x_busy = true;
 		memcpy(pin, src, bytes);
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(dst, pin, bytes, cudaMemcpyHostToDevice, c->stream));
 	}
@@ -458,6 +466,7 @@ CopyPlan copy_plan(size_t bytes)
 int copy_in_chunks(tie_cuda_ctx *c, const void *x, size_t bytes)
 {
 	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));  // the previous call's copies out of the staging are done
+	c->pin_x_busy = true;
 	if (!c->copy_pool && !(c->copy_pool = new (std::nothrow) CopyPool()))
 		return TIE_CUDA_ENOMEM;
 	const CopyPlan p = copy_plan(bytes);
@@ -983,9 +992,34 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 	}
 	const void *src = x;
 	if (!x_pinned) {
-		TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+		if (c->pin_x_busy)
+			TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+		c->pin_x_busy = true;
 		memcpy(c->pin_x, x, bytes);
 		src = c->pin_x;
+	}
+	// one token: the kernel stores the row and the status word into the pinned staging itself, and the call returns when
+	// they are there: no copy behind the kernel, and no wait for the end of its grid (45 -> us a call)
+	if (one_kernel_step(c, *L, n_tokens, flags)) {
+		volatile unsigned *word = reinterpret_cast<volatile unsigned *>(c->pin_out) - 1;
+		constexpr unsigned PENDING = ~0u;
+		*word = PENDING;
+		GraphKey k = {2, layer, n_tokens, src, c->pin_out, bias_dev, nullptr, kflags};
+		TRY(run_maybe_graphed(c, graph, k, [&]() -> int {
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->s.x, src, bytes, cudaMemcpyHostToDevice, c->stream));
+			return moe_ffn_device(c, *L, c->s.x, c->pin_out, n_tokens, bias_dev, nullptr, flags, const_cast<unsigned *>(word));
+		}));
+		const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(500);
+		while (*word == PENDING && std::chrono::steady_clock::now() < until)
+			;
+		std::atomic_thread_fence(std::memory_order_acquire);
+		if (*word == PENDING)  // (work in front of it on the stream, a time-out in the kernel, or the chain ran instead)
+			TRY(check_status(c));
+		else
+			TRY(report_status(c, *word));
+		c->pin_x_busy = false;
+		memcpy(out, c->pin_out, bytes);
+		return TIE_CUDA_OK;
 	}
 	GraphKey k = {2, layer, n_tokens, src, out_pinned ? out : c->pin_out, bias_dev, nullptr, kflags};
 	TRY(run_maybe_graphed(c, graph, k, [&]() -> int {
@@ -1098,9 +1132,7 @@ int tie_cuda_moe_block_inplace(tie_cuda_ctx *c, int layer, float *hidden_dev, in
 			       TIE_CUDA_PATH_NO_PAIR)};
 	TRY(run_maybe_graphed(c, flags & TIE_CUDA_GRAPH, k, [&]() -> int {
 		// one token: the RMSNorm is part of the one-kernel step
-		if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR &&
-		    !(flags & (TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2)) &&
-		    decode_fused_supported(c, *L, n_tokens)) {
+		if (one_kernel_step(c, *L, n_tokens, flags)) {
 			const int rc = launch_decode_fused_blocks(c, *L, 1, hidden_dev);
 			if (rc != TIE_CUDA_ENOTSUP) {
 				if (!rc) {
@@ -1129,13 +1161,11 @@ int tie_cuda_moe_stack_inplace(tie_cuda_ctx *c, int first_layer, int n_layers, f
 	TIE_CUDA_TRY(c, cudaSetDevice(c->device));
 	const unsigned pflags = flags & (TIE_CUDA_PATH_MASK | TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2 |
 					 TIE_CUDA_PATH_NO_PAIR);
-	const bool decode_paths = (pflags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR &&
-				  !(pflags & (TIE_CUDA_PATH_LEGACY_STREAM | TIE_CUDA_PATH_DECODE_CHAIN | TIE_CUDA_ROUTE_LFM2));
 	GraphKey k = {8, first_layer, n_tokens, hidden_dev, nullptr, nullptr, reinterpret_cast<const void *>((size_t)n_layers), pflags};
 	TRY(run_maybe_graphed(c, flags & TIE_CUDA_GRAPH, k, [&]() -> int {
 		for (int l = first_layer; l < first_layer + n_layers; l++) {
 			Layer &L = c->layers[l];
-			if (decode_paths && decode_fused_supported(c, L, n_tokens)) {
+			if (one_kernel_step(c, L, n_tokens, pflags)) {
 				// one token: one launch for as many blocks as share a kernel
 				int n = 1;
 				while (l + n < first_layer + n_layers && c->layers[l + n].gate.kind == L.gate.kind &&

@@ -160,6 +160,7 @@ struct tie_cuda_ctx {
 	int first_expert = 0, n_local = 0;
 	// pinned staging for host-pointer calls
 	float *pin_x = nullptr, *pin_out_base = nullptr, *pin_out = nullptr;  // (pin_out_base: as Scratch::out_base)
+	bool pin_x_busy = true;	 // a copy out of pin_x may still be in flight
 	tie::CopyPool *copy_pool = nullptr;	    // helper threads for pageable batches, started at the first one
 	cudaEvent_t copy_ev[tie::COPY_CHUNKS] = {nullptr};
 	int *pin_idx = nullptr;

@@ -72,6 +72,7 @@ struct DfArgs {
 	float *logits, *h, *out, *topk_w;
 	int *topk_idx;
 	unsigned *status, *sync;  // sync[0]: arrivals, sync[1]: epoch
+	unsigned *host_status;	  // or null: out is host memory; the status word goes here once all of out is there
 	int n_expert, top_k, first_expert, n_local;
 	int rpt_gu, tiles_gu, rpt_dn, tiles_dn;
 	uint32_t off_b, off_c, off_v, off_n;  // shared-memory offsets: down tiles, images of x, products, normed x
@@ -415,8 +416,16 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 				drain();
 				// the last CTA out advances the epoch for the next launch
 				target += (unsigned)G;
-				if (alive && atomicAdd(a.sync, 1u) == target - 1u)
+				if (a.host_status)
+					__threadfence_system();
+				if (alive && atomicAdd(a.sync, 1u) == target - 1u) {
 					atomicExch(a.sync + 1, target);
+					if (a.host_status) {
+						const unsigned st = *(volatile unsigned *)a.status;
+						__threadfence_system();
+						*(volatile unsigned *)a.host_status = st;
+					}
+				}
 			}
 			return;
 		}
@@ -483,7 +492,7 @@ DfLayer df_layer(const Layer &L)
 
 template <WKind KG, int K, int F>
 static int df_launch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float *x, const float *bias, const float *residual, float *out,
-		     bool query_only, bool norm)
+		     bool query_only, bool norm, unsigned *host_status)
 {
 	const DfPlan p = df_plan<KG, K, F>(c);
 	if (!p.ok)
@@ -520,6 +529,7 @@ static int df_launch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float 
 	a.off_v = (uint32_t)p.off_v;
 	a.off_n = (uint32_t)p.off_n;
 	a.norm_eps = norm ? c->cfg.norm_eps : -1.0f;
+	a.host_status = host_status;
 	auto kern = decode1_fused<KG, K, F>;
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
 	cudaLaunchConfig_t cfg = {};
@@ -548,15 +558,15 @@ static int df_launch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float 
 #define TIE_DF_SHAPES(X) X(2048, 768) X(512, 256)
 
 static int df_dispatch(tie_cuda_ctx *c, const Layer &L, int n_layers, const float *x, const float *bias, const float *residual, float *out,
-		       bool query_only, bool norm)
+		       bool query_only, bool norm, unsigned *host_status)
 {
 	if (L.gate.kind != L.up.kind)
 		return TIE_CUDA_ENOTSUP;
 	const int K = c->cfg.hidden, F = c->cfg.ffn_dim;
 #define X(KK, FF)                                                                                                               \
 	if (K == KK && F == FF)                                                                                                 \
-		return L.gate.kind == W_Q4K ? df_launch<W_Q4K, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm) \
-					    : df_launch<W_Q6K_R8, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm);
+		return L.gate.kind == W_Q4K ? df_launch<W_Q4K, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm, host_status) \
+					    : df_launch<W_Q6K_R8, KK, FF>(c, L, n_layers, x, bias, residual, out, query_only, norm, host_status);
 	TIE_DF_SHAPES(X)
 #undef X
 	return TIE_CUDA_ENOTSUP;
@@ -566,18 +576,20 @@ bool decode_fused_supported(tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	if (n_tokens != 1 || !c->coop_ok || c->cfg.top_k > MAX_TOP_K || c->cfg.n_expert > 256)
 		return false;
-	return df_dispatch(c, L, 1, nullptr, nullptr, nullptr, nullptr, true, false) == TIE_CUDA_OK;
+	return df_dispatch(c, L, 1, nullptr, nullptr, nullptr, nullptr, true, false, nullptr) == TIE_CUDA_OK;
 }
 
-int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out)
+// host_status: out is pinned host memory, and the status word follows it there when the row is complete.
+int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
+			unsigned *host_status)
 {
-	return df_dispatch(c, L, 1, x, bias, residual, out, false, false);
+	return df_dispatch(c, L, 1, x, bias, residual, out, false, false, host_status);
 }
 
 // hidden += block(RMSNorm(hidden)), for n_layers consecutive blocks from L on (same gate / up kind, decode_fused_supported).
 int launch_decode_fused_blocks(tie_cuda_ctx *c, const Layer &L, int n_layers, float *hidden)
 {
-	return df_dispatch(c, L, n_layers, hidden, nullptr, hidden, hidden, false, true);
+	return df_dispatch(c, L, n_layers, hidden, nullptr, hidden, hidden, false, true, nullptr);
 }
 
 }  // namespace tie

@@ -21,7 +21,8 @@ int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, co
 int launch_router_rows(tie_cuda_ctx *c, const float *x, const float *w, int n_rows, int in_dim, float *out);
 // decode_fused.cu
 bool decode_fused_supported(tie_cuda_ctx *c, const Layer &L, int n_tokens);
-int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out);
+int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
+			unsigned *host_status = nullptr);
 int launch_decode_fused_blocks(tie_cuda_ctx *c, const Layer &L, int n_layers, float *hidden);
 DfLayer df_layer(const Layer &L);
 // sort.cu
