@@ -128,3 +128,52 @@ def test_host_buffers_pageable_and_pinned(be, n_tokens, pinned):
         be.moe_ffn_ptr(0, xh, out, n_tokens, moe.HOST)
         assert np.array_equal(bits(out.numpy()), bits(want.cpu().numpy()))
         out.fill_(float("nan"))
+
+
+# One launch for a run of blocks with the same gate / up kind: down tensors of both kinds in it, and a block in the
+# middle that needs a launch of its own.
+def test_one_token_stack_of_mixed_blocks(small_shape, ref_silu_table):
+    import torch
+    from tie_b200 import moe
+    s = small_shape
+    n_gu, n_dn = s.n_expert * s.ffn_dim * (s.hidden // 256), s.n_expert * s.hidden * (s.ffn_dim // 256)
+    b = moe.MoeBackend(hidden=s.hidden, n_expert=s.n_expert, top_k=s.top_k, ffn_dim=s.ffn_dim, max_tokens=4, silu_table=ref_silu_table,
+                       n_layers=7)
+    try:
+        for l in range(7):
+            m = synth.make_layer(30 + l, s)
+            if l in (1, 2, 5):
+                m.down, m.down_type = synth.q4k_blocks(30 + l, synth.STREAM_DOWN, n_dn), synth.GGML_Q4_K
+            if l == 3:
+                m.gate, m.gate_type = synth.q6k_blocks(33, synth.STREAM_GATE, n_gu), synth.GGML_Q6_K
+                m.up, m.up_type = synth.q6k_blocks(33, synth.STREAM_UP, n_gu), synth.GGML_Q6_K
+            b.upload_layer(l, m, ffn_norm_w=None if l == 4 else np.linspace(0.9, 1.1, s.hidden, dtype=np.float32))
+        h0 = torch.from_numpy(synth.make_x(6, 1, s.hidden)).cuda()
+        want, got = h0.clone(), h0.clone()
+        for l in range(7):
+            b.moe_block_inplace_ptr(l, want, 1, moe.DEVICE)
+        l0 = b.launch_count
+        b.moe_stack_inplace_ptr(0, 7, got, 1, moe.DEVICE)
+        assert b.launch_count - l0 == 3
+        assert np.array_equal(bits(got.cpu().numpy()), bits(want.cpu().numpy())) and np.isfinite(got.cpu().numpy()).all()
+    finally:
+        b.close()
+
+
+# One token on host buffers: the result comes without a copy, also when the stream is still busy and from a graph.
+def test_one_token_host_calls(be):
+    import torch
+    from tie_b200 import moe
+    out = np.empty((1, 2048), np.float32)
+    big = torch.from_numpy(synth.make_x(0, 1100)).cuda()
+    big_out = torch.empty_like(big)
+    for i in range(4):
+        x = synth.make_x(0, 1, first_token=700 + i)
+        want = torch.empty(1, 2048, device="cuda")
+        be.moe_ffn_ptr(0, torch.from_numpy(x).cuda(), want, 1, moe.DEVICE)
+        for flags in (0, moe.GRAPH):
+            for _ in range(3):
+                be.moe_ffn_ptr(0, big, big_out, 1100, moe.DEVICE | moe.NO_SYNC)
+            out[:] = np.nan
+            be.moe_ffn_ptr(0, x, out, 1, moe.HOST | flags)
+            assert np.array_equal(bits(out), bits(want.cpu().numpy()))

@@ -981,6 +981,34 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 			return TIE_CUDA_OK;
 		return check_status(c);
 	}
+	if (one_kernel_step(c, *L, n_tokens, flags)) {
+		// One token: the kernel stores its result and the status word into the pinned staging itself, and the call returns
+		// when they have arrived: no copy behind the kernel, no wait for the end of its grid (45 -> 37 us a call).
+		if (c->pin_x_busy)
+			TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
+		c->pin_x_busy = true;
+		memcpy(c->pin_x, x, bytes);
+		volatile unsigned *word = reinterpret_cast<volatile unsigned *>(c->pin_out) - 1;
+		constexpr unsigned PENDING = ~0u;
+		*word = PENDING;
+		std::atomic_thread_fence(std::memory_order_release);
+		GraphKey k = {2, layer, n_tokens, c->pin_x, c->pin_out, bias_dev, nullptr, kflags};
+		TRY(run_maybe_graphed(c, graph, k, [&]() -> int {
+			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->s.x, c->pin_x, bytes, cudaMemcpyHostToDevice, c->stream));
+			return moe_ffn_device(c, *L, c->s.x, c->pin_out, n_tokens, bias_dev, nullptr, flags, const_cast<unsigned *>(word));
+		}));
+		const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(500);
+		while (*word == PENDING && std::chrono::steady_clock::now() < until)
+			;
+		std::atomic_thread_fence(std::memory_order_acquire);
+		if (*word == PENDING)  // (work in front of it on the stream, a time-out in the kernel, or the chain ran instead)
+			TRY(check_status(c));
+		else
+			TRY(report_status(c, *word));
+		c->pin_x_busy = false;
+		memcpy(out, c->pin_out, bytes);
+		return TIE_CUDA_OK;
+	}
 	// host pointers: pinned user memory is copied directly, pageable memory goes through the
 	// context's pinned staging buffers
 	const bool x_pinned = is_pinned_host(x), out_pinned = is_pinned_host(out);
@@ -997,29 +1025,6 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 		c->pin_x_busy = true;
 		memcpy(c->pin_x, x, bytes);
 		src = c->pin_x;
-	}
-	// one token: the kernel stores the row and the status word into the pinned staging itself, and the call returns when
-	// they are there: no copy behind the kernel, and no wait for the end of its grid (45 -> us a call)
-	if (one_kernel_step(c, *L, n_tokens, flags)) {
-		volatile unsigned *word = reinterpret_cast<volatile unsigned *>(c->pin_out) - 1;
-		constexpr unsigned PENDING = ~0u;
-		*word = PENDING;
-		GraphKey k = {2, layer, n_tokens, src, c->pin_out, bias_dev, nullptr, kflags};
-		TRY(run_maybe_graphed(c, graph, k, [&]() -> int {
-			TIE_CUDA_TRY(c, cudaMemcpyAsync(c->s.x, src, bytes, cudaMemcpyHostToDevice, c->stream));
-			return moe_ffn_device(c, *L, c->s.x, c->pin_out, n_tokens, bias_dev, nullptr, flags, const_cast<unsigned *>(word));
-		}));
-		const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(500);
-		while (*word == PENDING && std::chrono::steady_clock::now() < until)
-			;
-		std::atomic_thread_fence(std::memory_order_acquire);
-		if (*word == PENDING)  // (work in front of it on the stream, a time-out in the kernel, or the chain ran instead)
-			TRY(check_status(c));
-		else
-			TRY(report_status(c, *word));
-		c->pin_x_busy = false;
-		memcpy(out, c->pin_out, bytes);
-		return TIE_CUDA_OK;
 	}
 	GraphKey k = {2, layer, n_tokens, src, out_pinned ? out : c->pin_out, bias_dev, nullptr, kflags};
 	TRY(run_maybe_graphed(c, graph, k, [&]() -> int {

@@ -184,6 +184,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			reinterpret_cast<float4 *>(ws)[tid] = wv;
 		}
 		__syncthreads();
+		if (layer == 0)
+			target = sh.base;
 		// ---------------- (RMSNorm of the row, every CTA for itself: rms_norm_f32_f32_f32_avx2, math_avx2.c:56-97) ----------------
 		if (a.norm_eps >= 0.0f) {
 			if (warp == 0) {
@@ -230,8 +232,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			if (lane == 0)
 				sh.x_inv[b] = inv;
 		}
-		if (layer == 0)
-			target = (__syncthreads(), sh.base);
 		DF_STAMP(1);
 		if (!df_grid_barrier(a.sync, target += (unsigned)G, &sh, a.status))
 			return;	 // nothing of this CTA is in flight yet
