@@ -26,16 +26,21 @@ namespace tie {
 constexpr int DEC_MAX_NB = 8;  // super-blocks per row
 
 // Sum of a row's products over its super-blocks, in order (decode_fused.cu adds in the same order).
+// A CTA walks n_tiles row tiles of its slot: the image of x is made once, a matrix's next tile is loaded into the
+// registers that its products have just left and lands under the other matrix's, and one more warp adds up a
+// tile and stores h while the others are at the next.
+// A block of 3 / 4 / 6 / 8 tokens 46.2 / 58.6 / 69.7 / 84.7 -> 44.4 / 57.2 / 64.6 / 84.8 us against a CTA per tile (4 tokens:
+// 53 MB in 16 us; the pipes are 20 - 45 % busy, the warps wait for one another, for loads and for the products).
 template <WKind KIND>
-__global__ void __launch_bounds__(DEC_MAX_NB * 32, 2)
-decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert, int nb,
+__global__ void __launch_bounds__((DEC_MAX_NB + 1) * 32, 2)
+decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert, int nb, int n_tiles,
 	       const float *__restrict__ x, int top_k, const int *__restrict__ topk_idx, float *__restrict__ h, int first_expert,
 	       int n_local, const float *__restrict__ silu, unsigned *__restrict__ status, int n_expert_all)
 {
 	__shared__ __align__(16) uint8_t img[DEC_MAX_NB][XImage<KIND>::BYTES];
-	__shared__ float red[DEC_MAX_NB][2][16];
+	__shared__ float red[2][DEC_MAX_NB][2][16];
 	const int slot = blockIdx.y;  // (token, j)
-	const int r0 = blockIdx.x * 16;
+	const int r0 = blockIdx.x * n_tiles * 16, r1 = min(r0 + n_tiles * 16, rows_per_expert);
 	pdl_wait();	// the router's top-k (and x) are visible from here on
 	pdl_trigger();	// the down kernel may start fetching its weights
 	const int ge = topk_idx[slot];
@@ -47,33 +52,45 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 		return;
 	}
 	const int lane = threadIdx.x & 31, b = threadIdx.x >> 5;
-	const size_t off = (size_t)le * expert_stride + tile_offset<KIND>(nb, r0);
+	if (b == nb) {
+		for (int r = r0, buf = 0; r < r1; r += 16, buf ^= 1) {
+			__syncthreads();
+			float sum = red[buf][0][lane >> 4][lane & 15];
+			for (int i = 1; i < nb; i++)
+				sum = __fadd_rn(sum, red[buf][i][lane >> 4][lane & 15]);
+			const float up = __shfl_down_sync(0xffffffffu, sum, 16);
+			if (lane < 16)
+				h[(size_t)slot * rows_per_expert + r + lane] = swiglu_lut(silu, sum, up);
+		}
+		return;
+	}
+	wg += (size_t)le * expert_stride;
+	wu += (size_t)le * expert_stride;
 	MmaRows<KIND> g, u;
-	g.load(wg + off, nb, b, lane);
-	u.load(wu + off, nb, b, lane);
+	g.load(wg + tile_offset<KIND>(nb, r0), nb, b, lane);
+	u.load(wu + tile_offset<KIND>(nb, r0), nb, b, lane);
 	const float4 *xp = reinterpret_cast<const float4 *>(x + (size_t)(slot / top_k) * nb * QK_K + b * QK_K) + 2 * lane;
 	const float4 x0 = xp[0], x1 = xp[1];
 	const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 	const float inv = x_image<KIND>(v, img[b], lane);
-	float2 r, s;
-	g.dot(img[b], inv, lane, r, s);
-	if ((lane & 3) == 0) {
-		red[b][0][lane >> 2] = r.x * s.x;
-		red[b][0][(lane >> 2) + 8] = r.y * s.y;
-	}
-	u.dot(img[b], inv, lane, r, s);
-	if ((lane & 3) == 0) {
-		red[b][1][lane >> 2] = r.x * s.x;
-		red[b][1][(lane >> 2) + 8] = r.y * s.y;
-	}
-	__syncthreads();
-	if (threadIdx.x < 32) {
-		float sum = red[0][lane >> 4][lane & 15];
-		for (int i = 1; i < nb; i++)
-			sum = __fadd_rn(sum, red[i][lane >> 4][lane & 15]);
-		const float up = __shfl_down_sync(0xffffffffu, sum, 16);
-		if (lane < 16)
-			h[(size_t)slot * rows_per_expert + r0 + lane] = swiglu_lut(silu, sum, up);
+	for (int r = r0, buf = 0; r < r1; r += 16, buf ^= 1) {
+		const bool more = r + 16 < r1;
+		float2 p, s;
+		g.dot(img[b], inv, lane, p, s);
+		if (more)
+			g.load(wg + tile_offset<KIND>(nb, r + 16), nb, b, lane);
+		if ((lane & 3) == 0) {
+			red[buf][b][0][lane >> 2] = p.x * s.x;
+			red[buf][b][0][(lane >> 2) + 8] = p.y * s.y;
+		}
+		u.dot(img[b], inv, lane, p, s);
+		if (more)
+			u.load(wu + tile_offset<KIND>(nb, r + 16), nb, b, lane);
+		if ((lane & 3) == 0) {
+			red[buf][b][1][lane >> 2] = p.x * s.x;
+			red[buf][b][1][(lane >> 2) + 8] = p.y * s.y;
+		}
+		__syncthreads();
 	}
 }
 
@@ -244,8 +261,8 @@ static size_t dec_down_smem(const Layer &L, int top_k)
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	// every (token, slot) row by itself up to the batch where grouping the experts' rows pays for its passes
-	// around the products (run_experts): 4 / 6 / 8 / 10 / 13 / 20 tokens of this model's shape 59 / 70 / 86 / 100 / 122 / 173 us
-	// a block here, 72 / 81 / 87 / 94 / 102 / 113 grouped
+	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 58 / 65 / 72 / 85 us
+	// a block here, 70 / 79 / 81 / 85 grouped; 10 / 13 / 20 tokens 100 / 122 / 173 here, 93 / 98 / 110 grouped
 	const int n_rows = n_tokens * c->cfg.top_k;
 	return (n_tokens <= 4 || 2 * n_rows <= c->n_local) && n_rows <= 65535 && L.gate.kind == L.up.kind &&
 	       L.gate.k <= DEC_MAX_NB * QK_K && L.gate.rows % 16 == 0 && L.down.rows % 16 == 0 && L.down.k <= DEC_MAX_NB * QK_K &&
@@ -267,7 +284,10 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 {
 	const int n_rows = n_tokens * c->cfg.top_k, nb = L.gate.k / QK_K;
 	auto kern = L.gate.kind == W_Q4K ? decode_gate_up<W_Q4K> : decode_gate_up<W_Q6K_R8>;
-	return launch_kernel(c, true, 1, kern, dim3(L.gate.rows / 16, n_rows), 32 * nb, 0, L.gate.ptr, L.up.ptr, L.gate.expert_stride, L.gate.rows, nb, x,
+	// as many tiles a CTA as bring the grid to one wave of two CTAs per SM
+	const int tiles = L.gate.rows / 16, n_tiles = (tiles * n_rows + 2 * c->sm_count - 1) / (2 * c->sm_count);
+	return launch_kernel(c, true, 1, kern, dim3((tiles + n_tiles - 1) / n_tiles, n_rows), 32 * (nb + 1), 0, L.gate.ptr, L.up.ptr,
+			  L.gate.expert_stride, L.gate.rows, nb, n_tiles, x,
 			  c->cfg.top_k, c->s.topk_idx, c->s.h, c->first_expert, c->n_local, c->silu, c->s.status,
 			  foreign_slots_ok ? c->cfg.n_expert : 0);
 }
