@@ -79,8 +79,6 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TRY(dev_alloc(c, &s.hq, s.rows_pad * XF));
 	TRY(dev_alloc(c, &s.route_counter, (T + 3) / 4));
 	TIE_CUDA_TRY(c, cudaMemset(s.route_counter, 0, (T + 3) / 4 * sizeof(int)));
-	TRY(dev_alloc(c, &s.counter, 1));
-	TIE_CUDA_TRY(c, cudaMemset(s.counter, 0, sizeof(int)));
 	TRY(dev_alloc(c, &s.dec_sync, 2));
 	TIE_CUDA_TRY(c, cudaMemset(s.dec_sync, 0, 2 * sizeof(unsigned)));
 	TRY(dev_alloc(c, &s.row_expert, R));
@@ -340,10 +338,7 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 	// decode and small batches: three launches — router with fused selection, gate/up, down + combine
 	if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR && !(flags & TIE_CUDA_PATH_LEGACY_STREAM) &&
 	    decode_supported(c, L, n_tokens)) {
-		if (lfm2 || n_tokens > 4)
-			TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
-		else
-			TRY(launch_router_decode_fused(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w));
+		TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
 		prof_mark(c, 1);
 		c->last_used_tc = false;
 		c->last_direct_rows = n_tokens * c->cfg.top_k;
@@ -777,7 +772,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	}
 	Scratch &s = c->s;
 	void *dev_ptrs[] = {s.x,     s.out_base, s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
-			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.counter, s.row_expert, c->silu,  c->row_x,
+			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.row_expert, c->silu,  c->row_x,
 			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
 			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
@@ -1409,7 +1404,7 @@ int tie_cuda_ep_publish(tie_cuda_ctx *c, int layer, const float *x, int n_tokens
 		TIE_CUDA_TRY(c, cudaSetDevice(c->device));
 		prof_mark(c, 0);
 		TRY(launch_ep_signal(c, 0));
-		TRY(launch_router_decode_fused(c, x, L->router_w, router_bias, n_tokens, c->s.logits, c->s.topk_idx, c->s.topk_w));
+		TRY(launch_router(c, x, L->router_w, router_bias, n_tokens, c->s.logits, c->s.topk_idx, c->s.topk_w));
 		prof_mark(c, 1);
 		prof_mark(c, 2);
 		ep.phase = 1;

@@ -101,7 +101,6 @@ struct Scratch {
 	__half *hq = nullptr;  // [Rpad][xq_cols(F)]
 	unsigned *status = nullptr;		    // [1], the word in front of out
 	int *route_counter = nullptr;		    // [(T + 3) / 4] CTAs done per token tile of the batched router (zero at rest)
-	int *counter = nullptr;			    // [1] last-CTA counter of the fused decode router (zero at rest)
 	unsigned *dec_sync = nullptr;		    // [2] arrivals and epoch of the one-kernel decode step's grid barriers
 	int *row_expert = nullptr;		    // [R] staging for expert_rows
 	// expert-parallel dispatch state (sort of this rank's rows over ALL experts)

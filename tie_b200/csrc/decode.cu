@@ -261,7 +261,7 @@ static size_t dec_down_smem(const Layer &L, int top_k)
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	// every (token, slot) row by itself up to the batch where grouping the experts' rows pays for its passes
-	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 58 / 65 / 72 / 85 us
+	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 51 / 63 / 70 / 83 us
 	// a block here, 70 / 79 / 81 / 85 grouped; 10 / 13 / 20 tokens 100 / 122 / 173 here, 93 / 98 / 110 grouped
 	const int n_rows = n_tokens * c->cfg.top_k;
 	return (n_tokens <= 4 || 2 * n_rows <= c->n_local) && n_rows <= 65535 && L.gate.kind == L.up.kind &&

@@ -7,7 +7,7 @@
 // with two grid-wide barriers:
 //
 //   R  CTA e < n_expert: logit e by warp 0, the AVX2 lane order replayed (8 chains of sequential fused
-//      multiply-adds, hsum tree: bit-exact, as router_decode_fused); other warps meanwhile make the
+//      multiply-adds, hsum tree: bit-exact, as router_batch); other warps meanwhile make the
 //      images of x (mma_dot.cuh) for its gate/up tile
 //   -- barrier --
 //      every CTA selects the experts itself from the logits (one warp, hardware max/min reductions:

@@ -9,8 +9,6 @@ struct EpPush;
 int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
 		  int *topk_idx, float *topk_w, int lfm2 = 0, const EpPush *push = nullptr, bool *push_taken = nullptr);
 int router_setup(tie_cuda_ctx *c);
-int launch_router_decode_fused(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
-			       int *topk_idx, float *topk_w);
 // decode.cu
 int decode_setup(tie_cuda_ctx *c);
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens);

@@ -12,6 +12,7 @@ __global__ void __launch_bounds__(128) rms_norm_rows(const float *__restrict__ x
 						     float *__restrict__ o, int n_tokens, int n, float eps)
 {
 	extern __shared__ float sm[];
+	pdl_trigger();	// (the router fetches its weights meanwhile)
 	const int wib = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int t = blockIdx.x * (blockDim.x >> 5) + wib;
 	if (t >= n_tokens)

@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__res
 // how many SMs pull the 1 MB of router weights, a large one the multiply-adds and the shared-memory loads
 // beside them (wider loads move no more per cycle), so the tile grows with the batch (TIE_RT_TILES).  The
 // CTA that finishes a token tile last (a counter per tile, nobody waits) selects for all its tokens.
+// A small grid starts beside the kernel in front of it and fetches its first weights before it waits for the tokens.
 // Measured (logits + selection): 4 tokens 14.4 -> 8.8 us, 13 28.7 -> 10.3, 64 28.7 -> 12.3, 333 29 -> 26, 512 29 -> 26.7,
 // 1000 41 -> 37, 2000 68 -> 54, 4096 94 -> 93.
 //
@@ -112,6 +113,7 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 	// rank's tokens into every rank's memory while the others compute the logits; they share nothing
 	// with them.
 	if (push.x && (int)blockIdx.y * TE >= n_expert) {
+		pdl_wait();
 		const int row = (int)blockIdx.y - n_expert / TE, cta = row * (int)gridDim.x + (int)blockIdx.x;
 		if (cta < push.n_ctas)
 			ep_push_tokens_cta(push, cta, push.n_ctas);
@@ -122,17 +124,17 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 	const int l = threadIdx.x & 7, g4 = threadIdx.x >> 5;
 	const int tg = ((threadIdx.x >> 3) & 1) + 2 * (g4 % (C::TG / 2)), eg = ((threadIdx.x >> 4) & 1) + 2 * (g4 / (C::TG / 2));
 	const int n_chunks = hidden / KC;
-	auto fetch = [&](int c) {  // (one group a call, an empty one past the end)
+	auto fetch = [&](int c, bool tokens, bool weights) {
 		if (c < n_chunks) {
 #pragma unroll
 			for (int j = 0; j < C::LD; j++) {
 				const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
 				const float *src = row < TT ? x + (size_t)min(t0 + row, n_tokens - 1) * hidden	// (rows past the end: computed, dropped)
 							    : w + (size_t)(e0 + row - TT) * hidden;
-				ptx::cp_async16(ptx::smem_u32(rsm + (c % C::STAGES) * C::STAGE + row * C::PITCH + 4 * c4), src + c * KC + 4 * c4);
+				if (row < TT ? tokens : weights)
+					ptx::cp_async16(ptx::smem_u32(rsm + (c % C::STAGES) * C::STAGE + row * C::PITCH + 4 * c4), src + c * KC + 4 * c4);
 			}
 		}
-		ptx::cp_async_commit();
 	};
 	float acc[TPT][EPT];
 #pragma unroll
@@ -142,11 +144,18 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 			acc[j][b] = 0.0f;
 #pragma unroll
 	for (int c = 0; c < C::STAGES - 1; c++)
-		fetch(c);
+		fetch(c, false, true);
+	pdl_wait();	// the tokens may be the work of the kernel before this one
+#pragma unroll
+	for (int c = 0; c < C::STAGES - 1; c++) {
+		fetch(c, true, false);
+		ptx::cp_async_commit();
+	}
 	for (int c = 0; c < n_chunks; c++) {
 		ptx::cp_async_wait<C::STAGES - 2>();
 		__syncthreads();  // (chunk c is here for everyone, and everyone is done with the buffer of chunk c - 1)
-		fetch(c + C::STAGES - 1);
+		fetch(c + C::STAGES - 1, true, true);
+		ptx::cp_async_commit();	 // (an empty group past the end)
 		const float *buf = rsm + (c % C::STAGES) * C::STAGE + l, *xs = buf + tg * C::PITCH, *ws = buf + (TT + eg) * C::PITCH;
 #pragma unroll C::UNROLL
 		for (int g = 0; g < KC / 8; g++) {
@@ -185,6 +194,9 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 		__threadfence();
 	}
 	__syncthreads();
+	// The decode kernels' CTAs may come now and wait for this grid: before the selection, not before the products (from
+	// the start of the grid a block of 6 tokens takes 69.4 us, from here 62.5, without 63.4).
+	pdl_trigger();
 	if (!s_last)
 		return;
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -251,86 +263,6 @@ __global__ void __launch_bounds__(128) router_topk(const float *__restrict__ log
 	topk_softmax_warp(logits, warp, lane, n_expert, top_k, topk_idx, topk_w);
 }
 
-// Decode: logits as in router_logits_decode, and the CTA that finishes last (a counter, no
-// waiting) runs the selection for all tokens, saving a launch on the latency-bound path.
-__global__ void __launch_bounds__(256) router_decode_fused(const float *__restrict__ x, const float *__restrict__ w,
-							   const float *__restrict__ bias, float *__restrict__ logits, int n_tokens,
-							   int hidden, int n_expert, int top_k, int *__restrict__ topk_idx,
-							   float *__restrict__ topk_w, int *__restrict__ counter)
-{
-	extern __shared__ float sm[];
-	__shared__ int s_last;
-	float *ws = sm;
-	float *xs = sm + hidden;
-	const int xstride = hidden + 8;
-	const int e = blockIdx.x;
-	// let a dependent-launched successor (the decode gate/up kernel) become resident now; it waits
-	// for this grid's results itself.  The wait below covers a predecessor that was itself
-	// launched the same way.
-	asm volatile("griddepcontrol.wait;" ::: "memory");
-	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-	// all loads of the staging are issued before the first store (at most 8 wide loads per thread)
-	{
-		const float4 *wr4 = reinterpret_cast<const float4 *>(w + (size_t)e * hidden);
-		const int nw = hidden / 4, nx = n_tokens * (hidden / 4);
-		float4 v[8];
-#pragma unroll
-		for (int j = 0; j < 8; j++) {
-			const int i = threadIdx.x + 256 * j;
-			if (i < nw)
-				v[j] = __ldg(wr4 + i);
-			else if (i - nw < nx && i >= nw)
-				v[j] = __ldg(reinterpret_cast<const float4 *>(x) + (i - nw));
-		}
-#pragma unroll
-		for (int j = 0; j < 8; j++) {
-			const int i = threadIdx.x + 256 * j;
-			if (i < nw) {
-				reinterpret_cast<float4 *>(ws)[i] = v[j];
-			} else if (i - nw < nx) {
-				const int k = i - nw, tt = k / (hidden / 4), c4 = k % (hidden / 4);
-				*reinterpret_cast<float4 *>(xs + (size_t)tt * xstride + 4 * c4) = v[j];
-			}
-		}
-		for (int i = threadIdx.x + 2048; i < nw + nx; i += 256) {  // sizes beyond 8 loads per thread
-			if (i < nw) {
-				reinterpret_cast<float4 *>(ws)[i] = __ldg(wr4 + i);
-			} else {
-				const int k = i - nw, tt = k / (hidden / 4), c4 = k % (hidden / 4);
-				*reinterpret_cast<float4 *>(xs + (size_t)tt * xstride + 4 * c4) = __ldg(reinterpret_cast<const float4 *>(x) + k);
-			}
-		}
-	}
-	__syncthreads();
-	const int tt = threadIdx.x >> 3, l = threadIdx.x & 7;
-	float acc = 0.0f;
-	if (tt < n_tokens) {
-		const float *xr = xs + (size_t)tt * xstride;
-#pragma unroll 16
-		for (int i = 0; i < hidden / 8; i++)
-			acc = __fmaf_rn(xr[8 * i + l], ws[8 * i + l], acc);
-	}
-	float r = hsum8_lanes(acc);
-	if (l == 0 && tt < n_tokens) {
-		if (bias)
-			r = __fadd_rn(r, bias[e]);
-		__stcg(&logits[(size_t)tt * n_expert + e], r);
-	}
-	__threadfence();
-	__syncthreads();
-	if (threadIdx.x == 0)
-		s_last = (atomicAdd(counter, 1) == (int)gridDim.x - 1);
-	__syncthreads();
-	if (!s_last)
-		return;
-	__threadfence();
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	for (int t = warp; t < n_tokens; t += 8)
-		topk_softmax_warp(logits, t, lane, n_expert, top_k, topk_idx, topk_w);
-	if (threadIdx.x == 0)
-		*counter = 0;
-}
-
 // lfm2 = 0: bias (optional) is added to the logits, top-k + softmax over the selected logits
 // (Qwen3-MoE).  lfm2 = 1: LFM2-MoE routing, bias (optional) is the selection bias exp_probs_b.
 // push (expert-parallel steps): the kernel of the logits takes the hand-over of this rank's tokens to
@@ -378,35 +310,25 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 	if (pick < 0)
 		return TIE_CUDA_ENOTSUP;
 	at = 0;
-#define TIE_RT_RUN(A, B, ...)                                                                                                              \
-	if (at++ == pick) {                                                                                                          \
-		using C = __VA_ARGS__;                                                                                               \
-		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                                    \
-		f.n_ctas = rt_push_ctas(c, grid.x * (E / C::TE), grid.x * RT_PUSH_ROWS);                                             \
-		router_batch<C><<<grid, C::THREADS, C::SMEM, c->stream>>>(x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2, \
-									  sel_bias, c->s.route_counter, f);                          \
+	// (dependent where it is one wave: a grid that waits beside its predecessor then takes nothing from it)
+	int rc = TIE_CUDA_OK;
+#define TIE_RT_RUN(A, B, ...)                                                                                              \
+	if (at++ == pick) {                                                                                                \
+		using C = __VA_ARGS__;                                                                                     \
+		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                          \
+		f.n_ctas = rt_push_ctas(c, grid.x * (E / C::TE), grid.x * RT_PUSH_ROWS);                                   \
+		rc = launch_kernel(c, (int)(grid.x * grid.y) <= c->sm_count, 1, router_batch<C>, grid, C::THREADS, C::SMEM, \
+				   x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2, sel_bias, c->s.route_counter, f); \
 	}
 	TIE_RT_TILES(TIE_RT_RUN)
 #undef TIE_RT_RUN
-	TIE_CUDA_LAUNCHED(c);
-	return TIE_CUDA_OK;
-}
-
-int launch_router_decode_fused(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
-			       int *topk_idx, float *topk_w)
-{
-	const int H = c->cfg.hidden, E = c->cfg.n_expert;
-	size_t smem = ((size_t)H + (size_t)n_tokens * (H + 8)) * sizeof(float);
-	router_decode_fused<<<E, 256, smem, c->stream>>>(x, w, bias, logits, n_tokens, H, E, c->cfg.top_k, topk_idx, topk_w, c->s.counter);
-	TIE_CUDA_LAUNCHED(c);
-	return TIE_CUDA_OK;
+	return rc;
 }
 
 // Opt-in shared-memory sizes are set once per context (never inside a stream capture).
 int router_setup(tie_cuda_ctx *c)
 {
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_decode_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
 #define TIE_RT_ATTR(A, B, ...) \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, __VA_ARGS__::SMEM));
 	TIE_RT_TILES(TIE_RT_ATTR)
