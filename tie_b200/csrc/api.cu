@@ -89,6 +89,7 @@ int alloc_scratch(tie_cuda_ctx *c)
 	TRY(dev_alloc(c, &s.ep_n_active, 1));
 	TRY(dev_alloc(c, &s.ep_perm, R));
 	TRY(dev_alloc(c, &s.ep_inv, R));
+	TRY(dev_alloc(c, &s.inv, R));
 	TIE_CUDA_TRY(c, cudaMemset(s.status, 0, sizeof(unsigned)));
 	TIE_CUDA_TRY(c, cudaMemset(s.n_active, 0, sizeof(int)));
 	// rows past the last real one are read (never used) by the tensor path: keep them finite
@@ -282,7 +283,7 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	prof_mark(c, 2);
 	if (use_tc) {
 		const bool sums = L.gate.kind == W_Q4K;	 // the Q4_K "min" term needs the sub-block sums of the inputs
-		TRY(launch_split_rows(c, x_src, c->s.perm, src_div, n_rows, c->cfg.hidden, c->s.xs_hi, c->s.xs_lo,
+		TRY(launch_split_rows(c, x_src, c->s.inv, src_div, n_rows / src_div, c->cfg.hidden, c->s.xs_hi, c->s.xs_lo,
 				      sums ? c->s.xq : nullptr));
 		prof_mark(c, 3);
 		TRY(launch_tc_gate_up(c, L, n_tile));
@@ -773,7 +774,7 @@ void tie_cuda_destroy(tie_cuda_ctx *c)
 	Scratch &s = c->s;
 	void *dev_ptrs[] = {s.x,     s.out_base, s.logits, s.bias,  s.topk_idx, s.topk_w, s.counts, s.offsets, s.tile_start, s.active, s.n_active,
 			    s.perm,  s.h,     s.y,	s.xs_hi, s.hs_hi,  s.row_expert, c->silu,  c->row_x,
-			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv,
+			    c->row_o, s.ep_counts, s.ep_offsets, s.ep_tile_start, s.ep_active, s.ep_n_active, s.ep_perm, s.ep_inv, s.inv,
 			    s.tile_info, s.xq, s.hq, s.dec_sync, c->df_table, s.sort_hist, s.route_counter};
 	for (void *p : dev_ptrs)
 		if (p)

@@ -90,6 +90,7 @@ struct Scratch {
 	int *active = nullptr;	    // [E]  compact list of experts with rows
 	int *n_active = nullptr;    // [1]
 	int *perm = nullptr;	    // [R]  sorted position -> row id
+	int *inv = nullptr;	    // [R] where row r stands in perm
 	int *sort_hist = nullptr;   // [slices][experts] rows per (slice of SORT_SLICE rows, expert)
 	size_t sort_hist_cap = 0;
 	float *h = nullptr;	    // [R][F]  fp32 activations (stream path), sorted order

@@ -27,7 +27,7 @@ DfLayer df_layer(const Layer &L);
 struct SortBufs {
 	int *counts, *offsets, *tile_start, *active, *n_active, *perm;
 	int4 *tile_info;  // optional: one entry per token tile (expert, first sorted row, rows, 0)
-	// optional (expert-parallel publish): inv[row id] = where the row stands in perm, and, with
+	// optional: inv[row id] = where the row stands in perm (-1: nowhere), and (expert-parallel publish), with
 	// owner_div = experts per GPU and top_k > 0, EP_FIRST_OF_TOKEN set in the entries of perm
 	int *inv = nullptr;
 	int owner_div = 0, top_k = 0;
@@ -46,7 +46,7 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 		   const int *pos = nullptr);
 int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, const int *perm, int src_div, int n_rows,
 		       float *rows_out, int *expert_out, int *inv);
-int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_div, int n_rows, int n_cols, __half *hi,
+int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out, int n_src, int n_cols, __half *hi,
 		      __half *lo, __half *xq);
 int launch_swiglu(tie_cuda_ctx *c, float *gate, const float *up, int n);
 // n_rows_dev != null: the row count is read on the device and n_rows CTAs stride over the rows

@@ -78,84 +78,97 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 	}
 }
 
-// Eight consecutive values v[0..7] (k = k0 .. k0+7, k0 a multiple of 8) -> their fp16 hi and lo
-// halves (hi = rn16(v), lo = rn16(v - hi)) in the operand order [k0, k2, k1, k3] per group of 4, as
-// one 16-byte store each; optionally the sum over the 32-wide sub-block the values belong to (four
-// neighbouring lanes hold one sub-block), split the same way.
-__device__ __forceinline__ void split8_store(const float v[8], int k0, __half *__restrict__ hi_row, __half *__restrict__ lo_row,
-					     __half *__restrict__ q_row, int lane)
-{
-	uint32_t h[4], l[4];
+// Eight consecutive values v[0..7] (k = k0 .. k0+7, k0 a multiple of 8) as their fp16 hi and lo
+// halves (hi = rn16(v), lo = rn16(v - hi)) in the operand order [k0, k2, k1, k3] per group of 4, and the
+// sum over the 32-wide sub-block they belong to (four neighbouring lanes hold one), split the same way.
+struct Split8 {
+	uint4 hi, lo;
+	__half sum_hi, sum_lo;
+	__device__ __forceinline__ void make(const float v[8], bool sums)
+	{
+		uint32_t h[4], l[4];
 #pragma unroll
-	for (int g = 0; g < 2; g++) {
-		const float a = v[4 * g], b = v[4 * g + 1], c = v[4 * g + 2], d = v[4 * g + 3];
-		const __half2 h0 = __floats2half2_rn(a, c), h1 = __floats2half2_rn(b, d);
-		const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-		const __half2 l0 = __floats2half2_rn(a - f0.x, c - f0.y), l1 = __floats2half2_rn(b - f1.x, d - f1.y);
-		h[2 * g] = *reinterpret_cast<const uint32_t *>(&h0);
-		h[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&h1);
-		l[2 * g] = *reinterpret_cast<const uint32_t *>(&l0);
-		l[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&l1);
-	}
-	*reinterpret_cast<uint4 *>(hi_row + k0) = make_uint4(h[0], h[1], h[2], h[3]);
-	*reinterpret_cast<uint4 *>(lo_row + k0) = make_uint4(l[0], l[1], l[2], l[3]);
-	if (q_row) {
-		float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-		sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-		sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-		if ((lane & 3) == 0) {
-			const __half hs = __float2half_rn(sum);
-			q_row[xq_index(k0 >> 5)] = hs;
-			q_row[xq_index(k0 >> 5) + 8] = __float2half_rn(sum - __half2float(hs));
+		for (int g = 0; g < 2; g++) {
+			const float a = v[4 * g], b = v[4 * g + 1], c = v[4 * g + 2], d = v[4 * g + 3];
+			const __half2 h0 = __floats2half2_rn(a, c), h1 = __floats2half2_rn(b, d);
+			const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+			const __half2 l0 = __floats2half2_rn(a - f0.x, c - f0.y), l1 = __floats2half2_rn(b - f1.x, d - f1.y);
+			h[2 * g] = *reinterpret_cast<const uint32_t *>(&h0);
+			h[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&h1);
+			l[2 * g] = *reinterpret_cast<const uint32_t *>(&l0);
+			l[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&l1);
+		}
+		hi = make_uint4(h[0], h[1], h[2], h[3]);
+		lo = make_uint4(l[0], l[1], l[2], l[3]);
+		if (sums) {
+			float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+			sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+			sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+			sum_hi = __float2half_rn(sum);
+			sum_lo = __float2half_rn(sum - __half2float(sum_hi));
 		}
 	}
-}
+	__device__ __forceinline__ void store(int k0, __half *__restrict__ hi_row, __half *__restrict__ lo_row, __half *__restrict__ q_row,
+					      int lane) const
+	{
+		*reinterpret_cast<uint4 *>(hi_row + k0) = hi;
+		*reinterpret_cast<uint4 *>(lo_row + k0) = lo;
+		if (q_row && (lane & 3) == 0) {
+			q_row[xq_index(k0 >> 5)] = sum_hi;
+			q_row[xq_index(k0 >> 5) + 8] = sum_lo;
+		}
+	}
+};
 
 constexpr int ROWS_WARPS = 8;  // warps per CTA of the row passes: one row per warp at a time
 
-// Gather rows into expert-sorted order and split each fp32 value v into fp16 hi + lo
+// Rows into expert-sorted order, each fp32 value v split into fp16 hi + lo
 // (hi = rn16(v), lo = rn16(v - hi)): hi+lo carries 22 significand bits, which the tensor-core
 // scheme needs to stay within the 1e-3 parity bound.  xq (optional, q_cols per row): the
 // sums of the row over its 32-wide sub-blocks, split the same way (the Q4_K "min" term).
-// A warp takes 1024 columns of a row at a time: eight values per lane and step (16-byte loads and
-// stores), four steps' loads in flight; n_cols must be a multiple of 256.
-__global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__restrict__ x, const int *__restrict__ perm, int src_div,
-							      int n_rows, int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
+// Source row t is read and split once and stored at its n_out places inv[t * n_out ..] (< 0: none; inv null: row
+// t).  Bound by the stores: 4096 tokens to 8 experts each are 276 MB, 62 us when every place read its
+// row again.  A warp takes STEPS x 256 columns of a row, eight values per lane and step (16-byte loads and
+// stores); n_cols must be a multiple of 256.
+template <int STEPS>
+__global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__restrict__ x, const int *__restrict__ inv, int n_out, int n_src,
+							      int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
 							      __half *__restrict__ xq, int q_cols)
 {
 	pdl_trigger();	// (a dense product launched behind this pass sets itself up meanwhile)
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const int upr = (n_cols + 1023) >> 10;	// units of 1024 columns per row
-	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_rows * upr; un += gridDim.x * ROWS_WARPS) {
-		const int p = un / upr;
-		// (after a call with row experts out of range the sort has placed fewer rows than it was given and
-		// the tail of perm is stale: an entry that is no row id of this call reads row 0)
-		unsigned rid = perm ? (unsigned)perm[p] : (unsigned)p;
-		if (perm && rid >= (unsigned)n_rows)
-			rid = 0;
-		const int src = perm ? (int)rid / src_div : p;
-		const float *xr = x + (size_t)src * n_cols;
-		__half *hr = hi + (size_t)p * n_cols, *lr = lo + (size_t)p * n_cols;
-		__half *qr = xq ? xq + (size_t)p * q_cols : nullptr;
-		{
-			const int k0 = (un - p * upr) * 1024 + lane * 8;
-			float4 v[4][2];
+	const int upr = (n_cols + STEPS * 256 - 1) / (STEPS * 256);  // units per row
+	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_src * upr; un += gridDim.x * ROWS_WARPS) {
+		const int t = un / upr, k0 = (un - t * upr) * STEPS * 256 + lane * 8;
+		const float *xr = x + (size_t)t * n_cols;
+		int place = t;
+		if (inv && lane < n_out)
+			place = inv[(size_t)t * n_out + lane];
+		float4 v[STEPS][2];
 #pragma unroll
-			for (int i = 0; i < 4; i++) {
-				const int k = k0 + i * 256;
-				if (k < n_cols) {
-					v[i][0] = *reinterpret_cast<const float4 *>(xr + k);
-					v[i][1] = *reinterpret_cast<const float4 *>(xr + k + 4);
-				}
+		for (int i = 0; i < STEPS; i++) {
+			const int k = k0 + i * 256;
+			if (k < n_cols) {  // (uniform over the warp: n_cols is a multiple of 256)
+				v[i][0] = *reinterpret_cast<const float4 *>(xr + k);
+				v[i][1] = *reinterpret_cast<const float4 *>(xr + k + 4);
 			}
+		}
+		Split8 p[STEPS];
 #pragma unroll
-			for (int i = 0; i < 4; i++) {
-				const int k = k0 + i * 256;
-				if (k < n_cols) {  // (uniform over the warp: n_cols is a multiple of 256)
-					const float f[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
-					split8_store(f, k, hr, lr, qr, lane);
-				}
+		for (int i = 0; i < STEPS; i++)
+			if (k0 + i * 256 < n_cols) {
+				const float f[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
+				p[i].make(f, xq != nullptr);
 			}
+		for (int j = 0; j < n_out; j++) {
+			const int at = __shfl_sync(0xffffffffu, place, j);
+			if (at < 0)
+				continue;
+#pragma unroll
+			for (int i = 0; i < STEPS; i++)
+				if (k0 + i * 256 < n_cols)
+					p[i].store(k0 + i * 256, hi + (size_t)at * n_cols, lo + (size_t)at * n_cols,
+						   xq ? xq + (size_t)at * q_cols : nullptr, lane);
 		}
 	}
 }
@@ -210,7 +223,9 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float
 					    swiglu_lut(tab, g0.z, u0.z) * scale, swiglu_lut(tab, g0.w, u0.w) * scale,
 					    swiglu_lut(tab, g1.x, u1.x) * scale, swiglu_lut(tab, g1.y, u1.y) * scale,
 					    swiglu_lut(tab, g1.z, u1.z) * scale, swiglu_lut(tab, g1.w, u1.w) * scale};
-			split8_store(f, k, hr, lr, qr, lane);
+			Split8 p;
+			p.make(f, qr != nullptr);
+			p.store(k, hr, lr, qr, lane);
 		}
 	}
 }
@@ -249,16 +264,19 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 	return TIE_CUDA_OK;
 }
 
-int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *perm, int src_div, int n_rows, int n_cols, __half *hi,
+int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out, int n_src, int n_cols, __half *hi,
 		      __half *lo, __half *xq)
 {
-	if (n_cols % 256)
+	if (n_cols % 256 || n_out > 32)
 		return TIE_CUDA_ENOTSUP;
-	const int want = (n_rows * ((n_cols + 1023) / 1024) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 8;
-	if (n_rows <= 0)
+	if (n_src <= 0)
 		return TIE_CUDA_OK;
-	split_rows<<<want < cap ? want : cap, ROWS_WARPS * 32, 0, c->stream>>>(x, perm, src_div, n_rows, n_cols, hi, lo, xq,
-										xq_cols(n_cols));
+	// units of 1024 columns where they are enough to fill the SMs a few times over, else of 256
+	const bool wide = (long long)n_src * ((n_cols + 1023) / 1024) >= 4ll * ROWS_WARPS * c->sm_count;
+	const long long units = (long long)n_src * (wide ? (n_cols + 1023) / 1024 : n_cols / 256), cap = c->sm_count * 8;
+	const long long want = (units + ROWS_WARPS - 1) / ROWS_WARPS;
+	auto kern = wide ? split_rows<4> : split_rows<1>;
+	kern<<<(int)(want < cap ? want : cap), ROWS_WARPS * 32, 0, c->stream>>>(x, inv, n_out, n_src, n_cols, hi, lo, xq, xq_cols(n_cols));
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }

@@ -166,6 +166,8 @@ __global__ void __launch_bounds__(SORT_THREADS) sort_scatter(const int *__restri
 		perm[pos] = entry;
 		if (inv)
 			inv[r] = pos;
+	} else if (inv && owner_div == 0 && blockIdx.x * SORT_SLICE + threadIdx.x < (unsigned)n_rows) {
+		inv[blockIdx.x * SORT_SLICE + threadIdx.x] = -1;
 	}
 }
 
@@ -175,7 +177,8 @@ constexpr int SORT_SMALL = 1024;
 __global__ void __launch_bounds__(SORT_SMALL) sort_small(const int *__restrict__ row_expert, int n_rows, int first_expert, int n_local,
 							 int n_tile, int *__restrict__ counts, int *__restrict__ offsets,
 							 int *__restrict__ tile_start, int *__restrict__ active, int *__restrict__ n_active,
-							 int *__restrict__ perm, int4 *__restrict__ tile_info, unsigned *__restrict__ status)
+							 int *__restrict__ perm, int4 *__restrict__ tile_info, int *__restrict__ inv,
+							 unsigned *__restrict__ status)
 {
 	__shared__ short cnt[SORT_SMALL / 32][SORT_MAX_E];  // rows of expert e in warp w's 32 rows; then: rows before warp w
 	__shared__ int start[SORT_MAX_E];
@@ -255,8 +258,11 @@ __global__ void __launch_bounds__(SORT_SMALL) sort_small(const int *__restrict__
 		}
 	}
 	__syncthreads();
-	if (le >= 0)  // (stable: warps and lanes are in row order)
-		perm[start[le] + cnt[warp][le] + rank] = r;
+	const int pos = le >= 0 ? start[le] + cnt[warp][le] + rank : -1;  // (stable: warps and lanes are in row order)
+	if (le >= 0)
+		perm[pos] = r;
+	if (inv && r < n_rows)
+		inv[r] = pos;
 }
 
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, int first_expert, int n_expert,
@@ -264,10 +270,10 @@ int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, 
 {
 	if (n_expert > 256)
 		return TIE_CUDA_ENOTSUP;
-	if (n_rows <= SORT_SMALL && !b.inv && !b.owner_div) {
+	if (n_rows <= SORT_SMALL && !b.owner_div) {
 		const int threads = n_rows <= SORT_MAX_E ? SORT_MAX_E : (n_rows + 31) / 32 * 32;
 		sort_small<<<1, threads, 0, c->stream>>>(row_expert, n_rows, first_expert, n_expert, n_tile, b.counts, b.offsets, b.tile_start,
-							 b.active, b.n_active, b.perm, b.tile_info, c->s.status);
+							 b.active, b.n_active, b.perm, b.tile_info, b.inv, c->s.status);
 		TIE_CUDA_LAUNCHED(c);
 		return TIE_CUDA_OK;
 	}
@@ -286,7 +292,7 @@ int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, 
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile)
 {
 	Scratch &s = c->s;
-	SortBufs b = {s.counts, s.offsets, s.tile_start, s.active, s.n_active, s.perm, s.tile_info};
+	SortBufs b = {s.counts, s.offsets, s.tile_start, s.active, s.n_active, s.perm, s.tile_info, s.inv};
 	return launch_sort(c, row_expert, n_rows, n_tile, c->first_expert, c->n_local, b);
 }
 
