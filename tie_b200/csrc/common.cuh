@@ -330,7 +330,7 @@ __device__ __forceinline__ void pdl_trigger()
 {
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// dependent: such a launch.  (The chain of a whole MoE call measured slower with it, 9 tokens 82 -> 84 us,
+// dependent: such a launch.  (The chain of a whole MoE call measured slower with all of its launches so, 9 tokens 82 -> 84 us,
 // 4096 945 -> 1006: CTAs resident early take SMs from their predecessor's tail.)
 template <class... P, class... A>
 int launch_kernel(tie_cuda_ctx *c, bool dependent, int cluster, void (*kern)(P...), dim3 grid, int threads, size_t smem, const A &...args)

@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__res
 							      int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
 							      __half *__restrict__ xq, int q_cols)
 {
-	pdl_trigger();	// (a dense product launched behind this pass sets itself up meanwhile)
+	pdl_trigger();	// (a dense product, or one of narrow tiles, sets itself up meanwhile)
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int upr = (n_cols + STEPS * 256 - 1) / (STEPS * 256);  // units per row
 	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_src * upr; un += gridDim.x * ROWS_WARPS) {
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float
 								     const int *__restrict__ n_rows_dev, int n_rows_host)
 {
 	__shared__ float tab[SILU_N];
+	pdl_trigger();	// (a down product of narrow tiles sets itself up meanwhile)
 	for (int i = threadIdx.x; i < SILU_N / 4; i += blockDim.x)
 		reinterpret_cast<float4 *>(tab)[i] = __ldg(reinterpret_cast<const float4 *>(silu) + i);
 	__syncthreads();

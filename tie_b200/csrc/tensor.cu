@@ -1057,14 +1057,17 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	// least 4 super-blocks.  Measured at 64 / 512 / 4096 tokens: rows of 8 super-blocks (gate/up) 68 / 79 / 355 us
 	// paired, 70 / 92 / 410 single (a pair fetches half the token bytes per CTA); rows of 3 (down) 59 / 73 / 310
 	// paired, 55 / 70 / 294 single (the hand-offs between two SMs are not amortised over so few).
+	// set up beside the pass in front (a CTA needs a whole SM, so they come as SMs fall idle): dense products and narrow
+	// tiles, where a launch is 10 - 70 us (9 tokens 84.3 -> 82.3 us, 64 137.5 -> 135.4; 4096 equal or slower)
+	const bool dependent = dense_rows > 0 || NT == 32;
 	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles : 1 << 30;	// (known for a dense tensor: no idle CTAs)
 	if (c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K) {
-		return launch_kernel(c, dense_rows > 0, 2, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
+		return launch_kernel(c, dependent, 2, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
 				     TcSmem<KIND, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
 				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
 				     s.status, t0.rows, d, xqd);
 	}
-	return launch_kernel(c, dense_rows > 0, 1, grouped_gemm_sb<KIND, RAW, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
+	return launch_kernel(c, dependent, 1, grouped_gemm_sb<KIND, RAW, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
 			     TcSmem<KIND, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
 			     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status,
 			     t0.rows, d, xqd);
