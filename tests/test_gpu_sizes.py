@@ -177,3 +177,24 @@ def test_one_token_host_calls(be):
             out[:] = np.nan
             be.moe_ffn_ptr(0, x, out, 1, moe.HOST | flags)
             assert np.array_equal(bits(out), bits(want.cpu().numpy()))
+
+
+# RMSNorm of rows of one CTA each: hidden below, at and above what its threads keep in registers (2048).
+@pytest.mark.parametrize("hidden", [512, 2048, 2304])
+def test_rms_norm_row_lengths(hidden, port_lib, ref_silu_table):
+    import torch
+    from tie_b200 import moe
+    s = synth.MoeShape(hidden=hidden, n_expert=16, top_k=2, ffn_dim=256)
+    layer = synth.make_layer(17, s)
+    norm = np.linspace(0.8, 1.2, hidden, dtype=np.float32)
+    b = moe.MoeBackend(hidden=hidden, n_expert=16, top_k=2, ffn_dim=256, max_tokens=8, silu_table=ref_silu_table)
+    try:
+        b.upload_layer(0, layer, ffn_norm_w=norm)
+        h0 = synth.make_x(18, 5, hidden)
+        normed = np.stack([port_lib.rms_norm(h0[i], norm, 1e-6) for i in range(5)])
+        ref = h0 + port_lib.PortMoe(layer, silu=ref_silu_table).moe_ffn(normed)[0]
+        h = torch.from_numpy(h0.copy()).cuda()
+        b.moe_block_inplace_ptr(0, h, 5, moe.DEVICE)
+        assert workloads.rel_rms_err(h.cpu().numpy(), ref).max() < TOL
+    finally:
+        b.close()
