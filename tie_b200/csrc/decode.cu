@@ -95,15 +95,27 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 }
 
 // The product of slot j's 16 staged rows with its h row, in this warp: lane (g, t = 0, 1) ends up with rows g, g + 8.
+// The row's next super-block is loaded under the products of the one before, and the tile is waited for (bar;
+// false in ok: it never landed) when the first image is made.  (A block of 3 / 4 / 8 tokens 40.6 / 47.3 / 79.3 -> 39.1 / 46.5 /
+// 76.4 us against all warps waiting for all tiles before their first load of h.)
 template <WKind KIND>
-__device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const float *hrow, uint8_t *img, int lane)
+__device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const float *hrow, uint8_t *img, int lane, uint32_t bar,
+					    unsigned *status, bool &ok)
 {
 	float2 out = make_float2(0.f, 0.f);
-	for (int b = 0; b < nb; b++) {
-		const float4 *hp = reinterpret_cast<const float4 *>(hrow + b * QK_K) + 2 * lane;
-		const float4 h0 = hp[0], h1 = hp[1];
+	const float4 *hp = reinterpret_cast<const float4 *>(hrow) + 2 * lane;
+	float4 h0 = hp[0], h1 = hp[1];
+	ok = true;
+	for (int b = 0; b < nb && ok; b++) {
 		const float v[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+		if (b + 1 < nb) {
+			hp += QK_K / 4;
+			h0 = hp[0];
+			h1 = hp[1];
+		}
 		const float inv = x_image<KIND>(v, img, lane);
+		if (b == 0)
+			ok = __all_sync(0xffffffffu, dec_wait(bar, status));
 		MmaRows<KIND> w;
 		w.load_smem(tile, nb, b, lane);
 		float2 r, s;
@@ -151,18 +163,18 @@ decode_down_combine(const uint8_t *__restrict__ wd, size_t expert_stride, int ro
 		}
 	}
 	pdl_wait();  // h of the gate/up kernel is visible from here on
-	__syncthreads();
-	const bool bad = s_bad != 0;
-	const bool mine = topk_idx[t * top_k + j] - first_expert >= 0 && topk_idx[t * top_k + j] - first_expert < n_local;
-	const bool ok = !mine || dec_wait(ptx::smem_u32(&bar[j]), status);
-	if (!__syncthreads_and(ok) || bad)
-		return;	 // (every tile that was requested has landed, or its wait has run out)
-	const float2 v = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane);
-	if ((lane & 3) == 0) {
-		red[j][lane >> 2] = v.x;
-		red[j][(lane >> 2) + 8] = v.y;
+	const int le = topk_idx[t * top_k + j] - first_expert;
+	bool ok = true;
+	if (le >= 0 && le < n_local) {
+		const float2 v = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane,
+						 ptx::smem_u32(&bar[j]), status, ok);
+		if ((lane & 3) == 0) {
+			red[j][lane >> 2] = v.x;
+			red[j][(lane >> 2) + 8] = v.y;
+		}
 	}
-	__syncthreads();
+	if (!__syncthreads_and(ok) || s_bad)
+		return;	 // (every tile that was requested has landed, or its wait has run out)
 	if (threadIdx.x < 16) {
 		float acc = 0.f;
 		for (int k = 0; k < top_k; k++)
@@ -238,7 +250,9 @@ decode_down_peer(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_
 		return;
 	if (!mine)
 		return;
-	const float2 r = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane);
+	bool there;
+	const float2 r = down_rows<KIND>(dsm + (size_t)j * tile_bytes, nb, h + (size_t)(t * top_k + j) * nb * QK_K, img[j], lane,
+					 ptx::smem_u32(&bar[j]), status, there);
 	// lanes of t = 0 hold row g, their neighbours of t = 1 store row g + 8
 	if ((lane & 3) < 2) {
 		const size_t at = (size_t)(t * top_k + j) * rows_per_expert + r0 + (lane >> 2) + 8 * (lane & 1);
@@ -261,8 +275,8 @@ static size_t dec_down_smem(const Layer &L, int top_k)
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
 	// every (token, slot) row by itself up to the batch where grouping the experts' rows pays for its passes
-	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 51 / 63 / 70 / 83 us
-	// a block here, 70 / 79 / 81 / 85 grouped; 10 / 13 / 20 tokens 100 / 122 / 173 here, 93 / 98 / 110 grouped
+	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 46 / 58 / 66 / 76 us
+	// a block here, 64 / 73 / 76 / 79 grouped; 10 / 13 / 20 tokens 100 / 122 / 173 here, 93 / 98 / 110 grouped
 	const int n_rows = n_tokens * c->cfg.top_k;
 	return (n_tokens <= 4 || 2 * n_rows <= c->n_local) && n_rows <= 65535 && L.gate.kind == L.up.kind &&
 	       L.gate.k <= DEC_MAX_NB * QK_K && L.gate.rows % 16 == 0 && L.down.rows % 16 == 0 && L.down.k <= DEC_MAX_NB * QK_K &&
