@@ -72,6 +72,23 @@ def test_per_row_and_grouped_products_around_the_change(be, port0, n_tokens):
     assert be.last_active_experts() == len(np.unique(ref_idx))
 
 
+# 128 row tiles a token: the Q4_K down kernel runs with two CTAs per SM at 2 and 4 tokens, with three at 3 and 8.
+@pytest.mark.parametrize("n_tokens", [2, 3, 4, 8])
+def test_per_row_q4k_down_around_a_wave(n_tokens, port_lib, ref_silu_table):
+    from tie_b200 import moe
+    s = synth.MoeShape(hidden=2048, n_expert=128, top_k=8, ffn_dim=256)
+    q6 = synth.make_layer(workloads.BASE_SEED + 6, s)
+    down = synth.q4k_blocks(6, synth.STREAM_DOWN, s.n_expert * s.hidden * (s.ffn_dim // 256))
+    layer = synth.MoeLayer(s, q6.router_w, q6.gate, q6.up, down, gate_type=synth.GGML_Q4_K, up_type=synth.GGML_Q4_K, down_type=synth.GGML_Q4_K)
+    b = moe.MoeBackend(ffn_dim=s.ffn_dim, max_tokens=8, silu_table=ref_silu_table)
+    b.upload_layer(0, layer, keep_host=True)
+    x = synth.make_x(0, n_tokens, first_token=50)
+    ref, _, _ = port_lib.PortMoe(layer, silu=ref_silu_table).moe_ffn(x)
+    out = b.moe_ffn(0, x)
+    b.close()
+    assert workloads.rel_rms_err(out, ref).max() < 1e-5
+
+
 # Rows per expert at the edges of 16-, 32- and 64-row tiles: tiles of 32 up to 24 rows an expert on average, of 64
 # above; the dispatch sort is one CTA up to 1024 rows.
 _EDGES = [0, 1, 15, 16, 17, 31, 32, 33, 63, 64, 65]

@@ -126,8 +126,10 @@ __device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const f
 	return out;
 }
 
-template <WKind KIND>
-__global__ void __launch_bounds__(MAX_TOP_K * 32, 2)
+// CTAS: resident per SM.  Q4_K tiles leave room for a third CTA, at 80 registers instead of 96; launch_decode_down_combine
+// says where it pays.
+template <WKind KIND, int CTAS = 2>
+__global__ void __launch_bounds__(MAX_TOP_K * 32, CTAS)
 decode_down_combine(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_expert, int nb, const float *__restrict__ h,
 		    int top_k, const int *__restrict__ topk_idx, const float *__restrict__ topk_w, const float *__restrict__ residual,
 		    float *__restrict__ out, int first_expert, int n_local, unsigned *__restrict__ status)
@@ -286,6 +288,7 @@ bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 // Opt-in shared-memory sizes, once per context.
 int decode_setup(tie_cuda_ctx *c)
 {
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<W_Q4K, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<W_Q4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_combine<W_Q6K_R8>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(decode_down_peer<W_Q4K>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM));
@@ -310,7 +313,11 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out)
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
-	auto kern = L.down.kind == W_Q4K ? decode_down_combine<W_Q4K> : decode_down_combine<W_Q6K_R8>;
+	// Q4_K: three CTAs per SM where that saves a wave (3 and 5 - 8 tokens of this model).  Blocks of which half have such a
+	// down tensor, at 6 / 8 tokens: 58.0 / 76.5 -> 57.5 / 75.6 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
+	const long long grid = (long long)(L.down.rows / 16) * n_tokens, two = 2 * c->sm_count, three = 3 * c->sm_count;
+	const bool many = (grid + three - 1) / three < (grid + two - 1) / two;
+	auto kern = L.down.kind != W_Q4K ? decode_down_combine<W_Q6K_R8> : many ? decode_down_combine<W_Q4K, 3> : decode_down_combine<W_Q4K>;
 	return launch_kernel(c, true, 1, kern, dim3(L.down.rows / 16, n_tokens), 32 * top_k, dec_down_smem(L, top_k), L.down.ptr, L.down.expert_stride,
 			  L.down.rows, nb, c->s.h, top_k, c->s.topk_idx, c->s.topk_w, residual, out, c->first_expert, c->n_local, c->s.status);
 }
