@@ -62,7 +62,7 @@ def test_router_tiles_and_both_selections(be, port0, n_tokens):
     assert np.abs(w / w_r - 1).max() < 2e-6
 
 
-# 8 tokens are the last batch of the per-row kernels with 128 experts and top-8.
+# 6 tokens are the last batch of the per-row kernels with 128 experts and top-8.
 @pytest.mark.parametrize("n_tokens", [6, 8, 9, 12])
 def test_per_row_and_grouped_products_around_the_change(be, port0, n_tokens):
     x = synth.make_x(0, n_tokens, first_token=90)
@@ -72,7 +72,7 @@ def test_per_row_and_grouped_products_around_the_change(be, port0, n_tokens):
     assert be.last_active_experts() == len(np.unique(ref_idx))
 
 
-# 128 row tiles a token: the Q4_K down kernel runs with two CTAs per SM at 2 and 4 tokens, with three at 3 and 8.
+# 128 row tiles a token: the Q4_K down kernel runs with two CTAs per SM at 2 and 4 tokens, with three at 3.
 @pytest.mark.parametrize("n_tokens", [2, 3, 4, 8])
 def test_per_row_q4k_down_around_a_wave(n_tokens, port_lib, ref_silu_table):
     from tie_b200 import moe
@@ -213,5 +213,65 @@ def test_rms_norm_row_lengths(hidden, port_lib, ref_silu_table):
         h = torch.from_numpy(h0.copy()).cuda()
         b.moe_block_inplace_ptr(0, h, 5, moe.DEVICE)
         assert workloads.rel_rms_err(h.cpu().numpy(), ref).max() < TOL
+    finally:
+        b.close()
+
+
+# Below twice as many rows as experts every product is exact to fp32, as for one token: rows grouped by expert, two to
+# a group (7 tokens on with 128 experts and top-8), have the bits of their tokens alone, whichever experts they share.
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("n_tokens", [6, 7, 9, 20, 31])
+def test_small_batches_have_the_bits_of_single_tokens(be, port0, n_tokens, shared):
+    x = synth.make_x(0, n_tokens, first_token=600)
+    bias = None
+    if shared:  # all tokens on the same eight experts: groups of two and a remainder
+        bias = np.zeros(128, dtype=np.float32)
+        bias[[0, 3, 17, 44, 45, 90, 126, 127]] = 1000.0
+    out = be.moe_ffn(0, x, router_bias=bias)
+    active = be.last_active_experts()
+    alone = np.concatenate([be.moe_ffn(0, x[i:i + 1], router_bias=bias) for i in range(n_tokens)])
+    assert np.array_equal(bits(out), bits(alone))
+    ref, ref_idx, _ = port0.moe_ffn(x, router_bias=bias)
+    assert workloads.rel_rms_err(out, ref).max() < 1e-5
+    assert active == len(np.unique(ref_idx))
+
+
+# Activations far from 1, and Q6_K scales over their whole range (products beyond 11 bits), with every kind of tensor.  The
+# CPU restatement itself is up to 1.0e-5 from 64-bit arithmetic at 0.03 (SwiGLU rounds gate + 10) and 1.4e-6 at 1 and 2e4.
+@pytest.mark.parametrize("kinds", ["q4k_q6k", "q6k_q4k", "q4k_q4k"])
+@pytest.mark.parametrize("scale", [0.03, 1.0, 2e4])
+@pytest.mark.parametrize("n_tokens", [5, 9, 15])
+def test_small_batches_over_the_range_of_activations(n_tokens, scale, kinds, small_shape, port_lib, ref_silu_table):
+    import torch
+    from tie_b200 import moe
+    s = small_shape  # 32 experts, top-4: grouped from 5 to 15 tokens
+    n_gu, n_dn = s.n_expert * s.ffn_dim * (s.hidden // 256), s.n_expert * s.hidden * (s.ffn_dim // 256)
+
+    def blocks(kind, stream, n):
+        if kind == "q4k":
+            return synth.q4k_blocks(55, stream, n), synth.GGML_Q4_K
+        b = np.array(synth.q6k_blocks(55, stream, n)).reshape(n, synth.Q6K_BYTES)
+        b[:, 192:208] = np.random.default_rng(stream).integers(-128, 128, (n, 16), dtype=np.int8).view(np.uint8)
+        return b.reshape(-1), synth.GGML_Q6_K
+
+    gu, dn = kinds.split("_")
+    (gate, gt), (up, _), (down, dt) = blocks(gu, synth.STREAM_GATE, n_gu), blocks(gu, synth.STREAM_UP, n_gu), blocks(dn, synth.STREAM_DOWN, n_dn)
+    layer = synth.MoeLayer(s, synth.make_layer(55, s).router_w, gate, up, down, gate_type=gt, up_type=gt, down_type=dt)
+    b = moe.MoeBackend(hidden=s.hidden, n_expert=s.n_expert, top_k=s.top_k, ffn_dim=s.ffn_dim, max_tokens=16, silu_table=ref_silu_table)
+    try:
+        b.upload_layer(0, layer, keep_host=True)
+        x = synth.make_x(9, n_tokens, s.hidden) * np.float32(scale)
+        ref, _, _ = port_lib.PortMoe(layer, silu=ref_silu_table).moe_ffn(x)
+        out = b.moe_ffn(0, x)
+        assert np.isfinite(out).all() and workloads.rel_rms_err(out, ref).max() < (3e-5 if scale < 1 else 1e-5)
+        # as many rows through the building block of expert parallelism (rows without an output to speak of: see above)
+        rows, row_expert = np.repeat(x, s.top_k, axis=0), np.random.default_rng(3).integers(0, s.n_expert, n_tokens * s.top_k).astype(np.int32)
+        y = torch.empty(rows.shape, device="cuda")
+        b.expert_rows_ptr(0, torch.from_numpy(rows).cuda(), torch.from_numpy(row_expert).cuda(), len(rows), y, moe.DEVICE)
+        y_ref = port_lib.PortMoe(layer, silu=ref_silu_table).expert_rows(rows, row_expert)
+        rms = np.sqrt((y_ref.astype(np.float64) ** 2).mean(1))
+        assert (np.abs(y.cpu().numpy() - y_ref).max(1) / np.maximum(rms, 1e-2 * np.median(rms))).max() < (1e-4 if scale < 1 else 3e-5)
+        alone = np.concatenate([b.moe_ffn(0, x[i:i + 1]) for i in range(n_tokens)])
+        assert np.array_equal(bits(out), bits(alone))
     finally:
         b.close()

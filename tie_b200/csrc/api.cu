@@ -269,7 +269,10 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	} else if (path == TIE_CUDA_PATH_STREAM) {
 		use_tc = false;
 	} else {
-		use_tc = tc_supported(c, L) && 2 * n_rows > c->n_local;  // (below: decode_supported, decode.cu)
+		// Below twice as many rows as experts the products stay exact to fp32 (decode.cu, decode_group.cu, else the streaming
+		// kernels), also where the tensor path's fp16 hi + lo would be faster (a block of 20 / 31 tokens 121 / 155 us there, 114 /
+		// 127 here).  Row lengths that none of them is built for come here from half as many rows as experts on.
+		use_tc = tc_supported(c, L) && (n_rows >= 2 * c->n_local || (2 * n_rows > c->n_local && !stream_supported(L)));
 	}
 	c->tc_no_pair = (flags & TIE_CUDA_PATH_NO_PAIR) != 0;
 	const int direct = (!use_tc && n_rows <= c->cfg.top_k && src_div == c->cfg.top_k) ? 1 : 0;
@@ -336,7 +339,23 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 			return TIE_CUDA_OK;
 		}
 	}
-	// decode and small batches: three launches — router with fused selection, gate/up, down + combine
+	// small batches: router with fused selection, the rows of each expert together, combine
+	if ((flags & (TIE_CUDA_PATH_MASK | TIE_CUDA_PATH_LEGACY_STREAM)) == 0 && decode_group_supported(c, L, n_tokens)) {
+		TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
+		prof_mark(c, 1);
+		c->last_used_tc = false;
+		c->last_direct_rows = n_tokens * c->cfg.top_k;
+		prof_mark(c, 2);
+		prof_mark(c, 3);
+		TRY(launch_group_gate_up(c, L, x, n_tokens));
+		prof_mark(c, 4);
+		TRY(launch_group_down(c, L, n_tokens, s.y));
+		prof_mark(c, 6);
+		TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out));
+		prof_mark(c, 7);
+		return TIE_CUDA_OK;
+	}
+	// decode: three launches — router with fused selection, gate/up, down + combine
 	if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR && !(flags & TIE_CUDA_PATH_LEGACY_STREAM) &&
 	    decode_supported(c, L, n_tokens)) {
 		TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
@@ -741,6 +760,8 @@ int tie_cuda_init(tie_cuda_ctx **out, const tie_cuda_config *cfg)
 	if ((rc = router_setup(c)) != TIE_CUDA_OK)
 		return fail(rc);
 	if ((rc = decode_setup(c)) != TIE_CUDA_OK)
+		return fail(rc);
+	if ((rc = decode_group_setup(c)) != TIE_CUDA_OK)
 		return fail(rc);
 	*out = c;
 	return TIE_CUDA_OK;

@@ -1,4 +1,4 @@
-// Decode and small batches (up to 8 tokens of this model's shape): the expert mat-vecs of every
+// Decode and small batches (up to 6 tokens of this model's shape): the expert mat-vecs of every
 // (token, slot) row on its own — no dispatch sort, no grouping — with the exact mma.sync products of
 // mma_dot.cuh.
 //
@@ -75,15 +75,15 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 	const float inv = x_image<KIND>(v, img[b], lane);
 	for (int r = r0, buf = 0; r < r1; r += 16, buf ^= 1) {
 		const bool more = r + 16 < r1;
-		float2 p, s;
-		g.dot(img[b], inv, lane, p, s);
+		float2 p = g.dot(one_row<KIND>(img[b], lane), lane), s = g.scale(inv);
 		if (more)
 			g.load(wg + tile_offset<KIND>(nb, r + 16), nb, b, lane);
 		if ((lane & 3) == 0) {
 			red[buf][b][0][lane >> 2] = p.x * s.x;
 			red[buf][b][0][(lane >> 2) + 8] = p.y * s.y;
 		}
-		u.dot(img[b], inv, lane, p, s);
+		p = u.dot(one_row<KIND>(img[b], lane), lane);
+		s = u.scale(inv);
 		if (more)
 			u.load(wu + tile_offset<KIND>(nb, r + 16), nb, b, lane);
 		if ((lane & 3) == 0) {
@@ -118,8 +118,7 @@ __device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const f
 			ok = __all_sync(0xffffffffu, dec_wait(bar, status));
 		MmaRows<KIND> w;
 		w.load_smem(tile, nb, b, lane);
-		float2 r, s;
-		w.dot(img, inv, lane, r, s);
+		const float2 r = w.dot(one_row<KIND>(img, lane), lane), s = w.scale(inv);
 		out.x = __fmaf_rn(s.x, r.x, out.x);
 		out.y = __fmaf_rn(s.y, r.y, out.y);
 	}
@@ -276,9 +275,7 @@ static size_t dec_down_smem(const Layer &L, int top_k)
 
 bool decode_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
-	// every (token, slot) row by itself up to the batch where grouping the experts' rows pays for its passes
-	// around the products (run_experts): 4 / 6 / 7 / 8 tokens of this model's shape 46 / 58 / 66 / 76 us
-	// a block here, 64 / 73 / 76 / 79 grouped; 10 / 13 / 20 tokens 100 / 122 / 173 here, 93 / 98 / 110 grouped
+	// (decode_group.cu takes what it is faster at from here)
 	const int n_rows = n_tokens * c->cfg.top_k;
 	return (n_tokens <= 4 || 2 * n_rows <= c->n_local) && n_rows <= 65535 && L.gate.kind == L.up.kind &&
 	       L.gate.k <= DEC_MAX_NB * QK_K && L.gate.rows % 16 == 0 && L.down.rows % 16 == 0 && L.down.k <= DEC_MAX_NB * QK_K &&

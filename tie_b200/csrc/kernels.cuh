@@ -17,6 +17,11 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 int launch_decode_down_peer(tie_cuda_ctx *c, const Layer &L, int n_tokens);
 int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out);
 int launch_router_rows(tie_cuda_ctx *c, const float *x, const float *w, int n_rows, int in_dim, float *out);
+// decode_group.cu
+int decode_group_setup(tie_cuda_ctx *c);
+bool decode_group_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens);
+int launch_group_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n_tokens);
+int launch_group_down(tie_cuda_ctx *c, const Layer &L, int n_tokens, float *y);
 // decode_fused.cu
 bool decode_fused_supported(tie_cuda_ctx *c, const Layer &L, int n_tokens);
 int launch_decode_fused(tie_cuda_ctx *c, const Layer &L, const float *x, const float *bias, const float *residual, float *out,
@@ -36,6 +41,7 @@ int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile);
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, int first_expert, int n_expert,
 		const SortBufs &b);
 // stream.cu
+bool stream_supported(const Layer &L);
 int launch_stream_gate_up(tie_cuda_ctx *c, const Layer &L, const float *xin, int src_div, const int *row_expert,
 			  int n_rows, int direct);
 int launch_stream_down(tie_cuda_ctx *c, const Layer &L, float *y, const int *row_expert, int n_rows, int direct);

@@ -97,17 +97,43 @@ __device__ __forceinline__ void mma_1688(float (&c)[4], uint32_t a0, uint32_t a1
 	    : "r"(a0), "r"(a1), "r"(b0));
 }
 
+// Where a lane's column of the MMA (column g = lane / 4) has its activations: a part of an image, and that part's sums.
+// A column that carries nothing reads zeros (ALL) or is off.
+template <bool ALL>
+struct MmaCol {
+	const uint8_t *x, *sums;
+	bool on;
+	__device__ __forceinline__ bool reads() const { return ALL || on; }
+};
+// one activation row: columns 0, 1, 2 are its parts
+template <WKind KIND>
+__device__ __forceinline__ MmaCol<false> one_row(const uint8_t *img, int lane)
+{
+	const int g = lane >> 2;
+	return {img + g * XImage<KIND>::PART, img + XImage<KIND>::SUMS + 16 * g, g < 3};
+}
+// two rows (the second image is `stride` bytes behind the first; n_rows = 1: there is none): columns 0 .. 2 and 4 .. 6
+template <WKind KIND>
+__device__ __forceinline__ MmaCol<true> two_rows(const uint8_t *img, int stride, int n_rows, const uint8_t *zeros, int lane)
+{
+	const int part = (lane >> 2) & 3, m = lane >> 4;
+	if (part == 3 || m >= n_rows)
+		return {zeros, zeros, false};
+	img += m * stride;
+	return {img + part * XImage<KIND>::PART, img + XImage<KIND>::SUMS + 16 * part, true};
+}
+
 // What lane (g = lane / 4, t = lane % 4) holds of the packed rows g and g + 8 of a 16-row tile.
 template <WKind KIND>
 struct MmaRows;
 
-// The products of a super-block: x[0] + x[1] is row g's, x[2] + x[3] row g + 8's, over the quad's lanes.
+// The products of a super-block: c[0] + c[1] is row g's, c[2] + c[3] row g + 8's, over two lanes of the quad.
 __device__ __forceinline__ float2 quad_rows(const float (&c)[4])
 {
-	float r0 = c[0] + c[1], r1 = c[2] + c[3];  // lane t = 0: columns 0, 1 (hi, mid); t = 1: 2 (lo), 3 (nothing)
+	float r0 = c[0] + c[1], r1 = c[2] + c[3];  // lane t = 0: columns 0, 1 (hi, mid); t = 1: 2 (lo), 3 (nothing); t = 2, 3: the second row's
 	r0 += __shfl_xor_sync(0xffffffffu, r0, 1);
 	r1 += __shfl_xor_sync(0xffffffffu, r1, 1);
-	return make_float2(r0, r1);  // (valid in lanes t = 0, 1)
+	return make_float2(r0, r1);  // (valid in lanes t = 0, 1; two_rows: the second row's in t = 2, 3)
 }
 
 template <>
@@ -140,10 +166,24 @@ struct MmaRows<W_Q4K> {
 			q[r][1] = odd ? u : v;
 		}
 	}
-	// the tile's products with the image are scale.x * r.x (row g) and scale.y * r.y (row g + 8)
-	__device__ __forceinline__ void dot(const uint8_t *img, float inv, int lane, float2 &r, float2 &scale) const
+	// the same from super-block b of a tile staged by itself (ChunkCopy)
+	__device__ __forceinline__ void load_chunk(const uint8_t *chunk, const uint8_t *, int, int, int lane)
 	{
 		const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+		for (int r = 0; r < 2; r++) {
+			const uint8_t *blk = chunk + (g + 8 * r) * Q4K_BYTES;
+			hdr[r] = *reinterpret_cast<const uint4 *>(blk);
+			q[r][0] = *reinterpret_cast<const uint4 *>(blk + 16 + 32 * t);
+			q[r][1] = *reinterpret_cast<const uint4 *>(blk + 32 + 32 * t);
+		}
+	}
+	__device__ __forceinline__ float2 scale(float inv) const { return make_float2(inv, inv); }
+	// the tile's products with a row are scale(inv).x * r.x (row g) and scale(inv).y * r.y (row g + 8)
+	template <bool ALL>
+	__device__ __forceinline__ float2 dot(const MmaCol<ALL> &col, int lane) const
+	{
+		const int t = lane & 3;
 		const __half2 k1024 = __float2half2_rn(1024.0f);
 		Q4kConsts c[2];
 		uint32_t mins[2];
@@ -163,14 +203,13 @@ struct MmaRows<W_Q4K> {
 			mins[w] = h2_bits(__hsub2(bits_h2(__byte_perm(mn, 0x64006400u, 0x7170u)), k1024));
 		}
 		float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f}, mm[4] = {0.f, 0.f, 0.f, 0.f};
-		const bool on = g < 3;	// columns 3 .. 7 carry nothing
-		const uint8_t *xp = img + g * XImage<W_Q4K>::PART + t * XImage<W_Q4K>::BLK;
-		const uint32_t bs = on ? *reinterpret_cast<const uint32_t *>(img + XImage<W_Q4K>::SUMS + 16 * g + 4 * t) : 0u;
+		const uint8_t *xp = col.x + t * XImage<W_Q4K>::BLK;
+		const uint32_t bs = col.reads() ? *reinterpret_cast<const uint32_t *>(col.sums + 4 * t) : 0u;
 		mma_1688(mm, mins[0], mins[1], bs);
 #pragma unroll
 		for (int i2 = 0; i2 < 4; i2++) {  // two words: 8 k of either sub-block
 			uint4 bl = make_uint4(0, 0, 0, 0), bh = bl;
-			if (on) {
+			if (col.reads()) {
 				bl = *reinterpret_cast<const uint4 *>(xp + 16 * i2);
 				bh = *reinterpret_cast<const uint4 *>(xp + 64 + 16 * i2);
 			}
@@ -191,8 +230,7 @@ struct MmaRows<W_Q4K> {
 			const uint32_t h = hdr[i >> 1].x;
 			s[i] = half_bits_to_float(h & 0xffffu) * (lo[i] + hi[i]) - half_bits_to_float(h >> 16) * mm[i];
 		}
-		r = quad_rows(s);
-		scale = make_float2(inv, inv);
+		return quad_rows(s);
 	}
 };
 
@@ -201,14 +239,15 @@ struct MmaRows<W_Q6K_R8> {
 	uint32_t a[2][4], b[2][4], h[2][4], sc[2][4];
 	float d[2];
 	// tile: first of the two R8 groups of 8 rows (each q6k_r8_group_bytes(nb) long)
-	template <bool SMEM>
-	__device__ __forceinline__ void load_t(const uint8_t *tile, int nb, int blk, int lane)
+	// chunk != null: the records lie there by themselves (ChunkCopy), only d is fetched from the tile
+	template <bool SMEM, bool CHUNK = false>
+	__device__ __forceinline__ void load_t(const uint8_t *tile, int nb, int blk, int lane, const uint8_t *chunk = nullptr)
 	{
 		const int g = lane >> 2, t = lane & 3;
 #pragma unroll
 		for (int r = 0; r < 2; r++) {
 			const uint8_t *grp = tile + r * q6k_r8_group_bytes(nb);
-			const uint8_t *rec = grp + (size_t)(g * nb + blk) * Q6K_RECORD;
+			const uint8_t *rec = CHUNK ? chunk + (g + 8 * r) * Q6K_RECORD : grp + (size_t)(g * nb + blk) * Q6K_RECORD;
 #pragma unroll
 			for (int pp = 0; pp < 4; pp++) {
 				const uint32_t *p = reinterpret_cast<const uint32_t *>(rec + 48 * pp + 4 * t);
@@ -219,16 +258,21 @@ struct MmaRows<W_Q6K_R8> {
 				sc[r][pp] = SMEM ? *ps : __ldg(ps);
 			}
 			const unsigned short *pd = reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, g, blk));
-			d[r] = half_bits_to_float(SMEM ? *pd : __ldg(pd));
+			d[r] = half_bits_to_float(SMEM && !CHUNK ? *pd : __ldg(pd));
 		}
 	}
 	__device__ __forceinline__ void load(const uint8_t *tile, int nb, int blk, int lane) { load_t<false>(tile, nb, blk, lane); }
 	__device__ __forceinline__ void load_smem(const uint8_t *tile, int nb, int blk, int lane) { load_t<true>(tile, nb, blk, lane); }
-	__device__ __forceinline__ void dot(const uint8_t *img, float inv, int lane, float2 &r, float2 &scale) const
+	__device__ __forceinline__ void load_chunk(const uint8_t *chunk, const uint8_t *tile, int nb, int blk, int lane)
 	{
-		const int g = lane >> 2, t = lane & 3;
-		const bool on = g < 3;
-		const uint8_t *xp = img + g * XImage<W_Q6K_R8>::PART + 8 * t;
+		load_t<true, true>(tile, nb, blk, lane, chunk);
+	}
+	__device__ __forceinline__ float2 scale(float inv) const { return make_float2(d[0] * inv, d[1] * inv); }
+	template <bool ALL>
+	__device__ __forceinline__ float2 dot(const MmaCol<ALL> &col, int lane) const
+	{
+		const int t = lane & 3;
+		const uint8_t *xp = col.x + 8 * t;
 		const __half2 k96 = __float2half2_rn(96.0f);
 		float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -246,7 +290,7 @@ struct MmaRows<W_Q6K_R8> {
 					w[i][1] = h2_bits(__hsub2(bits_h2(and_or(v >> 4, 0x03F003F0u, 0x54005400u)), k96));
 				}
 				uint2 x = make_uint2(0, 0);
-				if (on)
+				if (col.reads())
 					x = *reinterpret_cast<const uint2 *>(xp + 2 * (128 * (pp >> 1) + 16 * (pp & 1) + 32 * q));
 				float p[4] = {0.f, 0.f, 0.f, 0.f};
 				mma_16816(p, w[0][0], w[1][0], w[0][1], w[1][1], x.x, x.y);
@@ -259,8 +303,7 @@ struct MmaRows<W_Q6K_R8> {
 				s[3] = __fmaf_rn(s1, p[3], s[3]);
 			}
 		}
-		r = quad_rows(s);
-		scale = make_float2(d[0] * inv, d[1] * inv);
+		return quad_rows(s);
 	}
 };
 

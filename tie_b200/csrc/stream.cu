@@ -156,6 +156,16 @@ static int launch_stream_k(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor
 // Supported input dims are compiled in; anything else is TIE_CUDA_ENOTSUP.
 #define TIE_STREAM_DIMS(X) X(256) X(512) X(768) X(1024) X(1536) X(2048) X(4096)
 
+bool stream_supported(const Layer &L)
+{
+	auto ok = [](int k) {
+#define X(KK) k == KK ||
+		return TIE_STREAM_DIMS(X) false;
+#undef X
+	};
+	return L.gate.kind == L.up.kind && ok(L.gate.k) && ok(L.down.k);
+}
+
 int launch_stream_gate_up(tie_cuda_ctx *c, const Layer &L, const float *xin, int src_div, const int *row_expert,
 			  int n_rows, int direct)
 {
