@@ -147,6 +147,22 @@ def test_host_buffers_pageable_and_pinned(be, n_tokens, pinned):
         out.fill_(float("nan"))
 
 
+# The threads that help copying a pageable batch sleep once the call has returned: the process uses no processor time while
+# its caller sleeps (three helpers that poll on for 400 us would take up to 24 ms in 20 calls).
+def test_copy_helpers_sleep_after_the_call(be):
+    import time
+    from tie_b200 import moe
+    x = synth.make_x(0, 333)
+    out = np.empty_like(x)
+    used = 0.0
+    for _ in range(20):
+        be.moe_ffn_ptr(0, x, out, 333, moe.HOST | moe.GRAPH)
+        t0 = time.process_time()
+        time.sleep(0.002)
+        used += time.process_time() - t0
+    assert used < 6e-3
+
+
 # One launch for a run of blocks with the same gate / up kind: down tensors of both kinds in it, and a block in the
 # middle that needs a launch of its own.
 def test_one_token_stack_of_mixed_blocks(small_shape, ref_silu_table):

@@ -1030,6 +1030,14 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 	// context's pinned staging buffers
 	const bool x_pinned = is_pinned_host(x), out_pinned = is_pinned_host(out);
 	if (!x_pinned && !out_pinned && bytes >= COPY_MIN) {
+		struct Rest {  // (on every way out)
+			tie_cuda_ctx *c;
+			~Rest()
+			{
+				if (c->copy_pool)
+					c->copy_pool->rest();
+			}
+		} rest{c};
 		TRY(copy_in_chunks(c, x, bytes));
 		GraphKey k = {1, layer, n_tokens, c->s.x, c->s.out, bias_dev, nullptr, kflags | TIE_CUDA_DEVICE};
 		TRY(run_maybe_graphed(c, graph, k, [&]() { return moe_ffn_device(c, *L, c->s.x, c->s.out, n_tokens, bias_dev, nullptr, flags); }));

@@ -1,7 +1,7 @@
 // A few threads that copy memory in chunks beside the calling thread: what tie_cuda_moe_ffn moves between pageable
-// host buffers and the pinned staging.  One owner (the context's calling thread) at a time; after a copy the
-// helpers stay awake for SPIN_US (a call copies in, computes, copies out: waking a sleeping thread costs as much as
-// copying a chunk), then sleep.
+// host buffers and the pinned staging.  One owner (the context's calling thread) at a time.  Between the copies of a call
+// (in, compute, out: waking a sleeping thread costs as much as copying a chunk) the helpers stay awake, for SPIN_US at most;
+// when the call ends (rest) they sleep, so that the threads of a caller's own pool find the cores free.
 #pragma once
 
 #include <string.h>
@@ -21,6 +21,7 @@ class CopyPool {
 	std::thread helpers_[MAX_HELPERS];
 	int n_helpers_ = 0, inside_ = 0;  // helpers inside the current job (under mutex_)
 	std::atomic<uint64_t> job_{0};	  // (written under mutex_)
+	std::atomic<bool> in_call_{false};
 	bool open_ = false, quit_ = false;
 	char *dst_ = nullptr;
 	const char *src_ = nullptr;
@@ -37,7 +38,8 @@ class CopyPool {
 			if (seen) {
 				lk.unlock();
 				const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(SPIN_US);
-				while (job_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until)
+				while (in_call_.load(std::memory_order_relaxed) && job_.load(std::memory_order_acquire) == seen &&
+				       std::chrono::steady_clock::now() < until)
 					std::this_thread::yield();
 				lk.lock();
 			}
@@ -99,10 +101,13 @@ public:
 			allowed_.store(allowed, std::memory_order_relaxed);
 			left_.store(n, std::memory_order_release);
 			open_ = true;
+			in_call_.store(true, std::memory_order_relaxed);
 			job_.fetch_add(1, std::memory_order_release);
 		}
 		wake_.notify_all();
 	}
+	// The call that copied is over.
+	void rest() { in_call_.store(false, std::memory_order_relaxed); }
 	void allow(int n) { allowed_.store(n, std::memory_order_release); }
 	bool done(int i) const { return done_[i].load(std::memory_order_acquire); }
 	// Copies one chunk if there is one to copy.
