@@ -3,6 +3,9 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
 
 #include <atomic>
 #include <chrono>
@@ -453,6 +456,14 @@ int h2d(tie_cuda_ctx *c, void *dst, const void *src, size_t bytes, void *pin)
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(dst, pin, bytes, cudaMemcpyHostToDevice, c->stream));
 	}
 	return TIE_CUDA_OK;
+}
+
+// In a polling loop: leaves the core's pipeline to its other hardware thread.
+inline void cpu_pause()
+{
+#if defined(__x86_64__)
+	_mm_pause();
+#endif
 }
 
 size_t align_up(size_t v, size_t a)
@@ -1016,7 +1027,7 @@ int tie_cuda_moe_ffn_biased(tie_cuda_ctx *c, int layer, const float *x, float *o
 		}));
 		const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(500);
 		while (*word == PENDING && std::chrono::steady_clock::now() < until)
-			;
+			cpu_pause();
 		std::atomic_thread_fence(std::memory_order_acquire);
 		if (*word == PENDING)  // (work in front of it on the stream, a time-out in the kernel, or the chain ran instead)
 			TRY(check_status(c));
