@@ -39,8 +39,6 @@
 #include "tc_ptx.cuh"
 #include "decode_common.cuh"
 #include "router_topk.cuh"
-#define TIE_TIMING_DF_OWNER
-#include "timing.cuh"
 
 namespace tie {
 
@@ -154,7 +152,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 	const int n_chunks = gu_role ? (g1 - g0 + CH - 1) / CH : 0;
 	const uint32_t tile_gu = (uint32_t)(tile_offset<KG>(NBK, g1) - tile_offset<KG>(NBK, g0));
 
-	DF_STAMP(0);
 	if (tid == DF_THREADS - 1) {  // (not in a warp that the norm or the router waits for)
 		for (int c = 0; c < DF_MAX_CHUNKS; c++)
 			ptx::mbar_init(ptx::smem_u32(&sh.bar_gu[c]), 1);
@@ -237,10 +234,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			if (lane == 0)
 				sh.x_inv[b] = inv;
 		}
-		DF_STAMP(1);
 		if (!df_grid_barrier(a.sync, target += (unsigned)G, &sh, a.status))
 			return;	 // nothing of this CTA is in flight yet
-		DF_STAMP(2);
 
 		// ---------------- selection (every CTA for itself) and all weight requests ----------------
 		if (warp == 0) {
@@ -331,7 +326,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		};
 
 		// ---------------- G: gate, up, SwiGLU ----------------
-		DF_STAMP(3);
 		if (gu_role && !bad) {
 			// a job is (chunk of 16 rows, matrix, super-block); the products of a row's super-blocks are added up in order
 			const int jobs = n_chunks * 2 * NBK;
@@ -340,8 +334,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 				alive = __all_sync(0xffffffffu, dec_wait(ptx::smem_u32(&sh.bar_gu[chunk]), a.status, parity));
 				if (!alive)
 					break;
-				if (i == warp && lane == 0)
-					DF_STAMP(7);
 				if (i + DF_WARPS >= jobs && lane == 0)	// the warp's last
 					request_down();
 				MmaRows<KG> w;
@@ -365,10 +357,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 				}
 				__stcg(a.h + (size_t)slot * F + g0 + tid, swiglu_lut(a.silu, g, u));
 			}
-			DF_STAMP(8);
 		}
 		alive = __syncthreads_and(alive);
-		DF_STAMP(4);
 		if (!alive) {  // a copy never landed: leave, but not with copies in flight
 			if (tid == 0)
 				drain();
@@ -381,7 +371,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		}
 
 		// ---------------- D: down + combine ----------------
-		DF_STAMP(5);
 		const bool more = layer + 1 < a.n_layers && !bad;  // (bad is the same in every CTA: they all selected alike)
 		if (more && tid == 0) {	 // this CTA's share of the next block's router matrix -> L2
 			const uint32_t bytes = (uint32_t)a.n_expert * K * sizeof(float), per = ((bytes + G - 1) / G + 15u) & ~15u, o = per * (uint32_t)cta;
@@ -396,7 +385,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		if (dn_role && !bad) {
 			alive = dn_q6k ? df_down<W_Q6K_R8, F>(dsm, sd, prod, a.h, top_k, tile_dn, warp, lane, sh, a.status, parity)
 				       : df_down<W_Q4K, F>(dsm, sd, prod, a.h, top_k, tile_dn, warp, lane, sh, a.status, parity);
-			DF_STAMP(10);
 			alive = __syncthreads_and(alive);
 			if (alive) {
 				for (int lr = tid; lr < d1 - d0; lr += DF_THREADS) {
@@ -416,7 +404,6 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			}
 		}
 		__syncthreads();
-		DF_STAMP(6);
 		if (!alive || !more) {
 			if (tid == 0) {
 				drain();
