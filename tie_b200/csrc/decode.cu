@@ -5,7 +5,7 @@
 // Reference: process_expert_task (engine.c:916-964) for the selected experts of a token and the
 // weighted combine (model_qwen3.c:458-467).
 //
-//   decode_gate_up       CTA = (16 output rows, (token, slot)), warp = one super-block of the input row:
+//   decode_gate_up       CTA = (a run of 16-row tiles, (token, slot)), warp = one super-block of the input row:
 //                        gate and up products, summed over the warps -> SwiGLU -> h
 //   decode_down_combine  CTA = (16 output rows, token), warp = one slot: the packed rows of all slots are
 //                        requested (one bulk copy per slot) before the wait for h; a warp's super-blocks add up in
@@ -13,8 +13,8 @@
 //                        zero — the reference's combine — so no per-slot output and no combine pass exist.
 //
 // What bounds it: at 1-4 tokens latency (three dependent launches, 2-3 us each), above that the expansion of
-// the packed weights (about 230 instructions per warp for 16 rows x 256 Q4_K weights, 450 for Q6_K).
-// Rows that share an expert expand it once each (at 8 tokens 64 rows use about 51 experts).
+// the packed weights (330 instructions per warp for 16 rows x 256 Q4_K weights, loads and all; 600 for Q6_K, and 150 for the
+// image of h).  Rows that share an expert expand it once each.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma_dot.cuh"
@@ -29,8 +29,8 @@ constexpr int DEC_MAX_NB = 8;  // super-blocks per row
 // A CTA walks n_tiles row tiles of its slot: the image of x is made once, a matrix's next tile is loaded into the
 // registers that its products have just left and lands under the other matrix's, and one more warp adds up a
 // tile and stores h while the others are at the next.
-// A block of 3 / 4 / 6 / 8 tokens 46.2 / 58.6 / 69.7 / 84.7 -> 44.4 / 57.2 / 64.6 / 84.8 us against a CTA per tile (4 tokens:
-// 53 MB in 16 us; the pipes are 20 - 45 % busy, the warps wait for one another, for loads and for the products).
+// A block of 3 / 4 / 6 tokens 46.2 / 58.6 / 69.7 -> 44.4 / 57.2 / 64.6 us against a CTA per tile (4 tokens: 53 MB in 16 us;
+// the pipes are 20 - 45 % busy, the warps wait for one another, for loads and for the products).
 template <WKind KIND>
 __global__ void __launch_bounds__((DEC_MAX_NB + 1) * 32, 2)
 decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert, int nb, int n_tiles,
@@ -96,8 +96,8 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 
 // The product of slot j's 16 staged rows with its h row, in this warp: lane (g, t = 0, 1) ends up with rows g, g + 8.
 // The row's next super-block is loaded under the products of the one before, and the tile is waited for (bar;
-// false in ok: it never landed) when the first image is made.  (A block of 3 / 4 / 8 tokens 40.6 / 47.3 / 79.3 -> 39.1 / 46.5 /
-// 76.4 us against all warps waiting for all tiles before their first load of h.)
+// false in ok: it never landed) when the first image is made.  (A block of 3 / 4 tokens 40.6 / 47.3 -> 39.1 / 46.5 us against
+// all warps waiting for all tiles before their first load of h.)
 template <WKind KIND>
 __device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const float *hrow, uint8_t *img, int lane, uint32_t bar,
 					    unsigned *status, bool &ok)
@@ -310,8 +310,8 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out)
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
-	// Q4_K: three CTAs per SM where that saves a wave (3 and 5 - 8 tokens of this model).  Blocks of which half have such a
-	// down tensor, at 6 / 8 tokens: 58.0 / 76.5 -> 57.5 / 75.6 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
+	// Q4_K: three CTAs per SM where that saves a wave (3, 5 and 6 tokens of this model).  Blocks with such a down tensor, at 3 / 5
+	// / 6 tokens: 36.7 / 50.8 / 55.9 -> 36.3 / 49.8 / 55.0 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
 	const long long grid = (long long)(L.down.rows / 16) * n_tokens, two = 2 * c->sm_count, three = 3 * c->sm_count;
 	const bool many = (grid + three - 1) / three < (grid + two - 1) / two;
 	auto kern = L.down.kind != W_Q4K ? decode_down_combine<W_Q6K_R8> : many ? decode_down_combine<W_Q4K, 3> : decode_down_combine<W_Q4K>;

@@ -4,7 +4,7 @@
 // (model_qwen3.c:403-471).  The three-kernel decode path (decode.cu) pays three launches and
 // cannot keep the down tiles in flight under the gate/up kernel (the two kernels do not fit one
 // SM together).  Here one cooperative grid (one CTA per SM, all co-resident) walks the phases
-// with two grid-wide barriers:
+// with grid-wide barriers between them, two in a block and one behind it:
 //
 //   R  CTA e < n_expert: logit e by warp 0, the AVX2 lane order replayed (8 chains of sequential fused
 //      multiply-adds, hsum tree: bit-exact, as router_batch); other warps meanwhile make the
@@ -22,12 +22,11 @@
 //   -- barrier, the next block of a stack --
 //
 // A stack of blocks is one launch (the blocks may differ in the kind of the down tensor): a third barrier costs less
-// than the end of a grid and the start of the next, 22.7 -> 21.1 us a block, 20.3 with the norm weights loaded beside the row instead of behind its sum.
+// than the end of a grid and the start of the next, 22.7 -> 21.1 us a block, 20.2 with the norm weights loaded beside the row instead of behind its sum.
 //
-// Bound by latency: of 22.6 us for one block, 4.7 are RMSNorm + router chains, 3 the two grid
-// barriers, 1.7 the selection, 2 the first tile's arrival, 4 gate/up, 3 down, 3.4 launch and tail (the
-// 25.5 MB themselves would take 3.9).  28.9 us with scalar reductions and the row and the router matrix
-// loaded one after the other.
+// Bound by latency: of 23.5 us for one block with its weights in HBM, 4.0 are RMSNorm + router chains, 1.4 and 1.9 the
+// two grid barriers, 1.5 the selection, 3.0 the first tile's arrival, 4.5 gate/up, 3.3 the down products, 0.6 the combine, 3.3
+// launch and tail (the 25.5 MB themselves would take 3.9).
 //
 // The barriers count arrivals in a device word that only grows (targets are relative to an epoch
 // the last CTA of every launch advances), so the launch arguments never change and the kernel

@@ -1,11 +1,11 @@
 // Warp-level products of 16 packed weight rows x one super-block with ONE activation row on the
 // mma.sync tensor path, exact to fp32: the building block of the decode kernels (decode.cu,
-// decode_fused.cu), which stay bit-identical to one another because they share it.
+// decode_group.cu, decode_fused.cu), which stay bit-identical to one another because they share it.
 //
 // An activation row enters as THREE fp16 parts (hi, mid, lo: 33 significand bits after a power-of-two
-// scaling of the super-block, so an fp32 value is represented exactly) that sit in columns 0, 1, 2
-// of the MMA's 8: one m16n8k16 covers 16 rows x 16 k of all three, and the columns are added in fp32
-// at the end.  The weights are exact small integers in fp16 (tc_dequant.cuh): sc*q for Q4_K, q - 32
+// scaling of the super-block: fp32 values down to 2^-10 of the super-block's largest are represented exactly,
+// smaller ones to 2^-34 of the largest) that sit in columns 0, 1, 2 of the MMA's 8 (a second row's in 4, 5, 6):
+// one m16n8k16 covers 16 rows x 16 k of all three, and the columns are added in fp32 at the end.  The weights are exact small integers in fp16 (tc_dequant.cuh): sc*q for Q4_K, q - 32
 // for Q6_K, whose 16-wide scale groups are one MMA each and are scaled in fp32 afterwards (their
 // products sc*(q-32) would not always fit 11 bits).  A lane therefore expands packed words straight into its
 // fragment registers, 4.5 (Q4_K) to 7 (Q6_K) instructions per 4 weights where a scalar reduction needs 12 to

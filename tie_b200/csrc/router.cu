@@ -19,7 +19,7 @@
 
 namespace tie {
 
-// Large token counts: CTA = TT tokens x EPC experts; thread = (expert, lane); router weights come
+// tie_cuda_route_noalloc from 9 tokens: CTA = TT tokens x EPC experts; thread = (expert, lane); router weights come
 // straight from L2 (each loaded value feeds TT fused multiply-adds), x is staged in k-chunks.
 template <int TT, int EPC, int KC>
 __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__restrict__ x, const float *__restrict__ w,
@@ -215,10 +215,9 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 		counter[blockIdx.x] = 0;
 }
 
-// Decode-sized token counts (<= 8 tokens): one expert per CTA so the 1 MB of router weights is
-// pulled by many SMs at once; the row and the tokens are staged in shared memory with wide
-// loads, then thread (token, lane) runs the sequential chain.
-template <int MAXT>
+// The F32 row entry and tie_cuda_route_noalloc up to 8 tokens (MoE calls of every size run on router_batch): one
+// expert per CTA; the row and the tokens are staged in shared memory with wide loads, then thread (token, lane)
+// runs the sequential chain.
 __global__ void __launch_bounds__(64) router_logits_decode(const float *__restrict__ x, const float *__restrict__ w,
 							   const float *__restrict__ bias, float *__restrict__ logits,
 							   int n_tokens, int hidden, int n_expert)
@@ -328,7 +327,7 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 // Opt-in shared-memory sizes are set once per context (never inside a stream capture).
 int router_setup(tie_cuda_ctx *c)
 {
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
 #define TIE_RT_ATTR(A, B, ...) \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, __VA_ARGS__::SMEM));
 	TIE_RT_TILES(TIE_RT_ATTR)
@@ -342,7 +341,7 @@ int launch_router_rows(tie_cuda_ctx *c, const float *x, const float *w, int n_ro
 	size_t smem = ((size_t)in_dim + (size_t)(in_dim + 8)) * sizeof(float);
 	if (smem > 200 * 1024)
 		return TIE_CUDA_ENOTSUP;
-	router_logits_decode<8><<<n_rows, 64, smem, c->stream>>>(x, w, nullptr, out, 1, in_dim, n_rows);
+	router_logits_decode<<<n_rows, 64, smem, c->stream>>>(x, w, nullptr, out, 1, in_dim, n_rows);
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }
@@ -402,7 +401,7 @@ extern "C" int tie_cuda_route_noalloc(const float *x_dev, const float *router_w_
 			cudaGetLastError();
 			return TIE_CUDA_ECUDA;
 		}
-		if (cudaFuncSetAttribute(router_logits_decode<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
+		if (cudaFuncSetAttribute(router_logits_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) !=
 		    cudaSuccess) {
 			cudaGetLastError();
 			return TIE_CUDA_ECUDA;
@@ -413,7 +412,7 @@ extern "C" int tie_cuda_route_noalloc(const float *x_dev, const float *router_w_
 	setup_lock.unlock();
 	cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
 	if (n_tokens <= 8) {
-		router_logits_decode<8><<<n_expert, 64, smem, st>>>(x_dev, router_w_dev, router_bias_dev, logits, n_tokens, hidden, n_expert);
+		router_logits_decode<<<n_expert, 64, smem, st>>>(x_dev, router_w_dev, router_bias_dev, logits, n_tokens, hidden, n_expert);
 	} else {
 		constexpr int TT = 8, EPC = 16;
 		if (hidden % 256)
