@@ -15,7 +15,8 @@ value      tokens/s of the whole job, inputs resident in HBM, CUDA-event timed o
 e2e        the same through the reference-facing C-ABI call with HOST buffers (H2D and D2H inside)
 roofline   the dominant kernel (gate/up product) against the measured HBM peak
 cpu_baseline  the reference's own AVX2 path (oracle/_ref) — or the C restatement when that
-           library is absent — timed on this box's host cores on a bounded sample
+           library is absent — timed on this box's host cores on a bounded sample; --impl reference
+           runs nothing but the former, and says so where it is absent
 extra      decode (1 token), 64-, 4096- and 8192-token runs of the same block, the 48-block stack
 parity     (N > 1) sampled output rows of every rank against the CPU restatement, outside the timed regions
 
@@ -192,6 +193,10 @@ def run_reference_arm(args):
     on the batch size).  ms_per_step is the time of what ran."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    from oracle import ref
+    if not ref.available():  # (the restatement is not the reference: its rate would be taken for it)
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libtie_ref.so is not built: the reference's sources were not found"}))
         return
     world = int(os.environ.get("WORLD_SIZE", "1"))
     from tie_b200 import synth, workloads

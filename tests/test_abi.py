@@ -103,3 +103,15 @@ def test_reference_side_glue_compiles_against_the_reference_headers(tmp_path):
                            "-I", ref_dir, "-I", os.path.join(ROOT, "include"), "-I", os.path.dirname(src), "-o", str(obj)])
     syms = subprocess.check_output(["nm", "--defined-only", str(obj)], text=True)
     assert "tie_cuda_qwen3_load" in syms and "tie_cuda_qwen3_moe_ffn" in syms
+
+
+def test_reference_arm_of_the_benchmark_is_the_reference_or_nothing():
+    import json
+    import sys
+    from oracle import ref
+    if ref.available():
+        pytest.skip("the compiled reference is here")
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1", "--warmup", "1"],
+                       capture_output=True, text=True, timeout=300)
+    line = json.loads(r.stdout)
+    assert r.returncode == 0 and line["impl"] == "reference" and line["unavailable"] and "value" not in line
