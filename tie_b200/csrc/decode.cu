@@ -311,7 +311,7 @@ int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, co
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
 	// Q4_K: three CTAs per SM where that saves a wave (3, 5 and 6 tokens of this model).  Blocks with such a down tensor, at 3 / 5
-	// / 6 tokens: 36.7 / 50.8 / 55.9 -> 36.3 / 49.8 / 55.0 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
+	// / 6 tokens: 37.8 / 51.4 / 55.8 -> 37.6 / 50.0 / 54.7 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
 	const long long grid = (long long)(L.down.rows / 16) * n_tokens, two = 2 * c->sm_count, three = 3 * c->sm_count;
 	const bool many = (grid + three - 1) / three < (grid + two - 1) / two;
 	auto kern = L.down.kind != W_Q4K ? decode_down_combine<W_Q6K_R8> : many ? decode_down_combine<W_Q4K, 3> : decode_down_combine<W_Q4K>;

@@ -5,8 +5,8 @@
 // An activation row enters as THREE fp16 parts (hi, mid, lo: 33 significand bits after a power-of-two
 // scaling of the super-block: fp32 values down to 2^-10 of the super-block's largest are represented exactly,
 // smaller ones to 2^-34 of the largest) that sit in columns 0, 1, 2 of the MMA's 8 (a second row's in 4, 5, 6):
-// one m16n8k16 covers 16 rows x 16 k of all three, and the columns are added in fp32 at the end.  The weights are exact small integers in fp16 (tc_dequant.cuh): sc*q for Q4_K, q - 32
-// for Q6_K, whose 16-wide scale groups are one MMA each and are scaled in fp32 afterwards (their
+// one m16n8k16 covers 16 rows x 16 k of all three, and the columns are added in fp32 at the end.  The weights
+// are exact small integers in fp16 (tc_dequant.cuh): sc*q for Q4_K, q - 32 for Q6_K, whose 16-wide scale groups are one MMA each and are scaled in fp32 afterwards (their
 // products sc*(q-32) would not always fit 11 bits).  A lane therefore expands packed words straight into its
 // fragment registers, 4.5 (Q4_K) to 7 (Q6_K) instructions per 4 weights where a scalar reduction needs 12 to
 // 16, needs no activations in registers, and the k order inside a super-block is free: lane t of a
@@ -30,9 +30,19 @@ struct XImage {
 	static_assert(BYTES % 16 == 0, "image size");
 };
 
+// A float rounded to a multiple of the last bit of c = 1.5 x 2^n (it has to be below 2^(n-1)).
+__device__ __forceinline__ float on_grid(float v, float c)
+{
+	return __fsub_rn(__fadd_rn(v, c), c);
+}
+
 // One warp: 8 consecutive values per lane -> the image; returns the factor that undoes the scaling.
 // The values are scaled by a power of two so that the largest lies in [2^9, 2^10): sums of 32 stay
 // inside fp16, and a part's last bit is 2^-24.
+// The parts lie on fixed grids, multiples of 2^-1 and of 2^-12 (sums of 32: 2^4, 2^-7) and what is left: the tensor
+// cores cut the low bits off a sum at every step, always towards zero, and on a grid the products (at most 21 bits) add
+// up to what 24 bits hold, nearly always.  (Parts rounded each to its own 11 bits: a block of 1 - 8 tokens was 2.9e-7 -
+// 4.5e-7 from 64-bit arithmetic, in fp32 throughout 0.6e-7 - 2.9e-7.)
 template <WKind KIND>
 __device__ __forceinline__ float x_image(const float (&v)[8], uint8_t *img, int lane)
 {
@@ -55,11 +65,10 @@ __device__ __forceinline__ float x_image(const float (&v)[8], uint8_t *img, int 
 			float r0 = a[2 * h], r1 = a[2 * h + 1];
 #pragma unroll
 			for (int p = 0; p < 3; p++) {
-				const __half2 q = __floats2half2_rn(r0, r1);
-				const float2 f = __half22float2(q);
-				part[p][2 * g + h] = h2_bits(q);
-				r0 -= f.x;
-				r1 -= f.y;
+				const float c = p == 0 ? 0x1.8p22f : 0x1.8p11f, q0 = p < 2 ? on_grid(r0, c) : r0, q1 = p < 2 ? on_grid(r1, c) : r1;
+				part[p][2 * g + h] = h2_bits(__floats2half2_rn(q0, q1));
+				r0 -= q0;
+				r1 -= q1;
 			}
 		}
 	}
@@ -74,9 +83,9 @@ __device__ __forceinline__ float x_image(const float (&v)[8], uint8_t *img, int 
 		if ((lane & 3) == 0) {
 #pragma unroll
 			for (int p = 0; p < 3; p++) {
-				const __half q = __float2half_rn(sum);
-				reinterpret_cast<__half *>(img + XImage<KIND>::SUMS + 16 * p)[lane >> 2] = q;
-				sum -= __half2float(q);
+				const float q = p < 2 ? on_grid(sum, p == 0 ? 0x1.8p27f : 0x1.8p16f) : sum;
+				reinterpret_cast<__half *>(img + XImage<KIND>::SUMS + 16 * p)[lane >> 2] = __float2half_rn(q);
+				sum -= q;
 			}
 		}
 	}
