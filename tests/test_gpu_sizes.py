@@ -62,7 +62,7 @@ def test_router_tiles_and_both_selections(be, port0, n_tokens):
     assert np.abs(w / w_r - 1).max() < 2e-6
 
 
-# 6 tokens are the last batch of the per-row kernels with 128 experts and top-8.
+# 7 tokens are the last batch of the per-row kernels with 128 experts and top-8.
 @pytest.mark.parametrize("n_tokens", [6, 8, 9, 12])
 def test_per_row_and_grouped_products_around_the_change(be, port0, n_tokens):
     x = synth.make_x(0, n_tokens, first_token=90)
@@ -233,14 +233,14 @@ def test_rms_norm_row_lengths(hidden, port_lib, ref_silu_table):
         b.close()
 
 
-# Below twice as many rows as experts every product is exact to fp32, as for one token: rows grouped by expert, two to
-# a group (7 tokens on with 128 experts and top-8), have the bits of their tokens alone, whichever experts they share.
+# Below twice as many rows as experts every product is exact to fp32, as for one token: rows grouped by expert, four to
+# a group (8 tokens on with 128 experts and top-8), have the bits of their tokens alone, whichever experts they share.
 @pytest.mark.parametrize("shared", [False, True])
-@pytest.mark.parametrize("n_tokens", [6, 7, 9, 20, 31])
+@pytest.mark.parametrize("n_tokens", [7, 8, 9, 20, 31])
 def test_small_batches_have_the_bits_of_single_tokens(be, port0, n_tokens, shared):
     x = synth.make_x(0, n_tokens, first_token=600)
     bias = None
-    if shared:  # all tokens on the same eight experts: groups of two and a remainder
+    if shared:  # all tokens on the same eight experts: groups of four and a remainder
         bias = np.zeros(128, dtype=np.float32)
         bias[[0, 3, 17, 44, 45, 90, 126, 127]] = 1000.0
     out = be.moe_ffn(0, x, router_bias=bias)

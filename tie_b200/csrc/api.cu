@@ -273,7 +273,7 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 		use_tc = false;
 	} else {
 		// Below twice as many rows as experts the products stay exact to fp32 (decode.cu, decode_group.cu, else the streaming
-		// kernels), also where the tensor path's fp16 hi + lo would be faster (a block of 20 / 31 tokens 121 / 155 us there, 114 /
+		// kernels), also where the tensor path's fp16 hi + lo would be faster (a block of 20 / 31 tokens 115 / 139 us there, 114 /
 		// 127 here).  Row lengths that none of them is built for come here from half as many rows as experts on.
 		use_tc = tc_supported(c, L) && (n_rows >= 2 * c->n_local || (2 * n_rows > c->n_local && !stream_supported(L)));
 	}

@@ -1,4 +1,4 @@
-// Decode and small batches (up to 6 tokens of this model's shape): the expert mat-vecs of every
+// Decode and small batches (up to 7 tokens of this model's shape): the expert mat-vecs of every
 // (token, slot) row on its own — no dispatch sort, no grouping — with the exact mma.sync products of
 // mma_dot.cuh.
 //
@@ -75,14 +75,14 @@ decode_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, s
 	const float inv = x_image<KIND>(v, img[b], lane);
 	for (int r = r0, buf = 0; r < r1; r += 16, buf ^= 1) {
 		const bool more = r + 16 < r1;
-		float2 p = g.dot(one_row<KIND>(img[b], lane), lane), s = g.scale(inv);
+		float2 p = dot_one(g, one_row<KIND>(img[b], lane), lane), s = g.scale(inv);
 		if (more)
 			g.load(wg + tile_offset<KIND>(nb, r + 16), nb, b, lane);
 		if ((lane & 3) == 0) {
 			red[buf][b][0][lane >> 2] = p.x * s.x;
 			red[buf][b][0][(lane >> 2) + 8] = p.y * s.y;
 		}
-		p = u.dot(one_row<KIND>(img[b], lane), lane);
+		p = dot_one(u, one_row<KIND>(img[b], lane), lane);
 		s = u.scale(inv);
 		if (more)
 			u.load(wu + tile_offset<KIND>(nb, r + 16), nb, b, lane);
@@ -118,7 +118,7 @@ __device__ __forceinline__ float2 down_rows(const uint8_t *tile, int nb, const f
 			ok = __all_sync(0xffffffffu, dec_wait(bar, status));
 		MmaRows<KIND> w;
 		w.load_smem(tile, nb, b, lane);
-		const float2 r = w.dot(one_row<KIND>(img, lane), lane), s = w.scale(inv);
+		const float2 r = dot_one(w, one_row<KIND>(img, lane), lane), s = w.scale(inv);
 		out.x = __fmaf_rn(s.x, r.x, out.x);
 		out.y = __fmaf_rn(s.y, r.y, out.y);
 	}
@@ -310,8 +310,9 @@ int launch_decode_gate_up(tie_cuda_ctx *c, const Layer &L, const float *x, int n
 int launch_decode_down_combine(tie_cuda_ctx *c, const Layer &L, int n_tokens, const float *residual, float *out)
 {
 	const int top_k = c->cfg.top_k, nb = L.down.k / QK_K;
-	// Q4_K: three CTAs per SM where that saves a wave (3, 5 and 6 tokens of this model).  Blocks with such a down tensor, at 3 / 5
-	// / 6 tokens: 37.8 / 51.4 / 55.8 -> 37.6 / 50.0 / 54.7 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so not there.
+	// Q4_K: three CTAs per SM where that saves a wave (3 and 5 - 7 tokens of this model).  Blocks with such a down tensor, at 3 / 5
+	// / 6 / 7 tokens: 37.8 / 51.4 / 55.8 / 63.0 -> 37.6 / 50.0 / 54.7 / 61.9 us; at 2 (one wave) 32.3 -> 33.3, at 4 (two) equal, so
+	// not there.
 	const long long grid = (long long)(L.down.rows / 16) * n_tokens, two = 2 * c->sm_count, three = 3 * c->sm_count;
 	const bool many = (grid + three - 1) / three < (grid + two - 1) / two;
 	auto kern = L.down.kind != W_Q4K ? decode_down_combine<W_Q6K_R8> : many ? decode_down_combine<W_Q4K, 3> : decode_down_combine<W_Q4K>;

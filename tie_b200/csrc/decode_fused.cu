@@ -121,7 +121,7 @@ __device__ __forceinline__ bool df_down(uint8_t *dsm, const uint8_t *sd, float *
 			return false;
 		MmaRows<KD> w;
 		w.load_smem(sd + (size_t)j * tile_dn, NBF, b, lane);
-		const float2 r = w.dot(one_row<KD>(himg, lane), lane), s = w.scale(inv);
+		const float2 r = dot_one(w, one_row<KD>(himg, lane), lane), s = w.scale(inv);
 		if ((lane & 3) == 0) {
 			float2 *d = reinterpret_cast<float2 *>(prod) + i * 16 + (lane >> 2);
 			d[0] = make_float2(r.x, s.x);
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 					request_down();
 				MmaRows<KG> w;
 				w.load_smem((mat ? su : sg) + tile_offset<KG>(NBK, chunk * CH), NBK, b, lane);
-				const float2 r = w.dot(one_row<KG>(ximg + b * XImage<KG>::BYTES, lane), lane), s = w.scale(sh.x_inv[b]);
+				const float2 r = dot_one(w, one_row<KG>(ximg + b * XImage<KG>::BYTES, lane), lane), s = w.scale(sh.x_inv[b]);
 				if ((lane & 3) == 0) {
 					float *d = prod + ((chunk * 2 + mat) * NBK + b) * 16 + (lane >> 2);
 					d[0] = r.x * s.x;

@@ -1,22 +1,21 @@
-// Small batches between the per-row decode kernels and the grouped tensor-core products (7 to 31 tokens of this
+// Small batches between the per-row decode kernels and the grouped tensor-core products (8 to 31 tokens of this
 // model's shape): rows that share an expert share the expansion of its packed weights, on the exact mma.sync
 // products of mma_dot.cuh, so that a row has the bits that the per-row kernels (decode.cu) give it.
 //
 // Reference: process_expert_task (engine.c:916-964) for the selected experts of a batch's tokens.
 //
-//   group_gate_up   item = (group of up to two rows of one expert, 16 output rows), warp = one super-block of the gate
+//   group_gate_up   item = (group of up to four rows of one expert, 16 output rows), warp = one super-block of the gate
 //                   or of the up rows; one more warp adds the super-blocks up -> SwiGLU -> h
 //   group_down      item = the same over the down rows, a warp per item -> y [(token, slot)][hidden]; combine_rows
 //                   (misc.cu) adds the slots up
 //
-// Every CTA makes the list of groups from the selection itself (a microsecond; no sort, no further launch) and takes an
-// equal share of the items, in one wave.
+// Every CTA makes the list of groups from the selection itself (a microsecond; no sort, no further launch) and takes its
+// share of the items, in one wave.
 //
 // What bounds it: the expansion (about 400 instructions per warp for 16 rows x 256 Q4_K weights with their loads and
-// hand-offs, 600 for Q6_K), which an expert's every second row pays again.  Groups of four (two MMAs a fragment) took 1.75 times
-// as long a tile as groups of two and balanced worse: 13 / 31 tokens 95 / 157 -> 98 / 159 us a block.
-// A block of 9 / 13 / 20 / 31 tokens with Q6_K down: 77 / 93 / 121 / 155 us; row by row 80 / 126 / 181 / 249; the grouped
-// tensor-core products, which hold activations in 22 bits, 85 / 95 / 114 / 127.
+// hand-offs, 600 for Q6_K), which an expert's every fourth row pays again.
+// A block of 9 / 13 / 20 / 31 tokens with Q6_K down: 80 / 94 / 115 / 139 us (in groups of two rows 77 / 93 / 121 / 155); row by
+// row 80 / 126 / 181 / 249; the grouped tensor-core products, which hold activations in 22 bits, 85 / 96 / 114 / 127.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma_dot.cuh"
@@ -25,7 +24,7 @@
 
 namespace tie {
 
-constexpr int DG_ROWS = 2;	   // rows of a group: the parts of two fit the eight columns of an MMA
+constexpr int DG_ROWS = 4;	   // rows of a group: the parts of two fit the eight columns of an MMA, and two MMAs share a fragment
 constexpr int DG_MAX_TOKENS = 32;  // a bit each
 constexpr int DG_MAX_ROWS = 256, DG_MAX_EXPERTS = 256;
 constexpr int DG_MAX_NB = 8;  // super-blocks per row
@@ -34,13 +33,18 @@ constexpr int DG_DOWN_WARPS = 8;
 // tile, or the last warp at a tile adding it up itself: 15 - 25 % slower).
 constexpr int DG_STAGES = 8;
 
+// What a tile of a group of one or two rows costs, and of three or four (the second MMAs and their operands).  31 tokens with 4 : 7 /
+// 2 : 3 / 3 : 4 / 5 : 6: 153 / 143 / 139 / 134 us without the norm.
+constexpr int DG_COST1 = 5, DG_COST2 = 6;
+
 // The rows of a call by expert, in token order, cut in groups of DG_ROWS.
 struct GroupList {
 	unsigned tokens[DG_MAX_EXPERTS];  // per expert: who selected it
 	uint8_t id[DG_MAX_EXPERTS][DG_MAX_TOKENS / DG_ROWS];
 	uint8_t expert[DG_MAX_ROWS], size[DG_MAX_ROWS];
 	uint8_t row[DG_MAX_ROWS][DG_ROWS];
-	int first, last;  // this CTA's items, an equal share of them; item = group * tiles + tile
+	int cost[DG_MAX_ROWS];	// of a tile of every group before this one
+	int first, last;	// this CTA's items, item = group * tiles + tile
 
 	// By all threads of a CTA.  An expert occurs at most once among a token's slots (top-k), so a row's place among
 	// its expert's is the number of earlier tokens that selected the expert.
@@ -59,26 +63,41 @@ struct GroupList {
 		}
 		__syncthreads();
 		if (threadIdx.x < 32) {
-			int made = 0;
+			int made = 0, total = 0;
 			for (int i0 = 0; i0 < n_rows; i0 += 32) {
 				const int i = i0 + threadIdx.x, e = i < n_rows ? topk_idx[i] - first_expert : -1;
 				const bool on = e >= 0 && e < n_local;
 				const int place = on ? __popc(tokens[e] & ((1u << (i / top_k)) - 1u)) : 0;
-				const unsigned firsts = __ballot_sync(0xffffffffu, on && place % DG_ROWS == 0);
-				if (on && place % DG_ROWS == 0) {
-					const int g = made + __popc(firsts & ((1u << threadIdx.x) - 1u));
+				const bool lead = on && place % DG_ROWS == 0;
+				const int size_here = lead ? min(DG_ROWS, __popc(tokens[e]) - place) : 0;
+				const unsigned firsts = __ballot_sync(0xffffffffu, lead), wide = __ballot_sync(0xffffffffu, size_here > 2);
+				if (lead) {
+					const unsigned below = (1u << threadIdx.x) - 1u;
+					const int g = made + __popc(firsts & below);
 					id[e][place / DG_ROWS] = (uint8_t)g;
 					expert[g] = (uint8_t)e;
-					size[g] = (uint8_t)min(DG_ROWS, __popc(tokens[e]) - place);
+					size[g] = (uint8_t)size_here;
+					cost[g] = total + DG_COST1 * __popc(firsts & below) + (DG_COST2 - DG_COST1) * __popc(wide & below);
 				}
 				made += __popc(firsts);
+				total += DG_COST1 * __popc(firsts) + (DG_COST2 - DG_COST1) * __popc(wide);
 				__syncwarp();
 				if (on)	 // (the group's first row is an earlier one: same or earlier round)
 					row[id[e][place / DG_ROWS]][place % DG_ROWS] = (uint8_t)i;
 			}
+			// the CTA's share of the items: what starts between two equal steps of their cost
+			int bound[2];
+			for (int k = 0; k < 2; k++) {
+				const int c = (int)((long long)total * tiles * (blockIdx.x + k) / gridDim.x);
+				int g = -1;  // the last group that starts at or before c
+				for (int g0 = 0; g0 < made; g0 += 32)
+					g += __popc(__ballot_sync(0xffffffffu, g0 + (int)threadIdx.x < made && cost[g0 + threadIdx.x] * tiles <= c));
+				const int w = g < 0 ? 1 : (size[g] > 2 ? DG_COST2 : DG_COST1);
+				bound[k] = g < 0 ? 0 : g * tiles + min(tiles, (c - cost[g] * tiles + w - 1) / w);
+			}
 			if (threadIdx.x == 0) {
-				first = (int)((long long)made * tiles * blockIdx.x / gridDim.x);
-				last = (int)((long long)made * tiles * (blockIdx.x + 1) / gridDim.x);
+				first = bound[0];
+				last = bound[1];
 			}
 		}
 		__syncthreads();
@@ -141,6 +160,31 @@ struct TileCursor {
 	}
 };
 
+// h of a group's rows (ROWS at most) from a tile's products p, which lie [gate, up by half-warp][super-block][row][16]: all rows
+// together, as one after the other their sums and table look-ups take longer than a tile (31 tokens 159 -> 139 us).
+template <int ROWS>
+__device__ __forceinline__ void group_h(const float *p, int nb, int n, const uint8_t *row, float *h, int rows_per_expert, const float *silu, int lane)
+{
+	float sum[ROWS], act[ROWS];
+#pragma unroll
+	for (int m = 0; m < ROWS; m++)
+		sum[m] = p[m * 16];
+	for (int i = 1; i < nb; i++)
+#pragma unroll
+		for (int m = 0; m < ROWS; m++)
+			sum[m] = __fadd_rn(sum[m], p[(i * DG_ROWS + m) * 16]);
+#pragma unroll
+	for (int m = 0; m < ROWS; m++) {
+		const float up = __shfl_down_sync(0xffffffffu, sum[m], 16);
+		act[m] = m < n ? swiglu_lut(silu, sum[m], up) : 0.f;
+	}
+	if (lane < 16)
+#pragma unroll
+		for (int m = 0; m < ROWS; m++)
+			if (m < n)
+				h[(size_t)row[m] * rows_per_expert] = act[m];
+}
+
 template <WKind KIND>
 __global__ void __launch_bounds__((2 * DG_MAX_NB + 1) * 32, 1)
 group_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, size_t expert_stride, int rows_per_expert, int nb,
@@ -177,14 +221,11 @@ group_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, si
 			const int n = gl.size[g];
 			ok = ok && dec_wait(ptx::smem_u32(&full[st]), status, parity);
 			const float *p = red + ((size_t)st * 2 + (lane >> 4)) * nb * RED_ROWS + (lane & 15);
-			for (int m = 0; m < n; m++) {
-				float sum = p[m * 16];
-				for (int i = 1; i < nb; i++)
-					sum = __fadd_rn(sum, p[i * RED_ROWS + m * 16]);
-				const float up = __shfl_down_sync(0xffffffffu, sum, 16);
-				if (lane < 16)
-					h[(size_t)gl.row[g][m] * rows_per_expert + r0 + lane] = swiglu_lut(silu, sum, up);
-			}
+			float *hp = h + r0 + lane;
+			if (n <= 2)
+				group_h<2>(p, nb, n, gl.row[g], hp, rows_per_expert, silu, lane);
+			else
+				group_h<DG_ROWS>(p, nb, n, gl.row[g], hp, rows_per_expert, silu, lane);
 			__syncwarp();
 			if (lane == 0)
 				ptx::mbar_arrive(ptx::smem_u32(&empty[st]));
@@ -213,21 +254,22 @@ group_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, si
 	ptx::cp_async_commit();
 	int n = 0, slot = 0, st = 0;
 	uint32_t parity = 1;  // of the stage: the first round finds every one empty
-	MmaCol<true> col;
+	MmaCol<true> col[2];
 	for (int it = items.x; it < items.y; it++) {
 		if (it == items.x || now.left == tiles) {  // another group: the gate and the up warp of a super-block make its images together
 			n = gl.size[now.g];
 			asm volatile("bar.sync %0, 64;" ::"r"(1 + b) : "memory");
-			if (mat < n) {
-				const float4 *xp = reinterpret_cast<const float4 *>(x + (size_t)(gl.row[now.g][mat] / top_k) * nb * QK_K + b * QK_K) + 2 * lane;
+			for (int m = mat; m < n; m += 2) {
+				const float4 *xp = reinterpret_cast<const float4 *>(x + (size_t)(gl.row[now.g][m] / top_k) * nb * QK_K + b * QK_K) + 2 * lane;
 				const float4 x0 = xp[0], x1 = xp[1];
 				const float v[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-				const float f = x_image<KIND>(v, img + mat * XImage<KIND>::BYTES, lane);
+				const float f = x_image<KIND>(v, img + m * XImage<KIND>::BYTES, lane);
 				if (lane == 0)
-					inv[b][mat] = f;
+					inv[b][m] = f;
 			}
 			asm volatile("bar.sync %0, 64;" ::"r"(1 + b) : "memory");
-			col = two_rows<KIND>(img, XImage<KIND>::BYTES, n, zeros, lane);
+			col[0] = two_rows<KIND>(img, XImage<KIND>::BYTES, 0, n, zeros, lane);
+			col[1] = two_rows<KIND>(img, XImage<KIND>::BYTES, 2, n, zeros, lane);
 		}
 		ptx::cp_async_wait<0>();
 		__syncwarp();  // (everybody's pieces are there, and everybody is done with the other slot)
@@ -241,12 +283,21 @@ group_gate_up(const uint8_t *__restrict__ wg, const uint8_t *__restrict__ wu, si
 		wr.load_chunk(chunks + slot * ChunkCopy<KIND>::BYTES, now.tile, nb, b, lane);
 		ok = ok && dec_wait(ptx::smem_u32(&empty[st]), status, parity);
 		float *dst = red + ((size_t)(st * 2 + mat) * nb + b) * RED_ROWS;
-		const float2 r = wr.dot(col, lane);
-		if ((lane & 1) == 0 && (lane >> 1 & 1) < n) {  // lanes t = 0 of a quad have the first row, t = 2 the second
-			const int m = lane >> 1 & 1;
-			const float2 f = wr.scale(inv[b][m]);
-			dst[m * 16 + (lane >> 2)] = r.x * f.x;
-			dst[m * 16 + (lane >> 2) + 8] = r.y * f.y;
+		float2 r[2];
+		if (n > 2)
+			wr.dot(col, lane, r);
+		else
+			r[0] = r[1] = dot_one(wr, col[0], lane);
+		if ((lane & 1) == 0) {	// lanes t = 0 of a quad have the first row of a pair, t = 2 the second
+#pragma unroll
+			for (int p = 0; p < 2; p++) {
+				const int m = 2 * p + (lane >> 1 & 1);
+				if (m < n) {
+					const float2 f = wr.scale(inv[b][m]);
+					dst[m * 16 + (lane >> 2)] = r[p].x * f.x;
+					dst[m * 16 + (lane >> 2) + 8] = r[p].y * f.y;
+				}
+			}
 		}
 		__syncwarp();
 		if (lane == 0)
@@ -303,7 +354,7 @@ group_down(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_ex
 	settle(it, end);
 	if (lane == 0 && it < items.y)
 		request(it);
-	const int m = lane >> 1 & 1;  // of the group's rows
+	const int m = lane >> 1 & 1;  // of a pair of the group's rows
 	uint32_t parity = 0;
 	bool ok = true;
 	pdl_wait();  // h of the gate/up kernel is visible from here on
@@ -327,7 +378,7 @@ group_down(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_ex
 			settle(it, end);  // (the next item from here on)
 			ok = ok && __all_sync(0xffffffffu, dec_wait(ba, status, parity));
 			parity ^= 1;
-			float2 out = make_float2(0.f, 0.f);
+			float2 out[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 			for (int b = 0; b < nb && ok; b++) {
 				MmaRows<KIND> w;
 				w.load_smem(tile, nb, b, lane);
@@ -338,13 +389,25 @@ group_down(const uint8_t *__restrict__ wd, size_t expert_stride, int rows_per_ex
 						request(it);
 					}
 				}
-				const float2 r = w.dot(two_rows<KIND>(img + b * STRIDE, nb * STRIDE, n, zeros, lane), lane), f = w.scale(inv[m][b]);
-				out.x = __fmaf_rn(f.x, r.x, out.x);
-				out.y = __fmaf_rn(f.y, r.y, out.y);
+				const MmaCol<true> col[2] = {two_rows<KIND>(img + b * STRIDE, nb * STRIDE, 0, n, zeros, lane),
+							     two_rows<KIND>(img + b * STRIDE, nb * STRIDE, 2, n, zeros, lane)};
+				float2 r[2];
+				if (n > 2)
+					w.dot(col, lane, r);
+				else
+					r[0] = r[1] = dot_one(w, col[0], lane);
+#pragma unroll
+				for (int p = 0; p < 2; p++) {
+					const float2 f = w.scale(inv[2 * p + m][b]);
+					out[p].x = __fmaf_rn(f.x, r[p].x, out[p].x);
+					out[p].y = __fmaf_rn(f.y, r[p].y, out[p].y);
+				}
 			}
-			// lanes t = 0, 1 of a quad hold rows g and g + 8 of the first row, t = 2, 3 of the second
-			if (ok && m < n)
-				y[(size_t)gl.row[g][m] * rows_per_expert + r0 + (lane >> 2) + 8 * (lane & 1)] = lane & 1 ? out.y : out.x;
+			// lanes t = 0, 1 of a quad hold rows g and g + 8 of the first row of a pair, t = 2, 3 of the second
+#pragma unroll
+			for (int p = 0; p < 2; p++)
+				if (ok && 2 * p + m < n)
+					y[(size_t)gl.row[g][2 * p + m] * rows_per_expert + r0 + (lane >> 2) + 8 * (lane & 1)] = lane & 1 ? out[p].y : out[p].x;
 		}
 	}
 }
@@ -367,10 +430,10 @@ static size_t group_down_smem(const DevTensor &t)
 
 bool decode_group_supported(const tie_cuda_ctx *c, const Layer &L, int n_tokens)
 {
-	// from where few rows have their expert to themselves: 6 / 7 / 8 tokens of this model's shape 61.2 / 66.2 / 71.8 us a
-	// block here, 60.4 / 68.0 / 79.4 row by row (decode.cu); up to where the tensor path takes over (run_experts)
+	// from where few rows have their expert to themselves: 7 / 8 tokens of this model's shape 68.9 / 74.1 us a block here, 67.7 /
+	// 78.9 row by row (decode.cu); up to where the tensor path takes over (run_experts)
 	const int n_rows = n_tokens * c->cfg.top_k;
-	return n_tokens > 4 && 8 * n_rows > 3 * c->n_local && n_tokens <= DG_MAX_TOKENS && n_rows <= DG_MAX_ROWS && n_rows < 2 * c->n_local && c->n_local <= DG_MAX_EXPERTS &&
+	return n_tokens > 4 && 16 * n_rows > 7 * c->n_local && n_tokens <= DG_MAX_TOKENS && n_rows <= DG_MAX_ROWS && n_rows < 2 * c->n_local && c->n_local <= DG_MAX_EXPERTS &&
 	       L.gate.kind == L.up.kind && L.gate.k <= DG_MAX_NB * QK_K && L.gate.rows % 16 == 0 && L.down.rows % 16 == 0 &&
 	       L.down.k <= DG_MAX_NB * QK_K && group_down_smem(L.down) <= (size_t)DG_MAX_SMEM && group_gate_up_smem(L.gate) <= (size_t)DG_MAX_SMEM;
 }

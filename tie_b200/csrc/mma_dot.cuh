@@ -121,11 +121,11 @@ __device__ __forceinline__ MmaCol<false> one_row(const uint8_t *img, int lane)
 	const int g = lane >> 2;
 	return {img + g * XImage<KIND>::PART, img + XImage<KIND>::SUMS + 16 * g, g < 3};
 }
-// two rows (the second image is `stride` bytes behind the first; n_rows = 1: there is none): columns 0 .. 2 and 4 .. 6
+// rows m0 and m0 + 1 of n_rows (their images `stride` bytes apart): columns 0 .. 2 and 4 .. 6
 template <WKind KIND>
-__device__ __forceinline__ MmaCol<true> two_rows(const uint8_t *img, int stride, int n_rows, const uint8_t *zeros, int lane)
+__device__ __forceinline__ MmaCol<true> two_rows(const uint8_t *img, int stride, int m0, int n_rows, const uint8_t *zeros, int lane)
 {
-	const int part = (lane >> 2) & 3, m = lane >> 4;
+	const int part = (lane >> 2) & 3, m = m0 + (lane >> 4);
 	if (part == 3 || m >= n_rows)
 		return {zeros, zeros, false};
 	img += m * stride;
@@ -188,9 +188,10 @@ struct MmaRows<W_Q4K> {
 		}
 	}
 	__device__ __forceinline__ float2 scale(float inv) const { return make_float2(inv, inv); }
-	// the tile's products with a row are scale(inv).x * r.x (row g) and scale(inv).y * r.y (row g + 8)
-	template <bool ALL>
-	__device__ __forceinline__ float2 dot(const MmaCol<ALL> &col, int lane) const
+	// the tile's products with a row are scale(inv).x * r.x (row g) and scale(inv).y * r.y (row g + 8); NP MMAs, of one or two
+	// rows each, share the expanded weights
+	template <int NP, bool ALL>
+	__device__ __forceinline__ void dot(const MmaCol<ALL> (&col)[NP], int lane, float2 (&r)[NP]) const
 	{
 		const int t = lane & 3;
 		const __half2 k1024 = __float2half2_rn(1024.0f);
@@ -211,16 +212,25 @@ struct MmaRows<W_Q4K> {
 			c[w].ch = __hmul2(s_hi, __float2half2_rn(-64.0f));
 			mins[w] = h2_bits(__hsub2(bits_h2(__byte_perm(mn, 0x64006400u, 0x7170u)), k1024));
 		}
-		float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f}, mm[4] = {0.f, 0.f, 0.f, 0.f};
-		const uint8_t *xp = col.x + t * XImage<W_Q4K>::BLK;
-		const uint32_t bs = col.reads() ? *reinterpret_cast<const uint32_t *>(col.sums + 4 * t) : 0u;
-		mma_1688(mm, mins[0], mins[1], bs);
+		float lo[NP][4], hi[NP][4], mm[NP][4];
+#pragma unroll
+		for (int p = 0; p < NP; p++) {
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+				lo[p][i] = hi[p][i] = mm[p][i] = 0.f;
+			mma_1688(mm[p], mins[0], mins[1], col[p].reads() ? *reinterpret_cast<const uint32_t *>(col[p].sums + 4 * t) : 0u);
+		}
 #pragma unroll
 		for (int i2 = 0; i2 < 4; i2++) {  // two words: 8 k of either sub-block
-			uint4 bl = make_uint4(0, 0, 0, 0), bh = bl;
-			if (col.reads()) {
-				bl = *reinterpret_cast<const uint4 *>(xp + 16 * i2);
-				bh = *reinterpret_cast<const uint4 *>(xp + 64 + 16 * i2);
+			uint4 bl[NP], bh[NP];
+#pragma unroll
+			for (int p = 0; p < NP; p++) {
+				const uint8_t *xp = col[p].x + t * XImage<W_Q4K>::BLK;
+				bl[p] = bh[p] = make_uint4(0, 0, 0, 0);
+				if (col[p].reads()) {
+					bl[p] = *reinterpret_cast<const uint4 *>(xp + 16 * i2);
+					bh[p] = *reinterpret_cast<const uint4 *>(xp + 64 + 16 * i2);
+				}
 			}
 			const uint4 w0 = q[0][i2 >> 1], w1 = q[1][i2 >> 1];
 			const uint32_t wa[2] = {i2 & 1 ? w0.z : w0.x, i2 & 1 ? w0.w : w0.y}, wb[2] = {i2 & 1 ? w1.z : w1.x, i2 & 1 ? w1.w : w1.y};
@@ -229,17 +239,23 @@ struct MmaRows<W_Q4K> {
 				uint32_t l0[2], h0[2], l1[2], h1[2];
 				q4k_int_word(wa[j], c[0], l0, h0);
 				q4k_int_word(wb[j], c[1], l1, h1);
-				mma_16816(lo, l0[0], l1[0], l0[1], l1[1], j ? bl.z : bl.x, j ? bl.w : bl.y);
-				mma_16816(hi, h0[0], h1[0], h0[1], h1[1], j ? bh.z : bh.x, j ? bh.w : bh.y);
+#pragma unroll
+				for (int p = 0; p < NP; p++) {
+					mma_16816(lo[p], l0[0], l1[0], l0[1], l1[1], j ? bl[p].z : bl[p].x, j ? bl[p].w : bl[p].y);
+					mma_16816(hi[p], h0[0], h1[0], h0[1], h1[1], j ? bh[p].z : bh[p].x, j ? bh[p].w : bh[p].y);
+				}
 			}
 		}
-		float s[4];
 #pragma unroll
-		for (int i = 0; i < 4; i++) {
-			const uint32_t h = hdr[i >> 1].x;
-			s[i] = half_bits_to_float(h & 0xffffu) * (lo[i] + hi[i]) - half_bits_to_float(h >> 16) * mm[i];
+		for (int p = 0; p < NP; p++) {
+			float s[4];
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+				const uint32_t h = hdr[i >> 1].x;
+				s[i] = half_bits_to_float(h & 0xffffu) * (lo[p][i] + hi[p][i]) - half_bits_to_float(h >> 16) * mm[p][i];
+			}
+			r[p] = quad_rows(s);
 		}
-		return quad_rows(s);
 	}
 };
 
@@ -277,13 +293,17 @@ struct MmaRows<W_Q6K_R8> {
 		load_t<true, true>(tile, nb, blk, lane, chunk);
 	}
 	__device__ __forceinline__ float2 scale(float inv) const { return make_float2(d[0] * inv, d[1] * inv); }
-	template <bool ALL>
-	__device__ __forceinline__ float2 dot(const MmaCol<ALL> &col, int lane) const
+	template <int NP, bool ALL>
+	__device__ __forceinline__ void dot(const MmaCol<ALL> (&col)[NP], int lane, float2 (&r)[NP]) const
 	{
 		const int t = lane & 3;
-		const uint8_t *xp = col.x + 8 * t;
 		const __half2 k96 = __float2half2_rn(96.0f);
-		float s[4] = {0.f, 0.f, 0.f, 0.f};
+		float s[NP][4];
+#pragma unroll
+		for (int n = 0; n < NP; n++)
+#pragma unroll
+			for (int i = 0; i < 4; i++)
+				s[n][i] = 0.f;
 #pragma unroll
 		for (int pp = 0; pp < 4; pp++) {
 			const uint32_t sx[2] = {sc[0][pp] ^ 0x80808080u, sc[1][pp] ^ 0x80808080u};
@@ -298,22 +318,36 @@ struct MmaRows<W_Q6K_R8> {
 					w[i][0] = h2_bits(__hsub2(bits_h2(and_or(v << 4, 0x03F003F0u, 0x54005400u)), k96));
 					w[i][1] = h2_bits(__hsub2(bits_h2(and_or(v >> 4, 0x03F003F0u, 0x54005400u)), k96));
 				}
-				uint2 x = make_uint2(0, 0);
-				if (col.reads())
-					x = *reinterpret_cast<const uint2 *>(xp + 2 * (128 * (pp >> 1) + 16 * (pp & 1) + 32 * q));
-				float p[4] = {0.f, 0.f, 0.f, 0.f};
-				mma_16816(p, w[0][0], w[1][0], w[0][1], w[1][1], x.x, x.y);
 				// int8 scale -> float: 2^23 + (s + 128), less 2^23 + 128
 				const float s0 = __uint_as_float(__byte_perm(sx[0], 0x4B000000u, 0x7650u | q)) - 8388736.0f;
 				const float s1 = __uint_as_float(__byte_perm(sx[1], 0x4B000000u, 0x7650u | q)) - 8388736.0f;
-				s[0] = __fmaf_rn(s0, p[0], s[0]);
-				s[1] = __fmaf_rn(s0, p[1], s[1]);
-				s[2] = __fmaf_rn(s1, p[2], s[2]);
-				s[3] = __fmaf_rn(s1, p[3], s[3]);
+#pragma unroll
+				for (int n = 0; n < NP; n++) {
+					uint2 x = make_uint2(0, 0);
+					if (col[n].reads())
+						x = *reinterpret_cast<const uint2 *>(col[n].x + 8 * t + 2 * (128 * (pp >> 1) + 16 * (pp & 1) + 32 * q));
+					float p[4] = {0.f, 0.f, 0.f, 0.f};
+					mma_16816(p, w[0][0], w[1][0], w[0][1], w[1][1], x.x, x.y);
+					s[n][0] = __fmaf_rn(s0, p[0], s[n][0]);
+					s[n][1] = __fmaf_rn(s0, p[1], s[n][1]);
+					s[n][2] = __fmaf_rn(s1, p[2], s[n][2]);
+					s[n][3] = __fmaf_rn(s1, p[3], s[n][3]);
+				}
 			}
 		}
-		return quad_rows(s);
+#pragma unroll
+		for (int n = 0; n < NP; n++)
+			r[n] = quad_rows(s[n]);
 	}
 };
+
+template <WKind KIND, bool ALL>
+__device__ __forceinline__ float2 dot_one(const MmaRows<KIND> &w, const MmaCol<ALL> &col, int lane)
+{
+	const MmaCol<ALL> c[1] = {col};
+	float2 r[1];
+	w.dot(c, lane, r);
+	return r[0];
+}
 
 }  // namespace tie
