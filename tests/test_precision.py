@@ -83,3 +83,26 @@ def test_small_batches_are_as_exact_as_fp32(block, n_tokens, layer, bound):
     b, x, want = block
     n = min(n_tokens, N_EXACT)
     assert error(b.moe_ffn(layer, x[:n_tokens])[:n], want[layer, :n]) < bound
+
+
+# fp16 hi + lo halves (22 bits), with accumulators of their own for the two: 1.09e-6 and 1.37e-6 at the most; with their
+# products in turn in one accumulator 1.5e-6 and 1.9e-6.
+@pytest.mark.gpu
+@pytest.mark.parametrize("layer,bound", [(0, 1.1e-6), (1, 1.38e-6)], ids=["q6k_down", "q4k_down"])
+@pytest.mark.parametrize("n_tokens", [32, 512])
+def test_prompt_batches(block, n_tokens, layer, bound):
+    b, x, want = block
+    assert error(b.moe_ffn(layer, x[:n_tokens])[:N_EXACT], want[layer]) < bound
+
+
+# The same for one product: 2.9e-7 and 6.0e-7.
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [37, 256])
+@pytest.mark.parametrize("ggml_type,in_dim,out_dim", [(synth.GGML_Q4_K, 4096, 2048), (synth.GGML_Q6_K, 2048, 512)])
+def test_dense_products(block, ggml_type, in_dim, out_dim, batch):
+    b = block[0]
+    w = np.ascontiguousarray((synth.q4k_blocks if ggml_type == synth.GGML_Q4_K else synth.q6k_blocks)(5, 9, in_dim // 256 * out_dim))
+    b.register_tensor(w, ggml_type, in_dim)
+    x = synth.make_x(4, batch, in_dim)
+    got = b.mat_mat(w, x, np.empty((batch, out_dim), dtype=np.float32), batch, in_dim, out_dim)
+    assert error(got, x.astype(np.float64) @ dequant(w, ggml_type, in_dim).T) < 4e-7
