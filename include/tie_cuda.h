@@ -48,10 +48,10 @@ extern "C" {
 #define TIE_CUDA_GRAPH 4u
 /* expert-kernel selection (default: chosen from n_tokens) */
 #define TIE_CUDA_PATH_AUTO 0u
-#define TIE_CUDA_PATH_STREAM (1u << 8) /* CUDA-core streaming kernels (decode / small batches) */
+#define TIE_CUDA_PATH_STREAM (1u << 8) /* the decode kernels up to 8 tokens or so, else the CUDA-core streaming kernels */
 #define TIE_CUDA_PATH_TENSOR (2u << 8) /* tcgen05 grouped GEMM (prefill) */
 #define TIE_CUDA_PATH_MASK (3u << 8)
-#define TIE_CUDA_PATH_LEGACY_STREAM (1u << 10) /* with PATH_STREAM: use the general streaming kernels even for 1-4 tokens */
+#define TIE_CUDA_PATH_LEGACY_STREAM (1u << 10) /* with PATH_STREAM: use the general streaming kernels even where the decode kernels take the batch */
 #define TIE_CUDA_PATH_DECODE_CHAIN (1u << 11) /* one token: the chain of three decode kernels instead of the single cooperative one */
 #define TIE_CUDA_PATH_NO_PAIR (1u << 14) /* tensor path: one CTA per 128-row tile instead of CTA pairs sharing one MMA issue (M = 256) */
 /* Routing of the LFM2-MoE branch (model_lfm2.c:438-473) instead of the Qwen3-MoE one
