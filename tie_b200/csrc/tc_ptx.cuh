@@ -50,6 +50,25 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
 		: "memory");
 	return ok != 0;
 }
+// Three at once: the tests are in flight together (one after the other each costs its latency, also when all are complete).
+__device__ __forceinline__ bool mbar_try_wait3(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1, uint32_t bar2, uint32_t parity2)
+{
+	uint32_t ok;
+	asm volatile(
+		"{\n\t"
+		".reg .pred p, q, r;\n\t"
+		"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+		"mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+		"mbarrier.try_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+		"and.pred p, p, q;\n\t"
+		"and.pred p, p, r;\n\t"
+		"selp.u32 %0, 1, 0, p;\n\t"
+		"}"
+		: "=r"(ok)
+		: "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1), "r"(bar2), "r"(parity2)
+		: "memory");
+	return ok != 0;
+}
 // As try_wait, allowing the hardware to suspend the thread for up to `ns` nanoseconds while the
 // phase is incomplete (a suspended thread issues nothing; it resumes when the phase completes).
 __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t parity, uint32_t ns)

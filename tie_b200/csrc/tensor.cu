@@ -67,6 +67,9 @@ constexpr int TC_THREADS = (TC_PWARPS + TC_DWARPS + 3) * 32;  // + MMA issuer + 
 constexpr int TC_LREGS = 72, TC_PREGS = 64, TC_DREGS = 88;
 static_assert(32 * (TC_PWARPS * TC_PREGS + TC_DWARPS * TC_DREGS) + 3 * 32 * TC_LREGS <= TC_THREADS * TC_LREGS, "register split");
 constexpr int TC_UNITS = 4;  // slots of the weight ring in tensor memory, one per producer group: half a super-block each
+// Super-blocks whose MMAs are in flight or waited for, at most: who waits for one has seen those TC_DONE and more before
+// it retire, and none TC_DONE after it can before the wait is over (a phase parity tells neighbouring phases apart, no more).
+constexpr int TC_DONE = 8;
 constexpr int TC_NDS = 8;    // block-factor hand-off buffers (producers -> drain warps)
 constexpr long long TC_WAIT_CYCLES = 1ll << 30;	 // about half a second of SM clocks
 constexpr float TC_H_SCALE = 1.0f / 256.0f;	 // keeps SwiGLU outputs inside fp16 range; exact (power of two)
@@ -96,7 +99,7 @@ struct TcRing {
 	static constexpr int ROWS = PAIR ? NT / 2 : NT;			// token rows a CTA holds, at most
 	static constexpr int GROUP = TC_SPB * 2 * ROWS * TC_BK * 2;	// 16 .. 64 KB
 	static constexpr int GROUPS = TC_B_BYTES / GROUP;
-	static_assert(GROUPS <= TC_BG_MAX && (GROUPS & (GROUPS - 1)) == 0, "token ring");
+	static_assert(GROUPS <= TC_BG_MAX && GROUPS <= TC_DONE && (GROUPS & (GROUPS - 1)) == 0, "token ring");
 };
 // packed super-block of 128 rows: the 144-byte Q4_K blocks resp. the 208-byte Q6_K records
 // (192 bytes of quants + 16 bytes of scales) of the rows back to back, one TMA box.  Row strides
@@ -122,16 +125,13 @@ struct TcSmem {
 };
 
 struct TcShared {
-	uint64_t full[TC_UNITS];	// unit written by its producer group(s)
-	uint64_t empty[TC_UNITS];	// ... and consumed by the MMAs
-	uint64_t bfull[TC_BG_MAX];	// token tiles of a super-block landed (TMA transaction bytes)
-	uint64_t bempty[TC_BG_MAX];	// ... and consumed
+	uint64_t full[2];		// both units of a super-block written by their producer groups
+	uint64_t bfull[TC_BG_MAX];	// token tiles of a super-block (and a segment of sums) landed (TMA transaction bytes)
+	uint64_t done[TC_DONE];		// MMAs of a super-block retired: weight units, token tiles and sums are free, its accumulator is complete
 	uint64_t wfull[TC_NWF_MAX];	// packed super-block landed
 	uint64_t wempty[TC_NWB_MAX];	// ... and expanded
-	uint64_t pfull[2][TC_NBUF_MAX];	// accumulator complete (one super-block), per set of drain warps
+	uint64_t pfull[2][TC_NBUF_MAX];	// accumulator complete, per set of drain warps (where there are two)
 	uint64_t pempty[TC_NBUF_MAX];	// accumulator read out by the drain warps
-	uint64_t xfull[2];		// sub-block sums of a work item landed
-	uint64_t xempty[2];		// ... and consumed
 	uint64_t mempty[2];		// min sums of a work item read out by the drain warps
 	uint64_t fin;			// every commit has landed
 	uint32_t tmem_base;
@@ -382,14 +382,12 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	auto w_buf = [&](int wb) -> uint32_t { return tiles + Sm::OFF_W + wb * Sm::WBUF; };
 
 	if (threadIdx.x == 0) {
-		for (int s = 0; s < TC_UNITS; s++) {
-			ptx::mbar_init(ptx::smem_u32(&sh->full[s]), (PAIR ? 2 : 1) * 4);
-			ptx::mbar_init(ptx::smem_u32(&sh->empty[s]), 1);
-		}
-		for (int s = 0; s < TC_BG_MAX; s++) {
+		for (int s = 0; s < 2; s++)
+			ptx::mbar_init(ptx::smem_u32(&sh->full[s]), (PAIR ? 2 : 1) * 8);
+		for (int s = 0; s < TC_BG_MAX; s++)
 			ptx::mbar_init(ptx::smem_u32(&sh->bfull[s]), 1);
-			ptx::mbar_init(ptx::smem_u32(&sh->bempty[s]), 1);
-		}
+		for (int s = 0; s < TC_DONE; s++)
+			ptx::mbar_init(ptx::smem_u32(&sh->done[s]), 1);
 		for (int s = 0; s < Sm::NWF; s++)
 			ptx::mbar_init(ptx::smem_u32(&sh->wfull[s]), 1);
 		for (int s = 0; s < Sm::NWB; s++)
@@ -399,11 +397,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			ptx::mbar_init(ptx::smem_u32(&sh->pfull[1][s]), 1);
 			ptx::mbar_init(ptx::smem_u32(&sh->pempty[s]), (PAIR ? 2 : 1) * FOLDERS);
 		}
-		for (int s = 0; s < 2; s++) {
-			ptx::mbar_init(ptx::smem_u32(&sh->xfull[s]), 1);
-			ptx::mbar_init(ptx::smem_u32(&sh->xempty[s]), 1);
+		for (int s = 0; s < 2; s++)
 			ptx::mbar_init(ptx::smem_u32(&sh->mempty[s]), (PAIR ? 2 : 1) * FOLDERS);
-		}
 		ptx::mbar_init(ptx::smem_u32(&sh->fin), 1);
 		sh->abort = 0;
 		ptx::fence_barrier_init();
@@ -468,7 +463,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		ptx::setmaxnreg_dec<TC_PREGS>();
 		const int row = threadIdx.x & 127, grp = threadIdx.x >> 7, half = grp & 1;
 		const uint32_t slot = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cols::A + UNIT * grp;
-		const uint32_t full = ptx::smem_u32(&sh->full[grp]), empty = ptx::smem_u32(&sh->empty[grp]);
+		const uint32_t full = ptx::smem_u32(&sh->full[grp >> 1]);
 		const uint32_t n_sb = walker < total ? (uint32_t)((total - 1 - walker) / stride_t + 1) * (uint32_t)nb : 0u;
 		bool alive = true;
 		for (uint32_t n = grp >> 1; n < n_sb; n += 2) {
@@ -486,7 +481,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				uint32_t va[8], vb[8];
 				ex.piece(i, va, vb);
 				if (i == 0) {
-					if (n >= 2 && !tc_wait_warp(empty, ((n >> 1) & 1u) ^ 1u, abort_flag, status, lane)) {
+					const uint32_t m = n - 2u;  // the slot's last user
+					if (n >= 2 && !tc_wait_warp(ptx::smem_u32(&sh->done[m % TC_DONE]), (m / TC_DONE) & 1u, abort_flag, status, lane)) {
 						alive = false;
 						break;
 					}
@@ -604,7 +600,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					dnext = half_bits_to_float(
 						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
 				const uint32_t buf = n % NBUF;
-				if (!tc_wait_warp(ptx::smem_u32(&sh->pfull[set][buf]), SETS ? (pph >> buf) & 1u : (n / NBUF) & 1u, abort_flag, status, lane)) {
+				if (!tc_wait_warp(ptx::smem_u32(SETS ? &sh->pfull[set][buf] : &sh->done[n % TC_DONE]),
+						  SETS ? (pph >> buf) & 1u : (n / TC_DONE) & 1u, abort_flag, status, lane)) {
 					alive = false;
 					break;
 				}
@@ -652,6 +649,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		// One thread, one super-block at a time: the barriers it needs are tested together and branched on once
 		// — a wait in front of every stage cost this thread more than the stage's MMAs (8 MMAs of N = 16 take 93
 		// cycles to issue, 107 with the commit, 260 behind a test-and-branch; four stages behind one, 130 each).
+		// One commit tells everybody who waits for the super-block (a barrier each for the units, the token tiles and the
+		// accumulator were four, and the sums' barriers two more: prompt of 512 212.2 -> 210.5 us, 4096 -> 2048 projection of
+		// 512 tokens 24.4 -> 23.7).
 		if (rank == 0 && ptx::elect_one()) {
 			auto mma = [&](uint32_t d, uint32_t a, uint32_t b, uint32_t idesc, uint32_t acc) {
 				if (PAIR)
@@ -667,8 +667,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			};
 			uint32_t n = 0, tl = 0, xs_n = 0;  // super-blocks, work items, segments of sums so far
 			bool alive = true;
-			auto wait = [&](uint64_t *bar, uint32_t parity) {
-				alive = alive && tc_wait(ptx::smem_u32(bar), parity, abort_flag, status);
+			auto wait = [&](uint32_t bar, uint32_t parity) {
+				alive = alive && tc_wait(bar, parity, abort_flag, status);
 			};
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
 				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
@@ -679,30 +679,22 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				// hi rows and one MMA of twice the columns takes both
 				const bool stacked = 2 * item.n_mma <= NT;
 				const uint32_t dset = SETS ? tl & 1u : 0u;  // the set of drain warps that takes the item
-				for (int sbi = 0; sbi < nb && alive; sbi++, n++) {
-					const uint32_t buf = n % NBUF, j0 = 2u * (n & 1u), uph = (n >> 1) & 1u;
-					const uint32_t q = n & (Ring::GROUPS - 1), bph = (n / Ring::GROUPS) & 1u, pph = ((n / NBUF) & 1u) ^ 1u;
-					bool ready = ptx::mbar_try_wait(ptx::smem_u32(&sh->bfull[q]), bph);
-					ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->full[j0]), uph);
-					ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->full[j0 + 1]), uph);
-					if (n >= (uint32_t)NBUF)
-						ready &= ptx::mbar_try_wait(ptx::smem_u32(&sh->pempty[buf]), pph);
-					if (!ready) {
-						wait(&sh->bfull[q], bph);
-						if (n >= (uint32_t)NBUF)
-							wait(&sh->pempty[buf], pph);
-						wait(&sh->full[j0], uph);
-						wait(&sh->full[j0 + 1], uph);
+				for (int sbi = 0; sbi < nb; sbi++, n++) {
+					const uint32_t buf = n % NBUF, j0 = 2u * (n & 1u);
+					const uint32_t q = n & (Ring::GROUPS - 1);
+					const uint32_t fb = ptx::smem_u32(&sh->bfull[q]), fu = ptx::smem_u32(&sh->full[n & 1u]), pe = ptx::smem_u32(&sh->pempty[buf]);
+					// (the phase before a barrier's first counts as complete: the first uses of an accumulator do not wait)
+					const uint32_t fb_ph = (n / Ring::GROUPS) & 1u, fu_ph = (n >> 1) & 1u, pe_ph = ((n / NBUF) & 1u) ^ 1u;
+					if (!ptx::mbar_try_wait3(fb, fb_ph, fu, fu_ph, pe, pe_ph)) {
+						wait(fb, fb_ph);
+						wait(pe, pe_ph);
+						wait(fu, fu_ph);
 						if (!alive)
 							break;
 					}
 					ptx::tc_fence_after();
 					const uint32_t dP = tmem + NT * buf, bt = b_group(q);
 					const uint32_t xs = ptx::umma_desc_lo(xq_buf(xs_n & 1u) + (uint32_t)((sbi >> 2) & 1) * lo_off) + 2u * (sbi & 3);
-					// (dmin m)_hi (half 0), (dmin m)_lo (half 1) times the block's sums, hi and lo side by side in k
-					auto min_mma = [&](int h, uint32_t acc) {
-						mma(tmem + Cols::M + NT * dset, tmem + Cols::A + UNIT * (j0 + h) + 64u, xs, idesc, acc);
-					};
 					auto stages = [&](auto both) {
 						auto a_of = [&](int q4) { return tmem + Cols::A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1); };
 						auto b_of = [&](int q4) { return ptx::umma_desc_lo(bt + q4 * 2u * lo_off); };
@@ -717,42 +709,34 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 									mma(dP, a_of(q4) + 8 * kk, b_of(q4) + (lo_off >> 4) + 2 * kk, idesc, (q4 > 0 || kk > 0) ? 1u : 0u);
 						}
 #pragma unroll
-						for (int q4 = 0; q4 < TC_SPB; q4++) {
+						for (int q4 = 0; q4 < TC_SPB; q4++)
 #pragma unroll
 							for (int kk = 0; kk < TC_BK / 16; kk++)
 								mma(dP, a_of(q4) + 8 * kk, b_of(q4) + 2 * kk, both.value ? idesc2 : idesc,
 								    (!both.value || q4 > 0 || kk > 0) ? 1u : 0u);
-							if ((q4 & 1) && (!Q4 || (sbi & 7) != 0)) {
-								if (Q4)
-									min_mma(q4 >> 1, 1u);
-								commit(&sh->empty[j0 + (q4 >> 1)]);
-							}
-						}
 					};
 					if (stacked)
 						stages(std::true_type());
 					else
 						stages(std::false_type());
-					if (Q4 && (sbi & 7) == 0) {
-						// the first min sums of a segment: behind the stages, so that neither the sums' landing nor the
-						// drain of the previous item's accumulator holds those up
-						wait(&sh->xfull[xs_n & 1u], (xs_n >> 1) & 1u);
-						if (sbi == 0 && tl >= (uint32_t)Cols::NM)
-							wait(&sh->mempty[dset], ((SETS ? tl >> 1 : tl) & 1u) ^ 1u);
-						if (!alive)
-							break;
-						ptx::tc_fence_after();
-						min_mma(0, sbi > 0 ? 1u : 0u);
-						commit(&sh->empty[j0]);
-						min_mma(1, 1u);
-						commit(&sh->empty[j0 + 1]);
+					if (Q4) {
+						// (dmin m)_hi (first unit), (dmin m)_lo (second) times the block's sums, hi and lo side by side in k; an item's
+						// first ones behind its first stages, so that the drain of its accumulator's last item holds those up no more
+						if (sbi == 0) {
+							wait(ptx::smem_u32(&sh->mempty[dset]), ((SETS ? tl >> 1 : tl) & 1u) ^ 1u);
+							if (!alive)
+								break;
+							ptx::tc_fence_after();
+						}
+						const uint32_t dM = tmem + Cols::M + NT * dset, aM = tmem + Cols::A + UNIT * j0 + 64u;
+						mma(dM, aM, xs, idesc, sbi > 0 ? 1u : 0u);
+						mma(dM, aM + UNIT, xs, idesc, 1u);
+						if ((sbi & 7) == 7 || sbi == nb - 1)
+							xs_n++;
 					}
-					commit(&sh->bempty[q]);
-					if (Q4 && ((sbi & 7) == 7 || sbi == nb - 1)) {
-						commit(&sh->xempty[xs_n & 1u]);
-						xs_n++;
-					}
-					commit(&sh->pfull[dset][buf]);
+					commit(&sh->done[n % TC_DONE]);
+					if (SETS)
+						commit(&sh->pfull[dset][buf]);
 				}
 			}
 			// the last commits have to land in both CTAs' barriers before either CTA may leave
@@ -763,7 +747,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	} else if (warp == W_TOK) {
 		// ================= token loader: token operand and sub-block sums (TMA) =================
 		if (ptx::elect_one()) {
-			uint32_t tl = 0, n = 0, xs_n = 0;
+			uint32_t tl = 0, n = 0, xs_n = 0, x_end = 0;  // x_end: where the segment of sums before the current one ended
 			bool alive = true;
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
 				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
@@ -773,32 +757,38 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				const uint32_t row_bytes = (uint32_t)(16 << item.box) * 128u;  // of one 64-wide column tile, both CTAs
 				const int row0 = item.row0 + (PAIR ? (int)rank * (item.n_mma >> 1) : 0);
 				const CUtensorMap *tmp = item.box == 0 ? &tm0 : (item.box == 1 ? &tm1 : &tm2);
+				auto wait_done = [&](uint32_t m) {
+					return tc_wait<100>(ptx::smem_u32(&sh->done[m % TC_DONE]), (m / TC_DONE) & 1u, abort_flag, status);
+				};
 				for (int sbi = 0; sbi < nb; sbi++, n++) {
-					if (Q4 && (sbi & 7) == 0) {  // a segment of the sub-block sums (two buffers)
-						const uint32_t xi = xs_n & 1u;
-						if (xs_n >= 2u && !tc_wait<100>(ptx::smem_u32(&sh->xempty[xi]), ((xs_n >> 1) & 1u) ^ 1u, abort_flag, status)) {
-							alive = false;
-							break;
-						}
-						const uint32_t xb = ptx::smem_u32(&sh->xfull[xi]);
-						const CUtensorMap *tqp = item.box == 0 ? &tq0 : (item.box == 1 ? &tq1 : &tq2);
-						if (rank == 0)
-							ptx::mbar_arrive_expect_tx(xb, (uint32_t)xq_depth * row_bytes);
-						if (PAIR)
-							ptx::tma_load_3d_pair(xq_buf(xi), tqp, xb, 0, row0, sbi >> 2);
-						else
-							ptx::tma_load_3d(xq_buf(xi), tqp, xb, 0, row0, sbi >> 2);
-						xs_n++;
-					}
 					const uint32_t q = n & (Ring::GROUPS - 1);
-					if (n >= (uint32_t)Ring::GROUPS &&
-					    !tc_wait<100>(ptx::smem_u32(&sh->bempty[q]), ((n / Ring::GROUPS) & 1u) ^ 1u, abort_flag, status)) {
+					if (n >= (uint32_t)Ring::GROUPS && !wait_done(n - Ring::GROUPS)) {
 						alive = false;
 						break;
 					}
 					const uint32_t fb = ptx::smem_u32(&sh->bfull[q]);
+					uint32_t bytes = 2u * TC_SPB * row_bytes;
+					if (Q4 && (sbi & 7) == 0) {
+						// a segment of the sub-block sums comes with its first super-block (two buffers; the segment before the
+						// last one is over with the super-block in front of x_end, of which the wait above may have told)
+						if (xs_n >= 2u && x_end + Ring::GROUPS > n + 1u && !wait_done(x_end - 1u)) {
+							alive = false;
+							break;
+						}
+						x_end = n;
+						bytes += (uint32_t)xq_depth * row_bytes;
+					}
 					if (rank == 0)
-						ptx::mbar_arrive_expect_tx(fb, 2u * TC_SPB * row_bytes);
+						ptx::mbar_arrive_expect_tx(fb, bytes);
+					if (Q4 && (sbi & 7) == 0) {
+						const uint32_t xi = xs_n & 1u;
+						const CUtensorMap *tqp = item.box == 0 ? &tq0 : (item.box == 1 ? &tq1 : &tq2);
+						if (PAIR)
+							ptx::tma_load_3d_pair(xq_buf(xi), tqp, fb, 0, row0, sbi >> 2);
+						else
+							ptx::tma_load_3d(xq_buf(xi), tqp, fb, 0, row0, sbi >> 2);
+						xs_n++;
+					}
 					if (PAIR)
 						ptx::tma_load_4d_pair(b_group(q), tmp, fb, 0, row0, 0, sbi * TC_SPB);
 					else
