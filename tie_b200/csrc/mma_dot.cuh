@@ -297,7 +297,7 @@ struct MmaRows<W_Q6K_R8> {
 	__device__ __forceinline__ void dot(const MmaCol<ALL> (&col)[NP], int lane, float2 (&r)[NP]) const
 	{
 		const int t = lane & 3;
-		const __half2 k96 = __float2half2_rn(96.0f);
+		const __half2 k1056 = __float2half2_rn(1056.0f), k16th = __float2half2_rn(0.0625f), km96 = __float2half2_rn(-96.0f);
 		float s[NP][4];
 #pragma unroll
 		for (int n = 0; n < NP; n++)
@@ -307,17 +307,21 @@ struct MmaRows<W_Q6K_R8> {
 #pragma unroll
 		for (int pp = 0; pp < 4; pp++) {
 			const uint32_t sx[2] = {sc[0][pp] ^ 0x80808080u, sc[1][pp] ^ 0x80808080u};
+			uint32_t w[4][2][2];  // [q][row]
+#pragma unroll
+			for (int i = 0; i < 2; i++) {
+				q6k_word<4>(a[i][pp], h[i][pp], w[0][i], w[2][i]);
+				q6k_word<2>(b[i][pp], h[i][pp], w[1][i], w[3][i]);
+#pragma unroll
+				for (int e = 0; e < 2; e++) {
+					w[0][i][e] = h2_bits(__hsub2(bits_h2(w[0][i][e]), k1056));
+					w[1][i][e] = h2_bits(__hsub2(bits_h2(w[1][i][e]), k1056));
+					w[2][i][e] = h2_bits(__hfma2(bits_h2(w[2][i][e]), k16th, km96));
+					w[3][i][e] = h2_bits(__hfma2(bits_h2(w[3][i][e]), k16th, km96));
+				}
+			}
 #pragma unroll
 			for (int q = 0; q < 4; q++) {  // 16 weights: l + 32 q of the half, one scale
-				uint32_t w[2][2];
-#pragma unroll
-				for (int i = 0; i < 2; i++) {
-					const uint32_t lo4 = (q & 1 ? b[i][pp] : a[i][pp]) >> (q & 2 ? 4 : 0);
-					const uint32_t hh = q == 0 ? h[i][pp] << 4 : (q == 1 ? h[i][pp] << 2 : (q == 2 ? h[i][pp] : h[i][pp] >> 2));
-					const uint32_t v = and_or(hh, 0x30303030u, lo4 & 0x0F0F0F0Fu);
-					w[i][0] = h2_bits(__hsub2(bits_h2(and_or(v << 4, 0x03F003F0u, 0x54005400u)), k96));
-					w[i][1] = h2_bits(__hsub2(bits_h2(and_or(v >> 4, 0x03F003F0u, 0x54005400u)), k96));
-				}
 				// int8 scale -> float: 2^23 + (s + 128), less 2^23 + 128
 				const float s0 = __uint_as_float(__byte_perm(sx[0], 0x4B000000u, 0x7650u | q)) - 8388736.0f;
 				const float s1 = __uint_as_float(__byte_perm(sx[1], 0x4B000000u, 0x7650u | q)) - 8388736.0f;
@@ -327,7 +331,7 @@ struct MmaRows<W_Q6K_R8> {
 					if (col[n].reads())
 						x = *reinterpret_cast<const uint2 *>(col[n].x + 8 * t + 2 * (128 * (pp >> 1) + 16 * (pp & 1) + 32 * q));
 					float p[4] = {0.f, 0.f, 0.f, 0.f};
-					mma_16816(p, w[0][0], w[1][0], w[0][1], w[1][1], x.x, x.y);
+					mma_16816(p, w[q][0][0], w[q][1][0], w[q][0][1], w[q][1][1], x.x, x.y);
 					s[n][0] = __fmaf_rn(s0, p[0], s[n][0]);
 					s[n][1] = __fmaf_rn(s0, p[1], s[n][1]);
 					s[n][2] = __fmaf_rn(s1, p[2], s[n][2]);

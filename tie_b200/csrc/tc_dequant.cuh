@@ -10,7 +10,7 @@
 // taken out of tensor memory, so no low-order operand is needed for the weights.
 //
 // Quants become halves without conversion instructions: a 16-bit field 0x6400 | q is the half
-// 1024 + q, 0x6400 | (q << 4) is 1024 + 16 q, 0x5400 | (q << 4) is 64 + q (q < 64); one HFMA2 with
+// 1024 + q, 0x6400 | (q << 4) is 1024 + 16 q (q < 64); one HFMA2 with
 // a per-sub-block scale and offset then yields sc*q resp. sc*(q-32) for two weights (the product
 // inside the fused multiply-add is exact, so the result is the exact integer).  The two halves of
 // such a pair come from bytes 0 and 2 (or 1 and 3) of a 32-bit word, so within every group of 4
@@ -68,12 +68,18 @@ __device__ __forceinline__ void q4k_int_word(uint32_t w, const Q4kConsts &c, uin
 	hi[1] = h2_bits(__hfma2(bits_h2(and_or(w8, 0x00F000F0u, 0x64006400u)), c.sh, c.ch));
 }
 
-// Four 6-bit quants held as the bytes of q (0..63 each) -> sc*(q-32) pairs: out[0] = bytes (0, 2),
-// out[1] = bytes (1, 3).  s = half2(sc), c = half2(-96 sc).
-__device__ __forceinline__ void q6k_int_word(uint32_t q, __half2 s, __half2 c, uint32_t out[2])
+// Eight 6-bit quants: their low four bits are the bytes' low (first four) and high nibbles of a, their high two bits lie
+// in the bytes of h, SHIFT bits below bit 4 and below bit 8.  Both are ORed into mantissas where they stand, with
+// one shift of a and two of h for all eight (joined into bytes first, 18 instructions of the logic pipe instead of 11):
+// lo[0] = 1024 + q of bytes (0, 2), lo[1] of bytes (1, 3), hi[] = 1024 + 16 q.
+template <int SHIFT>
+__device__ __forceinline__ void q6k_word(uint32_t a, uint32_t h, uint32_t lo[2], uint32_t hi[2])
 {
-	out[0] = h2_bits(__hfma2(bits_h2(and_or(q << 4, 0x03F003F0u, 0x54005400u)), s, c));
-	out[1] = h2_bits(__hfma2(bits_h2(and_or(q >> 4, 0x03F003F0u, 0x54005400u)), s, c));
+	const uint32_t a8 = a >> 8, hl = h << SHIFT, hr = h >> (8 - SHIFT);
+	lo[0] = and_or(hl, 0x00300030u, and_or(a, 0x000F000Fu, 0x64006400u));
+	lo[1] = and_or(hr, 0x00300030u, and_or(a8, 0x000F000Fu, 0x64006400u));
+	hi[0] = and_or(hl, 0x03000300u, and_or(a, 0x00F000F0u, 0x64006400u));
+	hi[1] = and_or(hr, 0x03000300u, and_or(a8, 0x00F000F0u, 0x64006400u));
 }
 
 }  // namespace tie

@@ -218,6 +218,12 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr)
 	asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
 	return v;
 }
+__device__ __forceinline__ uint2 lds64(uint32_t addr)
+{
+	uint2 v;
+	asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
+	return v;
+}
 __device__ __forceinline__ uint32_t lds32(uint32_t addr)
 {
 	uint32_t v;
@@ -233,9 +239,8 @@ __device__ __forceinline__ __half2 byte_pair_1024(uint32_t w, uint32_t selector)
 }
 
 // Expansion of half a packed super-block (already in shared memory) by the producer thread of a row:
-// prepare() once, then piece(2q + i) makes 32 of the row's 64 weights of the half's stage q: columns
-// 8i .. 8i+7 and 16 + 8i .. of that stage.  (Pieces of 16 registers: a whole stage at a time spills at
-// the 72 registers 27 warps leave each thread.)
+// prepare() once, then four pieces of 32 weights.  Q4_K: piece(2q + i) makes columns 8i .. 8i+7 and 16 + 8i .. of the
+// half's stage q.  (Pieces of 16 registers: a whole stage at a time spills at the 72 registers 27 warps leave each thread.)
 template <WKind KIND>
 struct Expander;
 
@@ -294,30 +299,34 @@ struct Expander<W_Q6K_R8> {
 		qaddr = rec + 96u * half;
 		saddr = rec + 192u + 8u * half;
 	}
-	__device__ __forceinline__ void piece(int i, uint32_t va[8], uint32_t vb[8]) const
+	// sixteen weights of each stage: v[stage][0 .. 3] columns 8 hs + 4 k .. (k = i & 1), v[stage][4 .. 7] the same + 16.
+	// The operand is sc * (q - 32) / 16 (the drain multiplies d by 16): sc * (1024 + q) less sc * 1056 would leave fp16.
+	__device__ __forceinline__ void piece(int i, uint32_t v[2][8]) const
 	{
-		const int st = i >> 1, hs = i & 1;
-		const __half2 k1152 = __float2half2_rn(1152.0f), km96 = __float2half2_rn(-96.0f);
-		const uint32_t chunk = qaddr + 48u * hs;
-		const uint4 a = lds128(chunk), b = lds128(chunk + 16u), h = lds128(chunk + 32u);
-		// scales of the part: bytes {0,1} for st = 0, {2,3} for st = 1; int8 -> half as 1024 + (s ^ 0x80) - 1152
-		const uint32_t scx = lds32(saddr + 4u * hs) ^ 0x80808080u;
-		const __half2 sA = __hsub2(byte_pair_1024(scx, st ? 0x7252u : 0x7050u), k1152);
-		const __half2 sB = __hsub2(byte_pair_1024(scx, st ? 0x7353u : 0x7151u), k1152);
-		const __half2 cA = __hmul2(sA, km96), cB = __hmul2(sB, km96);
-		const uint32_t A[4] = {a.x, a.y, a.z, a.w}, B[4] = {b.x, b.y, b.z, b.w}, Hh[4] = {h.x, h.y, h.z, h.w};
+		const int hs = i >> 1, k = i & 1;
+		const __half2 k1152 = __float2half2_rn(1152.0f);
+		const uint32_t chunk = qaddr + 48u * hs + 8u * k;
+		const uint2 w[2] = {lds64(chunk), lds64(chunk + 16u)}, h = lds64(chunk + 32u);
+		const uint32_t scx = lds32(saddr + 4u * hs) ^ 0x80808080u;  // int8 -> half as 1024 + (s ^ 0x80) - 1152
 #pragma unroll
-		for (int k = 0; k < 4; k++) {
-			uint32_t qa, qb;
-			if (st == 0) {
-				qa = and_or(Hh[k] << 4, 0x30303030u, A[k] & 0x0F0F0F0Fu);
-				qb = and_or(Hh[k] << 2, 0x30303030u, B[k] & 0x0F0F0F0Fu);
-			} else {
-				qa = and_or(Hh[k], 0x30303030u, (A[k] >> 4) & 0x0F0F0F0Fu);
-				qb = and_or(Hh[k] >> 2, 0x30303030u, (B[k] >> 4) & 0x0F0F0F0Fu);
+		for (int ab = 0; ab < 2; ab++) {
+			const __half2 s0 = __hsub2(byte_pair_1024(scx, ab ? 0x7151u : 0x7050u), k1152), s1 = __hsub2(byte_pair_1024(scx, ab ? 0x7353u : 0x7252u), k1152);
+			const __half2 f0 = __hmul2(s0, __float2half2_rn(0.0625f)), c0 = __hmul2(s0, __float2half2_rn(-66.0f));
+			const __half2 f1 = __hmul2(s1, __float2half2_rn(1.0f / 256)), c1 = __hmul2(s1, __float2half2_rn(-6.0f));
+			const uint32_t a2[2] = {w[ab].x, w[ab].y}, h2[2] = {h.x, h.y};
+#pragma unroll
+			for (int j = 0; j < 2; j++) {
+				uint32_t lo[2], hi[2];
+				if (ab)
+					q6k_word<2>(a2[j], h2[j], lo, hi);
+				else
+					q6k_word<4>(a2[j], h2[j], lo, hi);
+#pragma unroll
+				for (int e = 0; e < 2; e++) {
+					v[0][4 * ab + 2 * j + e] = h2_bits(__hfma2(bits_h2(lo[e]), f0, c0));
+					v[1][4 * ab + 2 * j + e] = h2_bits(__hfma2(bits_h2(hi[e]), f1, c1));
+				}
 			}
-			q6k_int_word(qa, sA, cA, va + 2 * k);  // k = 16 hs + 4k .. of the stage
-			q6k_int_word(qb, sB, cB, vb + 2 * k);  // k = 32 + 16 hs + 4k ..
 		}
 	}
 };
@@ -478,8 +487,11 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			}
 #pragma unroll
 			for (int i = 0; i < 4; i++) {
-				uint32_t va[8], vb[8];
-				ex.piece(i, va, vb);
+				uint32_t v[2][8];
+				if constexpr (Q4)
+					ex.piece(i, v[0], v[1]);
+				else
+					ex.piece(i, v);
 				if (i == 0) {
 					const uint32_t m = n - 2u;  // the slot's last user
 					if (n >= 2 && !tc_wait_warp(ptx::smem_u32(&sh->done[m % TC_DONE]), (m / TC_DONE) & 1u, abort_flag, status, lane)) {
@@ -488,8 +500,14 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					}
 					ptx::tc_fence_after();
 				}
-				ptx::tmem_st8(slot + 32u * (i >> 1) + 8u * (i & 1), va);
-				ptx::tmem_st8(slot + 32u * (i >> 1) + 8u * (i & 1) + 16u, vb);
+				if constexpr (Q4) {
+					ptx::tmem_st8(slot + 32u * (i >> 1) + 8u * (i & 1), v[0]);
+					ptx::tmem_st8(slot + 32u * (i >> 1) + 8u * (i & 1) + 16u, v[1]);
+				} else {
+#pragma unroll
+					for (int c = 0; c < 4; c++)
+						ptx::tmem_st4(slot + 32u * (c >> 1) + 8u * (i >> 1) + 4u * (i & 1) + 16u * (c & 1), v[c >> 1] + 4 * (c & 1));
+				}
 			}
 			if (!alive)
 				break;
@@ -587,7 +605,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
 				}
 			};
-			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead
+			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead; times 16, which the operand lacks
 			const uint8_t *grp = nullptr;
 			float dnext = 0.0f;
 			if (!Q4) {
@@ -595,7 +613,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, 0))));
 			}
 			for (int sbi = 0; sbi < nb; sbi++, n++) {
-				float scale = dnext;
+				float scale = 16.0f * dnext;
 				if (!Q4 && sbi + 1 < nb)
 					dnext = half_bits_to_float(
 						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
