@@ -259,9 +259,9 @@ void prof_mark(tie_cuda_ctx *c, int id)
 
 // The expert part on device rows.  x_src: fp32 rows; row r reads x_src[r / src_div].
 // row_expert [n_rows] (device) gives the global expert of every row; y [n_rows][H] receives
-// the unweighted expert outputs in row order.
+// the unweighted expert outputs in row order, or where *pos is set to an array, row r at pos[r] (pos null: in row order).
 int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div, const int *row_expert, int n_rows, float *y,
-		unsigned flags)
+		unsigned flags, const int **pos = nullptr)
 {
 	const unsigned path = flags & TIE_CUDA_PATH_MASK;
 	bool use_tc;
@@ -296,7 +296,10 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 		prof_mark(c, 4);
 		TRY(launch_tc_swiglu(c, L, n_rows));
 		prof_mark(c, 5);
-		TRY(launch_tc_down(c, L, n_tile, y));
+		// A combine finds the rows where the sort put them: each tile's stores then go to neighbouring rows.
+		TRY(launch_tc_down(c, L, n_tile, y, pos != nullptr));
+		if (pos)
+			*pos = c->s.inv;
 		prof_mark(c, 6);
 	} else {
 		prof_mark(c, 3);
@@ -376,8 +379,9 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 	}
 	TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
 	prof_mark(c, 1);
-	TRY(run_experts(c, L, x, c->cfg.top_k, s.topk_idx, n_tokens * c->cfg.top_k, s.y, flags));
-	TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out));
+	const int *pos = nullptr;
+	TRY(run_experts(c, L, x, c->cfg.top_k, s.topk_idx, n_tokens * c->cfg.top_k, s.y, flags, &pos));
+	TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out, pos));
 	prof_mark(c, 7);
 	return TIE_CUDA_OK;
 }

@@ -68,7 +68,7 @@ bool tc_supported(const tie_cuda_ctx *c, const Layer &L);
 // n_tile: the token tiles of the sort, 32 or 64 rows
 int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile);
 int launch_tc_swiglu(tie_cuda_ctx *c, const Layer &L, int n_rows, const int *n_rows_dev = nullptr);
-int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_tile, float *y);
+int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_tile, float *y, bool sorted);
 int launch_tc_down_peer(tie_cuda_ctx *c, const Layer &L, const EpDst &dst);
 // ep.cu
 int launch_ep_signal(tie_cuda_ctx *c, int which);

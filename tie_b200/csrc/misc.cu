@@ -69,7 +69,8 @@ __global__ void __launch_bounds__(NORM_THREADS) rms_norm_rows(const float *__res
 
 // model_qwen3.c:458-467: acc = 0; acc += w_j * y_j, j ascending (fused multiply-add, as the
 // reference compiles it).  residual != null: out = residual + acc (math_avx2.c:731-751).
-// pos != null: the row of (t, j) is y[pos[t*top_k + j]] instead of y[t*top_k + j].
+// pos != null: the row of (t, j) is y[pos[t*top_k + j]] instead of y[t*top_k + j] (< 0, after a call that reports an
+// expert out of range: any row).
 __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y, const float *__restrict__ topk_w, int top_k,
 						    int hidden, const float *__restrict__ residual, float *__restrict__ out,
 						    const int *__restrict__ pos)
@@ -80,7 +81,7 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 #pragma unroll
 	for (int j = 0; j < MAX_TOP_K; j++) {
 		wj[j] = (j < top_k) ? topk_w[(size_t)t * top_k + j] : 0.f;
-		yrow[j] = (j < top_k) ? (size_t)(pos ? pos[(size_t)t * top_k + j] : t * top_k + j) * hidden : 0;
+		yrow[j] = (j < top_k) ? (size_t)(pos ? max(pos[(size_t)t * top_k + j], 0) : t * top_k + j) * hidden : 0;
 	}
 	for (int k = threadIdx.x * 4; k < hidden; k += blockDim.x * 4) {
 		float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
