@@ -71,7 +71,7 @@ int alloc_scratch(tie_cuda_ctx *c)
 	s.sort_hist_cap = ((R + SORT_SLICE - 1) / SORT_SLICE + 1) * E;
 	TRY(dev_alloc(c, &s.sort_hist, s.sort_hist_cap));
 	TRY(dev_alloc(c, &s.h, R * F));
-	TRY(dev_alloc(c, &s.y, R * (H > 2 * F ? H : 2 * F)));  // also holds the raw gate|up products of the tensor path
+	TRY(dev_alloc(c, &s.y, R * H));
 	// hi and lo halves of each split array share one allocation (lo right behind hi): one 3-D TMA box fetches both
 	TRY(dev_alloc(c, &s.xs_hi, 2 * s.rows_pad * H));
 	s.xs_lo = s.xs_hi + s.rows_pad * H;
@@ -120,8 +120,8 @@ void free_tensor(DevTensor &t)
 	t = DevTensor();
 }
 
-// Copy one stacked expert tensor to the device (re-ordering Q6_K into R8).
-int upload_tensor(tie_cuda_ctx *c, DevTensor &t, const void *host, int type, int rows, int k)
+// Copy one stacked expert tensor to the device (re-ordering Q6_K into R8).  half_tiles: gate or up (tc_make_weight_map).
+int upload_tensor(tie_cuda_ctx *c, DevTensor &t, const void *host, int type, int rows, int k, bool half_tiles)
 {
 	const size_t bb = block_bytes(type);
 	if (!bb)
@@ -158,7 +158,7 @@ int upload_tensor(tie_cuda_ctx *c, DevTensor &t, const void *host, int type, int
 	}
 	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
 	c->weight_bytes += t.bytes;
-	return tc_make_weight_map(c, t);
+	return tc_make_weight_map(c, t, half_tiles);
 }
 
 int add_reg(tie_cuda_ctx *c, const void *host, size_t bytes, const uint8_t *dev, int type, WKind kind, int rows, int k,
@@ -245,7 +245,7 @@ int report_status(tie_cuda_ctx *c, unsigned st)
 }
 
 // Phase marks: 0 start, 1 router done, 2 dispatch sort done, 3 input split done, 4 gate/up done,
-// 5 SwiGLU pass done (only where it is a pass of its own), 6 down done, 7 combine done.
+// 5 unused (SwiGLU is part of the gate/up product), 6 down done, 7 combine done.
 void prof_mark(tie_cuda_ctx *c, int id)
 {
 	if (!c->prof_on)
@@ -294,8 +294,6 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 		prof_mark(c, 3);
 		TRY(launch_tc_gate_up(c, L, n_tile));
 		prof_mark(c, 4);
-		TRY(launch_tc_swiglu(c, L, n_rows));
-		prof_mark(c, 5);
 		// A combine finds the rows where the sort put them: each tile's stores then go to neighbouring rows.
 		TRY(launch_tc_down(c, L, n_tile, y, pos != nullptr));
 		if (pos)
@@ -968,9 +966,9 @@ int tie_cuda_upload_moe_layer(tie_cuda_ctx *c, int layer, const void *router_w_f
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(L.norm_w, ffn_norm_w, (size_t)H * sizeof(float), cudaMemcpyHostToDevice, c->stream));
 	}
 	c->weight_bytes -= L.gate.bytes + L.up.bytes + L.down.bytes;
-	TRY(upload_tensor(c, L.gate, gate_exps, gate_type, F, H));
-	TRY(upload_tensor(c, L.up, up_exps, up_type, F, H));
-	TRY(upload_tensor(c, L.down, down_exps, down_type, H, F));
+	TRY(upload_tensor(c, L.gate, gate_exps, gate_type, F, H, true));
+	TRY(upload_tensor(c, L.up, up_exps, up_type, F, H, true));
+	TRY(upload_tensor(c, L.down, down_exps, down_type, H, F, false));
 	TIE_CUDA_TRY(c, cudaStreamSynchronize(c->stream));
 	TRY(add_reg(c, router_w_f32, (size_t)E * H * sizeof(float), reinterpret_cast<const uint8_t *>(L.router_w), TIE_GGML_TYPE_F32,
 		    W_Q4K, E, H));
@@ -1534,8 +1532,6 @@ int tie_cuda_ep_compute(tie_cuda_ctx *c, int layer, unsigned flags)
 	prof_mark(c, 3);
 	TRY(launch_tc_gate_up(c, *L, TC_TOKEN_TILE));
 	prof_mark(c, 4);
-	TRY(launch_tc_swiglu(c, *L, c->sm_count * 8, ep.n_rows));
-	prof_mark(c, 5);
 	EpDst dst;
 	for (int i = 0; i < ep.view.n_ranks; i++)
 		dst.y[i] = reinterpret_cast<float *>(ep.view.peer[i] + ep.view.off_y);
@@ -1696,7 +1692,7 @@ int tie_cuda_register_tensor(tie_cuda_ctx *c, const void *host_ptr, size_t n_byt
 		dense->expert_stride = n_bytes;
 		dense->bytes = n_bytes;
 		dense->host_ptr = host_ptr;
-		int rc = tc_make_weight_map(c, *dense, 1);
+		int rc = tc_make_weight_map(c, *dense, false, 1);
 		if (!rc && dense->has_map)
 			rc = tc_make_dense_view(c, *dense);
 		if (rc) {

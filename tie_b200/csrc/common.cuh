@@ -52,7 +52,7 @@ struct DevTensor {
 	size_t expert_stride = 0;  // bytes per expert
 	size_t bytes = 0;
 	const void *host_ptr = nullptr;	 // for the dispatch-row registry
-	CUtensorMap map;	 // Q4_K: byte map for the tensor-core path's weight loader
+	CUtensorMap map;	 // byte map for the tensor-core path's weight loader
 	bool has_map = false;
 	DenseView *view = nullptr;  // stand-alone tensors only (owned)
 };
@@ -260,7 +260,7 @@ __device__ __forceinline__ void q4k_scale_min(const uint32_t sc[3], int j, int &
 // The reference's table-driven SwiGLU exactly as its AVX2 kernel evaluates it
 // (math_avx2.c:908-950, built with -ffast-math: the division by 20 is a multiply by 0.05f):
 // no range check — outside [-10,10] the first/last table segment is extrapolated.
-__device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float g, float u)
+__device__ __forceinline__ int silu_index(float g, float &frac)
 {
 	float pos = __fmul_rn(__fmul_rn(__fadd_rn(g, 10.0f), 8191.0f), 0.05f);
 	float r = rintf(pos);
@@ -270,7 +270,13 @@ __device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float
 	else
 		idx = (int)r;
 	idx = max(0, min(idx, SILU_N - 2));
-	float frac = __fsub_rn(pos, (float)idx);
+	frac = __fsub_rn(pos, (float)idx);
+	return idx;
+}
+__device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float g, float u)
+{
+	float frac;
+	const int idx = silu_index(g, frac);
 	float y1 = tab[idx], y2 = tab[idx + 1];
 	return __fmul_rn(__fmaf_rn(__fsub_rn(y2, y1), frac, y1), u);
 }

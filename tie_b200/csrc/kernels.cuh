@@ -55,19 +55,15 @@ int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, c
 int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out, int n_src, int n_cols, __half *hi,
 		      __half *lo, __half *xq);
 int launch_swiglu(tie_cuda_ctx *c, float *gate, const float *up, int n);
-// n_rows_dev != null: the row count is read on the device and n_rows CTAs stride over the rows
-int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *xq,
-			const int *n_rows_dev = nullptr);
 // tensor.cu
 int tc_setup(tie_cuda_ctx *c);
-int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, int n_experts = -1);  // default: the context's local experts
+int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, bool half_tiles, int n_experts = -1);  // default: the context's local experts
 bool tc_dense_supported(const tie_cuda_ctx *c, const DevTensor &t);
 int tc_make_dense_view(tie_cuda_ctx *c, DevTensor &t);
 int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y);
 bool tc_supported(const tie_cuda_ctx *c, const Layer &L);
 // n_tile: the token tiles of the sort, 32 or 64 rows
 int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile);
-int launch_tc_swiglu(tie_cuda_ctx *c, const Layer &L, int n_rows, const int *n_rows_dev = nullptr);
 int launch_tc_down(tie_cuda_ctx *c, const Layer &L, int n_tile, float *y, bool sorted);
 int launch_tc_down_peer(tie_cuda_ctx *c, const Layer &L, const EpDst &dst);
 // ep.cu

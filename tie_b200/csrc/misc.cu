@@ -221,44 +221,6 @@ __global__ void __launch_bounds__(256) gather_rows(const float *__restrict__ x, 
 	}
 }
 
-// gu [row][gate(ffn) | up(ffn)] fp32 -> h = SwiGLU(gate, up) * scale, split into fp16 hi + lo and
-// stored in the k order of the tensor-core operand tiles ([k0, k2, k1, k3] per group of 4).
-// The warps stride over units of 256 columns of a row, with the 32 KB table in shared memory (two
-// look-ups per element: from global memory they were what bound the pass).  ffn must be a multiple
-// of 256.
-__global__ void __launch_bounds__(ROWS_WARPS * 32) swiglu_split_rows(const float *__restrict__ gu, int ffn, float scale,
-								     const float *__restrict__ silu, __half *__restrict__ hi,
-								     __half *__restrict__ lo, __half *__restrict__ xq, int q_cols,
-								     const int *__restrict__ n_rows_dev, int n_rows_host)
-{
-	__shared__ float tab[SILU_N];
-	pdl_trigger();	// (a down product of narrow tiles sets itself up meanwhile)
-	for (int i = threadIdx.x; i < SILU_N / 4; i += blockDim.x)
-		reinterpret_cast<float4 *>(tab)[i] = __ldg(reinterpret_cast<const float4 *>(silu) + i);
-	__syncthreads();
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const size_t n_rows = n_rows_dev ? (size_t)*n_rows_dev : (size_t)n_rows_host;
-	const size_t upr = (size_t)(ffn >> 8);
-	for (size_t un = (size_t)blockIdx.x * ROWS_WARPS + warp; un < n_rows * upr; un += (size_t)gridDim.x * ROWS_WARPS) {
-		const size_t r = un / upr;
-		const float *g = gu + r * 2 * ffn, *u = g + ffn;
-		__half *hr = hi + r * ffn, *lr = lo + r * ffn;
-		__half *qr = xq ? xq + r * q_cols : nullptr;
-		{
-			const int k = (int)(un - r * upr) * 256 + lane * 8;
-			const float4 g0 = *reinterpret_cast<const float4 *>(g + k), g1 = *reinterpret_cast<const float4 *>(g + k + 4);
-			const float4 u0 = *reinterpret_cast<const float4 *>(u + k), u1 = *reinterpret_cast<const float4 *>(u + k + 4);
-			const float f[8] = {swiglu_lut(tab, g0.x, u0.x) * scale, swiglu_lut(tab, g0.y, u0.y) * scale,
-					    swiglu_lut(tab, g0.z, u0.z) * scale, swiglu_lut(tab, g0.w, u0.w) * scale,
-					    swiglu_lut(tab, g1.x, u1.x) * scale, swiglu_lut(tab, g1.y, u1.y) * scale,
-					    swiglu_lut(tab, g1.z, u1.z) * scale, swiglu_lut(tab, g1.w, u1.w) * scale};
-			Split8 p;
-			p.make(f, qr != nullptr);
-			p.store(k, hr, lr, qr, lane);
-		}
-	}
-}
-
 __global__ void __launch_bounds__(256) swiglu_kernel(float *__restrict__ gate, const float *__restrict__ up, int n,
 						     const float *__restrict__ silu)
 {
@@ -313,20 +275,6 @@ int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, c
 		       float *rows_out, int *expert_out, int *inv)
 {
 	gather_rows<<<n_rows, 256, 0, c->stream>>>(x, row_expert, perm, src_div, c->cfg.hidden, rows_out, expert_out, inv);
-	TIE_CUDA_LAUNCHED(c);
-	return TIE_CUDA_OK;
-}
-
-int launch_swiglu_split(tie_cuda_ctx *c, const float *gu, int n_rows, int ffn, float scale, __half *hi, __half *lo, __half *xq,
-			const int *n_rows_dev)
-{
-	if (ffn % 256)
-		return TIE_CUDA_ENOTSUP;
-	// (n_rows_dev: the row count is read on the device and n_rows is the grid the caller wants)
-	const int want = (n_rows * (ffn / 256) + ROWS_WARPS - 1) / ROWS_WARPS, cap = c->sm_count * 4;
-	const int grid = n_rows_dev ? n_rows : (want < cap ? want : cap);
-	swiglu_split_rows<<<grid > 0 ? grid : 1, ROWS_WARPS * 32, 0, c->stream>>>(gu, ffn, scale, c->silu, hi, lo, xq, xq_cols(ffn),
-										   n_rows_dev, n_rows);
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }

@@ -15,7 +15,7 @@
 // inside the fused multiply-add is exact, so the result is the exact integer).  The two halves of
 // such a pair come from bytes 0 and 2 (or 1 and 3) of a 32-bit word, so within every group of 4
 // consecutive k the operand tiles hold the order [k0, k2, k1, k3]; the token operand is written in
-// the same order (split_rows, swiglu_split_rows), so the contraction is unchanged.
+// the same order (split_rows, the gate/up epilogue), so the contraction is unchanged.
 #pragma once
 
 #include "common.cuh"

@@ -59,14 +59,24 @@ namespace tie {
 constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;
 constexpr int TC_SPB = QK_K / TC_BK;	  // stages per super-block
-constexpr int TC_PWARPS = 16;		  // producer warps: four groups of 128 threads
-constexpr int TC_DWARPS = 8;		  // drain warps
-constexpr int TC_THREADS = (TC_PWARPS + TC_DWARPS + 3) * 32;  // + MMA issuer + token loader + weight loader
-// Registers: the kernel is launched with 72 per thread; the producers give 8 of theirs to the drain warps,
+constexpr int TC_THREADS = (16 + 8 + 3) * 32;  // producer and drain warps (TcRoles), MMA issuer, token loader, weight loader
+// Narrow tiles (up to 32 tokens): four groups of producer warps, whose expansion paces them, and two sets of four drain
+// warps.  The sets take the work items in turn, so that one finishes its rows while the other folds the next item's super-blocks.
+// Wide tiles: eight drain warps a set, half of the tokens for each four.  Gate and up, whose rows take longest to
+// finish, have two such sets and two producer groups (4096 tokens 422 -> 387 us, 512 98 -> 90); the others one set and four groups
+// (down product of 4096 tokens 217 us, in the form of gate and up 233).
+// Registers: the kernel is launched with 72 per thread; the producers give of theirs to the drain warps,
 // whose 32 sums per thread otherwise spill (gate/up at 512 tokens 96 -> 90 us, at 4096 414 -> 385 us).
-constexpr int TC_LREGS = 72, TC_PREGS = 64, TC_DREGS = 88;
-static_assert(32 * (TC_PWARPS * TC_PREGS + TC_DWARPS * TC_DREGS) + 3 * 32 * TC_LREGS <= TC_THREADS * TC_LREGS, "register split");
-constexpr int TC_UNITS = 4;  // slots of the weight ring in tensor memory, one per producer group: half a super-block each
+constexpr int TC_LREGS = 72;
+template <bool GU, int NT>
+struct TcRoles {
+	static constexpr int PGROUPS = GU && NT > 32 ? 2 : 4, PWARPS = 4 * PGROUPS, DWARPS = 24 - PWARPS;
+	static constexpr int NSETS = GU || NT == 32 ? 2 : 1, SET = DWARPS / NSETS;
+	static constexpr int PARTS = SET / 4;  // how many ways a set splits the tokens
+	static constexpr int PREGS = PGROUPS == 4 ? 64 : 56, DREGS = PGROUPS == 4 ? 88 : 80;
+	static_assert(PARTS == (NT == 32 ? 1 : 2) && PWARPS * PREGS + DWARPS * DREGS <= 24 * TC_LREGS, "roles");
+};
+constexpr int TC_UNITS = 4;  // slots of the weight ring in tensor memory: half a super-block each
 // Super-blocks whose MMAs are in flight or waited for, at most: who waits for one has seen those TC_DONE and more before
 // it retire, and none TC_DONE after it can before the wait is over (a phase parity tells neighbouring phases apart, no more).
 constexpr int TC_DONE = 8;
@@ -106,7 +116,7 @@ struct TcRing {
 // of 9 and 13 x 16 bytes: 16-byte reads by 32 consecutive rows are bank-conflict free.
 constexpr int TC_Q6_ROW = Q6K_RECORD;
 constexpr int TC_NWB_MAX = 4, TC_NWF_MAX = 6;
-template <WKind KIND, bool PAIR, int NT>
+template <WKind KIND, bool GU, bool PAIR, int NT>
 struct TcSmem {
 	static constexpr bool Q4 = KIND == W_Q4K;
 	static constexpr int NWB = Q4 && PAIR ? 4 : 3;	// packed super-blocks in flight
@@ -118,7 +128,8 @@ struct TcSmem {
 	static constexpr int OFF_W = TC_B_BYTES;
 	static constexpr int OFF_XQ = OFF_W + NWB * WBUF;
 	static constexpr int OFF_DS = OFF_XQ + 2 * XQ;	// block factors (Q4_K)
-	static constexpr int OFF_BAR = OFF_DS + (Q4 ? TC_NDS * TC_BM * 4 : 0);
+	static constexpr int OFF_PSUM = OFF_DS + (Q4 ? TC_NDS * TC_BM * 4 : 0);	 // gate and up: sums handed from drain warp to drain warp
+	static constexpr int OFF_BAR = OFF_PSUM + (GU ? 8 * 32 * 4 : 0);
 	static constexpr int SMEM = OFF_BAR + 512 + 1024 /* alignment slack */;
 	static_assert(WBUF % 1024 == 0 && NWB <= TC_NWB_MAX, "packed super-block buffers");
 	static_assert(SMEM <= 226 * 1024, "shared memory budget");  // (1 KB is left to the static variables)
@@ -133,6 +144,7 @@ struct TcShared {
 	uint64_t pfull[2][TC_NBUF_MAX];	// accumulator complete, per set of drain warps (where there are two)
 	uint64_t pempty[TC_NBUF_MAX];	// accumulator read out by the drain warps
 	uint64_t mempty[2];		// min sums of a work item read out by the drain warps
+	uint64_t sfull[8], sempty[8];	// gate and up: half a sub-block's sums handed to the warp of the other half, and taken
 	uint64_t fin;			// every commit has landed
 	uint32_t tmem_base;
 	uint32_t abort;
@@ -174,11 +186,11 @@ __device__ __forceinline__ bool tc_wait_warp(uint32_t bar, uint32_t parity, vola
 	return __all_sync(0xffffffffu, tc_wait<BACKOFF_NS>(bar, parity, abort_flag, status));
 }
 
-// A work item: a token tile (expert le, sorted rows [row0, row0 + n_valid)) x a 128-row tile.
+// A work item: a token tile (expert le, sorted rows [row0, row0 + n_valid)) x a 128-row tile (GU: 64 rows of either matrix).
 struct TcItem {
 	int le, row0, n_valid, n_mma;  // n_mma: n_valid rounded up to 16, the N of the MMAs
 	int box;	  // 0, 1, 2: the tile's token boxes hold 16, 32 or 64 rows (half of that per CTA of a pair)
-	int mat_sel, m0;  // which matrix (RAW: 0 gate, 1 up) and first row inside it
+	int m0;	      // first row of the matrix
 };
 
 // The first TC_ITEMS work items of a CTA are decoded into shared memory when the kernel starts, all at
@@ -186,29 +198,26 @@ struct TcItem {
 // cost each role about a thousand cycles per item (measured: gate/up at 512 tokens 90 -> 88 us).
 constexpr int TC_ITEMS = 128;
 // m_items: work items per token tile (128-row tiles, or pairs of them); a CTA of a pair takes the
-// tile 2 * item + its rank.  Packed: expert, first row, rows, first weight row | matrix << 30.
+// tile 2 * item + its rank.  tile_rows: rows of the matrix a tile takes.  Packed: expert, first row, rows, first weight row.
 template <bool PAIR, int NT>
-__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int rows_per_matrix,
-					  uint32_t rank)
+__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int tile_rows, uint32_t rank)
 {
 	const int slot = t / m_items, mi = t - slot * m_items;
 	const int4 ti = tile_info ? __ldg(tile_info + slot) : make_int4(0, slot * NT, min(NT, n_rows - slot * NT), 0);
-	const int m = (PAIR ? 2 * mi + (int)rank : mi) * TC_BM, sel = m >= rows_per_matrix ? 1 : 0;
-	return make_int4(ti.x, ti.y, ti.z, (m - sel * rows_per_matrix) | sel << 30);
+	return make_int4(ti.x, ti.y, ti.z, (PAIR ? 2 * mi + (int)rank : mi) * tile_rows);
 }
 template <bool PAIR, int NT>
 __device__ __forceinline__ TcItem tc_item(int t, int tl, const int4 *s_items, int m_items, const int4 *__restrict__ tile_info,
-					  int n_rows, int rows_per_matrix, uint32_t rank)
+					  int n_rows, int tile_rows, uint32_t rank)
 {
-	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR, NT>(t, m_items, tile_info, n_rows, rows_per_matrix, rank);
+	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR, NT>(t, m_items, tile_info, n_rows, tile_rows, rank);
 	TcItem it;
 	it.le = ti.x;
 	it.row0 = ti.y;
 	it.n_valid = ti.z;
 	it.n_mma = (ti.z + 15) & ~15;
 	it.box = ti.z <= 16 ? 0 : (ti.z <= 32 ? 1 : 2);
-	it.mat_sel = ti.w >> 30;
-	it.m0 = ti.w & 0x3FFFFFFF;
+	it.m0 = ti.w;
 	return it;
 }
 
@@ -331,9 +340,13 @@ struct Expander<W_Q6K_R8> {
 	}
 };
 
-// RAW: products are stored as fp32 in expert-sorted row order, y[row0 + n][matrix * rows + mrow]
-// (gate | up of one row side by side) for the SwiGLU pass; the 128-row tiles then run over w0
-// followed by w1.  Otherwise (down) they are times out_scale (a power of two) in sorted order, or, with perm, in
+// GU (gate and up): a tile is 64 rows of w0 and the same of w1, sixteen of each in the tensor-memory lanes of a
+// warp, so that the SwiGLU of a row is one shuffle away in the drain: h * out_scale, split into fp16 hi + lo, goes to the down
+// product's operand (and its sub-block sums, where that is Q4_K).  The products themselves stay on the chip: as
+// fp32 rows for a pass of its own they were 2 x 200 MB at 4096 tokens.  (Products and pass -> product with SwiGLU: 64 tokens
+// 69 + 10 -> 70 us, 512 86 + 13 -> 90, 4096 368 + 57 -> 387.)  The table is read through the 28 KB of L1 that shared memory
+// leaves; its middle 20 KB in shared memory took a weight buffer's place, 64 tokens 70 -> 76 us.
+// Otherwise (down, dense) products times out_scale (a power of two) are stored in sorted order, or, with perm, in
 // the order of the rows y[perm[row0 + n]].
 // tm0/1/2: maps of the split token operand ([hi | lo][rows][k], box 64 k x 16/32/64 rows x 2; half
 // of the rows for a CTA of a pair); tq0/1/2: the same of its sub-block sums; tw0 / tw1: byte maps of
@@ -349,7 +362,14 @@ struct Expander<W_Q6K_R8> {
 // PEER (expert parallelism over peer memory, down product only): sorted row p belongs to row
 // dst.row[p] & 0xFFFFFF of rank dst.row[p] >> 24 and is stored there, into that rank's memory
 // (dst.y[rank], plain stores over NVLink, 128 contiguous bytes per warp and row).
-template <WKind KIND, bool RAW, bool PEER = false, bool PAIR = false, int NT = TC_TOKEN_TILE>
+struct GuOut {
+	__half *hi = nullptr;	 // [rows][rows of the matrix], the k order of the operand tiles
+	size_t lo = 0;		 // the lo halves lie so many values behind
+	__half *sums = nullptr;	 // [rows][sum_cols] or null
+	int sum_cols = 0;
+	const float *silu = nullptr;
+};
+template <WKind KIND, bool GU, bool PEER = false, bool PAIR = false, int NT = TC_TOKEN_TILE>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
 		const __grid_constant__ CUtensorMap tm2, const __grid_constant__ CUtensorMap tq0,
@@ -358,15 +378,17 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		const uint8_t *__restrict__ w1, size_t expert_stride, int k_dim, const int4 *__restrict__ tile_info,
 		const int *__restrict__ tile_start, int n_local, int m_tiles, float *__restrict__ y, const int *__restrict__ perm,
 		int out_stride, float out_scale, unsigned *__restrict__ status, int rows_per_matrix, const EpDst dst,
-		const int xq_depth)
+		const int xq_depth, const GuOut gu)
 {
-	static_assert(!(RAW && PEER), "peer destinations exist for the down product only");
-	using Sm = TcSmem<KIND, PAIR, NT>;
+	static_assert(!(GU && PEER), "peer destinations exist for the down product only");
+	using Sm = TcSmem<KIND, GU, PAIR, NT>;
+	constexpr int TILE_ROWS = GU ? TC_BM / 2 : TC_BM;  // of a matrix
 	using Ring = TcRing<PAIR, NT>;
 	using Cols = TcCols<KIND, NT>;
 	constexpr int NBUF = Cols::NBUF;
-	constexpr bool SETS = NT == 32;	 // two sets of drain warps, taking the work items in turn
-	constexpr int FOLDERS = SETS ? TC_DWARPS / 2 : TC_DWARPS;  // drain warps that read an accumulator
+	using Roles = TcRoles<GU, NT>;
+	constexpr int PARTS = Roles::PARTS;
+	constexpr int FOLDERS = Roles::SET;  // drain warps that read an accumulator
 	constexpr bool Q4 = KIND == W_Q4K;
 	constexpr uint32_t UNIT = Cols::UNIT;
 	extern __shared__ uint8_t smem_raw[];
@@ -384,6 +406,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	uint8_t *smem = smem_raw + (tiles - raw);
 	TcShared *sh = reinterpret_cast<TcShared *>(smem + Sm::OFF_BAR);
 	float *ds = reinterpret_cast<float *>(smem + Sm::OFF_DS);  // [TC_NDS][128] d of the rows (Q4_K)
+	float *psum = reinterpret_cast<float *>(smem + Sm::OFF_PSUM);
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
 	// token tiles of a super-block: four stages of the CTA's hi rows followed by its lo rows
@@ -409,12 +432,16 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		}
 		for (int s = 0; s < 2; s++)
 			ptx::mbar_init(ptx::smem_u32(&sh->mempty[s]), (PAIR ? 2 : 1) * FOLDERS);
+		for (int s = 0; s < 8; s++) {
+			ptx::mbar_init(ptx::smem_u32(&sh->sfull[s]), 1);
+			ptx::mbar_init(ptx::smem_u32(&sh->sempty[s]), 1);
+		}
 		ptx::mbar_init(ptx::smem_u32(&sh->fin), 1);
 		sh->abort = 0;
 		ptx::fence_barrier_init();
 		ptx::fence_proxy_async_smem();
 	}
-	constexpr int W_MMA = TC_PWARPS + TC_DWARPS, W_TOK = W_MMA + 1, W_WGT = W_TOK + 1;
+	constexpr int W_MMA = Roles::PWARPS + Roles::DWARPS, W_TOK = W_MMA + 1, W_WGT = W_TOK + 1;
 	if (warp == W_MMA) {  // the MMA warp owns the tensor-memory allocation (pairs: one warp of each CTA, together)
 		if (PAIR) {
 			ptx::tmem_alloc_pair(ptx::smem_u32(&sh->tmem_base), TC_TMEM_COLS);
@@ -436,9 +463,11 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	}
 	if (warp == W_WGT && lane == 0) {
 		ptx::prefetch_tmap(&tw0);
-		if (RAW)
+		if (GU)
 			ptx::prefetch_tmap(&tw1);
 	}
+	if (GU)
+		pdl_trigger();	// (a down product of narrow tiles sets itself up as the SMs fall idle)
 	pdl_wait();  // what the kernels before this one wrote is visible from here on
 	if (threadIdx.x == 0)
 		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
@@ -448,7 +477,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	if (threadIdx.x < TC_ITEMS) {
 		const int t = walker + threadIdx.x * stride_t;
 		if (t < total)
-			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, rows_per_matrix, rank);
+			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, TILE_ROWS, rank);
 	}
 	__syncthreads();
 	if (PAIR)
@@ -464,24 +493,26 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			ptx::mbar_arrive(ptx::smem_u32(bar));
 	};
 
-	if (warp < TC_PWARPS) {
+	if (warp < Roles::PWARPS) {
 		// ================= producers: packed blocks (shared memory) -> integer A tiles (tensor memory) =================
-		// Four groups of four warps (one warp per 32-row quadrant of tensor memory).  A unit is half a
+		// Groups of four warps (one warp per 32-row quadrant of tensor memory).  A unit is half a
 		// super-block: two 64-k stages and, for Q4_K, the hi (first half) or lo columns of its dmin * m
-		// products.  Group j makes half j & 1 of every other super-block and owns slot j of the ring; a
+		// products.  Group j makes half j & 1 of every super-block (four groups: of every other); a
 		// first piece is expanded in registers BEFORE the slot is waited for.
-		ptx::setmaxnreg_dec<TC_PREGS>();
+		ptx::setmaxnreg_dec<Roles::PREGS>();
+		constexpr uint32_t STEP = Roles::PGROUPS / 2;
 		const int row = threadIdx.x & 127, grp = threadIdx.x >> 7, half = grp & 1;
-		const uint32_t slot = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cols::A + UNIT * grp;
-		const uint32_t full = ptx::smem_u32(&sh->full[grp >> 1]);
+		// (GU: lanes 0 - 15 of a warp take rows of the gate box, 16 - 31 the same rows of the up box behind it)
+		const int wrow = GU ? ((row & 16) << 2) + ((row >> 5) << 4) + (row & 15) : row;
+		const uint32_t slot0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cols::A + UNIT * (STEP == 2 ? grp : half);
 		const uint32_t n_sb = walker < total ? (uint32_t)((total - 1 - walker) / stride_t + 1) * (uint32_t)nb : 0u;
 		bool alive = true;
-		for (uint32_t n = grp >> 1; n < n_sb; n += 2) {
-			const uint32_t wb = n % Sm::NWB;
+		for (uint32_t n = STEP == 2 ? grp >> 1 : 0; n < n_sb; n += STEP) {
+			const uint32_t wb = n % Sm::NWB, slot = slot0 + (STEP == 1 ? 2 * UNIT * (n & 1u) : 0u);
 			if (!tc_wait_warp(ptx::smem_u32(&sh->wfull[n % Sm::NWF]), (n / Sm::NWF) & 1u, abort_flag, status, lane))
 				break;
 			Expander<KIND> ex;
-			ex.prepare(w_buf(wb), row, half);
+			ex.prepare(w_buf(wb), wrow, half);
 			if constexpr (Q4) {
 				if (half == 0)
 					ds[(n & (TC_NDS - 1)) * TC_BM + row] = ex.d();
@@ -522,40 +553,38 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			ptx::tc_fence_before();
 			__syncwarp();
 			if (lane == 0) {
-				if (PAIR)
-					ptx::mbar_arrive_leader(full);
-				else
-					ptx::mbar_arrive(full);
+				arrive_issuer(&sh->full[STEP == 2 ? grp >> 1 : n & 1u]);
 				// this warp's half of the packed super-block is expanded: the buffer goes back to the weight loader
 				ptx::mbar_arrive(ptx::smem_u32(&sh->wempty[wb]));
 			}
 		}
 	} else if (warp < W_MMA) {
 		// ================= drain warps: partial sums of a super-block -> fp32 rows =================
-		ptx::setmaxnreg_inc<TC_DREGS>();
-		const int dw = warp - TC_PWARPS, quad = warp & 3, part = dw >> 2;
+		ptx::setmaxnreg_inc<Roles::DREGS>();
+		const int dw = warp - Roles::PWARPS, quad = warp & 3, part = (dw >> 2) % PARTS, set = Roles::NSETS == 2 ? dw / Roles::SET : 0;
 		const int lrow = quad * 32 + lane;
 		const uint32_t tlane = tmem + ((uint32_t)(quad * 32) << 16);
-		const int set = SETS ? part : 0;
+		const bool upper = GU && (lane & 16);  // a lane of up rows
+		uint32_t handed = 0;		       // GU: sums handed over (or taken) so far
 		uint32_t n = 0;	   // super-blocks so far
-		uint32_t pph = 0;  // SETS, per accumulator: parity of this set's next wait (it takes only its items' uses)
+		uint32_t pph = 0;  // per accumulator: parity of this set's next wait (it takes only its items' uses)
 		bool alive = true;
 		int dtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, dtl++) {
-			if (SETS && (dtl & 1) != set) {	 // the other set's item
+			if (Roles::NSETS == 2 && (dtl & 1) != set) {  // the other set's item
 				n += nb;
 				continue;
 			}
-			const TcItem item = tc_item<PAIR, NT>(t, dtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
-			const int mrow = item.m0 + lrow;
-			// tokens of this warp: with two sets the whole tile, else half of it (the first or the second by part).
+			const TcItem item = tc_item<PAIR, NT>(t, dtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
+			const int mrow = item.m0 + (GU ? quad * 16 + (lane & 15) : lrow);
+			// tokens of this warp: the whole tile, or half of it (the first or the second by part).
 			// Where twice the columns fit an accumulator, the hi and lo products have columns of their own (one MMA
 			// for both), which for a pair lie [hi lo] per CTA's half of the tokens.
 			const bool stacked = 2 * item.n_mma <= NT;
-			const int ntok = SETS ? item.n_mma : (item.n_mma > 32 ? 32 : item.n_mma >> 1);
-			const int tok0 = SETS ? 0 : part * ntok;
+			const int ntok = PARTS == 1 ? item.n_mma : (item.n_mma > 32 ? 32 : item.n_mma >> 1);
+			const int tok0 = part * ntok;
 			const bool two = ntok == 32;
-			const uint32_t c_hi = PAIR ? part * item.n_mma : tok0, c_lo = PAIR ? c_hi + ntok : item.n_mma + tok0;  // (not SETS)
+			const uint32_t c_hi = PAIR ? part * item.n_mma : tok0, c_lo = PAIR ? c_hi + ntok : item.n_mma + tok0;  // (two parts)
 			float acc[32];
 #pragma unroll
 			for (int j = 0; j < 32; j++)
@@ -574,10 +603,10 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					ptx::tmem_ld_wait();
 				} else if (both) {
 					uint32_t u[16];
-					ptx::tmem_ld16(tlane + col + (SETS ? 0u : c_hi), v);
-					ptx::tmem_ld16(tlane + col + (SETS ? 16u : c_lo), u);
+					ptx::tmem_ld16(tlane + col + (PARTS == 1 ? 0u : c_hi), v);
+					ptx::tmem_ld16(tlane + col + (PARTS == 1 ? 16u : c_lo), u);
 					ptx::tmem_ld_wait();
-					if (SETS && PAIR) {  // [hi lo] of tokens 0 .. 7, then of 8 .. 15
+					if (PARTS == 1 && PAIR) {  // [hi lo] of tokens 0 .. 7, then of 8 .. 15
 #pragma unroll
 						for (int j = 0; j < 8; j++) {
 							v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(v[8 + j]));
@@ -610,39 +639,111 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			const uint8_t *grp = nullptr;
 			float dnext = 0.0f;
 			if (!Q4) {
-				grp = (item.mat_sel ? w1 : w0) + (size_t)item.le * expert_stride + (size_t)(mrow >> 3) * q6k_r8_group_bytes(nb);
+				grp = (upper ? w1 : w0) + (size_t)item.le * expert_stride + (size_t)(mrow >> 3) * q6k_r8_group_bytes(nb);
 				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, 0))));
 			}
 			for (int sbi = 0; sbi < nb; sbi++, n++) {
-				float scale = 16.0f * out_scale * dnext;
+				float scale = (GU ? 16.0f : 16.0f * out_scale) * dnext;
 				if (!Q4 && sbi + 1 < nb)
 					dnext = half_bits_to_float(
 						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
 				const uint32_t buf = n % NBUF;
-				if (!tc_wait_warp(ptx::smem_u32(SETS ? &sh->pfull[set][buf] : &sh->done[n % TC_DONE]),
-						  SETS ? (pph >> buf) & 1u : (n / TC_DONE) & 1u, abort_flag, status, lane)) {
+				if (!tc_wait_warp(ptx::smem_u32(Roles::NSETS == 2 ? &sh->pfull[set][buf] : &sh->done[n % TC_DONE]),
+						  Roles::NSETS == 2 ? (pph >> buf) & 1u : (n / TC_DONE) & 1u, abort_flag, status, lane)) {
 					alive = false;
 					break;
 				}
-				if (SETS)
+				if (Roles::NSETS == 2)
 					pph ^= 1u << buf;
 				ptx::tc_fence_after();
 				if (Q4)
-					scale = out_scale * ds[(n & (TC_NDS - 1)) * TC_BM + lrow];
+					scale = (GU ? 1.0f : out_scale) * ds[(n & (TC_NDS - 1)) * TC_BM + lrow];
 				fold(NT * buf, stacked, scale, &sh->pempty[buf]);
 			}
 			if (!alive)
 				break;
 			// the min sums (Q4_K) were complete with the last super-block
 			if (Q4)
-				fold(Cols::M + NT * set, false, -out_scale, &sh->mempty[set]);
-			// rows of this work item: lanes hold consecutive output columns (coalesced 128-byte stores)
+				fold(Cols::M + NT * (set % Cols::NM), false, GU ? -1.0f : -out_scale, &sh->mempty[set % Cols::NM]);
 			const int n_rows = min(ntok, item.n_valid - tok0);
 			const int p0 = item.row0 + tok0;  // sorted position of the first row
+			if constexpr (GU) {
+				// Lane l holds gate (l < 16) or up rows of all the warp's tokens and makes h of row l & 15 for half of them.
+				auto finish = [&](auto half_tokens) {
+					constexpr int H = half_tokens.value;
+					const int j0 = upper ? H : 0;
+					// (the order [k0, k2, k1, k3] of every group of 4)
+					const int k = (mrow & ~3) | (mrow & 1) << 1 | (mrow >> 1 & 1);
+					__half *hp = gu.hi + (size_t)(p0 + j0) * rows_per_matrix + k;
+					float h[H];
+#pragma unroll
+					for (int j = 0; j < H; j++) {
+						const float other = __shfl_xor_sync(0xffffffffu, upper ? acc[j] : acc[H + j], 16);
+						const float mine = upper ? acc[H + j] : acc[j];
+						h[j] = swiglu_lut(gu.silu, upper ? other : mine, upper ? mine : other) * out_scale;
+					}
+#pragma unroll
+					for (int j = 0; j < H; j++) {
+						if (j0 + j < n_rows) {
+							const __half hi = __float2half_rn(h[j]);
+							hp[0] = hi;
+							hp[gu.lo] = __float2half_rn(h[j] - __half2float(hi));
+						}
+						hp += rows_per_matrix;
+					}
+					if (gu.sums) {
+						// sums over the warp's 16 rows (a token each for lane & (H - 1)), added to those of the sub-block's other 16
+#pragma unroll
+						for (int w = 8; w >= 1; w >>= 1) {
+							if (w >= H) {
+#pragma unroll
+								for (int j = 0; j < H; j++)
+									h[j] += __shfl_xor_sync(0xffffffffu, h[j], w);
+								continue;
+							}
+							const bool keep_hi = lane & w;
+#pragma unroll
+							for (int j = 0; j < w; j++) {
+								const float send = keep_hi ? h[j] : h[w + j], keep = keep_hi ? h[w + j] : h[j];
+								h[j] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+							}
+						}
+						const int tok = j0 + (lane & (H - 1)), pair = (dw >> 2) * 2 + (quad >> 1);
+						const uint32_t sf = ptx::smem_u32(&sh->sfull[pair]), se = ptx::smem_u32(&sh->sempty[pair]);
+						float *ps = psum + pair * 32 + lane;
+						if (quad & 1) {
+							alive = tc_wait_warp(se, (handed & 1u) ^ 1u, abort_flag, status, lane);
+							*ps = h[0];
+							__syncwarp();
+							if (lane == 0)
+								ptx::mbar_arrive(sf);
+						} else {
+							alive = tc_wait_warp(sf, handed & 1u, abort_flag, status, lane);
+							const float sum = h[0] + *ps;
+							__syncwarp();
+							if (lane == 0)
+								ptx::mbar_arrive(se);
+							if (alive && tok < n_rows && (lane & 15) < H) {
+								const __half hi = __float2half_rn(sum);
+								__half *q = gu.sums + (size_t)(p0 + tok) * gu.sum_cols + xq_index(mrow >> 5);
+								q[0] = hi;
+								q[8] = __float2half_rn(sum - __half2float(hi));
+							}
+						}
+						handed++;
+					}
+				};
+				if (two)
+					finish(std::integral_constant<int, 16>());
+				else
+					finish(std::integral_constant<int, 8>());
+				continue;
+			}
+			// rows of this work item: lanes hold consecutive output columns (coalesced 128-byte stores)
 			// (in sorted order a tile's stores go to neighbouring rows: scattered to the rows' own places, 8 KB apart in 268 MB
 			// at 4096 tokens, the down product took 238 us there instead of 217, 61 instead of 55 at 512)
-			if (RAW || (!PEER && !perm)) {
-				float *yr = y + (size_t)p0 * out_stride + (RAW ? (size_t)item.mat_sel * rows_per_matrix : 0) + mrow;
+			if (!PEER && !perm) {
+				float *yr = y + (size_t)p0 * out_stride + mrow;
 #pragma unroll
 				for (int j0 = 0; j0 < 32; j0 += 8) {
 					if (j0 + 8 <= n_rows) {
@@ -700,14 +801,14 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				alive = alive && tc_wait(bar, parity, abort_flag, status);
 			};
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
 				const uint32_t idesc = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, item.n_mma);
 				const uint32_t idesc2 = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, 2 * item.n_mma);
 				const uint32_t lo_off = (uint32_t)((PAIR ? 8 : 16) << item.box) * 128u;
 				// a tile whose hi and lo products fit an accumulator side by side fills its box, so the lo rows follow the
 				// hi rows and one MMA of twice the columns takes both
 				const bool stacked = 2 * item.n_mma <= NT;
-				const uint32_t dset = SETS ? tl & 1u : 0u;  // the set of drain warps that takes the item
+				const uint32_t dset = Roles::NSETS == 2 ? tl & 1u : 0u, mset = Cols::NM == 2 ? dset : 0u;  // the set of drain warps that takes the item, its min sums
 				for (int sbi = 0; sbi < nb; sbi++, n++) {
 					const uint32_t buf = n % NBUF, j0 = 2u * (n & 1u);
 					const uint32_t q = n & (Ring::GROUPS - 1);
@@ -752,19 +853,19 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						// (dmin m)_hi (first unit), (dmin m)_lo (second) times the block's sums, hi and lo side by side in k; an item's
 						// first ones behind its first stages, so that the drain of its accumulator's last item holds those up no more
 						if (sbi == 0) {
-							wait(ptx::smem_u32(&sh->mempty[dset]), ((SETS ? tl >> 1 : tl) & 1u) ^ 1u);
+							wait(ptx::smem_u32(&sh->mempty[mset]), ((tl / Cols::NM) & 1u) ^ 1u);
 							if (!alive)
 								break;
 							ptx::tc_fence_after();
 						}
-						const uint32_t dM = tmem + Cols::M + NT * dset, aM = tmem + Cols::A + UNIT * j0 + 64u;
+						const uint32_t dM = tmem + Cols::M + NT * mset, aM = tmem + Cols::A + UNIT * j0 + 64u;
 						mma(dM, aM, xs, idesc, sbi > 0 ? 1u : 0u);
 						mma(dM, aM + UNIT, xs, idesc, 1u);
 						if ((sbi & 7) == 7 || sbi == nb - 1)
 							xs_n++;
 					}
 					commit(&sh->done[n % TC_DONE]);
-					if (SETS)
+					if (Roles::NSETS == 2)
 						commit(&sh->pfull[dset][buf]);
 				}
 			}
@@ -779,7 +880,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			uint32_t tl = 0, n = 0, xs_n = 0, x_end = 0;  // x_end: where the segment of sums before the current one ended
 			bool alive = true;
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
 				// one box per super-block: four stages of 64 k x (hi, lo) x the CTA's token rows.  The CTAs of a pair
 				// take the first and the second half of the tile's n_mma columns; all the bytes are counted on
 				// the leader's barrier, whose token loader announces them.
@@ -832,7 +933,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		bool alive = true;
 		int wtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, wtl++) {
-			const TcItem item = tc_item<PAIR, NT>(t, wtl, s_items, m_items, tile_info, n_local, rows_per_matrix, rank);
+			const TcItem item = tc_item<PAIR, NT>(t, wtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
 			for (int sbi = 0; sbi < nb; sbi++) {
 				if (wc >= (uint32_t)Sm::NWB && !tc_wait_warp<100>(ptx::smem_u32(&sh->wempty[wb]), wph ^ 1u, abort_flag, status, lane)) {
 					alive = false;
@@ -841,12 +942,16 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				const uint32_t bar = ptx::smem_u32(&sh->wfull[wc % Sm::NWF]);
 				if (ptx::elect_one()) {
 					ptx::mbar_arrive_expect_tx(bar, Sm::WBUF);
-					if (Q4)	 // box = (one block, 128 rows)
-						ptx::tma_load_2d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, sbi * Q4K_BYTES,
-								 item.le * rows_per_matrix + item.m0);
-					else  // box = (one record, 8 rows of a group, 16 groups)
-						ptx::tma_load_3d(w_buf(wb), item.mat_sel ? &tw1 : &tw0, bar, sbi * TC_Q6_ROW, 0,
-								 (item.le * rows_per_matrix + item.m0) >> 3);
+					const int row = item.le * rows_per_matrix + item.m0;
+#pragma unroll
+					for (int m = 0; m < (GU ? 2 : 1); m++) {
+						const CUtensorMap *tw = m ? &tw1 : &tw0;
+						const uint32_t at = w_buf(wb) + m * (Sm::WBUF / 2);
+						if (Q4)	 // box = (one block, 128 or 64 rows)
+							ptx::tma_load_2d(at, tw, bar, sbi * Q4K_BYTES, row);
+						else  // box = (one record, 8 rows of a group, 16 or 8 groups)
+							ptx::tma_load_3d(at, tw, bar, sbi * TC_Q6_ROW, 0, row >> 3);
+					}
 				}
 				wc++;
 				if (++wb == Sm::NWB) {
@@ -958,8 +1063,9 @@ static int make_sums_tmap(tie_cuda_ctx *c, CUtensorMap *tm, void *base, size_t r
 }
 
 // Byte map of an expert tensor for the weight loader.  Q4_K: [experts x rows][row bytes], box = one
-// 144-byte block x 128 rows.  Q6_K: [groups][8 rows][row records], box = one 208-byte record x 8 x 16.
-int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, int n_experts)
+// 144-byte block x 128 rows.  Q6_K: [groups][8 rows][row records], box = one 208-byte record x 8 x 16.  half_tiles: boxes of
+// half the rows (gate and up, which share a tile).
+int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, bool half_tiles, int n_experts)
 {
 	if (n_experts <= 0)
 		n_experts = c->n_local;
@@ -967,9 +1073,10 @@ int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, int n_experts)
 	if (t.rows % TC_BM || t.k % QK_K)
 		return TIE_CUDA_OK;
 	const int nb = t.k / QK_K;
+	const unsigned box_rows = half_tiles ? TC_BM / 2 : TC_BM;
 	if (t.kind == W_Q4K) {
 		int rc = encode_2d(c, &t.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, t.ptr, (size_t)t.rows * n_experts, (size_t)nb * Q4K_BYTES,
-				   Q4K_BYTES, TC_BM, CU_TENSOR_MAP_SWIZZLE_NONE);
+				   Q4K_BYTES, box_rows, CU_TENSOR_MAP_SWIZZLE_NONE);
 		if (rc)
 			return rc;
 	} else {
@@ -980,7 +1087,7 @@ int tc_make_weight_map(tie_cuda_ctx *c, DevTensor &t, int n_experts)
 		}
 		cuuint64_t dims[3] = {(cuuint64_t)nb * Q6K_RECORD, 8, (cuuint64_t)t.rows * n_experts / 8};
 		cuuint64_t strides[2] = {(cuuint64_t)nb * Q6K_RECORD, (cuuint64_t)q6k_r8_group_bytes(nb)};
-		cuuint32_t box[3] = {Q6K_RECORD, 8, TC_BM / 8};
+		cuuint32_t box[3] = {Q6K_RECORD, 8, box_rows / 8};
 		cuuint32_t estr[3] = {1, 1, 1};
 		CUresult r = enc(&t.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, t.ptr, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
 				 CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1009,26 +1116,26 @@ int tc_setup(tie_cuda_ctx *c)
 			if (rc)
 				return rc;
 		}
-#define TC_ATTR(KIND, RAW) \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<KIND, false, 64>::SMEM)); \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, false, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
-					     TcSmem<KIND, false, 32>::SMEM));                                                                         \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, false, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
-					     TcSmem<KIND, true, 32>::SMEM))
+#define TC_ATTR(KIND, GU) \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<KIND, GU, false, 64>::SMEM)); \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, false, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
+					     TcSmem<KIND, GU, false, 32>::SMEM));                                                                         \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, false, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,                \
+					     TcSmem<KIND, GU, true, 32>::SMEM))
 	TC_ATTR(W_Q4K, false);
 	TC_ATTR(W_Q4K, true);
 	TC_ATTR(W_Q6K_R8, false);
 	TC_ATTR(W_Q6K_R8, true);
 #undef TC_ATTR
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q4K, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     TcSmem<W_Q4K, false, 64>::SMEM));
+					     TcSmem<W_Q4K, false, false, 64>::SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q6K_R8, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					     TcSmem<W_Q6K_R8, false, 64>::SMEM));
+					     TcSmem<W_Q6K_R8, false, false, 64>::SMEM));
 	// the CTA-pair forms; how many pairs the device holds at once sizes their (persistent) grids
-#define TC_ATTR_PAIR(KIND, RAW, PEER)                                                                                          \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, PEER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-					     TcSmem<KIND, true, 64>::SMEM));                                                   \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, RAW, PEER, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 0))
+#define TC_ATTR_PAIR(KIND, GU, PEER)                                                                                          \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, PEER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+					     TcSmem<KIND, GU, true, 64>::SMEM));                                                   \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, PEER, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 0))
 	TC_ATTR_PAIR(W_Q4K, false, false);
 	TC_ATTR_PAIR(W_Q4K, true, false);
 	TC_ATTR_PAIR(W_Q4K, false, true);
@@ -1040,7 +1147,7 @@ int tc_setup(tie_cuda_ctx *c)
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(c->sm_count & ~1);
 		cfg.blockDim = dim3(TC_THREADS);
-		cfg.dynamicSmemBytes = TcSmem<W_Q4K, true, 64>::SMEM;
+		cfg.dynamicSmemBytes = TcSmem<W_Q4K, true, true, 64>::SMEM;
 		cudaLaunchAttribute attr[1];
 		attr[0].id = cudaLaunchAttributeClusterDimension;
 		attr[0].val.clusterDim.x = 2;
@@ -1060,19 +1167,20 @@ int tc_setup(tie_cuda_ctx *c)
 }
 
 // arr: 0 = the split inputs x (gate/up), 1 = the split activations h (down).
-template <WKind KIND, bool RAW, bool PEER = false, int NT = TC_TOKEN_TILE>
+template <WKind KIND, bool GU, bool PEER = false, int NT = TC_TOKEN_TILE>
 static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1, int arr, float *y, float out_scale,
-		       bool sorted_out = false, const EpDst *dst = nullptr, int dense_rows = 0, const DenseView *view = nullptr)
+		       bool sorted_out = false, const EpDst *dst = nullptr, int dense_rows = 0, const DenseView *view = nullptr,
+		       const GuOut &gu = GuOut())
 {
 	Scratch &s = c->s;
 	const int4 *tile_info = dense_rows ? nullptr : s.tile_info;
 	const int n_experts = dense_rows ? dense_rows : c->n_local;
-	const int m_tiles = (RAW ? 2 : 1) * t0.rows / TC_BM;
+	const int m_tiles = (GU ? 2 : 1) * t0.rows / TC_BM;
 	const CUtensorMap &w0m = t0.map;
-	const CUtensorMap &w1m = t1 ? t1->map : t0.map;
+	const CUtensorMap &w1m = GU ? t1->map : t0.map;
 	const uint8_t *w1p = t1 ? t1->ptr : nullptr;
 	const int *perm = sorted_out ? nullptr : s.perm;
-	const int out_stride = RAW ? 2 * t0.rows : t0.rows;
+	const int out_stride = t0.rows;
 	const EpDst d = dst ? *dst : EpDst();
 	const int k_dim = t0.k;
 	const int xqd = xq_depth((size_t)xq_cols(t0.k));
@@ -1088,15 +1196,15 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	const bool dependent = dense_rows > 0 || NT == 32;
 	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles : 1 << 30;	// (known for a dense tensor: no idle CTAs)
 	if (c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K) {
-		return launch_kernel(c, dependent, 2, grouped_gemm_sb<KIND, RAW, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
-				     TcSmem<KIND, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
+		return launch_kernel(c, dependent, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
+				     TcSmem<KIND, GU, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
 				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
-				     s.status, t0.rows, d, xqd);
+				     s.status, t0.rows, d, xqd, gu);
 	}
-	return launch_kernel(c, dependent, 1, grouped_gemm_sb<KIND, RAW, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
-			     TcSmem<KIND, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
+	return launch_kernel(c, dependent, 1, grouped_gemm_sb<KIND, GU, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
+			     TcSmem<KIND, GU, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
 			     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status,
-			     t0.rows, d, xqd);
+			     t0.rows, d, xqd, gu);
 }
 
 static bool tc_tensor_ok(const DevTensor &t)
@@ -1110,24 +1218,20 @@ bool tc_supported(const tie_cuda_ctx *c, const Layer &L)
 }
 
 // xs_hi/xs_lo (and xq for Q4_K) must hold the split inputs in sorted order; the sort must
-// have been run with n_tile (32 or 64).  Gate and up run as independent 128-row tiles; the raw fp32
-// products go to the scratch s.y as [row][gate | up].
+// have been run with n_tile (32 or 64).  Leaves the SwiGLU outputs, scaled and split, in hs_hi/hs_lo (and their sums in hq
+// where the down matrix is Q4_K).
 int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile)
 {
-	if (n_tile == 32)
-		return (L.gate.kind == W_Q4K) ? launch_tc_t<W_Q4K, true, false, 32>(c, L.gate, &L.up, 0, c->s.y, 1.0f)
-					      : launch_tc_t<W_Q6K_R8, true, false, 32>(c, L.gate, &L.up, 0, c->s.y, 1.0f);
-	return (L.gate.kind == W_Q4K) ? launch_tc_t<W_Q4K, true>(c, L.gate, &L.up, 0, c->s.y, 1.0f)
-				      : launch_tc_t<W_Q6K_R8, true>(c, L.gate, &L.up, 0, c->s.y, 1.0f);
-}
-
-// Element-wise SwiGLU of the raw gate | up products, scaled and split into hs_hi/hs_lo (and
-// hq when the down matrix is Q4_K).
-int launch_tc_swiglu(tie_cuda_ctx *c, const Layer &L, int n_rows, const int *n_rows_dev)
-{
-	const bool sums = L.down.kind == W_Q4K;
-	return launch_swiglu_split(c, c->s.y, n_rows, L.gate.rows, TC_H_SCALE, c->s.hs_hi, c->s.hs_lo, sums ? c->s.hq : nullptr,
-				   n_rows_dev);
+	Scratch &s = c->s;
+	GuOut gu;
+	gu.hi = s.hs_hi;
+	gu.lo = (size_t)(s.hs_lo - s.hs_hi);
+	gu.sums = L.down.kind == W_Q4K ? s.hq : nullptr;
+	gu.sum_cols = xq_cols(L.gate.rows);
+	gu.silu = c->silu;
+	auto launch = n_tile == 32 ? (L.gate.kind == W_Q4K ? launch_tc_t<W_Q4K, true, false, 32> : launch_tc_t<W_Q6K_R8, true, false, 32>)
+				   : (L.gate.kind == W_Q4K ? launch_tc_t<W_Q4K, true> : launch_tc_t<W_Q6K_R8, true>);
+	return launch(c, L.gate, &L.up, 0, nullptr, TC_H_SCALE, true, nullptr, 0, nullptr, gu);
 }
 
 // reads hs_hi/hs_lo; writes y in sorted order or (sorted false) y[perm[p]].
