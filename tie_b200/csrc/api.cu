@@ -284,13 +284,12 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	const int n_tile = n_rows <= 24 * c->n_local ? 32 : TC_TOKEN_TILE;
 	c->last_direct_rows = direct ? n_rows : -1;
 	c->last_used_tc = use_tc;
-	if (!direct)
+	if (!direct && !use_tc)
 		TRY(launch_sort(c, row_expert, n_rows, n_tile));
 	prof_mark(c, 2);
 	if (use_tc) {
 		const bool sums = L.gate.kind == W_Q4K;	 // the Q4_K "min" term needs the sub-block sums of the inputs
-		TRY(launch_split_rows(c, x_src, c->s.inv, src_div, n_rows / src_div, c->cfg.hidden, c->s.xs_hi, c->s.xs_lo,
-				      sums ? c->s.xq : nullptr));
+		TRY(launch_dispatch(c, x_src, row_expert, n_rows / src_div, src_div, n_tile, sums, pos != nullptr));
 		prof_mark(c, 3);
 		TRY(launch_tc_gate_up(c, L, n_tile));
 		prof_mark(c, 4);
@@ -1738,7 +1737,7 @@ int tie_cuda_mat_mat(tie_cuda_ctx *c, const void *w_host, const float *x, float 
 	}
 	// the batch, split into fp16 hi + lo (and its sub-block sums for Q4_K), in the tensor's view of the x arrays
 	const bool sums = reg->dense->kind == W_Q4K;
-	TRY(launch_split_rows(c, x_dev, nullptr, 1, batch_len, in_dim, s.xs_hi, s.xs_hi + v.lo_off, sums ? s.xq : nullptr));
+	TRY(launch_split_rows(c, x_dev, batch_len, in_dim, s.xs_hi, s.xs_hi + v.lo_off, sums ? s.xq : nullptr));
 	TRY(launch_tc_dense(c, *reg->dense, batch_len, o_dev));
 	if (!dev) {
 		TIE_CUDA_TRY(c, cudaMemcpyAsync(o, o_dev, (size_t)batch_len * out_dim * sizeof(float), cudaMemcpyDeviceToHost, c->stream));

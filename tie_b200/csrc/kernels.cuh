@@ -40,6 +40,8 @@ struct SortBufs {
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile);
 int launch_sort(tie_cuda_ctx *c, const int *row_expert, int n_rows, int n_tile, int first_expert, int n_expert,
 		const SortBufs &b);
+// dispatch.cu
+int launch_dispatch(tie_cuda_ctx *c, const float *x, const int *row_expert, int n_src, int n_out, int n_tile, bool sums, bool after_router);
 // stream.cu
 bool stream_supported(const Layer &L);
 int launch_stream_gate_up(tie_cuda_ctx *c, const Layer &L, const float *xin, int src_div, const int *row_expert,
@@ -52,8 +54,7 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 		   const int *pos = nullptr);
 int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, const int *perm, int src_div, int n_rows,
 		       float *rows_out, int *expert_out, int *inv);
-int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out, int n_src, int n_cols, __half *hi,
-		      __half *lo, __half *xq);
+int launch_split_rows(tie_cuda_ctx *c, const float *x, int n_src, int n_cols, __half *hi, __half *lo, __half *xq);
 int launch_swiglu(tie_cuda_ctx *c, float *gate, const float *up, int n);
 // tensor.cu
 int tc_setup(tie_cuda_ctx *c);

@@ -2,6 +2,7 @@
 // the fp16 hi/lo split of activations for the tensor-core path, and the table SwiGLU on its own.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "split8.cuh"
 
 namespace tie {
 
@@ -106,98 +107,24 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 	}
 }
 
-// Eight consecutive values v[0..7] (k = k0 .. k0+7, k0 a multiple of 8) as their fp16 hi and lo
-// halves (hi = rn16(v), lo = rn16(v - hi)) in the operand order [k0, k2, k1, k3] per group of 4, and the
-// sum over the 32-wide sub-block they belong to (four neighbouring lanes hold one), split the same way.
-struct Split8 {
-	uint4 hi, lo;
-	__half sum_hi, sum_lo;
-	__device__ __forceinline__ void make(const float v[8], bool sums)
-	{
-		uint32_t h[4], l[4];
-#pragma unroll
-		for (int g = 0; g < 2; g++) {
-			const float a = v[4 * g], b = v[4 * g + 1], c = v[4 * g + 2], d = v[4 * g + 3];
-			const __half2 h0 = __floats2half2_rn(a, c), h1 = __floats2half2_rn(b, d);
-			const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-			const __half2 l0 = __floats2half2_rn(a - f0.x, c - f0.y), l1 = __floats2half2_rn(b - f1.x, d - f1.y);
-			h[2 * g] = *reinterpret_cast<const uint32_t *>(&h0);
-			h[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&h1);
-			l[2 * g] = *reinterpret_cast<const uint32_t *>(&l0);
-			l[2 * g + 1] = *reinterpret_cast<const uint32_t *>(&l1);
-		}
-		hi = make_uint4(h[0], h[1], h[2], h[3]);
-		lo = make_uint4(l[0], l[1], l[2], l[3]);
-		if (sums) {
-			float sum = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
-			sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-			sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-			sum_hi = __float2half_rn(sum);
-			sum_lo = __float2half_rn(sum - __half2float(sum_hi));
-		}
-	}
-	__device__ __forceinline__ void store(int k0, __half *__restrict__ hi_row, __half *__restrict__ lo_row, __half *__restrict__ q_row,
-					      int lane) const
-	{
-		*reinterpret_cast<uint4 *>(hi_row + k0) = hi;
-		*reinterpret_cast<uint4 *>(lo_row + k0) = lo;
-		if (q_row && (lane & 3) == 0) {
-			q_row[xq_index(k0 >> 5)] = sum_hi;
-			q_row[xq_index(k0 >> 5) + 8] = sum_lo;
-		}
-	}
-};
-
 constexpr int ROWS_WARPS = 8;  // warps per CTA of the row passes: one row per warp at a time
 
-// Rows into expert-sorted order, each fp32 value v split into fp16 hi + lo
-// (hi = rn16(v), lo = rn16(v - hi)): hi+lo carries 22 significand bits, which the tensor-core
-// scheme needs to stay within the 1e-3 parity bound.  xq (optional, q_cols per row): the
-// sums of the row over its 32-wide sub-blocks, split the same way (the Q4_K "min" term).
-// Source row t is read and split once and stored at its n_out places inv[t * n_out ..] (< 0: none; inv null: row
-// t).  Bound by the stores: 4096 tokens to 8 experts each are 276 MB, 62 us when every place read its
-// row again.  A warp takes STEPS x 256 columns of a row, eight values per lane and step (16-byte loads and
+// The rows of a dense product's batch, split (Split8), and their sub-block sums (xq, optional, q_cols per row: the Q4_K
+// "min" term).  A warp takes STEPS x 256 columns of a row, eight values per lane and step (16-byte loads and
 // stores); n_cols must be a multiple of 256.
 template <int STEPS>
-__global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__restrict__ x, const int *__restrict__ inv, int n_out, int n_src,
-							      int n_cols, __half *__restrict__ hi, __half *__restrict__ lo,
-							      __half *__restrict__ xq, int q_cols)
+__global__ void __launch_bounds__(ROWS_WARPS * 32) split_rows(const float *__restrict__ x, int n_src, int n_cols, __half *__restrict__ hi,
+							      __half *__restrict__ lo, __half *__restrict__ xq, int q_cols)
 {
-	pdl_trigger();	// (a dense product, or one of narrow tiles, sets itself up meanwhile)
+	pdl_trigger();	// (the product sets itself up meanwhile)
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	const int upr = (n_cols + STEPS * 256 - 1) / (STEPS * 256);  // units per row
 	for (int un = blockIdx.x * ROWS_WARPS + warp; un < n_src * upr; un += gridDim.x * ROWS_WARPS) {
-		const int t = un / upr, k0 = (un - t * upr) * STEPS * 256 + lane * 8;
-		const float *xr = x + (size_t)t * n_cols;
-		int place = t;
-		if (inv && lane < n_out)
-			place = inv[(size_t)t * n_out + lane];
-		float4 v[STEPS][2];
-#pragma unroll
-		for (int i = 0; i < STEPS; i++) {
-			const int k = k0 + i * 256;
-			if (k < n_cols) {  // (uniform over the warp: n_cols is a multiple of 256)
-				v[i][0] = *reinterpret_cast<const float4 *>(xr + k);
-				v[i][1] = *reinterpret_cast<const float4 *>(xr + k + 4);
-			}
-		}
-		Split8 p[STEPS];
-#pragma unroll
-		for (int i = 0; i < STEPS; i++)
-			if (k0 + i * 256 < n_cols) {
-				const float f[8] = {v[i][0].x, v[i][0].y, v[i][0].z, v[i][0].w, v[i][1].x, v[i][1].y, v[i][1].z, v[i][1].w};
-				p[i].make(f, xq != nullptr);
-			}
-		for (int j = 0; j < n_out; j++) {
-			const int at = __shfl_sync(0xffffffffu, place, j);
-			if (at < 0)
-				continue;
-#pragma unroll
-			for (int i = 0; i < STEPS; i++)
-				if (k0 + i * 256 < n_cols)
-					p[i].store(k0 + i * 256, hi + (size_t)at * n_cols, lo + (size_t)at * n_cols,
-						   xq ? xq + (size_t)at * q_cols : nullptr, lane);
-		}
+		const int t = un / upr;
+		SplitUnit<STEPS> u;
+		u.load(x + (size_t)t * n_cols, (un - t * upr) * STEPS * 256 + lane * 8, n_cols);
+		u.split(xq != nullptr);
+		u.store(hi + (size_t)t * n_cols, lo + (size_t)t * n_cols, xq ? xq + (size_t)t * q_cols : nullptr, lane);
 	}
 }
 
@@ -254,10 +181,9 @@ int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_t
 	return TIE_CUDA_OK;
 }
 
-int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out, int n_src, int n_cols, __half *hi,
-		      __half *lo, __half *xq)
+int launch_split_rows(tie_cuda_ctx *c, const float *x, int n_src, int n_cols, __half *hi, __half *lo, __half *xq)
 {
-	if (n_cols % 256 || n_out > 32)
+	if (n_cols % 256)
 		return TIE_CUDA_ENOTSUP;
 	if (n_src <= 0)
 		return TIE_CUDA_OK;
@@ -266,7 +192,7 @@ int launch_split_rows(tie_cuda_ctx *c, const float *x, const int *inv, int n_out
 	const long long units = (long long)n_src * (wide ? (n_cols + 1023) / 1024 : n_cols / 256), cap = c->sm_count * 8;
 	const long long want = (units + ROWS_WARPS - 1) / ROWS_WARPS;
 	auto kern = wide ? split_rows<4> : split_rows<1>;
-	kern<<<(int)(want < cap ? want : cap), ROWS_WARPS * 32, 0, c->stream>>>(x, inv, n_out, n_src, n_cols, hi, lo, xq, xq_cols(n_cols));
+	kern<<<(int)(want < cap ? want : cap), ROWS_WARPS * 32, 0, c->stream>>>(x, n_src, n_cols, hi, lo, xq, xq_cols(n_cols));
 	TIE_CUDA_LAUNCHED(c);
 	return TIE_CUDA_OK;
 }

@@ -3,7 +3,8 @@
 //
 // The reference has no such step — it walks tokens one by one and fans the 8 selected experts
 // out to 8 pool threads (model_qwen3.c:415-456).  Here all (token, slot) rows are grouped by
-// expert so that each expert's weights are streamed once per call.
+// expert so that each expert's weights are streamed once per call.  (The grouped products sort and split their rows in one
+// launch, dispatch.cu; this sort serves the streaming kernels and the expert-parallel exchange.)
 //
 // The rows are cut into slices of SORT_SLICE rows, one CTA per slice, one row per thread; a warp
 // finds the rows of equal expert among its 32 (match_any) and every row is read twice:
