@@ -74,8 +74,9 @@ __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__res
 // beside them (wider loads move no more per cycle), so the tile grows with the batch (TIE_RT_TILES).  The
 // CTA that finishes a token tile last (a counter per tile, nobody waits) selects for all its tokens.
 // A small grid starts beside the kernel in front of it and fetches its first weights before it waits for the tokens.
-// Measured (logits + selection): 4 tokens 14.4 -> 8.8 us, 13 28.7 -> 10.3, 64 28.7 -> 12.3, 333 29 -> 26, 512 29 -> 26.7,
-// 1000 41 -> 37, 2000 68 -> 54, 4096 94 -> 93.
+// A copy's addresses are made once a call, not once a chunk (with the sums over the lanes below, an event on either side: 64
+// tokens 16.4 us as before, 512 30.7 -> 26.7, 1000 41.1 -> 37.2, 2000 59.4 -> 52, 4096 100.4 -> 92.2).  Two AVX2 lanes per thread
+// on packed multiply-adds, alone or with a loading warp in front, were equal or slower at every size.
 //
 // The hand-over of the tokens in an expert-parallel step rides along as one more row of CTAs, of
 // which as many work as there are SMs the logits' CTAs leave free (at least 16): CTAs that share an
@@ -97,7 +98,7 @@ struct RtCfg {
 	static constexpr int STAGES = 3, SMEM = STAGES * STAGE * (int)sizeof(float);
 	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : 8;
 	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte copies per thread and chunk
-	static_assert((TT + TE) * (KC / 4) % THREADS == 0 && TG % 2 == 0 && EG % 2 == 0 && KC % 32 == 0, "router tile");
+	static_assert(THREADS % (KC / 4) == 0 && TT % (THREADS / (KC / 4)) == 0 && (TT + TE) * (KC / 4) % THREADS == 0 && TG % 2 == 0 && EG % 2 == 0 && KC % 32 == 0, "router tile");
 };
 
 template <class C>
@@ -124,16 +125,22 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 	const int l = threadIdx.x & 7, g4 = threadIdx.x >> 5;
 	const int tg = ((threadIdx.x >> 3) & 1) + 2 * (g4 % (C::TG / 2)), eg = ((threadIdx.x >> 4) & 1) + 2 * (g4 / (C::TG / 2));
 	const int n_chunks = hidden / KC;
+	// what this thread copies of a chunk: 16 bytes of LD rows, ROWS apart; the addresses are made once
+	constexpr int ROWS = C::THREADS / (KC / 4);
+	const int row0 = threadIdx.x / (KC / 4), c4 = threadIdx.x % (KC / 4);
+	const float *src[C::LD];
+#pragma unroll
+	for (int j = 0; j < C::LD; j++)
+		src[j] = 4 * c4 + (j * ROWS < TT ? x + (size_t)min(t0 + row0 + j * ROWS, n_tokens - 1) * hidden  // (rows past the end: computed, dropped)
+						 : w + (size_t)(e0 + row0 + j * ROWS - TT) * hidden);
+	const uint32_t dst0 = ptx::smem_u32(rsm + row0 * C::PITCH + 4 * c4);
 	auto fetch = [&](int c, bool tokens, bool weights) {
 		if (c < n_chunks) {
+			const uint32_t dst = dst0 + (uint32_t)((c % C::STAGES) * C::STAGE) * 4u;
 #pragma unroll
-			for (int j = 0; j < C::LD; j++) {
-				const int i = threadIdx.x + C::THREADS * j, row = i / (KC / 4), c4 = i % (KC / 4);
-				const float *src = row < TT ? x + (size_t)min(t0 + row, n_tokens - 1) * hidden	// (rows past the end: computed, dropped)
-							    : w + (size_t)(e0 + row - TT) * hidden;
-				if (row < TT ? tokens : weights)
-					ptx::cp_async16(ptx::smem_u32(rsm + (c % C::STAGES) * C::STAGE + row * C::PITCH + 4 * c4), src + c * KC + 4 * c4);
-			}
+			for (int j = 0; j < C::LD; j++)
+				if (j * ROWS < TT ? tokens : weights)
+					ptx::cp_async16(dst + (uint32_t)(j * ROWS * C::PITCH) * 4u, src[j] + (size_t)c * KC);
 		}
 	};
 	float acc[TPT][EPT];
@@ -173,18 +180,40 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 					acc[j][b] = __fmaf_rn(xv[j], wv[b], acc[j][b]);
 		}
 	}
+	// hsum8_lanes of every (token, expert) of the 8 threads: ((l0 + l4) + (l1 + l5)) + ((l2 + l6) + (l3 + l7)).  A thread adds
+	// and passes on half of what it has per step, as far as that goes: 7/8 of a shuffle a chain instead of 3, and every thread
+	// stores (4096 tokens 100.4 -> 93.5 us, 512 30.7 -> 28.8).
+	constexpr int N = TPT * EPT;
+	float *v = &acc[0][0];
+	int at = 0;  // of the thread's sums in the flat order [j][b]
+	int left = N;
 #pragma unroll
-	for (int j = 0; j < TPT; j++) {
-		const int t = t0 + tg + C::TG * j;
+	for (int step = 0; step < 3; step++) {
+		const int bit = step == 0 ? 4 : (step == 1 ? 1 : 2);
+		if (left > 1) {
+			left /= 2;
+			const bool upper = l & bit;
+			at += upper ? left : 0;
 #pragma unroll
-		for (int b = 0; b < EPT; b++) {
-			const int e = e0 + eg + C::EG * b;
-			float v = hsum8_lanes(acc[j][b]);  // lanes l = 0..7 are 8 consecutive threads
-			if (l == 0 && t < n_tokens) {
-				if (bias)
-					v = __fadd_rn(v, bias[e]);
-				__stcg(logits + (size_t)t * n_expert + e, v);
-			}
+			for (int n = 0; n < N / 2; n++)
+				if (n < left) {
+					const float keep = upper ? v[left + n] : v[n], send = upper ? v[n] : v[left + n];
+					v[n] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, bit));
+				}
+		} else {
+			v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], bit));
+		}
+	}
+	constexpr int OUT = N >= 8 ? N / 8 : 1;
+#pragma unroll
+	for (int n = 0; n < OUT; n++) {
+		const int j = (at + n) / EPT, b = (at + n) % EPT, t = t0 + tg + C::TG * j, e = e0 + eg + C::EG * b;
+		// (fewer chains than threads: the first of those that have the same sum)
+		if (t < n_tokens && (N >= 8 || (N == 4 ? !(l & 2) : (N == 2 ? !(l & 3) : l == 0)))) {
+			float r = v[n];
+			if (bias)
+				r = __fadd_rn(r, bias[e]);
+			__stcg(logits + (size_t)t * n_expert + e, r);
 		}
 	}
 	__syncthreads();
@@ -272,13 +301,13 @@ __global__ void __launch_bounds__(128) router_topk(const float *__restrict__ log
 // operand load costs less per token, and more for the batch that leaves it half empty or one CTA over.
 #define TIE_RT_TILES(X)                            \
 	X(100, 820, RtCfg<8, 8, 64, 64, 64>)   \
-	X(70, 465, RtCfg<8, 4, 32, 64, 64>)    \
-	X(145, 223, RtCfg<4, 8, 16, 64, 64>)   \
-	X(105, 140, RtCfg<4, 4, 16, 32, 64>)   \
-	X(104, 101, RtCfg<2, 4, 16, 16, 256>)  \
-	X(85, 70, RtCfg<2, 2, 8, 16, 256>)     \
-	X(70, 53, RtCfg<1, 2, 8, 8, 512>)      \
-	X(65, 31, RtCfg<1, 1, 4, 4, 512>)
+	X(102, 410, RtCfg<8, 4, 32, 64, 64>)   \
+	X(155, 212, RtCfg<4, 8, 16, 64, 64>)   \
+	X(133, 130, RtCfg<4, 4, 16, 32, 64>)   \
+	X(123, 101, RtCfg<2, 4, 16, 16, 256>)  \
+	X(115, 69, RtCfg<2, 2, 8, 16, 256>)    \
+	X(110, 51, RtCfg<1, 2, 8, 8, 512>)     \
+	X(95, 28, RtCfg<1, 1, 4, 4, 512>)
 int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
 		  int *topk_idx, float *topk_w, int lfm2, const EpPush *push, bool *push_taken)
 {
