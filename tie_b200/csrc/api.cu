@@ -279,9 +279,9 @@ int run_experts(tie_cuda_ctx *c, const Layer &L, const float *x_src, int src_div
 	}
 	c->tc_no_pair = (flags & TIE_CUDA_PATH_NO_PAIR) != 0;
 	const int direct = (!use_tc && n_rows <= c->cfg.top_k && src_div == c->cfg.top_k) ? 1 : 0;
-	// tiles of 32 tokens where hardly any expert has more rows than that (the next tile would expand its
-	// weights again), else of 64
-	const int n_tile = n_rows <= 24 * c->n_local ? 32 : TC_TOKEN_TILE;
+	// tiles of 32 tokens up to 27 rows an expert on average, else of 64: experts of more rows expand their weights once more per
+	// tile, and wide tiles have fewer producers (25 rows an expert: 161 us with tiles of 32, 167 of 64; 28: equal; 32: 206 and 189)
+	const int n_tile = n_rows <= 27 * c->n_local ? 32 : TC_TOKEN_TILE;
 	c->last_direct_rows = direct ? n_rows : -1;
 	c->last_used_tc = use_tc;
 	if (!direct && !use_tc)

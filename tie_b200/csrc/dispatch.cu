@@ -43,7 +43,7 @@ dispatch_rows(const float *__restrict__ x, int n_cols, const int *__restrict__ r
 		(&hist[0][0])[tid] = 0;
 	__syncthreads();
 	pdl_wait();
-	pdl_trigger();	// (products of narrow tiles set themselves up meanwhile)
+	pdl_trigger();	// (the gate/up product sets itself up meanwhile)
 	constexpr int AHEAD = 8;
 	for (int r0 = warp * 32; r0 < n_rows; r0 += AHEAD * DISP_THREADS) {
 		int le[AHEAD];

@@ -467,7 +467,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			ptx::prefetch_tmap(&tw1);
 	}
 	if (GU)
-		pdl_trigger();	// (a down product of narrow tiles sets itself up as the SMs fall idle)
+		pdl_trigger();	// (the down product sets itself up as the SMs fall idle)
 	pdl_wait();  // what the kernels before this one wrote is visible from here on
 	if (threadIdx.x == 0)
 		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
@@ -1191,17 +1191,17 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	// least 4 super-blocks.  Measured at 64 / 512 / 4096 tokens: rows of 8 super-blocks (gate/up) 68 / 79 / 355 us
 	// paired, 70 / 92 / 410 single (a pair fetches half the token bytes per CTA); rows of 3 (down) 59 / 73 / 310
 	// paired, 55 / 70 / 294 single (the hand-offs between two SMs are not amortised over so few).
-	// set up beside the pass in front (a CTA needs a whole SM, so they come as SMs fall idle): dense products and narrow
-	// tiles, where a launch is 10 - 70 us (9 tokens 84.3 -> 82.3 us, 64 137.5 -> 135.4; 4096 equal or slower)
-	const bool dependent = dense_rows > 0 || NT == 32;
+	// Set up beside the kernel in front: a CTA needs a whole SM, so they come as SMs fall idle (9 tokens 84.3 -> 82.3 us, 64 137.5 ->
+	// 135.4; since no pass stands between the two products wide tiles gain too: a step of 400 / 512 / 4096 tokens 167.1 / 188.7 /
+	// 929 -> 164.8 / 183.5 / 926).
 	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles : 1 << 30;	// (known for a dense tensor: no idle CTAs)
 	if (c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K) {
-		return launch_kernel(c, dependent, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
+		return launch_kernel(c, true, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
 				     TcSmem<KIND, GU, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
 				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
 				     s.status, t0.rows, d, xqd, gu);
 	}
-	return launch_kernel(c, dependent, 1, grouped_gemm_sb<KIND, GU, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
+	return launch_kernel(c, true, 1, grouped_gemm_sb<KIND, GU, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
 			     TcSmem<KIND, GU, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
 			     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status,
 			     t0.rows, d, xqd, gu);
