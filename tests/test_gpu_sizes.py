@@ -212,6 +212,26 @@ def test_one_token_host_calls(be):
             assert np.array_equal(bits(out), bits(want.cpu().numpy()))
 
 
+# Up to some 70 tokens the router makes the RMSNorm of a block's tokens itself: the same bits as behind the norm kernel (what the
+# chain flag asks for), around the router's tiles of 4 and 8 tokens, rows of fewer float4 than its threads, and above its last size.
+@pytest.mark.parametrize("hidden", [512, 1536, 2048])
+@pytest.mark.parametrize("n_tokens", [2, 3, 4, 5, 8, 9, 31, 33, 63, 65, 90])
+def test_block_norm_inside_the_router(hidden, n_tokens, ref_silu_table):
+    import torch
+    from tie_b200 import moe
+    s = synth.MoeShape(hidden=hidden, n_expert=32, top_k=4, ffn_dim=256)
+    b = moe.MoeBackend(hidden=s.hidden, n_expert=s.n_expert, top_k=s.top_k, ffn_dim=s.ffn_dim, max_tokens=96, silu_table=ref_silu_table)
+    try:
+        b.upload_layer(0, synth.make_layer(40, s), ffn_norm_w=np.linspace(0.5, 1.5, s.hidden, dtype=np.float32))
+        h0 = torch.from_numpy(synth.make_x(8, n_tokens, s.hidden)).cuda()
+        want, got = h0.clone(), h0.clone()
+        b.moe_block_inplace_ptr(0, want, n_tokens, moe.DEVICE | moe.PATH_DECODE_CHAIN)
+        b.moe_block_inplace_ptr(0, got, n_tokens, moe.DEVICE)
+        assert np.array_equal(bits(got.cpu().numpy()), bits(want.cpu().numpy())) and not torch.equal(got, h0)
+    finally:
+        b.close()
+
+
 # RMSNorm of rows of one CTA each: hidden below, at and above what its threads keep in registers (2048).
 @pytest.mark.parametrize("hidden", [512, 2048, 2304])
 def test_rms_norm_row_lengths(hidden, port_lib, ref_silu_table):

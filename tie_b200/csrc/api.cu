@@ -324,13 +324,20 @@ bool one_kernel_step(tie_cuda_ctx *c, const Layer &L, int n_tokens, unsigned fla
 	       decode_fused_supported(c, L, n_tokens);
 }
 
+// normed: x is the residual stream, and the router makes its RMSNorm (router_norm_supported) into that buffer.
 int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_tokens, const float *bias_dev,
-		   const float *residual, unsigned flags, unsigned *host_status = nullptr)
+		   const float *residual, unsigned flags, unsigned *host_status = nullptr, float *normed = nullptr)
 {
 	Scratch &s = c->s;
 	const int lfm2 = (flags & TIE_CUDA_ROUTE_LFM2) ? 1 : 0;
+	auto route = [&]() {
+		const int rc = launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2, nullptr, nullptr, L.norm_w, normed);
+		if (normed)
+			x = normed;
+		return rc;
+	};
 	prof_mark(c, 0);
-	if (one_kernel_step(c, L, n_tokens, flags)) {
+	if (!normed && one_kernel_step(c, L, n_tokens, flags)) {
 		const int rc = launch_decode_fused(c, L, x, bias_dev, residual, out, host_status);
 		if (rc != TIE_CUDA_ENOTSUP) {  // (not supported after all: the chain below)
 			if (rc)
@@ -344,7 +351,7 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 	}
 	// small batches: router with fused selection, the rows of each expert together, combine
 	if ((flags & (TIE_CUDA_PATH_MASK | TIE_CUDA_PATH_LEGACY_STREAM)) == 0 && decode_group_supported(c, L, n_tokens)) {
-		TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
+		TRY(route());
 		prof_mark(c, 1);
 		c->last_used_tc = false;
 		c->last_direct_rows = n_tokens * c->cfg.top_k;
@@ -361,7 +368,7 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 	// decode: three launches — router with fused selection, gate/up, down + combine
 	if ((flags & TIE_CUDA_PATH_MASK) != TIE_CUDA_PATH_TENSOR && !(flags & TIE_CUDA_PATH_LEGACY_STREAM) &&
 	    decode_supported(c, L, n_tokens)) {
-		TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
+		TRY(route());
 		prof_mark(c, 1);
 		c->last_used_tc = false;
 		c->last_direct_rows = n_tokens * c->cfg.top_k;
@@ -374,13 +381,23 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 		prof_mark(c, 7);
 		return TIE_CUDA_OK;
 	}
-	TRY(launch_router(c, x, L.router_w, bias_dev, n_tokens, s.logits, s.topk_idx, s.topk_w, lfm2));
+	TRY(route());
 	prof_mark(c, 1);
 	const int *pos = nullptr;
 	TRY(run_experts(c, L, x, c->cfg.top_k, s.topk_idx, n_tokens * c->cfg.top_k, s.y, flags, &pos));
 	TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out, pos));
 	prof_mark(c, 7);
 	return TIE_CUDA_OK;
+}
+
+// RMSNorm -> FFN -> residual add on the stream, in place.
+int moe_block_device(tie_cuda_ctx *c, Layer &L, float *hidden, int n_tokens, unsigned flags)
+{
+	// (asked for the chain of kernels, the norm is one of them too)
+	if (!(flags & TIE_CUDA_PATH_DECODE_CHAIN) && router_norm_supported(c, n_tokens))
+		return moe_ffn_device(c, L, hidden, hidden, n_tokens, nullptr, hidden, flags, nullptr, c->s.x);
+	TRY(launch_rms_norm(c, hidden, L.norm_w, c->s.x, n_tokens));
+	return moe_ffn_device(c, L, c->s.x, hidden, n_tokens, nullptr, hidden, flags);
 }
 
 struct GraphKey {
@@ -1184,8 +1201,7 @@ int tie_cuda_moe_block_inplace(tie_cuda_ctx *c, int layer, float *hidden_dev, in
 				return rc;
 			}
 		}
-		TRY(launch_rms_norm(c, hidden_dev, L->norm_w, c->s.x, n_tokens));
-		return moe_ffn_device(c, *L, c->s.x, hidden_dev, n_tokens, nullptr, hidden_dev, flags);
+		return moe_block_device(c, *L, hidden_dev, n_tokens, flags);
 	}));
 	if (flags & TIE_CUDA_NO_SYNC)
 		return TIE_CUDA_OK;
@@ -1221,8 +1237,7 @@ int tie_cuda_moe_stack_inplace(tie_cuda_ctx *c, int first_layer, int n_layers, f
 					continue;
 				}
 			}
-			TRY(launch_rms_norm(c, hidden_dev, L.norm_w, c->s.x, n_tokens));
-			TRY(moe_ffn_device(c, L, c->s.x, hidden_dev, n_tokens, nullptr, hidden_dev, pflags));
+			TRY(moe_block_device(c, L, hidden_dev, n_tokens, pflags));
 		}
 		return TIE_CUDA_OK;
 	}));

@@ -7,7 +7,10 @@ namespace tie {
 // router.cu
 struct EpPush;
 int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
-		  int *topk_idx, float *topk_w, int lfm2 = 0, const EpPush *push = nullptr, bool *push_taken = nullptr);
+		  int *topk_idx, float *topk_w, int lfm2 = 0, const EpPush *push = nullptr, bool *push_taken = nullptr,
+		  const float *norm_w = nullptr, float *norm_out = nullptr);
+// norm_out: x is the residual stream, its RMSNorm (weights norm_w or null) goes there and is what is routed
+bool router_norm_supported(const tie_cuda_ctx *c, int n_tokens);
 int router_setup(tie_cuda_ctx *c);
 // decode.cu
 int decode_setup(tie_cuda_ctx *c);

@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(EPC * 8) router_logits_tile(const float *__res
 // which as many work as there are SMs the logits' CTAs leave free (at least 16): CTAs that share an
 // SM with the logits take load/store slots from them (32 working CTAs lengthened the kernel by 10 us
 // at 4 GPUs, 128 by 18 us).
+constexpr int RT_NORM_SMEM = 200 * 1024;
 constexpr int RT_PUSH_ROWS = 1;
 static int rt_push_ctas(const tie_cuda_ctx *c, int logits_ctas, int most)
 {
@@ -98,14 +99,25 @@ struct RtCfg {
 	static constexpr int STAGES = 3, SMEM = STAGES * STAGE * (int)sizeof(float);
 	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : 8;
 	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte copies per thread and chunk
+	// the form with the RMSNorm in front: whole rows in shared memory, and COLS float4 of each in a thread's registers
+	static constexpr bool NORM = TT <= 8 && KC == 512;
+	static constexpr int COLS = NORM ? 16 / TT : 0;
 	static_assert(THREADS % (KC / 4) == 0 && TT % (THREADS / (KC / 4)) == 0 && (TT + TE) * (KC / 4) % THREADS == 0 && TG % 2 == 0 && EG % 2 == 0 && KC % 32 == 0, "router tile");
 };
 
-template <class C>
-__global__ void __launch_bounds__(C::THREADS, C::THREADS >= 512 ? 1 : 2)
+// NORM: x is the residual stream; the CTA makes the RMSNorm of its tokens itself (rms_norm_rows, the same operations in the same
+// order) while the router weights arrive, and the CTAs of the first experts store it for the kernels behind.  A launch of
+// its own is 3.4 us of a block of 4 tokens (8 blocks of 4 tokens 366.1 -> 356.6 us, 4 of 13 356.1 -> 349.0).
+struct RtNorm {
+	const float *w = nullptr;  // or null: weight 1
+	float *out = nullptr;
+	float eps = 0.f;
+};
+template <class C, bool NORM>
+__global__ void __launch_bounds__(C::THREADS, C::THREADS >= 512 || NORM ? 1 : 2)
 router_batch(const float *__restrict__ x, const float *__restrict__ w, const float *__restrict__ bias, float *__restrict__ logits,
 	     int n_tokens, int hidden, int n_expert, int top_k, int *__restrict__ topk_idx, float *__restrict__ topk_w, int lfm2,
-	     const float *__restrict__ sel_bias, int *__restrict__ counter, const EpPush push)
+	     const float *__restrict__ sel_bias, int *__restrict__ counter, const EpPush push, const RtNorm norm)
 {
 	constexpr int TPT = C::TPT, EPT = C::EPT, TT = C::TT, TE = C::TE, KC = C::KC;
 	extern __shared__ __align__(16) float rsm[];
@@ -152,24 +164,80 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 #pragma unroll
 	for (int c = 0; c < C::STAGES - 1; c++)
 		fetch(c, false, true);
-	pdl_wait();	// the tokens may be the work of the kernel before this one
+	const int px = hidden + 8;	// NORM: pitch of the rows
+	float *rows = rsm + C::STAGES * C::STAGE;
+	if constexpr (NORM) {
+		__shared__ float s_inv[TT];
+		constexpr int COLS = C::COLS;
+		float4 v[TT][COLS], g[COLS];
+		auto col = [&](int k) { return threadIdx.x + k * C::THREADS; };
 #pragma unroll
-	for (int c = 0; c < C::STAGES - 1; c++) {
-		fetch(c, true, false);
-		ptx::cp_async_commit();
+		for (int k = 0; k < COLS; k++)
+			g[k] = norm.w && 4 * col(k) < hidden ? __ldg(reinterpret_cast<const float4 *>(norm.w) + col(k)) : make_float4(1.f, 1.f, 1.f, 1.f);
+		pdl_wait();
+#pragma unroll
+		for (int k = 0; k < COLS; k++)
+#pragma unroll
+			for (int j = 0; j < TT; j++)
+				if (4 * col(k) < hidden)
+					v[j][k] = reinterpret_cast<const float4 *>(x + (size_t)min(t0 + j, n_tokens - 1) * hidden)[col(k)];
+#pragma unroll
+		for (int k = 0; k < COLS; k++)
+#pragma unroll
+			for (int j = 0; j < TT; j++)
+				if (4 * col(k) < hidden)
+					*reinterpret_cast<float4 *>(rows + j * px + 4 * col(k)) = v[j][k];
+		__syncthreads();
+		if (threadIdx.x < 8 * TT) {  // a thread per lane of a row's sum of squares
+			const float *r = rows + (threadIdx.x >> 3) * px + (threadIdx.x & 7);
+			float a = 0.f;
+#pragma unroll 32
+			for (int i = 0; i < hidden / 8; i++)
+				a = __fmaf_rn(r[8 * i], r[8 * i], a);
+			const float ss = hsum8_lanes(a);
+			if ((threadIdx.x & 7) == 0)
+				s_inv[threadIdx.x >> 3] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)hidden), norm.eps)));
+		}
+		__syncthreads();
+#pragma unroll
+		for (int j = 0; j < TT; j++) {
+			const float inv = s_inv[j];
+#pragma unroll
+			for (int k = 0; k < COLS; k++)
+				if (4 * col(k) < hidden) {
+					const float4 a = v[j][k], b = g[k];
+					const float4 o = make_float4(__fmul_rn(__fmul_rn(a.x, b.x), inv), __fmul_rn(__fmul_rn(a.y, b.y), inv),
+								     __fmul_rn(__fmul_rn(a.z, b.z), inv), __fmul_rn(__fmul_rn(a.w, b.w), inv));
+					*reinterpret_cast<float4 *>(rows + j * px + 4 * col(k)) = o;
+					if (blockIdx.y == 0 && t0 + j < n_tokens)
+						reinterpret_cast<float4 *>(norm.out + (size_t)(t0 + j) * hidden)[col(k)] = o;
+				}
+		}
+#pragma unroll
+		for (int c = 0; c < C::STAGES - 1; c++)
+			ptx::cp_async_commit();  // (all the weights asked for so far are in the first group)
+	} else {
+		pdl_wait();	// the tokens may be the work of the kernel before this one
+#pragma unroll
+		for (int c = 0; c < C::STAGES - 1; c++) {
+			fetch(c, true, false);
+			ptx::cp_async_commit();
+		}
 	}
 	for (int c = 0; c < n_chunks; c++) {
 		ptx::cp_async_wait<C::STAGES - 2>();
 		__syncthreads();  // (chunk c is here for everyone, and everyone is done with the buffer of chunk c - 1)
-		fetch(c + C::STAGES - 1, true, true);
+		fetch(c + C::STAGES - 1, !NORM, true);
 		ptx::cp_async_commit();	 // (an empty group past the end)
-		const float *buf = rsm + (c % C::STAGES) * C::STAGE + l, *xs = buf + tg * C::PITCH, *ws = buf + (TT + eg) * C::PITCH;
+		const float *buf = rsm + (c % C::STAGES) * C::STAGE + l, *ws = buf + (TT + eg) * C::PITCH;
+		const float *xs = NORM ? rows + l + tg * px + c * KC : buf + tg * C::PITCH;
+		const int xpitch = NORM ? px : C::PITCH;
 #pragma unroll C::UNROLL
 		for (int g = 0; g < KC / 8; g++) {
 			float xv[TPT], wv[EPT];
 #pragma unroll
 			for (int j = 0; j < TPT; j++)
-				xv[j] = xs[C::TG * j * C::PITCH + 8 * g];
+				xv[j] = xs[C::TG * j * xpitch + 8 * g];
 #pragma unroll
 			for (int b = 0; b < EPT; b++)
 				wv[b] = ws[C::EG * b * C::PITCH + 8 * g];
@@ -308,18 +376,9 @@ __global__ void __launch_bounds__(128) router_topk(const float *__restrict__ log
 	X(115, 69, RtCfg<2, 2, 8, 16, 256>)    \
 	X(110, 51, RtCfg<1, 2, 8, 8, 512>)     \
 	X(95, 28, RtCfg<1, 1, 4, 4, 512>)
-int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
-		  int *topk_idx, float *topk_w, int lfm2, const EpPush *push, bool *push_taken)
+static int pick_tile(const tie_cuda_ctx *c, int n_tokens)
 {
-	const int H = c->cfg.hidden, E = c->cfg.n_expert, K = c->cfg.top_k;
-	EpPush f = {};
-	if (push)
-		f = *push;
-	if (push_taken)
-		*push_taken = push != nullptr;
-	const float *sel_bias = lfm2 ? bias : nullptr;
-	if (lfm2)
-		bias = nullptr;
+	const int H = c->cfg.hidden, E = c->cfg.n_expert;
 	int pick = -1, at = 0;
 	long long best = 0;
 #define TIE_RT_PICK(A, B, ...)                                                                             \
@@ -335,9 +394,45 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 	}
 	TIE_RT_TILES(TIE_RT_PICK)
 #undef TIE_RT_PICK
+	return pick;
+}
+
+// Can the router's kernel for this batch make the RMSNorm too?  (Small tiles: each CTA makes all of its tokens'.)
+bool router_norm_supported(const tie_cuda_ctx *c, int n_tokens)
+{
+	const int H = c->cfg.hidden, pick = pick_tile(c, n_tokens);
+	int at = 0;
+	bool ok = false;
+#define TIE_RT_NORM(A, B, ...)                                                                                              \
+	if (at++ == pick) {                                                                                                 \
+		using C = __VA_ARGS__;                                                                                      \
+		ok = C::NORM && H / 4 <= C::COLS * C::THREADS && C::SMEM + C::TT * (H + 8) * sizeof(float) <= RT_NORM_SMEM; \
+	}
+	TIE_RT_TILES(TIE_RT_NORM)
+#undef TIE_RT_NORM
+	return ok;
+}
+
+int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *bias, int n_tokens, float *logits,
+		  int *topk_idx, float *topk_w, int lfm2, const EpPush *push, bool *push_taken, const float *norm_w, float *norm_out)
+{
+	const int H = c->cfg.hidden, E = c->cfg.n_expert, K = c->cfg.top_k;
+	EpPush f = {};
+	if (push)
+		f = *push;
+	if (push_taken)
+		*push_taken = push != nullptr;
+	const float *sel_bias = lfm2 ? bias : nullptr;
+	if (lfm2)
+		bias = nullptr;
+	const int pick = pick_tile(c, n_tokens);
 	if (pick < 0)
 		return TIE_CUDA_ENOTSUP;
-	at = 0;
+	int at = 0;
+	RtNorm norm;
+	norm.w = norm_w;
+	norm.out = norm_out;
+	norm.eps = c->cfg.norm_eps;
 	// (dependent where it is one wave: a grid that waits beside its predecessor then takes nothing from it)
 	int rc = TIE_CUDA_OK;
 #define TIE_RT_RUN(A, B, ...)                                                                                              \
@@ -345,8 +440,16 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 		using C = __VA_ARGS__;                                                                                     \
 		dim3 grid((n_tokens + C::TT - 1) / C::TT, E / C::TE + (push ? RT_PUSH_ROWS : 0));                          \
 		f.n_ctas = rt_push_ctas(c, grid.x * (E / C::TE), grid.x * RT_PUSH_ROWS);                                   \
-		rc = launch_kernel(c, (int)(grid.x * grid.y) <= c->sm_count, 1, router_batch<C>, grid, C::THREADS, C::SMEM, \
-				   x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, lfm2, sel_bias, c->s.route_counter, f); \
+		const bool dependent = (int)(grid.x * grid.y) <= c->sm_count;                                              \
+		auto run = [&](auto kern, size_t smem) {                                                                   \
+			return launch_kernel(c, dependent, 1, kern, grid, C::THREADS, smem, x, w, bias, logits, n_tokens, H, E, K, topk_idx, topk_w, \
+					     lfm2, sel_bias, c->s.route_counter, f, norm);                                 \
+		};                                                                                                         \
+		if constexpr (C::NORM)                                                                                     \
+			rc = norm_out ? run(router_batch<C, true>, C::SMEM + C::TT * (H + 8) * sizeof(float))               \
+				      : run(router_batch<C, false>, C::SMEM);                                               \
+		else                                                                                                       \
+			rc = norm_out ? TIE_CUDA_EINVAL : run(router_batch<C, false>, C::SMEM);                            \
 	}
 	TIE_RT_TILES(TIE_RT_RUN)
 #undef TIE_RT_RUN
@@ -357,8 +460,13 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 int router_setup(tie_cuda_ctx *c)
 {
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_logits_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-#define TIE_RT_ATTR(A, B, ...) \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<__VA_ARGS__>, cudaFuncAttributeMaxDynamicSharedMemorySize, __VA_ARGS__::SMEM));
+#define TIE_RT_ATTR(A, B, ...)                                                                                                               \
+	{                                                                                                                                    \
+		using C = __VA_ARGS__;                                                                                                       \
+		TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));         \
+		if constexpr (C::NORM)                                                                                                       \
+			TIE_CUDA_TRY(c, cudaFuncSetAttribute(router_batch<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_NORM_SMEM)); \
+	}
 	TIE_RT_TILES(TIE_RT_ATTR)
 #undef TIE_RT_ATTR
 	return TIE_CUDA_OK;
