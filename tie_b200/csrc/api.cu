@@ -361,7 +361,7 @@ int moe_ffn_device(tie_cuda_ctx *c, Layer &L, const float *x, float *out, int n_
 		prof_mark(c, 4);
 		TRY(launch_group_down(c, L, n_tokens, s.y));
 		prof_mark(c, 6);
-		TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out));
+		TRY(launch_combine(c, s.y, s.topk_w, n_tokens, residual, out, nullptr, true));
 		prof_mark(c, 7);
 		return TIE_CUDA_OK;
 	}

@@ -54,7 +54,7 @@ int launch_stream_matvec(tie_cuda_ctx *c, const uint8_t *wexp, WKind kind, int k
 // misc.cu
 int launch_rms_norm(tie_cuda_ctx *c, const float *x, const float *w, float *o, int n_tokens);
 int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_tokens, const float *residual, float *out,
-		   const int *pos = nullptr);
+		   const int *pos = nullptr, bool dependent = false);
 int launch_gather_rows(tie_cuda_ctx *c, const float *x, const int *row_expert, const int *perm, int src_div, int n_rows,
 		       float *rows_out, int *expert_out, int *inv);
 int launch_split_rows(tie_cuda_ctx *c, const float *x, int n_src, int n_cols, __half *hi, __half *lo, __half *xq);

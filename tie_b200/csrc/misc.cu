@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(256) combine_rows(const float *__restrict__ y,
 						    const int *__restrict__ pos)
 {
 	const int t = blockIdx.x;
+	pdl_wait();
 	float wj[MAX_TOP_K];
 	size_t yrow[MAX_TOP_K];
 #pragma unroll
@@ -174,11 +175,9 @@ int launch_rms_norm(tie_cuda_ctx *c, const float *x, const float *w, float *o, i
 }
 
 int launch_combine(tie_cuda_ctx *c, const float *y, const float *topk_w, int n_tokens, const float *residual, float *out,
-		   const int *pos)
+		   const int *pos, bool dependent)
 {
-	combine_rows<<<n_tokens, 256, 0, c->stream>>>(y, topk_w, c->cfg.top_k, c->cfg.hidden, residual, out, pos);
-	TIE_CUDA_LAUNCHED(c);
-	return TIE_CUDA_OK;
+	return launch_kernel(c, dependent, 1, combine_rows, dim3(n_tokens), 256, 0, y, topk_w, c->cfg.top_k, c->cfg.hidden, residual, out, pos);
 }
 
 int launch_split_rows(tie_cuda_ctx *c, const float *x, int n_src, int n_cols, __half *hi, __half *lo, __half *xq)
