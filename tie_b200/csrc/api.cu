@@ -71,7 +71,7 @@ int alloc_scratch(tie_cuda_ctx *c)
 	s.sort_hist_cap = ((R + SORT_SLICE - 1) / SORT_SLICE + 1) * E;
 	TRY(dev_alloc(c, &s.sort_hist, s.sort_hist_cap));
 	TRY(dev_alloc(c, &s.h, R * F));
-	TRY(dev_alloc(c, &s.y, R * H));
+	TRY(dev_alloc(c, &s.y, R * (H > 2 * F ? H : 2 * F)));  // (tie_cuda_mat_mat on host buffers counts on as much)
 	// hi and lo halves of each split array share one allocation (lo right behind hi): one 3-D TMA box fetches both
 	TRY(dev_alloc(c, &s.xs_hi, 2 * s.rows_pad * H));
 	s.xs_lo = s.xs_hi + s.rows_pad * H;
