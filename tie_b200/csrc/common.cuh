@@ -19,6 +19,7 @@ constexpr int Q6K_BYTES = 210;	  // sizeof(block_q6_k), gguf.h:101-106
 constexpr int MAX_TOP_K = 8;
 constexpr int TC_TOKEN_TILE = 64;  // rows of one expert per token tile of the tensor-core path (or 32: run_experts)
 constexpr int SILU_N = TIE_CUDA_SILU_TABLE_SIZE;
+constexpr int TC_MAX_PARTS = 8;	  // parts that a dense product's rows are split into, at most
 constexpr int SORT_SLICE = 256;   // rows per CTA of the dispatch sort
 constexpr int OUT_PAD = 64;	  // floats in front of the output rows: the status word is the last of them
 constexpr int COPY_CHUNKS = 16;	  // pageable host batches are copied in at most this many chunks
@@ -188,6 +189,7 @@ struct tie_cuda_ctx {
 	CUtensorMap tmap[12];
 	CUtensorMap tmap_half[12];  // the same with boxes of half the rows: what a CTA of a pair fetches
 	bool tmaps_ok = false;
+	int tc_clusters[tie::TC_MAX_PARTS + 1] = {0};  // clusters of n CTAs of the grouped product the device holds at once
 	int tc_pairs = 0;	    // CTA pairs the device holds at once (0: the pair kernels are not used)
 	bool tc_no_pair = false;    // this call asked for the single-CTA grouped GEMM (TIE_CUDA_PATH_NO_PAIR)
 	// host registry for dispatch rows

@@ -259,6 +259,19 @@ __device__ __forceinline__ void cluster_sync_all()
 {
 	asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same shared-memory address in CTA `rank` of the cluster, and 16 bytes from such an address.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t local_smem_addr, uint32_t rank)
+{
+	uint32_t r;
+	asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
+	return r;
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t cluster_smem_addr)
+{
+	float4 v;
+	asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(cluster_smem_addr) : "memory");
+	return v;
+}
 // The shared::cluster address of the same variable in the leader CTA of the pair (for the leader: its own).
 __device__ __forceinline__ uint32_t leader_addr(uint32_t local_smem_addr)
 {

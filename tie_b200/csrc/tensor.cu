@@ -191,6 +191,7 @@ struct TcItem {
 	int le, row0, n_valid, n_mma;  // n_mma: n_valid rounded up to 16, the N of the MMAs
 	int box;	  // 0, 1, 2: the tile's token boxes hold 16, 32 or 64 rows (half of that per CTA of a pair)
 	int m0;	      // first row of the matrix
+	int part;     // SPLIT: which part of the rows' super-blocks (else 0)
 };
 
 // The first TC_ITEMS work items of a CTA are decoded into shared memory when the kernel starts, all at
@@ -199,20 +200,28 @@ struct TcItem {
 constexpr int TC_ITEMS = 128;
 // m_items: work items per token tile (128-row tiles, or pairs of them); a CTA of a pair takes the
 // tile 2 * item + its rank.  tile_rows: rows of the matrix a tile takes.  Packed: expert, first row, rows, first weight row.
-template <bool PAIR, int NT>
-__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int tile_rows, uint32_t rank)
+// SPLIT (dense only): n_parts neighbouring items are the parts of one tile; the part stands in place of the expert.
+template <bool PAIR, int NT, bool SPLIT>
+__device__ __forceinline__ int4 tc_decode(int t, int m_items, const int4 *__restrict__ tile_info, int n_rows, int tile_rows, uint32_t rank,
+					  int n_parts)
 {
+	int part = 0;
+	if (SPLIT) {
+		part = t % n_parts;
+		t /= n_parts;
+	}
 	const int slot = t / m_items, mi = t - slot * m_items;
 	const int4 ti = tile_info ? __ldg(tile_info + slot) : make_int4(0, slot * NT, min(NT, n_rows - slot * NT), 0);
-	return make_int4(ti.x, ti.y, ti.z, (PAIR ? 2 * mi + (int)rank : mi) * tile_rows);
+	return make_int4(SPLIT ? part : ti.x, ti.y, ti.z, (PAIR ? 2 * mi + (int)rank : mi) * tile_rows);
 }
-template <bool PAIR, int NT>
+template <bool PAIR, int NT, bool SPLIT>
 __device__ __forceinline__ TcItem tc_item(int t, int tl, const int4 *s_items, int m_items, const int4 *__restrict__ tile_info,
-					  int n_rows, int tile_rows, uint32_t rank)
+					  int n_rows, int tile_rows, uint32_t rank, int n_parts)
 {
-	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR, NT>(t, m_items, tile_info, n_rows, tile_rows, rank);
+	const int4 ti = tl < TC_ITEMS ? s_items[tl] : tc_decode<PAIR, NT, SPLIT>(t, m_items, tile_info, n_rows, tile_rows, rank, n_parts);
 	TcItem it;
-	it.le = ti.x;
+	it.le = SPLIT ? 0 : ti.x;
+	it.part = SPLIT ? ti.x : 0;
 	it.row0 = ti.y;
 	it.n_valid = ti.z;
 	it.n_mma = (ti.z + 15) & ~15;
@@ -369,7 +378,11 @@ struct GuOut {
 	int sum_cols = 0;
 	const float *silu = nullptr;
 };
-template <WKind KIND, bool GU, bool PEER = false, bool PAIR = false, int NT = TC_TOKEN_TILE>
+// SPLIT: a dense product whose tiles leave most of the device idle (2048 -> 512 of 37 tokens: 8 tiles) divides the super-blocks of a
+// row among the n_parts CTAs of a cluster, one work item each.  They leave their sums in shared memory, and each adds up its
+// share of the tile's tokens from all of them, in the order of the parts.  (Through global memory, the last to come adding
+// up, 37 tokens took 27 us instead of 15.)
+template <WKind KIND, bool GU, bool PEER = false, bool PAIR = false, int NT = TC_TOKEN_TILE, bool SPLIT = false>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1,
 		const __grid_constant__ CUtensorMap tm2, const __grid_constant__ CUtensorMap tq0,
@@ -378,8 +391,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		const uint8_t *__restrict__ w1, size_t expert_stride, int k_dim, const int4 *__restrict__ tile_info,
 		const int *__restrict__ tile_start, int n_local, int m_tiles, float *__restrict__ y, const int *__restrict__ perm,
 		int out_stride, float out_scale, unsigned *__restrict__ status, int rows_per_matrix, const EpDst dst,
-		const int xq_depth, const GuOut gu)
+		const int xq_depth, const GuOut gu, const int n_parts)
 {
+	static_assert(!SPLIT || (!GU && !PEER && !PAIR), "parts of plain products only");
 	static_assert(!(GU && PEER), "peer destinations exist for the down product only");
 	using Sm = TcSmem<KIND, GU, PAIR, NT>;
 	constexpr int TILE_ROWS = GU ? TC_BM / 2 : TC_BM;  // of a matrix
@@ -399,7 +413,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	const int walker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
 	const int stride_t = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
 	const int m_items = PAIR ? m_tiles / 2 : m_tiles;
-	const int nb = k_dim / QK_K;
+	const int nb = k_dim / QK_K, nbl = SPLIT ? nb / n_parts : nb;  // super-blocks of a row, and of a work item
 
 	const uint32_t raw = ptx::smem_u32(smem_raw);
 	const uint32_t tiles = (raw + 1023u) & ~1023u;
@@ -470,14 +484,14 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		pdl_trigger();	// (the down product sets itself up as the SMs fall idle)
 	pdl_wait();  // what the kernels before this one wrote is visible from here on
 	if (threadIdx.x == 0)
-		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items;
+		s_total = (*(volatile unsigned *)status & ST_WAIT_TIMEOUT) ? 0 : (tile_info ? tile_start[n_local] : (n_local + NT - 1) / NT) * m_items * (SPLIT ? n_parts : 1);
 	ptx::tc_fence_before();
 	__syncthreads();
 	const int total = s_total;  // (a CTA without work items goes through the motions: it holds tensor memory, its peer waits for it)
 	if (threadIdx.x < TC_ITEMS) {
 		const int t = walker + threadIdx.x * stride_t;
 		if (t < total)
-			s_items[threadIdx.x] = tc_decode<PAIR, NT>(t, m_items, tile_info, n_local, TILE_ROWS, rank);
+			s_items[threadIdx.x] = tc_decode<PAIR, NT, SPLIT>(t, m_items, tile_info, n_local, TILE_ROWS, rank, n_parts);
 	}
 	__syncthreads();
 	if (PAIR)
@@ -505,7 +519,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		// (GU: lanes 0 - 15 of a warp take rows of the gate box, 16 - 31 the same rows of the up box behind it)
 		const int wrow = GU ? ((row & 16) << 2) + ((row >> 5) << 4) + (row & 15) : row;
 		const uint32_t slot0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Cols::A + UNIT * (STEP == 2 ? grp : half);
-		const uint32_t n_sb = walker < total ? (uint32_t)((total - 1 - walker) / stride_t + 1) * (uint32_t)nb : 0u;
+		const uint32_t n_sb = walker < total ? (uint32_t)((total - 1 - walker) / stride_t + 1) * (uint32_t)nbl : 0u;
 		bool alive = true;
 		for (uint32_t n = STEP == 2 ? grp >> 1 : 0; n < n_sb; n += STEP) {
 			const uint32_t wb = n % Sm::NWB, slot = slot0 + (STEP == 1 ? 2 * UNIT * (n & 1u) : 0u);
@@ -572,10 +586,10 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		int dtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, dtl++) {
 			if (Roles::NSETS == 2 && (dtl & 1) != set) {  // the other set's item
-				n += nb;
+				n += nbl;
 				continue;
 			}
-			const TcItem item = tc_item<PAIR, NT>(t, dtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
+			const TcItem item = tc_item<PAIR, NT, SPLIT>(t, dtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank, n_parts);
 			const int mrow = item.m0 + (GU ? quad * 16 + (lane & 15) : lrow);
 			// tokens of this warp: the whole tile, or half of it (the first or the second by part).
 			// Where twice the columns fit an accumulator, the hi and lo products have columns of their own (one MMA
@@ -636,17 +650,18 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				}
 			};
 			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead; times 16, which the operand lacks
+			const int sb0 = item.part * nbl;
 			const uint8_t *grp = nullptr;
 			float dnext = 0.0f;
 			if (!Q4) {
 				grp = (upper ? w1 : w0) + (size_t)item.le * expert_stride + (size_t)(mrow >> 3) * q6k_r8_group_bytes(nb);
-				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, 0))));
+				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sb0))));
 			}
-			for (int sbi = 0; sbi < nb; sbi++, n++) {
+			for (int sbi = 0; sbi < nbl; sbi++, n++) {
 				float scale = (GU ? 16.0f : 16.0f * out_scale) * dnext;
-				if (!Q4 && sbi + 1 < nb)
+				if (!Q4 && sbi + 1 < nbl)
 					dnext = half_bits_to_float(
-						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sbi + 1))));
+						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sb0 + sbi + 1))));
 				const uint32_t buf = n % NBUF;
 				if (!tc_wait_warp(ptx::smem_u32(Roles::NSETS == 2 ? &sh->pfull[set][buf] : &sh->done[n % TC_DONE]),
 						  Roles::NSETS == 2 ? (pph >> buf) & 1u : (n / TC_DONE) & 1u, abort_flag, status, lane)) {
@@ -743,20 +758,22 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			// (in sorted order a tile's stores go to neighbouring rows: scattered to the rows' own places, 8 KB apart in 268 MB
 			// at 4096 tokens, the down product took 238 us there instead of 217, 61 instead of 55 at 512)
 			if (!PEER && !perm) {
-				float *yr = y + (size_t)p0 * out_stride + mrow;
+				// (SPLIT: [token][128 rows] in the token ring, which the item's MMAs are done with)
+				float *yr = SPLIT ? reinterpret_cast<float *>(smem) + tok0 * TC_BM + lrow : y + (size_t)p0 * out_stride + mrow;
+				const unsigned ystep = SPLIT ? TC_BM : out_stride;
 #pragma unroll
 				for (int j0 = 0; j0 < 32; j0 += 8) {
 					if (j0 + 8 <= n_rows) {
 #pragma unroll
 						for (int j = 0; j < 8; j++)
-							yr[(size_t)(unsigned)j * (unsigned)out_stride] = acc[j0 + j];
+							yr[(size_t)(unsigned)j * ystep] = acc[j0 + j];
 					} else {
 #pragma unroll
 						for (int j = 0; j < 8; j++)
 							if (j0 + j < n_rows)
-								yr[(size_t)(unsigned)j * (unsigned)out_stride] = acc[j0 + j];
+								yr[(size_t)(unsigned)j * ystep] = acc[j0 + j];
 					}
-					yr += 8 * (size_t)out_stride;
+					yr += 8 * (size_t)ystep;
 					asm volatile("" ::: "memory");	// (the addresses of eight rows at a time: hoisted together they spill)
 				}
 			} else {
@@ -801,7 +818,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				alive = alive && tc_wait(bar, parity, abort_flag, status);
 			};
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
+				const TcItem item = tc_item<PAIR, NT, SPLIT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank, n_parts);
 				const uint32_t idesc = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, item.n_mma);
 				const uint32_t idesc2 = ptx::umma_idesc_f16(PAIR ? 2 * TC_BM : TC_BM, 2 * item.n_mma);
 				const uint32_t lo_off = (uint32_t)((PAIR ? 8 : 16) << item.box) * 128u;
@@ -809,7 +826,8 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				// hi rows and one MMA of twice the columns takes both
 				const bool stacked = 2 * item.n_mma <= NT;
 				const uint32_t dset = Roles::NSETS == 2 ? tl & 1u : 0u, mset = Cols::NM == 2 ? dset : 0u;  // the set of drain warps that takes the item, its min sums
-				for (int sbi = 0; sbi < nb; sbi++, n++) {
+				for (int sbi = 0; sbi < nbl; sbi++, n++) {
+					const int g = item.part * nbl + sbi;  // of the row
 					const uint32_t buf = n % NBUF, j0 = 2u * (n & 1u);
 					const uint32_t q = n & (Ring::GROUPS - 1);
 					const uint32_t fb = ptx::smem_u32(&sh->bfull[q]), fu = ptx::smem_u32(&sh->full[n & 1u]), pe = ptx::smem_u32(&sh->pempty[buf]);
@@ -824,7 +842,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					}
 					ptx::tc_fence_after();
 					const uint32_t dP = tmem + NT * buf, bt = b_group(q);
-					const uint32_t xs = ptx::umma_desc_lo(xq_buf(xs_n & 1u) + (uint32_t)((sbi >> 2) & 1) * lo_off) + 2u * (sbi & 3);
+					const uint32_t xs = ptx::umma_desc_lo(xq_buf(xs_n & 1u) + (uint32_t)((g >> 2) & 1) * lo_off) + 2u * (g & 3);
 					auto stages = [&](auto both) {
 						auto a_of = [&](int q4) { return tmem + Cols::A + UNIT * (j0 + (q4 >> 1)) + 32u * (q4 & 1); };
 						auto b_of = [&](int q4) { return ptx::umma_desc_lo(bt + q4 * 2u * lo_off); };
@@ -861,7 +879,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						const uint32_t dM = tmem + Cols::M + NT * mset, aM = tmem + Cols::A + UNIT * j0 + 64u;
 						mma(dM, aM, xs, idesc, sbi > 0 ? 1u : 0u);
 						mma(dM, aM + UNIT, xs, idesc, 1u);
-						if ((sbi & 7) == 7 || sbi == nb - 1)
+						if ((g & 7) == 7 || sbi == nbl - 1)
 							xs_n++;
 					}
 					commit(&sh->done[n % TC_DONE]);
@@ -880,7 +898,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 			uint32_t tl = 0, n = 0, xs_n = 0, x_end = 0;  // x_end: where the segment of sums before the current one ended
 			bool alive = true;
 			for (int t = walker; t < total && alive; t += stride_t, tl++) {
-				const TcItem item = tc_item<PAIR, NT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
+				const TcItem item = tc_item<PAIR, NT, SPLIT>(t, (int)tl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank, n_parts);
 				// one box per super-block: four stages of 64 k x (hi, lo) x the CTA's token rows.  The CTAs of a pair
 				// take the first and the second half of the tile's n_mma columns; all the bytes are counted on
 				// the leader's barrier, whose token loader announces them.
@@ -890,7 +908,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				auto wait_done = [&](uint32_t m) {
 					return tc_wait<100>(ptx::smem_u32(&sh->done[m % TC_DONE]), (m / TC_DONE) & 1u, abort_flag, status);
 				};
-				for (int sbi = 0; sbi < nb; sbi++, n++) {
+				for (int sbi = 0; sbi < nbl; sbi++, n++) {
+					const int g = item.part * nbl + sbi;
+					const bool sums = Q4 && (sbi == 0 || (g & 7) == 0);
 					const uint32_t q = n & (Ring::GROUPS - 1);
 					if (n >= (uint32_t)Ring::GROUPS && !wait_done(n - Ring::GROUPS)) {
 						alive = false;
@@ -898,7 +918,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					}
 					const uint32_t fb = ptx::smem_u32(&sh->bfull[q]);
 					uint32_t bytes = 2u * TC_SPB * row_bytes;
-					if (Q4 && (sbi & 7) == 0) {
+					if (sums) {
 						// a segment of the sub-block sums comes with its first super-block (two buffers; the segment before the
 						// last one is over with the super-block in front of x_end, of which the wait above may have told)
 						if (xs_n >= 2u && x_end + Ring::GROUPS > n + 1u && !wait_done(x_end - 1u)) {
@@ -910,19 +930,19 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 					}
 					if (rank == 0)
 						ptx::mbar_arrive_expect_tx(fb, bytes);
-					if (Q4 && (sbi & 7) == 0) {
+					if (sums) {
 						const uint32_t xi = xs_n & 1u;
 						const CUtensorMap *tqp = item.box == 0 ? &tq0 : (item.box == 1 ? &tq1 : &tq2);
 						if (PAIR)
-							ptx::tma_load_3d_pair(xq_buf(xi), tqp, fb, 0, row0, sbi >> 2);
+							ptx::tma_load_3d_pair(xq_buf(xi), tqp, fb, 0, row0, (g >> 3) * 2);
 						else
-							ptx::tma_load_3d(xq_buf(xi), tqp, fb, 0, row0, sbi >> 2);
+							ptx::tma_load_3d(xq_buf(xi), tqp, fb, 0, row0, (g >> 3) * 2);
 						xs_n++;
 					}
 					if (PAIR)
-						ptx::tma_load_4d_pair(b_group(q), tmp, fb, 0, row0, 0, sbi * TC_SPB);
+						ptx::tma_load_4d_pair(b_group(q), tmp, fb, 0, row0, 0, g * TC_SPB);
 					else
-						ptx::tma_load_4d(b_group(q), tmp, fb, 0, row0, 0, sbi * TC_SPB);
+						ptx::tma_load_4d(b_group(q), tmp, fb, 0, row0, 0, g * TC_SPB);
 				}
 			}
 		}
@@ -933,8 +953,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		bool alive = true;
 		int wtl = 0;
 		for (int t = walker; t < total && alive; t += stride_t, wtl++) {
-			const TcItem item = tc_item<PAIR, NT>(t, wtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank);
-			for (int sbi = 0; sbi < nb; sbi++) {
+			const TcItem item = tc_item<PAIR, NT, SPLIT>(t, wtl, s_items, m_items, tile_info, n_local, TILE_ROWS, rank, n_parts);
+			for (int sbi = 0; sbi < nbl; sbi++) {
+				const int g = item.part * nbl + sbi;
 				if (wc >= (uint32_t)Sm::NWB && !tc_wait_warp<100>(ptx::smem_u32(&sh->wempty[wb]), wph ^ 1u, abort_flag, status, lane)) {
 					alive = false;
 					break;
@@ -948,9 +969,9 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						const CUtensorMap *tw = m ? &tw1 : &tw0;
 						const uint32_t at = w_buf(wb) + m * (Sm::WBUF / 2);
 						if (Q4)	 // box = (one block, 128 or 64 rows)
-							ptx::tma_load_2d(at, tw, bar, sbi * Q4K_BYTES, row);
+							ptx::tma_load_2d(at, tw, bar, g * Q4K_BYTES, row);
 						else  // box = (one record, 8 rows of a group, 16 or 8 groups)
-							ptx::tma_load_3d(at, tw, bar, sbi * TC_Q6_ROW, 0, row >> 3);
+							ptx::tma_load_3d(at, tw, bar, g * TC_Q6_ROW, 0, row >> 3);
 					}
 				}
 				wc++;
@@ -969,6 +990,25 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 	}
 	ptx::tc_fence_before();
 	__syncthreads();
+	if constexpr (SPLIT) {
+		ptx::cluster_sync_all();
+		const int4 it = s_items[0];  // (one item a CTA; the parts of a tile differ in the part only)
+		const uint32_t me = ptx::cluster_ctarank();
+		for (int i = threadIdx.x; total > 0 && i < (it.z - (int)me + n_parts - 1) / n_parts * (TC_BM / 4); i += TC_THREADS) {
+			const int tok = (int)me + i / (TC_BM / 4) * n_parts, col = i % (TC_BM / 4) * 4;
+			float4 v[TC_MAX_PARTS];
+#pragma unroll
+			for (int k = 0; k < TC_MAX_PARTS; k++)
+				if (k < n_parts)
+					v[k] = ptx::ld_cluster(ptx::cluster_addr(tiles + (uint32_t)(tok * TC_BM + col) * 4u, k));
+#pragma unroll
+			for (int k = 1; k < TC_MAX_PARTS; k++)
+				if (k < n_parts)
+					v[0] = make_float4(__fadd_rn(v[0].x, v[k].x), __fadd_rn(v[0].y, v[k].y), __fadd_rn(v[0].z, v[k].z), __fadd_rn(v[0].w, v[k].w));
+			*reinterpret_cast<float4 *>(y + (size_t)(it.y + tok) * out_stride + it.w + col) = v[0];
+		}
+		ptx::cluster_sync_all();  // (nobody's shared memory goes while it is read)
+	}
 	if (PAIR)
 		ptx::cluster_sync_all();  // neither CTA leaves while its peer may still signal its barriers or read its memories
 	if (warp == W_MMA) {
@@ -1131,6 +1171,15 @@ int tc_setup(tie_cuda_ctx *c)
 					     TcSmem<W_Q4K, false, false, 64>::SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q6K_R8, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 					     TcSmem<W_Q6K_R8, false, false, 64>::SMEM));
+	// the forms that split a dense product's rows
+#define TC_ATTR_SPLIT(KIND, NT)                                                                                                                   \
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, false, false, false, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+					     TcSmem<KIND, false, false, NT>::SMEM))
+	TC_ATTR_SPLIT(W_Q4K, 32);
+	TC_ATTR_SPLIT(W_Q4K, 64);
+	TC_ATTR_SPLIT(W_Q6K_R8, 32);
+	TC_ATTR_SPLIT(W_Q6K_R8, 64);
+#undef TC_ATTR_SPLIT
 	// the CTA-pair forms; how many pairs the device holds at once sizes their (persistent) grids
 #define TC_ATTR_PAIR(KIND, GU, PEER)                                                                                          \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, PEER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
@@ -1162,15 +1211,38 @@ int tc_setup(tie_cuda_ctx *c)
 		}
 		c->tc_pairs = n_clusters < c->sm_count / 2 ? n_clusters : c->sm_count / 2;
 	}
+	// and how many clusters of n CTAs, for products whose rows are split (the SMs of a GPC are not a multiple of every n)
+	for (int n = 2; n <= TC_MAX_PARTS; n++) {
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(c->sm_count / n * n);
+		cfg.blockDim = dim3(TC_THREADS);
+		cfg.dynamicSmemBytes = TcSmem<W_Q4K, false, false, 64>::SMEM;
+		cudaLaunchAttribute attr[1];
+		attr[0].id = cudaLaunchAttributeClusterDimension;
+		attr[0].val.clusterDim.x = n;
+		attr[0].val.clusterDim.y = 1;
+		attr[0].val.clusterDim.z = 1;
+		cfg.attrs = attr;
+		cfg.numAttrs = 1;
+		if (cudaOccupancyMaxActiveClusters(&c->tc_clusters[n], grouped_gemm_sb<W_Q4K, false, false, false, 64, true>, &cfg) != cudaSuccess) {
+			cudaGetLastError();
+			c->tc_clusters[n] = 0;
+		}
+	}
 	c->tmaps_ok = true;
 	return TIE_CUDA_OK;
 }
 
+static bool tc_paired(const tie_cuda_ctx *c, int m_tiles, int k_dim)
+{
+	return c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K;
+}
+
 // arr: 0 = the split inputs x (gate/up), 1 = the split activations h (down).
-template <WKind KIND, bool GU, bool PEER = false, int NT = TC_TOKEN_TILE>
+template <WKind KIND, bool GU, bool PEER = false, int NT = TC_TOKEN_TILE, bool SPLIT = false>
 static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1, int arr, float *y, float out_scale,
 		       bool sorted_out = false, const EpDst *dst = nullptr, int dense_rows = 0, const DenseView *view = nullptr,
-		       const GuOut &gu = GuOut())
+		       const GuOut &gu = GuOut(), int n_parts = 1)
 {
 	Scratch &s = c->s;
 	const int4 *tile_info = dense_rows ? nullptr : s.tile_info;
@@ -1194,17 +1266,18 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	// Set up beside the kernel in front: a CTA needs a whole SM, so they come as SMs fall idle (9 tokens 84.3 -> 82.3 us, 64 137.5 ->
 	// 135.4; since no pass stands between the two products wide tiles gain too: a step of 400 / 512 / 4096 tokens 167.1 / 188.7 /
 	// 929 -> 164.8 / 183.5 / 926).
-	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles : 1 << 30;	// (known for a dense tensor: no idle CTAs)
-	if (c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K) {
-		return launch_kernel(c, true, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
+	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles * n_parts : 1 << 30;	// (known for a dense tensor: no idle CTAs)
+	if constexpr (!SPLIT) {
+		if (tc_paired(c, m_tiles, k_dim))
+			return launch_kernel(c, true, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
 				     TcSmem<KIND, GU, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
 				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
-				     s.status, t0.rows, d, xqd, gu);
+				     s.status, t0.rows, d, xqd, gu, n_parts);
 	}
-	return launch_kernel(c, true, 1, grouped_gemm_sb<KIND, GU, PEER, false, NT>, dim3(min(c->sm_count, items)), TC_THREADS,
+	return launch_kernel(c, true, n_parts, grouped_gemm_sb<KIND, GU, PEER, false, NT, SPLIT>, dim3(min(c->sm_count, items)), TC_THREADS,
 			     TcSmem<KIND, GU, false, NT>::SMEM, mf[0], mf[1], mf[2], mfq[0], mfq[1], mfq[2], w0m, w1m, t0.ptr, w1p,
 			     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale, s.status,
-			     t0.rows, d, xqd, gu);
+			     t0.rows, d, xqd, gu, n_parts);
 }
 
 static bool tc_tensor_ok(const DevTensor &t)
@@ -1231,7 +1304,7 @@ int launch_tc_gate_up(tie_cuda_ctx *c, const Layer &L, int n_tile)
 	gu.silu = c->silu;
 	auto launch = n_tile == 32 ? (L.gate.kind == W_Q4K ? launch_tc_t<W_Q4K, true, false, 32> : launch_tc_t<W_Q6K_R8, true, false, 32>)
 				   : (L.gate.kind == W_Q4K ? launch_tc_t<W_Q4K, true> : launch_tc_t<W_Q6K_R8, true>);
-	return launch(c, L.gate, &L.up, 0, nullptr, TC_H_SCALE, true, nullptr, 0, nullptr, gu);
+	return launch(c, L.gate, &L.up, 0, nullptr, TC_H_SCALE, true, nullptr, 0, nullptr, gu, 1);
 }
 
 // reads hs_hi/hs_lo; writes y in sorted order or (sorted false) y[perm[p]].
@@ -1288,11 +1361,25 @@ int tc_make_dense_view(tie_cuda_ctx *c, DevTensor &t)
 int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y)
 {
 	// tiles of 64 rows share a weight tile's expansion; tiles of 32 where those leave SMs idle
-	if ((n_rows + 63) / 64 * (t.rows / TC_BM) <= c->sm_count / 2)
-		return t.kind == W_Q4K ? launch_tc_t<W_Q4K, false, false, 32>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view)
-				       : launch_tc_t<W_Q6K_R8, false, false, 32>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view);
-	return t.kind == W_Q4K ? launch_tc_t<W_Q4K, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view)
-			       : launch_tc_t<W_Q6K_R8, false>(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view);
+	const int m_tiles = t.rows / TC_BM, nb = t.k / QK_K;
+	const bool narrow = (n_rows + 63) / 64 * m_tiles <= c->sm_count / 2;
+	const int tiles = (narrow ? (n_rows + 31) / 32 : (n_rows + 63) / 64) * m_tiles;
+	// As many parts of a row as divide it and fit the device at once.  2048 -> 512 of 37 tokens 14.8 -> 10.9 us, 4096 -> 2048 of 64
+	// 19.6 -> 12.9; a second wave of clusters costs more than the parts give (2048 -> 512 of 100 tokens, 16 clusters of 8: 16.9).
+	int parts = 1;
+	for (int n = 2; n <= TC_MAX_PARTS; n++)
+		if (nb % n == 0 && tiles <= c->tc_clusters[n])
+			parts = n;
+	auto run = [&](auto launch) { return launch(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view, GuOut(), parts); };
+	const bool q4 = t.kind == W_Q4K;
+	if (parts > 1) {
+		if (narrow)
+			return q4 ? run(launch_tc_t<W_Q4K, false, false, 32, true>) : run(launch_tc_t<W_Q6K_R8, false, false, 32, true>);
+		return q4 ? run(launch_tc_t<W_Q4K, false, false, 64, true>) : run(launch_tc_t<W_Q6K_R8, false, false, 64, true>);
+	}
+	if (narrow)
+		return q4 ? run(launch_tc_t<W_Q4K, false, false, 32>) : run(launch_tc_t<W_Q6K_R8, false, false, 32>);
+	return q4 ? run(launch_tc_t<W_Q4K, false>) : run(launch_tc_t<W_Q6K_R8, false>);
 }
 
 // The down product of an expert-parallel step: row p goes to the rank and row dst->row[p] names.
