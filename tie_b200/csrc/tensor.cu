@@ -1233,9 +1233,9 @@ int tc_setup(tie_cuda_ctx *c)
 	return TIE_CUDA_OK;
 }
 
-static bool tc_paired(const tie_cuda_ctx *c, int m_tiles, int k_dim)
+static bool tc_paired(const tie_cuda_ctx *c, int m_tiles, int k_dim, int min_blocks)
 {
-	return c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= 4 * QK_K;
+	return c->tc_pairs > 0 && !c->tc_no_pair && m_tiles % 2 == 0 && k_dim >= min_blocks * QK_K;
 }
 
 // arr: 0 = the split inputs x (gate/up), 1 = the split activations h (down).
@@ -1262,13 +1262,16 @@ static int launch_tc_t(tie_cuda_ctx *c, const DevTensor &t0, const DevTensor *t1
 	// pairs of CTAs (one MMA issue for two 128-row tiles) where the 128-row tiles pair up and a work item has at
 	// least 4 super-blocks.  Measured at 64 / 512 / 4096 tokens: rows of 8 super-blocks (gate/up) 68 / 79 / 355 us
 	// paired, 70 / 92 / 410 single (a pair fetches half the token bytes per CTA); rows of 3 (down) 59 / 73 / 310
-	// paired, 55 / 70 / 294 single (the hand-offs between two SMs are not amortised over so few).
+	// paired, 55 / 70 / 294 single (the hand-offs between two SMs are not amortised over so few).  Wide tiles of Q6_K rows, which
+	// expand longest, from 3 on: since their rows are stored in order, 512 / 1000 / 4096 tokens 56.3 / 76.8 / 228 paired,
+	// 56.3 / 78.8 / 236 single (narrow, 64: 50.2 and 48.2; wide Q4_K 52 / 73.7 / 224 and 50.2 / 72.7 / 225).
+	const int min_blocks = KIND == W_Q6K_R8 && NT > 32 && !PEER ? 3 : 4;
 	// Set up beside the kernel in front: a CTA needs a whole SM, so they come as SMs fall idle (9 tokens 84.3 -> 82.3 us, 64 137.5 ->
 	// 135.4; since no pass stands between the two products wide tiles gain too: a step of 400 / 512 / 4096 tokens 167.1 / 188.7 /
 	// 929 -> 164.8 / 183.5 / 926).
 	const int items = dense_rows ? (dense_rows + NT - 1) / NT * m_tiles * n_parts : 1 << 30;	// (known for a dense tensor: no idle CTAs)
 	if constexpr (!SPLIT) {
-		if (tc_paired(c, m_tiles, k_dim))
+		if (tc_paired(c, m_tiles, k_dim, min_blocks))
 			return launch_kernel(c, true, 2, grouped_gemm_sb<KIND, GU, PEER, true, NT>, dim3(2 * min(c->tc_pairs, items / 2)), TC_THREADS,
 				     TcSmem<KIND, GU, true, NT>::SMEM, mh[0], mh[1], mh[2], mhq[0], mhq[1], mhq[2], w0m, w1m, t0.ptr, w1p,
 				     t0.expert_stride, k_dim, tile_info, s.tile_start, n_experts, m_tiles, y, perm, out_stride, out_scale,
