@@ -32,6 +32,8 @@
 // the last CTA of every launch advances), so the launch arguments never change and the kernel
 // replays from a CUDA graph.  Every spin is bounded; a CTA that gives up flags the status word,
 // waits (bounded) for its own copies in flight and returns.
+#include <type_traits>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "mma_dot.cuh"
@@ -87,8 +89,8 @@ __device__ __forceinline__ bool df_grid_barrier(unsigned *counter, unsigned targ
 {
 	__syncthreads();
 	if (threadIdx.x == 0) {
-		__threadfence();
-		atomicAdd(counter, 1u);
+		// (release: what the CTA wrote before its barrier above is visible to whoever sees the count)
+		asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
 		const long long t0 = clock64();
 		int ok = 1;
 		while ((int)(df_ld_acquire(counter) - target) < 0) {
@@ -168,7 +170,17 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		const uint32_t parity = (uint32_t)layer & 1u;  // (every copy barrier completes once a layer)
 
 		// The row, its norm weights and the CTA's row of the router matrix are on their way before anything is computed.
-		float *ws = reinterpret_cast<float *>(dsm), *xn = reinterpret_cast<float *>(dsm + a.off_n);
+		// For the sequential chains both lie as [AVX2 lane][step] too: a thread of a chain gets four steps per load (one each:
+		// 16 blocks 320 us, so 305, with the two lines on the barrier and the selection; the tile area is free until the selection).
+		constexpr int TP = K / 8 + 4;
+		float *wt = reinterpret_cast<float *>(dsm), *xt = wt + 8 * TP, *xn = reinterpret_cast<float *>(dsm + a.off_n);
+		auto transposed = [&](float *t, const float4 &v) {  // 4 tid .. of the row
+			float *d = t + 4 * (tid & 1) * TP + (tid >> 1);
+			d[0] = v.x;
+			d[TP] = v.y;
+			d[2 * TP] = v.z;
+			d[3 * TP] = v.w;
+		};
 		static_assert(K / 4 <= DF_THREADS, "one 16-byte load per thread");
 		const float *router_w = layer ? sh.lay.router_w : a.first.router_w, *norm_w = layer ? sh.lay.norm_w : a.first.norm_w;
 		float4 xv = make_float4(0.f, 0.f, 0.f, 0.f), nv = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -180,7 +192,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			if (a.norm_eps >= 0.0f && norm_w)
 				nv = __ldg(reinterpret_cast<const float4 *>(norm_w) + tid);
 			reinterpret_cast<float4 *>(xn)[tid] = xv;
-			reinterpret_cast<float4 *>(ws)[tid] = wv;
+			transposed(xt, xv);
+			transposed(wt, wv);
 		}
 		__syncthreads();
 		if (layer == 0)
@@ -190,10 +203,14 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			if (warp == 0) {
 				float acc = 0.0f;
 				if (lane < 8) {
-#pragma unroll 32
-					for (int i = 0; i < K / 8; i++) {
-						const float v = xn[8 * i + lane];
-						acc = __fmaf_rn(v, v, acc);
+					const float4 *t = reinterpret_cast<const float4 *>(xt + lane * TP);
+#pragma unroll 16
+					for (int i = 0; i < K / 32; i++) {
+						const float4 v = t[i];
+						acc = __fmaf_rn(v.x, v.x, acc);
+						acc = __fmaf_rn(v.y, v.y, acc);
+						acc = __fmaf_rn(v.z, v.z, acc);
+						acc = __fmaf_rn(v.w, v.w, acc);
 					}
 				}
 				const float ss = hsum8_lanes(acc);  // (l + l4), then + 1, then + 2: the reference's tree
@@ -202,10 +219,12 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 			}
 			__syncthreads();
 			const float inv = sh.inv;
-			if (tid < K / 4)
-				reinterpret_cast<float4 *>(xn)[tid] =
-					make_float4(__fmul_rn(__fmul_rn(xv.x, nv.x), inv), __fmul_rn(__fmul_rn(xv.y, nv.y), inv),
-						    __fmul_rn(__fmul_rn(xv.z, nv.z), inv), __fmul_rn(__fmul_rn(xv.w, nv.w), inv));
+			if (tid < K / 4) {
+				const float4 o = make_float4(__fmul_rn(__fmul_rn(xv.x, nv.x), inv), __fmul_rn(__fmul_rn(xv.y, nv.y), inv),
+							     __fmul_rn(__fmul_rn(xv.z, nv.z), inv), __fmul_rn(__fmul_rn(xv.w, nv.w), inv));
+				reinterpret_cast<float4 *>(xn)[tid] = o;
+				transposed(xt, o);
+			}
 			__syncthreads();
 		}
 
@@ -213,9 +232,15 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 		if (warp == 0 && cta < a.n_expert) {
 			float acc = 0.0f;
 			if (lane < 8) {
-#pragma unroll 32
-				for (int i = 0; i < K / 8; i++)
-					acc = __fmaf_rn(xn[8 * i + lane], ws[8 * i + lane], acc);
+				const float4 *tx = reinterpret_cast<const float4 *>(xt + lane * TP), *tw = reinterpret_cast<const float4 *>(wt + lane * TP);
+#pragma unroll 16
+				for (int i = 0; i < K / 32; i++) {
+					const float4 u = tx[i], v = tw[i];
+					acc = __fmaf_rn(u.x, v.x, acc);
+					acc = __fmaf_rn(u.y, v.y, acc);
+					acc = __fmaf_rn(u.z, v.z, acc);
+					acc = __fmaf_rn(u.w, v.w, acc);
+				}
 			}
 			float r = hsum8_lanes(acc);
 			if (lane == 0) {
@@ -238,14 +263,20 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 
 		// ---------------- selection (every CTA for itself) and all weight requests ----------------
 		if (warp == 0) {
-			unsigned key[1][8];
+			auto select = [&](auto per) {
+				unsigned key[1][per.value];
 #pragma unroll
-			for (int i = 0; i < 8; i++)
-				key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
-			int mine[1];
-			topk_warp<1, 8>(key, lane, top_k, mine);
-			if (lane < top_k)
-				sh.idx[lane] = mine[0];
+				for (int i = 0; i < per.value; i++)
+					key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
+				int mine[1];
+				topk_warp<1, per.value>(key, lane, top_k, mine);
+				if (lane < top_k)
+					sh.idx[lane] = mine[0];
+			};
+			if (a.n_expert <= 128)
+				select(std::integral_constant<int, 4>());
+			else
+				select(std::integral_constant<int, 8>());
 		}
 		__syncthreads();
 		bool bad = false;
@@ -466,7 +497,7 @@ static DfPlan df_plan(const tie_cuda_ctx *c)
 		return p;
 	const size_t tile_gu = (size_t)p.rpt_gu * df_row_bytes<KG>(K), tile_dn = (size_t)p.rpt_dn * df_row_bytes<W_Q6K_R8>(F);  // (the larger kind)
 	size_t area_a = 2 * tile_gu;
-	area_a = max(area_a, (size_t)2 * K * sizeof(float));				 // router staging
+	area_a = max(area_a, (size_t)2 * (K + 32) * sizeof(float));			 // the row and the router row, by AVX2 lane
 	area_a = max(area_a, (size_t)DF_WARPS * max(XImage<W_Q4K>::BYTES, XImage<W_Q6K_R8>::BYTES));  // images of h
 	p.off_b = (area_a + 127) / 128 * 128;
 	p.off_c = (p.off_b + (size_t)top_k * tile_dn + 127) / 128 * 128;
