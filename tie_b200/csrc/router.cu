@@ -97,7 +97,7 @@ struct RtCfg {
 	static constexpr int TG = TT / TPT, EG = TE / EPT, THREADS = 8 * TG * EG;
 	static constexpr int PITCH = KC + 8, STAGE = (TT + TE) * PITCH;  // floats; two rows apart by a quarter of the banks
 	static constexpr int STAGES = 3, SMEM = STAGES * STAGE * (int)sizeof(float);
-	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : 8;
+	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : (TPT * EPT > 2 ? 8 : 32);  // (one or two chains a thread: their loads go far ahead)
 	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte copies per thread and chunk
 	// the form with the RMSNorm in front: whole rows in shared memory, and COLS float4 of each in a thread's registers
 	static constexpr bool NORM = TT <= 8 && KC == 512;
@@ -107,7 +107,8 @@ struct RtCfg {
 
 // NORM: x is the residual stream; the CTA makes the RMSNorm of its tokens itself (rms_norm_rows, the same operations in the same
 // order) while the router weights arrive, and the CTAs of the first experts store it for the kernels behind.  A launch of
-// its own is 3.4 us of a block of 4 tokens (8 blocks of 4 tokens 366.1 -> 356.6 us, 4 of 13 356.1 -> 349.0).
+// its own is 3.4 us of a block of 4 tokens (8 blocks of 4 tokens 366.1 -> 356.6 us, 4 of 13 356.1 -> 349.0; with the chains' loads
+// further ahead, here and in the products of the smallest tiles, another 2 and 1 %).
 struct RtNorm {
 	const float *w = nullptr;  // or null: weight 1
 	float *out = nullptr;
@@ -164,7 +165,7 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 #pragma unroll
 	for (int c = 0; c < C::STAGES - 1; c++)
 		fetch(c, false, true);
-	const int px = hidden + 8;	// NORM: pitch of the rows
+	const int px = hidden + 8, tp = hidden / 8 + 4;	 // NORM: pitch of the rows, and of their lanes before that
 	float *rows = rsm + C::STAGES * C::STAGE;
 	if constexpr (NORM) {
 		__shared__ float s_inv[TT];
@@ -185,15 +186,25 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 		for (int k = 0; k < COLS; k++)
 #pragma unroll
 			for (int j = 0; j < TT; j++)
-				if (4 * col(k) < hidden)
-					*reinterpret_cast<float4 *>(rows + j * px + 4 * col(k)) = v[j][k];
+				if (4 * col(k) < hidden) {  // for the sums, as [AVX2 lane][step]: four steps of a chain per load
+					float *d = rows + j * (hidden + 32) + 4 * (col(k) & 1) * tp + (col(k) >> 1);
+					d[0] = v[j][k].x;
+					d[tp] = v[j][k].y;
+					d[2 * tp] = v[j][k].z;
+					d[3 * tp] = v[j][k].w;
+				}
 		__syncthreads();
 		if (threadIdx.x < 8 * TT) {  // a thread per lane of a row's sum of squares
-			const float *r = rows + (threadIdx.x >> 3) * px + (threadIdx.x & 7);
+			const float4 *r = reinterpret_cast<const float4 *>(rows + (threadIdx.x >> 3) * (hidden + 32) + (threadIdx.x & 7) * tp);
 			float a = 0.f;
-#pragma unroll 32
-			for (int i = 0; i < hidden / 8; i++)
-				a = __fmaf_rn(r[8 * i], r[8 * i], a);
+#pragma unroll 16
+			for (int i = 0; i < hidden / 32; i++) {
+				const float4 u = r[i];
+				a = __fmaf_rn(u.x, u.x, a);
+				a = __fmaf_rn(u.y, u.y, a);
+				a = __fmaf_rn(u.z, u.z, a);
+				a = __fmaf_rn(u.w, u.w, a);
+			}
 			const float ss = hsum8_lanes(a);
 			if ((threadIdx.x & 7) == 0)
 				s_inv[threadIdx.x >> 3] = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)hidden), norm.eps)));
@@ -406,7 +417,7 @@ bool router_norm_supported(const tie_cuda_ctx *c, int n_tokens)
 #define TIE_RT_NORM(A, B, ...)                                                                                              \
 	if (at++ == pick) {                                                                                                 \
 		using C = __VA_ARGS__;                                                                                      \
-		ok = C::NORM && H / 4 <= C::COLS * C::THREADS && C::SMEM + C::TT * (H + 8) * sizeof(float) <= RT_NORM_SMEM; \
+		ok = C::NORM && H / 4 <= C::COLS * C::THREADS && C::SMEM + C::TT * (H + 32) * sizeof(float) <= RT_NORM_SMEM; \
 	}
 	TIE_RT_TILES(TIE_RT_NORM)
 #undef TIE_RT_NORM
@@ -446,7 +457,7 @@ int launch_router(tie_cuda_ctx *c, const float *x, const float *w, const float *
 					     lfm2, sel_bias, c->s.route_counter, f, norm);                                 \
 		};                                                                                                         \
 		if constexpr (C::NORM)                                                                                     \
-			rc = norm_out ? run(router_batch<C, true>, C::SMEM + C::TT * (H + 8) * sizeof(float))               \
+			rc = norm_out ? run(router_batch<C, true>, C::SMEM + C::TT * (H + 32) * sizeof(float))               \
 				      : run(router_batch<C, false>, C::SMEM);                                               \
 		else                                                                                                       \
 			rc = norm_out ? TIE_CUDA_EINVAL : run(router_batch<C, false>, C::SMEM);                            \
