@@ -21,9 +21,9 @@
 //   * a weight loader thread brings the packed blocks of one super-block x 128 rows into shared
 //     memory with TMA (three or four super-blocks in flight: the HBM latency is hidden by the
 //     hardware, not by registers, and no thread issues scattered 16-byte loads);
-//   * 16 producer warps, in four groups of 128 threads (one per weight row), expand them (one HFMA2 per two
+//   * producer warps, in four (or two: TcRoles) groups of 128 threads (one per weight row), expand them (one HFMA2 per two
 //     weights) and write the A tiles to TENSOR MEMORY (tcgen05.st) into a ring of four units of half a
-//     super-block, one per group;
+//     super-block;
 //   * a token loader thread issues TMA tile loads of the token operand (hi/lo fp16, expert-sorted
 //     rows: only rows the expert really has) and of the sub-block sums, into rings of their own;
 //   * one MMA issuer thread walks the super-blocks: P += A.B_lo over the block's 16-wide k steps, then
@@ -31,9 +31,9 @@
 //     columns: one MMA over hi and lo rows, into columns side by side), a super-block per accumulator
 //     buffer, two buffers of 64 columns in turn (NT = 32, launches of narrow tiles: four of 32), and the block's min sums into a
 //     buffer of their own;
-//   * 8 drain warps take a finished super-block out of tensor memory (tcgen05.ld), hand the buffer back
+//   * drain warps take a finished super-block out of tensor memory (tcgen05.ld), hand the buffer back
 //     at once, fold the values into fp32 registers with d (-1 for the min sums), and after the last
-//     super-block of a work item store the rows — while the MMAs of the next super-blocks / work
+//     super-block of a work item finish and store the rows — while the MMAs of the next super-blocks / work
 //     item already run.
 // All hand-offs go through mbarriers (tcgen05.commit on the MMA side).  Every wait
 // is bounded: on a timeout the CTA raises ST_WAIT_TIMEOUT in the status word, all roles leave their
