@@ -46,8 +46,8 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch of the two grouped-GEMM launches of the
 # 512-token workload, from the ncu capture of `python bench.py --only prefill512`; a change to that
 # kernel needs a new capture (the traffic is set by the packed weights and the operand arrays, not
-# by the kernel's schedule, and has stayed within 1 % over the kernel's revisions).
-NCU_DRAM_BYTES_PER_LAUNCH = {"gate_up": 261237504 + 18816512, "down": 177829120 + 15746560}  # read + written
+# by the kernel's schedule; with SwiGLU in the gate/up product its rows are half as many bytes).
+NCU_DRAM_BYTES_PER_LAUNCH = {"gate_up": 261399808 + 11544576, "down": 177821696 + 16302336}  # read + written
 NCU_DRAM_SOURCE = "ncu capture of grouped_gemm_sb on `bench.py --only prefill512`"
 
 
