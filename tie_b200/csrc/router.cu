@@ -296,10 +296,11 @@ router_batch(const float *__restrict__ x, const float *__restrict__ w, const flo
 		}
 	}
 	__syncthreads();
-	if (threadIdx.x == 0) {	 // (one fence for the CTA: the barrier has ordered its stores before this thread)
-		__threadfence();
-		s_last = atomicAdd(counter + blockIdx.x, 1) == n_expert / TE - 1;
-		__threadfence();
+	if (threadIdx.x == 0) {
+		// (releases the CTA's logits, which the barrier has ordered before this thread, and acquires those of the others)
+		int done;
+		asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], 1;" : "=r"(done) : "l"(counter + blockIdx.x) : "memory");
+		s_last = done == n_expert / TE - 1;
 	}
 	__syncthreads();
 	// The decode kernels' CTAs may come now and wait for this grid: before the selection, not before the products (from
