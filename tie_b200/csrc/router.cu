@@ -97,7 +97,7 @@ struct RtCfg {
 	static constexpr int TG = TT / TPT, EG = TE / EPT, THREADS = 8 * TG * EG;
 	static constexpr int PITCH = KC + 8, STAGE = (TT + TE) * PITCH;  // floats; two rows apart by a quarter of the banks
 	static constexpr int STAGES = 3, SMEM = STAGES * STAGE * (int)sizeof(float);
-	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : (TPT * EPT > 2 ? 8 : 32);  // (one or two chains a thread: their loads go far ahead)
+	static constexpr int UNROLL = TPT * EPT >= 64 ? 2 : (TPT * EPT > 8 ? 8 : 32);  // (few chains a thread: their loads go far ahead)
 	static constexpr int LD = (TT + TE) * (KC / 4) / THREADS;  // 16-byte copies per thread and chunk
 	// the form with the RMSNorm in front: whole rows in shared memory, and COLS float4 of each in a thread's registers
 	static constexpr bool NORM = TT <= 8 && KC == 512;
