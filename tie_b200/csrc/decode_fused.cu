@@ -269,7 +269,8 @@ __global__ void __launch_bounds__(DF_THREADS, 1) decode1_fused(const DfArgs a)
 				for (int i = 0; i < per.value; i++)
 					key[0][i] = lane + 32 * i < a.n_expert ? score_key(__ldcg(a.logits + lane + 32 * i)) : 0u;
 				int mine[1];
-				topk_warp<1, per.value>(key, lane, top_k, mine);
+				unsigned best[1];
+				topk_warp<1, per.value>(key, lane, top_k, mine, best);
 				if (lane < top_k)
 					sh.idx[lane] = mine[0];
 			};

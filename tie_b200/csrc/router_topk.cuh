@@ -22,25 +22,33 @@ __device__ __forceinline__ unsigned score_key(float v)
 	return (u & 0x80000000u) ? ~u : u | 0x80000000u;
 }
 
+// The score of a key (of -0: +0).
+__device__ __forceinline__ float key_score(unsigned key)
+{
+	return __uint_as_float(key & 0x80000000u ? key ^ 0x80000000u : ~key);
+}
+
 // find_top_k (engine.c:891-914) by one warp for NT tokens at once: key[n][i] is the key of expert
 // lane + 32 i (0: none, or taken).  A round is two hardware reductions, the largest key and, among its
 // holders, the lowest expert: ties keep the lower index.  Lane r < top_k ends up with the expert of
-// rank r (or -1) of token n in mine[n].
+// rank r (or -1) of token n in mine[n], and its key in best[n].
 template <int NT, int PER>
-__device__ __forceinline__ void topk_warp(unsigned (&key)[NT][PER], int lane, int top_k, int (&mine)[NT])
+__device__ __forceinline__ void topk_warp(unsigned (&key)[NT][PER], int lane, int top_k, int (&mine)[NT], unsigned (&best)[NT])
 {
 #pragma unroll
-	for (int n = 0; n < NT; n++)
+	for (int n = 0; n < NT; n++) {
 		mine[n] = -1;
+		best[n] = 0u;
+	}
 	for (int r = 0; r < top_k; r++) {
 		unsigned top[NT], e[NT];
 #pragma unroll
 		for (int n = 0; n < NT; n++) {
-			unsigned best = key[n][0];
+			unsigned largest = key[n][0];
 #pragma unroll
 			for (int i = 1; i < PER; i++)
-				best = max(best, key[n][i]);
-			top[n] = __reduce_max_sync(0xffffffffu, best);
+				largest = max(largest, key[n][i]);
+			top[n] = __reduce_max_sync(0xffffffffu, largest);
 		}
 #pragma unroll
 		for (int n = 0; n < NT; n++) {
@@ -55,8 +63,10 @@ __device__ __forceinline__ void topk_warp(unsigned (&key)[NT][PER], int lane, in
 #pragma unroll
 			for (int i = 0; i < PER; i++)
 				key[n][i] = e[n] == (unsigned)(lane + 32 * i) ? 0u : key[n][i];
-			if (lane == r && top[n] != 0u)	// (0: fewer experts than top_k)
+			if (lane == r && top[n] != 0u) {  // (0: fewer experts than top_k)
 				mine[n] = (int)e[n];
+				best[n] = top[n];
+			}
 		}
 	}
 }
@@ -92,13 +102,15 @@ __device__ __forceinline__ void topk_tokens(float *__restrict__ logits, const fl
 			}
 		}
 	int mine[NT];
-	topk_warp<NT, PER>(key, lane, top_k, mine);
+	unsigned best[NT];
+	topk_warp<NT, PER>(key, lane, top_k, mine, best);
 	__syncwarp();
 #pragma unroll
 	for (int n = 0; n < NT; n++) {
 		if (n >= n_real)
 			break;
-		float v = mine[n] >= 0 ? __ldcg(logits + (size_t)(t + n) * n_expert + mine[n]) : 0.0f;
+		// (a selected logit is its key again, not a load behind the selection; LFM2 gates are not what was selected on)
+		float v = mine[n] < 0 ? 0.0f : (lfm2 ? __ldcg(logits + (size_t)(t + n) * n_expert + mine[n]) : key_score(best[n]));
 		const float mx = __shfl_sync(0xffffffffu, v, 0);  // (scores are sorted descending: lane 0 holds the max)
 		if (!lfm2)
 			v = lane < top_k ? expf(__fsub_rn(v, mx)) : 0.0f;
