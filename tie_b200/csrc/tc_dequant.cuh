@@ -5,14 +5,16 @@
 //   Q6_K: w = d * (sc_b * (q - 32))            (sc_b int8, q 6-bit)         math_scalar.c:257-287
 // with d, dmin constant over the super-block.  The integer products sc_b*q (<= 945) and
 // sc_b*(q-32) are what the tensor cores multiply: they are EXACT in fp16 up to 2048 (the Q6_K
-// product can reach 4096; above 2048 an odd product is rounded to even, a relative 2^-12 on that
-// one weight).  The fp32 factors d and dmin are applied when a super-block's partial sums are
+// product can reach 4096; above 2048 an odd product is off by 1, at most 2^-11 of that one
+// weight).  The fp32 factors d and dmin are applied when a super-block's partial sums are
 // taken out of tensor memory, so no low-order operand is needed for the weights.
 //
 // Quants become halves without conversion instructions: a 16-bit field 0x6400 | q is the half
-// 1024 + q, 0x6400 | (q << 4) is 1024 + 16 q (q < 64); one HFMA2 with
-// a per-sub-block scale and offset then yields sc*q resp. sc*(q-32) for two weights (the product
-// inside the fused multiply-add is exact, so the result is the exact integer).  The two halves of
+// 1024 + q, 0x6400 | (q << 4) is 1024 + 16 q (q < 64); one HFMA2 with a per-sub-block scale and
+// offset then yields sc*q for two weights (the offset is a half and the product inside the fused
+// multiply-add is exact, so the result is the integer, rounded once where it has more than 11
+// bits).  The same for sc*(q-32) from 1024 + 16 q, whose offset -96 sc is a half; from 1024 + q it would
+// be -1056 sc, which is none, so 1056 is subtracted first (exactly) and the product rounds.  The two halves of
 // such a pair come from bytes 0 and 2 (or 1 and 3) of a 32-bit word, so within every group of 4
 // consecutive k the operand tiles hold the order [k0, k2, k1, k3]; the token operand is written in
 // the same order (split_rows, the gate/up epilogue), so the contraction is unchanged.

@@ -318,19 +318,19 @@ struct Expander<W_Q6K_R8> {
 		saddr = rec + 192u + 8u * half;
 	}
 	// sixteen weights of each stage: v[stage][0 .. 3] columns 8 hs + 4 k .. (k = i & 1), v[stage][4 .. 7] the same + 16.
-	// The operand is sc * (q - 32) / 16 (the drain multiplies d by 16): sc * (1024 + q) less sc * 1056 would leave fp16.
+	// Low nibbles: 1056 is subtracted in front of the product.  sc * 1056 behind it is no half, nor a sixteenth of it for odd
+	// scales from 63 up, whose weights were off by up to half a step.  High nibbles: 96 * sc has 9 bits.
 	__device__ __forceinline__ void piece(int i, uint32_t v[2][8]) const
 	{
 		const int hs = i >> 1, k = i & 1;
-		const __half2 k1152 = __float2half2_rn(1152.0f);
+		const __half2 k1152 = __float2half2_rn(1152.0f), k1056 = __float2half2_rn(1056.0f);
 		const uint32_t chunk = qaddr + 48u * hs + 8u * k;
 		const uint2 w[2] = {lds64(chunk), lds64(chunk + 16u)}, h = lds64(chunk + 32u);
 		const uint32_t scx = lds32(saddr + 4u * hs) ^ 0x80808080u;  // int8 -> half as 1024 + (s ^ 0x80) - 1152
 #pragma unroll
 		for (int ab = 0; ab < 2; ab++) {
 			const __half2 s0 = __hsub2(byte_pair_1024(scx, ab ? 0x7151u : 0x7050u), k1152), s1 = __hsub2(byte_pair_1024(scx, ab ? 0x7353u : 0x7252u), k1152);
-			const __half2 f0 = __hmul2(s0, __float2half2_rn(0.0625f)), c0 = __hmul2(s0, __float2half2_rn(-66.0f));
-			const __half2 f1 = __hmul2(s1, __float2half2_rn(1.0f / 256)), c1 = __hmul2(s1, __float2half2_rn(-6.0f));
+			const __half2 f1 = __hmul2(s1, __float2half2_rn(0.0625f)), c1 = __hmul2(s1, __float2half2_rn(-96.0f));
 			const uint32_t a2[2] = {w[ab].x, w[ab].y}, h2[2] = {h.x, h.y};
 #pragma unroll
 			for (int j = 0; j < 2; j++) {
@@ -341,7 +341,7 @@ struct Expander<W_Q6K_R8> {
 					q6k_word<4>(a2[j], h2[j], lo, hi);
 #pragma unroll
 				for (int e = 0; e < 2; e++) {
-					v[0][4 * ab + 2 * j + e] = h2_bits(__hfma2(bits_h2(lo[e]), f0, c0));
+					v[0][4 * ab + 2 * j + e] = h2_bits(__hmul2(__hsub2(bits_h2(lo[e]), k1056), s0));
 					v[1][4 * ab + 2 * j + e] = h2_bits(__hfma2(bits_h2(hi[e]), f1, c1));
 				}
 			}
@@ -649,7 +649,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 						acc[j] = __fmaf_rn(scale, __uint_as_float(v[j]), acc[j]);
 				}
 			};
-			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead; times 16, which the operand lacks
+			// Q6_K: d of (row, super-block) straight from global memory, one super-block ahead
 			const int sb0 = item.part * nbl;
 			const uint8_t *grp = nullptr;
 			float dnext = 0.0f;
@@ -658,7 +658,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 				dnext = half_bits_to_float(__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sb0))));
 			}
 			for (int sbi = 0; sbi < nbl; sbi++, n++) {
-				float scale = (GU ? 16.0f : 16.0f * out_scale) * dnext;
+				float scale = (GU ? 1.0f : out_scale) * dnext;
 				if (!Q4 && sbi + 1 < nbl)
 					dnext = half_bits_to_float(
 						__ldg(reinterpret_cast<const unsigned short *>(grp + q6k_r8_d_off(nb, mrow & 7, sb0 + sbi + 1))));
