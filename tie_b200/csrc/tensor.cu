@@ -393,7 +393,7 @@ grouped_gemm_sb(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 		int out_stride, float out_scale, unsigned *__restrict__ status, int rows_per_matrix, const EpDst dst,
 		const int xq_depth, const GuOut gu, const int n_parts)
 {
-	static_assert(!SPLIT || (!GU && !PEER && !PAIR), "parts of plain products only");
+	static_assert(!SPLIT || (!GU && !PEER && !PAIR && NT == 32), "parts of plain products in narrow tiles only");
 	static_assert(!(GU && PEER), "peer destinations exist for the down product only");
 	using Sm = TcSmem<KIND, GU, PAIR, NT>;
 	constexpr int TILE_ROWS = GU ? TC_BM / 2 : TC_BM;  // of a matrix
@@ -1171,15 +1171,11 @@ int tc_setup(tie_cuda_ctx *c)
 					     TcSmem<W_Q4K, false, false, 64>::SMEM));
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q6K_R8, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
 					     TcSmem<W_Q6K_R8, false, false, 64>::SMEM));
-	// the forms that split a dense product's rows
-#define TC_ATTR_SPLIT(KIND, NT)                                                                                                                   \
-	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, false, false, false, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-					     TcSmem<KIND, false, false, NT>::SMEM))
-	TC_ATTR_SPLIT(W_Q4K, 32);
-	TC_ATTR_SPLIT(W_Q4K, 64);
-	TC_ATTR_SPLIT(W_Q6K_R8, 32);
-	TC_ATTR_SPLIT(W_Q6K_R8, 64);
-#undef TC_ATTR_SPLIT
+	// the forms that split a dense product's rows (narrow tiles only: launch_tc_dense)
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q4K, false, false, false, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+					     TcSmem<W_Q4K, false, false, 32>::SMEM));
+	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<W_Q6K_R8, false, false, false, 32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+					     TcSmem<W_Q6K_R8, false, false, 32>::SMEM));
 	// the CTA-pair forms; how many pairs the device holds at once sizes their (persistent) grids
 #define TC_ATTR_PAIR(KIND, GU, PEER)                                                                                          \
 	TIE_CUDA_TRY(c, cudaFuncSetAttribute(grouped_gemm_sb<KIND, GU, PEER, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
@@ -1211,12 +1207,13 @@ int tc_setup(tie_cuda_ctx *c)
 		}
 		c->tc_pairs = n_clusters < c->sm_count / 2 ? n_clusters : c->sm_count / 2;
 	}
-	// and how many clusters of n CTAs, for products whose rows are split (the SMs of a GPC are not a multiple of every n)
+	// and how many clusters of n CTAs, for products whose rows are split (the SMs of a GPC are not a multiple of every n; either
+	// kind of weights takes an SM per CTA)
 	for (int n = 2; n <= TC_MAX_PARTS; n++) {
 		cudaLaunchConfig_t cfg = {};
 		cfg.gridDim = dim3(c->sm_count / n * n);
 		cfg.blockDim = dim3(TC_THREADS);
-		cfg.dynamicSmemBytes = TcSmem<W_Q4K, false, false, 64>::SMEM;
+		cfg.dynamicSmemBytes = TcSmem<W_Q4K, false, false, 32>::SMEM;
 		cudaLaunchAttribute attr[1];
 		attr[0].id = cudaLaunchAttributeClusterDimension;
 		attr[0].val.clusterDim.x = n;
@@ -1224,7 +1221,7 @@ int tc_setup(tie_cuda_ctx *c)
 		attr[0].val.clusterDim.z = 1;
 		cfg.attrs = attr;
 		cfg.numAttrs = 1;
-		if (cudaOccupancyMaxActiveClusters(&c->tc_clusters[n], grouped_gemm_sb<W_Q4K, false, false, false, 64, true>, &cfg) != cudaSuccess) {
+		if (cudaOccupancyMaxActiveClusters(&c->tc_clusters[n], grouped_gemm_sb<W_Q4K, false, false, false, 32, true>, &cfg) != cudaSuccess) {
 			cudaGetLastError();
 			c->tc_clusters[n] = 0;
 		}
@@ -1369,17 +1366,15 @@ int launch_tc_dense(tie_cuda_ctx *c, const DevTensor &t, int n_rows, float *y)
 	const int tiles = (narrow ? (n_rows + 31) / 32 : (n_rows + 63) / 64) * m_tiles;
 	// As many parts of a row as divide it and fit the device at once.  2048 -> 512 of 37 tokens 14.8 -> 10.9 us, 4096 -> 2048 of 64
 	// 19.6 -> 12.9; a second wave of clusters costs more than the parts give (2048 -> 512 of 100 tokens, 16 clusters of 8: 16.9).
+	// (Clusters of two and more are half as many as SMs at the most, so tiles of 64 are never split: these are more.)
 	int parts = 1;
-	for (int n = 2; n <= TC_MAX_PARTS; n++)
+	for (int n = 2; narrow && n <= TC_MAX_PARTS; n++)
 		if (nb % n == 0 && tiles <= c->tc_clusters[n])
 			parts = n;
 	auto run = [&](auto launch) { return launch(c, t, nullptr, 0, y, 1.0f, true, nullptr, n_rows, t.view, GuOut(), parts); };
 	const bool q4 = t.kind == W_Q4K;
-	if (parts > 1) {
-		if (narrow)
-			return q4 ? run(launch_tc_t<W_Q4K, false, false, 32, true>) : run(launch_tc_t<W_Q6K_R8, false, false, 32, true>);
-		return q4 ? run(launch_tc_t<W_Q4K, false, false, 64, true>) : run(launch_tc_t<W_Q6K_R8, false, false, 64, true>);
-	}
+	if (parts > 1)
+		return q4 ? run(launch_tc_t<W_Q4K, false, false, 32, true>) : run(launch_tc_t<W_Q6K_R8, false, false, 32, true>);
 	if (narrow)
 		return q4 ? run(launch_tc_t<W_Q4K, false, false, 32>) : run(launch_tc_t<W_Q6K_R8, false, false, 32>);
 	return q4 ? run(launch_tc_t<W_Q4K, false>) : run(launch_tc_t<W_Q6K_R8, false>);
