@@ -262,7 +262,7 @@ __device__ __forceinline__ void q4k_scale_min(const uint32_t sc[3], int j, int &
 // The reference's table-driven SwiGLU exactly as its AVX2 kernel evaluates it
 // (math_avx2.c:908-950, built with -ffast-math: the division by 20 is a multiply by 0.05f):
 // no range check — outside [-10,10] the first/last table segment is extrapolated.
-__device__ __forceinline__ int silu_index(float g, float &frac)
+__device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float g, float u)
 {
 	float pos = __fmul_rn(__fmul_rn(__fadd_rn(g, 10.0f), 8191.0f), 0.05f);
 	float r = rintf(pos);
@@ -272,13 +272,7 @@ __device__ __forceinline__ int silu_index(float g, float &frac)
 	else
 		idx = (int)r;
 	idx = max(0, min(idx, SILU_N - 2));
-	frac = __fsub_rn(pos, (float)idx);
-	return idx;
-}
-__device__ __forceinline__ float swiglu_lut(const float *__restrict__ tab, float g, float u)
-{
-	float frac;
-	const int idx = silu_index(g, frac);
+	float frac = __fsub_rn(pos, (float)idx);
 	float y1 = tab[idx], y2 = tab[idx + 1];
 	return __fmul_rn(__fmaf_rn(__fsub_rn(y2, y1), frac, y1), u);
 }

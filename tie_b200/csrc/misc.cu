@@ -157,12 +157,6 @@ __global__ void __launch_bounds__(256) swiglu_kernel(float *__restrict__ gate, c
 		gate[i] = swiglu_lut(silu, gate[i], up[i]);
 }
 
-// Distinct experts with at least one row (for the traffic accounting of benchmarks).
-__global__ void copy_int(const int *src, int *dst)
-{
-	*dst = *src;
-}
-
 int launch_rms_norm(tie_cuda_ctx *c, const float *x, const float *w, float *o, int n_tokens)
 {
 	const int H = c->cfg.hidden;

@@ -48,17 +48,6 @@ struct Q4kConsts {
 	__half2 sh, ch;	 // high nibbles: (1024 + 16 q) * (s/16) -   64 s
 };
 
-__device__ __forceinline__ Q4kConsts q4k_int_consts(int s_lo, int s_hi)
-{
-	Q4kConsts c;
-	const float fl = (float)s_lo, fh = (float)s_hi;
-	c.sl = __float2half2_rn(fl);
-	c.cl = __float2half2_rn(-1024.0f * fl);
-	c.sh = __float2half2_rn(fh * 0.0625f);
-	c.ch = __float2half2_rn(-64.0f * fh);
-	return c;
-}
-
 // One 32-bit word of Q4_K quants (4 bytes = 4 low + 4 high nibbles) -> sc*q as half2 pairs:
 // lo[0] = bytes (0, 2), lo[1] = bytes (1, 3) of the low nibbles; hi[] the same of the high ones.
 __device__ __forceinline__ void q4k_int_word(uint32_t w, const Q4kConsts &c, uint32_t lo[2], uint32_t hi[2])
