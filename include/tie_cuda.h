@@ -322,9 +322,10 @@ uint64_t tie_cuda_launch_count(const tie_cuda_ctx *c);
  * call (read back from the device; synchronises). */
 int tie_cuda_last_active_experts(tie_cuda_ctx *c);
 /* Per-phase device times of a call, from CUDA events on the context's stream (off by default).
- * phase_ms[TIE_CUDA_N_PHASES]: router, dispatch sort, input split, gate/up product, SwiGLU pass
- * (zero where the gate/up kernel applies it itself), down product, combine — of the most recent
- * tie_cuda_moe_ffn* / _block_inplace call.
+ * phase_ms[TIE_CUDA_N_PHASES]: router, dispatch sort, input split, gate/up product with SwiGLU, 0 (the
+ * place of a SwiGLU pass), down product, combine — of the most recent tie_cuda_moe_ffn* /
+ * _block_inplace call.  Where one launch sorts and splits, its time is the split's; the sort's is the
+ * gap between two events.
  * tie_cuda_get_profile synchronises; returns 1 if that call used the tensor-core kernels, 0 if
  * the streaming kernels, negative on error. */
 #define TIE_CUDA_N_PHASES 7

@@ -244,8 +244,9 @@ int report_status(tie_cuda_ctx *c, unsigned st)
 	return TIE_CUDA_OK;
 }
 
-// Phase marks: 0 start, 1 router done, 2 dispatch sort done, 3 input split done, 4 gate/up done,
-// 5 unused (SwiGLU is part of the gate/up product), 6 down done, 7 combine done.
+// Phase marks: 0 start, 1 router done, 2 dispatch sort done, 3 input split done (run_experts' grouped path: sort and split, one
+// launch between 2 and 3), 4 gate/up with SwiGLU done, 6 down done, 7 combine done.  (5 would be a SwiGLU pass; its place in
+// phase_ms stays.)
 void prof_mark(tie_cuda_ctx *c, int id)
 {
 	if (!c->prof_on)

@@ -399,9 +399,9 @@ def bench_main(args, metric, unit, tokens_per_rank, load_peaks, ClockSampler, co
             prof, _ = be.get_profile()
             acc = prof if acc is None else {k: acc[k] + v for k, v in prof.items()}
         be.set_profiling(False)
-        names = {"router": "router (+ tokens to the peers)", "sort": "sort + publish", "split": "wait for the peers' lists + row layout", "gate_up": "gate/up product",
-                 "swiglu": "SwiGLU pass", "down": "down product (stores rows to their sources)", "combine": "wait for owners + combine"}
-        phases = {names[k]: v / n_prof for k, v in acc.items()}
+        names = {"router": "router (+ tokens to the peers)", "sort": "sort + publish", "split": "wait for the peers' lists + row layout", "gate_up": "gate/up product with SwiGLU",
+                 "down": "down product (stores rows to their sources)", "combine": "wait for owners + combine"}
+        phases = {names[k]: v / n_prof for k, v in acc.items() if k in names}
 
     # ---- parity of this rank's output rows against the CPU checker (outside every timed region) ----
     parity_rows, parity_err = 0, 0.0

@@ -40,7 +40,7 @@ EXPORTS = [
 ]
 EP_HANDLE_BYTES = 64
 EP_PEER_POINTERS, EP_PEER_IPC_HANDLES = 0, 1
-PHASES = ["router", "sort", "split", "gate_up", "swiglu", "down", "combine"]
+PHASES = ["router", "sort", "split", "gate_up", "swiglu", "down", "combine"]  # swiglu: 0, gate_up makes it (tie_cuda_get_profile)
 
 
 class TieCudaError(RuntimeError):
