@@ -47,7 +47,7 @@ FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0}
 # 512-token workload, from the ncu capture of `python bench.py --only prefill512`; a change to that
 # kernel needs a new capture (the traffic is set by the packed weights and the operand arrays, not
 # by the kernel's schedule; with SwiGLU in the gate/up product its rows are half as many bytes).
-NCU_DRAM_BYTES_PER_LAUNCH = {"gate_up": 261399808 + 11544576, "down": 177821696 + 16302336}  # read + written
+NCU_DRAM_BYTES_PER_LAUNCH = {"gate_up": 261473280 + 13178880, "down": 177821952 + 16162816}  # read + written
 NCU_DRAM_SOURCE = "ncu capture of grouped_gemm_sb on `bench.py --only prefill512`"
 
 
@@ -532,9 +532,9 @@ def main():
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic",
         "config": config_of(shape, T),
-        "config_detail": {"arithmetic": "packed weights expanded on the fly to exact integer fp16 operands (block factors applied in fp32 per "
-                                        "super-block); activations split into fp16 hi + lo: one tcgen05.mma per 16-wide k step over the stacked "
-                                        "hi|lo rows for tiles of up to 64 tokens, two for larger tiles; fp32 accumulate",
+        "config_detail": {"arithmetic": "packed weights expanded on the fly to integer fp16 operands, exact up to 2048 (block factors applied in fp32 "
+                                        "per super-block); activations split into fp16 hi + lo: one tcgen05.mma per 16-wide k step over the stacked "
+                                        "hi|lo rows for tiles that half fill an accumulator, two for fuller ones; fp32 accumulate",
                           "l2": "weights touched per step (392 MB) exceed the 126 MB L2; no flush"},
         "clocks": clocks, "e2e": e2e, "gpu_launches": int(launches), "roofline": roofline, "cpu_baseline": cpu, "extra": extra,
     }

@@ -204,8 +204,9 @@ def wide(request, layer0, ref_silu_table):
     b.close()
 
 
-# A weight above 2048 is off by 1 at the most, 2^-11 of itself (scales uniform over int8: 1.5e-4 of a product of many).  Against
-# the rounded weights what is left is the activations' 22 bits: twice what prompts of the usual weights reach.
+# A weight above 2048 is off by 1 at the most, 2^-11 of itself: 1.4e-4 of a product with scales uniform over int8, 2.5e-4 where
+# gate and up both have them.  Against the rounded weights what is left is the activations' 22 bits: 8.0e-7 to 9.1e-7 here,
+# twice the bound of prompts of the usual weights allowed.
 WIDE, WIDE_OPERAND = 3e-4, 2.8e-6
 
 

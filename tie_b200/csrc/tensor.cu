@@ -8,7 +8,7 @@
 // Formulation: out^T = W . x^T.  Weight rows fill the 128-row M dimension of the MMA (expert row
 // counts are multiples of 128), the ragged token count of an expert is the N dimension (tiles of
 // up to 64 tokens).  A weight of a 256-wide super-block is d * (integer) - dmin * (integer)
-// (tc_dequant.cuh), so the tensor cores multiply EXACT small-integer fp16 weights with the
+// (tc_dequant.cuh), so the tensor cores multiply integer fp16 weights, exact up to 2048, with the
 // activations (split into fp16 hi + lo: 22 significand bits; one fp16 is not accurate enough
 // for the 1e-3 parity bound) and the fp32 block factors are applied once per super-block:
 //   out[r][n] = sum_B d[r][B] * sum_{k in B} (sc*q)[r][k] * x[n][k]  -  sum_b (dmin*m)[r][b] * xsum[n][b]
